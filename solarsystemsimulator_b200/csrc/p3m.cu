@@ -15,8 +15,9 @@
 //   sort    : stable radix sort by cell (devscan.cuh), particles gathered in
 //             that order as (x, y, z, m)
 //   bounds  : first and last sorted particle of every cell
-//   items   : one work item per group of 32 particles of a cell (cells
-//             hold from none to many thousands in a clustered state)
+//   items   : one work item per group of 64 or 32 particles of a cell (cells
+//             hold from none to many thousands in a clustered state), listed
+//             by the power of two of its source chunks, longest first
 //   pairs   : persistent warps take items from a counter (a dense cell's
 //             items spread over many warps). Every pair is evaluated once
 //             (the two accelerations are m_j h d and -m_i h d): an item pairs
@@ -25,7 +26,8 @@
 //             higher index (13 or so of the 26, periodic). The sources are
 //             staged through the warp's shared memory in chunks of 32,
 //             relative to the item's cell corner, so that f32 differences
-//             keep the positions' resolution; lane l meets sources (l + k)
+//             keep the positions' resolution; a lane holds two targets (64
+//             particles an item); lane l meets sources (l + k)
 //             and (l + k + 16) mod 32 at step k, in packed f32x2 arithmetic,
 //             and the sources' sums rotate through the lanes with them, so
 //             that both sides accumulate in registers. Both go to an f32
@@ -74,23 +76,50 @@ __global__ void k_pp_bounds(const unsigned long long* __restrict__ keys, long lo
     if (q == n - 1 || keys[q + 1] != k) last[k] = (int)(q + 1);
 }
 
-// items of each cell: ceil(count / 32)
-__global__ void k_pp_groups(const int* __restrict__ first, const int* __restrict__ last, long long cells,
-                            long long* __restrict__ groups) {
-    const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c < cells) groups[c] = (last[c] - first[c] + 31) / 32;
+// Work lists of items by length. An item's length is the number of source
+// chunks of 32 its warp walks: the later ones of its cell and those of the
+// neighbouring cells of higher index; class = floor(log2(length)). The
+// warps take the longest class first: an item of a collapsed halo's cell is
+// one warp's work for milliseconds, and the ones taken last set the tail. Items
+// have 64 targets (two per lane, which share the sources' loads and rotation);
+// in a cell whose first item is PP_LONG chunks or longer they have 32, since
+// there one warp's walk would bound the kernel.
+constexpr int PP_CLASSES = 16;
+constexpr int PP_LONG = 256;
+constexpr int PP_TWO = 1 << 30;                     // flag beside an item's cell (< 2^30): 64 targets
+
+__device__ __forceinline__ int pp_chunks(const int* first, const int* last, long long c) {
+    return (last[c] - first[c] + 31) / 32;
 }
 
-// item list: (cell, first target) of every group, in cell order; the
-// number of items into *n_items
-__global__ void k_pp_items(const int* __restrict__ first, const long long* __restrict__ offs, long long cells,
-                           const long long* __restrict__ groups, int2* __restrict__ items,
-                           unsigned* __restrict__ n_items) {
+// (cell, first target) of every item into the list of its class (thread per
+// cell; an item's length falls along its cell, so a class is one stretch)
+__global__ void k_pp_items(const int* __restrict__ first, const int* __restrict__ last, int M, long long cells,
+                           long long max_items, int2* __restrict__ items, unsigned* __restrict__ n_items) {
     const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= cells) return;
-    const long long g = groups[c], o = offs[c];
-    for (long long k = 0; k < g; ++k) items[o + k] = make_int2((int)c, first[c] + 32 * (int)k);
-    if (c == cells - 1) *n_items = (unsigned)(o + g);
+    const int g = pp_chunks(first, last, c);
+    if (g == 0) return;
+    const int cx = (int)(c % M), cy = (int)((c / M) % M), cz = (int)(c / ((long long)M * M));
+    long long near = 0;
+    for (int nb = 0; nb < 27; ++nb) {
+        if (nb == 13) continue;
+        const int nx = (cx + nb % 3 - 1 + M) % M, ny = (cy + (nb / 3) % 3 - 1 + M) % M, nz = (cz + nb / 9 - 1 + M) % M;
+        const long long nc = ((long long)nz * M + ny) * M + nx;
+        if (nc > c) near += pp_chunks(first, last, nc);
+    }
+    const int step = near + g >= PP_LONG ? 1 : 2;           // groups of 32 targets an item takes
+    const int tag = (int)c | (step == 2 ? PP_TWO : 0);
+    const int gi = (g + step - 1) / step;
+    for (int k = 0; k < gi;) {
+        const long long len = near + g - step * k;          // >= 1
+        const int cls = min(PP_CLASSES - 1, 63 - __clzll(len));
+        // down to length 2^cls the class stays the same (class 15 is open above)
+        const int run = (int)min((long long)(gi - k), (len - (1ll << cls)) / step + 1);
+        const unsigned at = atomicAdd(n_items + cls, (unsigned)run);
+        for (int j = 0; j < run; ++j) items[cls * max_items + at + j] = make_int2(tag, first[c] + 32 * step * (k + j));
+        k += run;
+    }
 }
 
 struct PPArgs {
@@ -103,8 +132,10 @@ struct PPArgs {
     double box;
     double G;
     float alpha, rc2, eps2;
-    const int2* items;
-    const unsigned* n_items;
+    float m;                        // the particles' common mass (UNI)
+    const int2* items;              // PP_CLASSES lists of max_items
+    const unsigned* n_items;        // their lengths
+    long long max_items;
     unsigned* next;                 // work counter (zero at launch)
     float* acc;                     // 3 x n, by cell-order position (zero at launch)
     long long n;
@@ -157,69 +188,165 @@ __device__ __forceinline__ f2x shfl2(f2x v, int from) {
 // e^{-x^2} t (a1 + a2 t + ... + a5 t^4), t = 1 / (1 + p x) (Abramowitz &
 // Stegun 7.1.26, |error| <= 1.5e-7), so g shares its Gaussian with the
 // second term 2 x e^{-x^2} / sqrt(pi). No branches: out of range (and for
-// coincident particles, where the arithmetic is not finite) the caller
+// coincident particles, where the erfc form is not finite) the caller
 // selects 0. Two pairs at a time in packed f32x2 arithmetic; the reciprocal
 // square roots, the exponential and the reciprocal are f32 MUFU operations.
-__device__ __forceinline__ f2x pp_h2(f2x R2, const f2x* K) {
-    // K: alpha, -log2(e), p, 1, a1..a5, 2/sqrt(pi), eps^2, -1 (each in both halves)
+//
+// Where alpha r_cut <= 3 (k_pp_pairs<POLY>) pairs at r >= eps take a cheaper
+// form: (1 - g(x)) / x^3 = S(x^2) with S(t) = (4 / sqrt(pi)) int_0^1 u^2 e^{-t u^2} du,
+// entire and positive, so the first term is -alpha^3 S(alpha^2 r^2), S on [0, 9]
+// a polynomial of degree 12 in w = 1 - t / 9 (weighted minimax fit of that
+// integral, weight max(t^{3/2}, 0.6): the error counts relative to the Newtonian
+// term): 3.7e-7 at most, 9.3e-8 rms in f32, where the erfc form has 5.9e-7 and
+// 1.1e-7. It takes 17 FMA-pipe operations and one MUFU a pair against 21 and
+// four: the special function unit no longer bounds the kernel. A step (warp
+// uniform) with a pair closer than eps takes the erfc form, which keeps close
+// pairs' rounding as it was.
+__device__ __forceinline__ f2x dup(float v) { return pk2(v, v); }
+
+struct PPConst {
+    f2x alpha, eps2;
+    f2x w1, w0, na3;             // POLY: w = w0 + w1 (r^2 + eps^2), -alpha^3
+    float hi, lo;                // POLY: r^2 + eps^2 at r_cut, at r = eps
+};
+
+__device__ __forceinline__ f2x pp_h2_poly(f2x R2E, const PPConst& k) {
+    constexpr float C[13] = {0.0370207495f,  0.0553906112f, 0.0686928646f, 0.0762103807f, 0.108367381f,
+                             -0.0975710749f, 0.928968487f,  -2.53256823f,  5.40020339f,   -7.24256426f,
+                             6.4283471f,     -3.28619025f,  0.807945481f};
+    float s0, s1;
+    upk2(R2E, s0, s1);
+    const f2x SI = pk2(sss_rsqrt_approx_f32(s0), sss_rsqrt_approx_f32(s1));
+    const f2x W = fma2(R2E, k.w1, k.w0);
+    f2x P = dup(C[12]);
+#pragma unroll
+    for (int j = 11; j >= 0; --j) P = fma2(P, W, dup(C[j]));
+    return fma2(P, k.na3, mul2(mul2(SI, SI), SI));
+}
+
+__device__ __forceinline__ f2x pp_h2(f2x R2, f2x alpha, f2x eps2) {
     float r0, r1;
     upk2(R2, r0, r1);
     const f2x RI = pk2(sss_rsqrt_approx_f32(r0), sss_rsqrt_approx_f32(r1));
     const f2x INV3 = mul2(mul2(RI, RI), RI);
-    const f2x X = mul2(K[0], mul2(R2, RI));
+    const f2x X = mul2(alpha, mul2(R2, RI));
     float v0, v1;
-    upk2(mul2(mul2(X, X), K[1]), v0, v1);
+    upk2(mul2(mul2(X, X), dup(-1.44269504f)), v0, v1);
     const f2x EX = pk2(ex2_approx(v0), ex2_approx(v1));
     float d0, d1;
-    upk2(fma2(K[2], X, K[3]), d0, d1);
+    upk2(fma2(dup(0.3275911f), X, dup(1.0f)), d0, d1);
     const f2x T = pk2(rcp_approx(d0), rcp_approx(d1));
-    const f2x POLY = mul2(T, fma2(T, fma2(T, fma2(T, fma2(T, K[8], K[7]), K[6]), K[5]), K[4]));
-    const f2x G = mul2(EX, fma2(K[9], X, POLY));
+    f2x P = fma2(T, dup(1.061405429f), dup(-1.453152027f));
+    P = fma2(T, P, dup(1.421413741f));
+    P = fma2(T, P, dup(-0.284496736f));
+    P = fma2(T, P, dup(0.254829592f));
+    const f2x Gx = mul2(EX, fma2(dup(1.12837917f), X, mul2(T, P)));
     float s0, s1;
-    upk2(add2(R2, K[10]), s0, s1);
+    upk2(add2(R2, eps2), s0, s1);
     const f2x SI = pk2(sss_rsqrt_approx_f32(s0), sss_rsqrt_approx_f32(s1));
-    return fma2(add2(G, K[11]), INV3, mul2(mul2(SI, SI), SI));
+    return fma2(add2(Gx, dup(-1.0f)), INV3, mul2(mul2(SI, SI), SI));
 }
 
-// One chunk of sources against the lanes' targets, two sources per step:
+// Stage a chunk's sources (lane l holds source l) as the packed pairs the
+// steps use: entry j = sources j and (j + da) mod 32, so that a step's operands
+// are two 16-byte shared loads and no register moves.
+__device__ __forceinline__ void pp_stage(ulonglong2* stage, int lane, int da, float x, float y, float z, float m) {
+    const int o = (lane + da) & 31;
+    const float x1 = __shfl_sync(0xffffffffu, x, o), y1 = __shfl_sync(0xffffffffu, y, o);
+    const float z1 = __shfl_sync(0xffffffffu, z, o), m1 = __shfl_sync(0xffffffffu, m, o);
+    __syncwarp();                                          // the previous chunk is consumed
+    stage[lane] = make_ulonglong2(pk2(x, x1), pk2(y, y1));
+    stage[32 + lane] = make_ulonglong2(pk2(z, z1), pk2(m, m1));
+    __syncwarp();
+}
+
+// A lane's target (negated, both halves) and its sums, one half per source of a step.
+struct PPTarget {
+    f2x nx, ny, nz, nm;
+    f2x ax, ay, az;
+};
+
+// One chunk of sources against the lanes' G targets, two sources per step:
 // offsets (a, a + da) for steps a = a0 .. a1 - 1 (source (lane + offset) mod
-// 32); `own` masks offset 16 on lanes 16 .. 31 (the item's own chunk, whose
-// pairs (l, l + 16) and (l + 16, l) coincide). Both sources' sums rotate
+// 32); OWN masks offset 16 on lanes 16 .. 31 (32 particles among themselves,
+// whose pairs (l, l + 16) and (l + 16, l) coincide). Both sources' sums rotate
 // through the lanes and end on their own lanes, then go to the accumulator.
-__device__ __forceinline__ void pp_chunk2(const float4* stage, int lane, int a0, int a1, int da, bool own,
-                                          f2x NTX, f2x NTY, f2x NTZ, f2x NTM, const f2x* K,
-                                          const PPArgs& q, f2x& AX, f2x& AY, f2x& AZ, long long src0, int m) {
+// UNI: all masses equal; the sums leave the mass out until the end. FMA-pipe
+// bound: 26 operations a pair (28 with masses; erfc form 33 and 35), with the 6
+// shuffles and two 16-byte shared loads of a step shared by its 2 G pairs.
+// 1,048,576 particles collapsed into halos (7.2e9 candidate pairs, 5.1e9 in
+// range): 10.4 ms a step against 15.4 with the erfc
+// form alone, sources packed by register moves and items in cell order (the
+// last heavy items then ran on by themselves). All items of 32 targets: 10.4; all
+// of 64: 11.2 (a heavy cell's walk is the kernel's length). Sorting particles
+// inside a cell and testing chunk boxes saves only a fifth of these pairs.
+template <int G, bool POLY, bool UNI, bool OWN, int A0, int A1, int DA>
+__device__ __forceinline__ void pp_chunk2(const ulonglong2* stage, int lane, PPTarget (&T)[2], const PPConst& k,
+                                          const PPArgs& q, long long src0, int m) {
     f2x BX = 0ull, BY = 0ull, BZ = 0ull;             // sums of sources (lane + a) and (lane + a + da)
-#pragma unroll 2
-    for (int a = a0; a < a1; ++a) {
-        const float4 sa = stage[(lane + a) & 31], sb = stage[(lane + a + da) & 31];
-        const f2x DX = add2(pk2(sa.x, sb.x), NTX), DY = add2(pk2(sa.y, sb.y), NTY), DZ = add2(pk2(sa.z, sb.z), NTZ);
-        const f2x R2 = fma2(DX, DX, fma2(DY, DY, mul2(DZ, DZ)));
-        float r0, r1;
-        upk2(R2, r0, r1);
-        const bool in0 = r0 < q.rc2 && r0 > 0.0f;
-        const bool in1 = r1 < q.rc2 && r1 > 0.0f && !(own && a + da == 16 && lane >= 16);
-        if (__any_sync(0xffffffffu, in0 || in1)) {                  // (warp-uniform)
-            float h0, h1;
-            upk2(pp_h2(R2, K), h0, h1);
-            const f2x H = pk2(in0 ? h0 : 0.0f, in1 ? h1 : 0.0f);
-            const f2x HJ = mul2(H, pk2(sa.w, sb.w)), HI = mul2(H, NTM);
-            AX = fma2(HJ, DX, AX);
-            AY = fma2(HJ, DY, AY);
-            AZ = fma2(HJ, DZ, AZ);
-            BX = fma2(HI, DX, BX);
-            BY = fma2(HI, DY, BY);
-            BZ = fma2(HI, DZ, BZ);
+    const int from = (lane + 1) & 31;
+#pragma unroll (G == 1 ? 2 : 1)
+    for (int a = A0; a < A1; ++a) {
+        const ulonglong2 xy = stage[(lane + a) & 31], zm = stage[32 + ((lane + a) & 31)];
+        f2x DX[G], DY[G], DZ[G], H[G];
+        bool near = !POLY;
+        if (POLY) {
+            float least = 3e38f;
+#pragma unroll
+            for (int g = 0; g < G; ++g) {
+                DX[g] = add2(xy.x, T[g].nx);
+                DY[g] = add2(xy.y, T[g].ny);
+                DZ[g] = add2(zm.x, T[g].nz);
+                H[g] = fma2(DX[g], DX[g], fma2(DY[g], DY[g], fma2(DZ[g], DZ[g], k.eps2)));
+                float r0, r1;
+                upk2(H[g], r0, r1);
+                least = fminf(least, fminf(r0, r1));
+            }
+            near = __any_sync(0xffffffffu, least < k.lo);
         }
-        if (a + 1 < a1) {                                          // take the next lane's sums (sources + 1)
-            const int from = (lane + 1) & 31;
+        if (POLY && !near) {
+#pragma unroll
+            for (int g = 0; g < G; ++g) {
+                float r0, r1, h0, h1;
+                upk2(H[g], r0, r1);
+                const bool in0 = r0 < k.hi, in1 = r1 < k.hi && !(OWN && a + DA == 16 && lane >= 16);
+                upk2(pp_h2_poly(H[g], k), h0, h1);
+                H[g] = pk2(in0 ? h0 : 0.0f, in1 ? h1 : 0.0f);
+            }
+        } else {
+#pragma unroll
+            for (int g = 0; g < G; ++g) {
+                DX[g] = add2(xy.x, T[g].nx);
+                DY[g] = add2(xy.y, T[g].ny);
+                DZ[g] = add2(zm.x, T[g].nz);
+                const f2x R2 = fma2(DX[g], DX[g], fma2(DY[g], DY[g], mul2(DZ[g], DZ[g])));
+                float r0, r1, h0, h1;
+                upk2(R2, r0, r1);
+                const bool in0 = r0 < q.rc2 && r0 > 0.0f;
+                const bool in1 = r1 < q.rc2 && r1 > 0.0f && !(OWN && a + DA == 16 && lane >= 16);
+                upk2(pp_h2(R2, k.alpha, k.eps2), h0, h1);
+                H[g] = pk2(in0 ? h0 : 0.0f, in1 ? h1 : 0.0f);
+            }
+        }
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+            PPTarget& t = T[g];
+            const f2x HJ = UNI ? H[g] : mul2(H[g], zm.y), HI = UNI ? H[g] : mul2(H[g], t.nm);
+            t.ax = fma2(HJ, DX[g], t.ax);
+            t.ay = fma2(HJ, DY[g], t.ay);
+            t.az = fma2(HJ, DZ[g], t.az);
+            BX = fma2(HI, DX[g], BX);
+            BY = fma2(HI, DY[g], BY);
+            BZ = fma2(HI, DZ[g], BZ);
+        }
+        if (a + 1 < A1) {                                          // take the next lane's sums (sources + 1)
             BX = shfl2(BX, from);
             BY = shfl2(BY, from);
             BZ = shfl2(BZ, from);
         }
     }
     // lane l holds sources (l + a1 - 1) and (l + a1 - 1 + da): deliver both to their lanes
-    const int fa = (lane - (a1 - 1)) & 31, fb = (lane - (a1 - 1 + da)) & 31;
+    const int fa = (lane - (A1 - 1)) & 31, fb = (lane - (A1 - 1 + DA)) & 31;
     float xa, xb, ya, yb, za, zb, t0, t1;
     upk2(shfl2(BX, fa), xa, t0);
     upk2(shfl2(BX, fb), t1, xb);
@@ -228,89 +355,140 @@ __device__ __forceinline__ void pp_chunk2(const float4* stage, int lane, int a0,
     upk2(shfl2(BZ, fa), za, t0);
     upk2(shfl2(BZ, fb), t1, zb);
     if (lane < m) {
-        atomicAdd(q.acc + src0 + lane, xa + xb);
-        atomicAdd(q.acc + q.n + src0 + lane, ya + yb);
-        atomicAdd(q.acc + 2 * q.n + src0 + lane, za + zb);
+        const float nm = UNI ? -q.m : 1.0f;
+        atomicAdd(q.acc + src0 + lane, nm * (xa + xb));
+        atomicAdd(q.acc + q.n + src0 + lane, nm * (ya + yb));
+        atomicAdd(q.acc + 2 * q.n + src0 + lane, nm * (za + zb));
     }
 }
 
-__global__ void __launch_bounds__(PP_WARPS * 32) k_pp_pairs(const PPArgs q) {
-    __shared__ float4 sh[PP_WARPS][32];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int M = q.M;
-    const unsigned total = *q.n_items;
-    float4* stage = sh[w];
-    const f2x K[12] = {pk2(q.alpha, q.alpha), pk2(-1.44269504f, -1.44269504f), pk2(0.3275911f, 0.3275911f),
-                       pk2(1.0f, 1.0f), pk2(0.254829592f, 0.254829592f), pk2(-0.284496736f, -0.284496736f),
-                       pk2(1.421413741f, 1.421413741f), pk2(-1.453152027f, -1.453152027f),
-                       pk2(1.061405429f, 1.061405429f), pk2(1.12837917f, 1.12837917f), pk2(q.eps2, q.eps2),
-                       pk2(-1.0f, -1.0f)};
-    for (;;) {
-        unsigned it = 0;
-        if (lane == 0) it = atomicAdd(q.next, 1u);
-        it = __shfl_sync(0xffffffffu, it, 0);
-        if (it >= total) break;
-        const int2 item = q.items[it];
-        const int c = item.x, t0 = item.y, cl = q.last[c];
-        const int t = t0 + lane;
-        const bool act = t < cl;
-        const int cx = c % M, cy = (c / M) % M, cz = c / (M * M);
-        const double ox = cx * q.l, oy = cy * q.l, oz = cz * q.l;
-        float tx = 0.0f, ty = 0.0f, tz = 0.0f, tm = 0.0f;
-        if (act) {
+// The sources [s0, s1) (shifted by s) against the lanes' G targets, chunk by chunk.
+template <int G, bool POLY, bool UNI>
+__device__ __forceinline__ void pp_walk(ulonglong2* stage, int lane, PPTarget (&T)[2], const PPConst& k,
+                                        const PPArgs& q, int s0, int s1, double sx, double sy, double sz) {
+    for (int j0 = s0; j0 < s1; j0 += 32) {
+        const int j = j0 + lane;
+        float x = 1e18f, y = 1e18f, z = 1e18f, m = 0.0f;            // padding: out of range of everything
+        if (j < s1) {
+            const double4 p = q.src[j];
+            x = (float)(p.x + sx);
+            y = (float)(p.y + sy);
+            z = (float)(p.z + sz);
+            m = (float)p.w;
+        }
+        pp_stage(stage, lane, 16, x, y, z, m);
+        pp_chunk2<G, POLY, UNI, false, 0, 16, 16>(stage, lane, T, k, q, j0, min(32, s1 - j0));
+    }
+}
+
+// An item: the targets from t0 of a cell as G = 1 or 2 groups of 32. Every target meets its sources in
+// ascending order, whatever the group it is in.
+template <int G, bool POLY, bool UNI>
+__device__ __forceinline__ void pp_item(ulonglong2* stage, int lane, const PPArgs& q, int c, int t0,
+                                        const PPConst& k) {
+    const int M = q.M, cl = q.last[c];
+    const int cx = c % M, cy = (c / M) % M, cz = c / (M * M);
+    const double ox = cx * q.l, oy = cy * q.l, oz = cz * q.l;
+    PPTarget T[2];
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+        const int t = t0 + 32 * g + lane;
+        float tx = -1e18f, ty = -1e18f, tz = -1e18f, tm = 0.0f;     // padding: out of range, of padding sources too
+        if (t < cl) {
             const double4 p = q.src[t];
             tx = (float)(p.x - ox);
             ty = (float)(p.y - oy);
             tz = (float)(p.z - oz);
             tm = (float)p.w;
         }
-        const f2x NTX = pk2(-tx, -tx), NTY = pk2(-ty, -ty), NTZ = pk2(-tz, -tz), NTM = pk2(-tm, -tm);
-        f2x AX = 0ull, AY = 0ull, AZ = 0ull;
-        // the item's own particles with each other (offsets 1 .. 16 as (j, j + 8), j = 1 .. 8)
-        __syncwarp();
-        stage[lane] = make_float4(tx, ty, tz, tm);
-        __syncwarp();
-        pp_chunk2(stage, lane, 1, 9, 8, true, NTX, NTY, NTZ, NTM, K, q, AX, AY, AZ, t0, min(32, cl - t0));
-        // the later particles of the cell, then the neighbouring cells of higher index
-        for (int nb = -1; nb < 27; ++nb) {
-            int s0, s1;
-            double sx = -ox, sy = -oy, sz = -oz;                    // source shift: periodic image - corner
-            if (nb < 0) {
-                s0 = t0 + 32;
-                s1 = cl;
-            } else {
-                if (nb == 13) continue;                            // the cell itself
-                int nx = cx + nb % 3 - 1, ny = cy + (nb / 3) % 3 - 1, nz = cz + nb / 9 - 1;
-                if (nx < 0) { nx += M; sx -= q.box; } else if (nx >= M) { nx -= M; sx += q.box; }
-                if (ny < 0) { ny += M; sy -= q.box; } else if (ny >= M) { ny -= M; sy += q.box; }
-                if (nz < 0) { nz += M; sz -= q.box; } else if (nz >= M) { nz -= M; sz += q.box; }
-                const int nc = (nz * M + ny) * M + nx;
-                if (nc < c) continue;                              // that cell's items take these pairs
-                s0 = q.first[nc];
-                s1 = q.last[nc];
-            }
-            for (int j0 = s0; j0 < s1; j0 += 32) {
-                const int j = j0 + lane;
-                __syncwarp();                                      // the previous chunk is consumed
-                float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                if (j < s1) {
-                    const double4 p = q.src[j];
-                    v = make_float4((float)(p.x + sx), (float)(p.y + sy), (float)(p.z + sz), (float)p.w);
-                }
-                stage[lane] = v;
-                __syncwarp();
-                pp_chunk2(stage, lane, 0, 16, 16, false, NTX, NTY, NTZ, NTM, K, q, AX, AY, AZ, j0, min(32, s1 - j0));
-            }
+        T[g] = PPTarget{dup(-tx), dup(-ty), dup(-tz), dup(-tm), 0ull, 0ull, 0ull};
+    }
+    // each group's particles with each other (offsets 1 .. 16 as (j, j + 8), j = 1 .. 8), then the first with the second
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+        const int t = t0 + 32 * g + lane;
+        const bool act = t < cl;
+        float x, y, z, m, h;
+        upk2(T[g].nx, x, h);
+        upk2(T[g].ny, y, h);
+        upk2(T[g].nz, z, h);
+        upk2(T[g].nm, m, h);
+        pp_stage(stage, lane, 8, act ? -x : 1e18f, act ? -y : 1e18f, act ? -z : 1e18f, -m);
+        PPTarget one[2];
+        one[0] = T[g];
+        pp_chunk2<1, POLY, UNI, true, 1, 9, 8>(stage, lane, one, k, q, t0 + 32 * g, min(32, cl - t0 - 32 * g));
+        T[g] = one[0];
+    }
+    if (G == 2) pp_walk<1, POLY, UNI>(stage, lane, T, k, q, t0 + 32, min(cl, t0 + 64), -ox, -oy, -oz);
+    // the later particles of the cell, then the neighbouring cells of higher index
+    for (int nb = -1; nb < 27; ++nb) {
+        int s0, s1;
+        double sx = -ox, sy = -oy, sz = -oz;                    // source shift: periodic image - corner
+        if (nb < 0) {
+            s0 = t0 + 32 * G;
+            s1 = cl;
+        } else {
+            if (nb == 13) continue;                            // the cell itself
+            int nx = cx + nb % 3 - 1, ny = cy + (nb / 3) % 3 - 1, nz = cz + nb / 9 - 1;
+            if (nx < 0) { nx += M; sx -= q.box; } else if (nx >= M) { nx -= M; sx += q.box; }
+            if (ny < 0) { ny += M; sy -= q.box; } else if (ny >= M) { ny -= M; sy += q.box; }
+            if (nz < 0) { nz += M; sz -= q.box; } else if (nz >= M) { nz -= M; sz += q.box; }
+            const int nc = (nz * M + ny) * M + nx;
+            if (nc < c) continue;                              // that cell's items take these pairs
+            s0 = q.first[nc];
+            s1 = q.last[nc];
         }
-        if (act) {
-            float x0, x1, y0, y1, z0, z1;
-            upk2(AX, x0, x1);
-            upk2(AY, y0, y1);
-            upk2(AZ, z0, z1);
-            atomicAdd(q.acc + t, x0 + x1);
-            atomicAdd(q.acc + q.n + t, y0 + y1);
-            atomicAdd(q.acc + 2 * q.n + t, z0 + z1);
+        pp_walk<G, POLY, UNI>(stage, lane, T, k, q, s0, s1, sx, sy, sz);
+    }
+    const float m = UNI ? q.m : 1.0f;
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+        const int t = t0 + 32 * g + lane;
+        float x0, x1, y0, y1, z0, z1;
+        upk2(T[g].ax, x0, x1);
+        upk2(T[g].ay, y0, y1);
+        upk2(T[g].az, z0, z1);
+        if (t < cl) {
+            atomicAdd(q.acc + t, m * (x0 + x1));
+            atomicAdd(q.acc + q.n + t, m * (y0 + y1));
+            atomicAdd(q.acc + 2 * q.n + t, m * (z0 + z1));
         }
+    }
+}
+
+template <bool POLY, bool UNI>
+__global__ void __launch_bounds__(PP_WARPS * 32) k_pp_pairs(const PPArgs q) {
+    __shared__ ulonglong2 sh[PP_WARPS][64];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    // lane k < PP_CLASSES: end of class 15 - k in the order the items are taken
+    unsigned end = lane < PP_CLASSES ? q.n_items[PP_CLASSES - 1 - lane] : 0;
+#pragma unroll
+    for (int o = 1; o < PP_CLASSES; o <<= 1) {
+        const unsigned y = __shfl_up_sync(0xffffffffu, end, o);
+        if (lane >= o) end += y;
+    }
+    const unsigned total = __shfl_sync(0xffffffffu, end, PP_CLASSES - 1);
+    ulonglong2* stage = sh[w];
+    PPConst k;
+    const float a9 = q.alpha * q.alpha / 9.0f;
+    k.alpha = dup(q.alpha);
+    k.eps2 = dup(q.eps2);
+    k.w1 = dup(-a9);
+    k.w0 = dup(fmaf(q.eps2, a9, 1.0f));
+    k.na3 = dup(-q.alpha * q.alpha * q.alpha);
+    k.hi = q.rc2 + q.eps2;
+    k.lo = 2.0f * q.eps2;
+    for (;;) {
+        unsigned it = 0;
+        if (lane == 0) it = atomicAdd(q.next, 1u);
+        it = __shfl_sync(0xffffffffu, it, 0);
+        if (it >= total) break;
+        const int b = __popc(__ballot_sync(0xffffffffu, lane < PP_CLASSES && end <= it));
+        const unsigned before = __shfl_sync(0xffffffffu, end, max(b - 1, 0));
+        const int2 item = q.items[(PP_CLASSES - 1 - b) * q.max_items + (it - (b ? before : 0u))];
+        const int c = item.x & (PP_TWO - 1);
+        if ((item.x & PP_TWO) && q.last[c] - item.y > 32) pp_item<2, POLY, UNI>(stage, lane, q, c, item.y, k);
+        else pp_item<1, POLY, UNI>(stage, lane, q, c, item.y, k);
     }
 }
 
@@ -352,9 +530,10 @@ extern "C" int sss_pm3_short(sss_pm3* p, const sss_pm3_particles* s, double G, d
     auto take = [&](size_t bytes) { const size_t o = off; off += (bytes + 255) & ~(size_t)255; return o; };
     const size_t o_k0 = take(8 * n), o_k1 = take(8 * n), o_v0 = take(4 * n), o_v1 = take(4 * n);
     const size_t o_src = take(32 * n), o_first = take(4 * cells), o_last = take(4 * cells);
-    const size_t o_rs = take(8 * std::max(sss_dev::radix_scratch(n), sss_dev::scan_scratch(cells)));
-    const size_t o_grp = take(8 * cells), o_off = take(8 * cells);
-    const size_t o_items = take(8 * (size_t)(n / 32 + cells + 1)), o_cnt = take(8), o_acc = take(12 * n);
+    const size_t o_rs = take(8 * sss_dev::radix_scratch(n));
+    const long long max_items = n / 32 + std::min<long long>(cells, n);
+    const size_t o_items = take(8 * (size_t)max_items * PP_CLASSES), o_cnt = take(4 * (PP_CLASSES + 1));
+    const size_t o_acc = take(12 * n);
     void* scr = nullptr;
     int rc = sss_scratch(ctx, off, &scr);
     if (rc) return rc;
@@ -366,10 +545,8 @@ extern "C" int sss_pm3_short(sss_pm3* p, const sss_pm3_particles* s, double G, d
     double4* src = (double4*)(B + o_src);
     int* first = (int*)(B + o_first);
     int* last = (int*)(B + o_last);
-    long long* groups = (long long*)(B + o_grp);
-    long long* offs = (long long*)(B + o_off);
     int2* items = (int2*)(B + o_items);
-    unsigned* counters = (unsigned*)(B + o_cnt);                  // [0] items, [1] work counter
+    unsigned* counters = (unsigned*)(B + o_cnt);                  // items per class, work counter
     const Pm3Parts parts = pm3_parts(s);
     const double l = p->box / M;
     k_pp_keys<<<blocks_for(n, 256), 256, 0, st>>>(parts, M, 1.0 / l, k0, v0);
@@ -381,11 +558,8 @@ extern "C" int sss_pm3_short(sss_pm3* p, const sss_pm3_particles* s, double G, d
     SSS_CUDA_TRY(ctx, cudaMemsetAsync(last, 0, 4 * (size_t)cells, st));
     k_pp_bounds<<<blocks_for(n, 256), 256, 0, st>>>(k0, n, first, last);
     SSS_LAUNCH_CHECK(ctx, "k_pp_bounds");
-    k_pp_groups<<<blocks_for(cells, 256), 256, 0, st>>>(first, last, cells, groups);
-    SSS_LAUNCH_CHECK(ctx, "k_pp_groups");
-    SSS_CUDA_TRY(ctx, sss_dev::exclusive_scan(groups, offs, cells, (long long*)(B + o_rs), st, ctx->d_status));
-    SSS_CUDA_TRY(ctx, cudaMemsetAsync(counters, 0, 8, st));
-    k_pp_items<<<blocks_for(cells, 256), 256, 0, st>>>(first, offs, cells, groups, items, counters);
+    SSS_CUDA_TRY(ctx, cudaMemsetAsync(counters, 0, 4 * (PP_CLASSES + 1), st));
+    k_pp_items<<<blocks_for(cells, 128), 128, 0, st>>>(first, last, M, cells, max_items, items, counters);
     SSS_LAUNCH_CHECK(ctx, "k_pp_items");
     PPArgs q;
     q.src = src;
@@ -401,14 +575,20 @@ extern "C" int sss_pm3_short(sss_pm3* p, const sss_pm3_particles* s, double G, d
     q.eps2 = (float)(eps * eps);
     q.items = items;
     q.n_items = counters;
-    q.next = counters + 1;
+    q.max_items = max_items;
+    q.next = counters + PP_CLASSES;
+    q.m = (float)s->mass_const;
     q.acc = (float*)(B + o_acc);
     q.n = n;
     SSS_CUDA_TRY(ctx, cudaMemsetAsync(q.acc, 0, 12 * (size_t)n, st));
+    // the polynomial's range is t <= 9; without a softening in f32 there is no r < eps test
+    const bool poly = alpha * r_cut <= 3.0000001 && q.eps2 > 0.0f;
+    void (*pairs)(const PPArgs) = poly ? (s->m ? k_pp_pairs<true, false> : k_pp_pairs<true, true>)
+                                       : (s->m ? k_pp_pairs<false, false> : k_pp_pairs<false, true>);
     int per_sm = 0;
-    SSS_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pp_pairs, PP_WARPS * 32, 0));
+    SSS_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pairs, PP_WARPS * 32, 0));
     const unsigned grid = (unsigned)(ctx->num_sms * std::max(per_sm, 1));
-    k_pp_pairs<<<grid, PP_WARPS * 32, 0, st>>>(q);
+    pairs<<<grid, PP_WARPS * 32, 0, st>>>(q);
     SSS_LAUNCH_CHECK(ctx, "k_pp_pairs");
     Pm3Epi e{mode, hdt, dt, p->box, snap};
     k_pp_finish<<<blocks_for(n, 256), 256, 0, st>>>(q, parts, e);

@@ -80,3 +80,34 @@ def test_bad_arguments():
     from solarsystemsimulator_b200 import pm3d
     with pytest.raises(ValueError):
         pm3d.PMPeriodic3D(8, 1.0, 1.0, 0, 2, 1.0, short_range=True)        # r_cut > box / 3
+
+
+@pytest.mark.parametrize("n,spread", [(2, 0.02), (31, 0.02), (33, 0.02), (64, 0.02), (65, 0.02), (97, 0.3), (9000, 0.02)])
+@pytest.mark.parametrize("x_cut,eps", [(3.0, 1e-3), (3.0, 0.0), (3.5, 1e-3)])
+@pytest.mark.parametrize("equal", [True, False])
+def test_pair_term_item_shapes(n, spread, x_cut, eps, equal):
+    """Group, item and work-list remainders (one and two groups of 32, a cell
+    above the long-walk limit), the polynomial and the erfc form, equal and
+    own masses. Per target the error is bounded by the sums over its pairs of
+    the Newtonian term times 1e-6 (the factor's error) plus three times the
+    rounding of an offset (2 cells to f32) over r, plus one rounding per
+    accumulated term."""
+    from oracle import pm3d as opm
+    from solarsystemsimulator_b200 import pm3d
+    rng = np.random.default_rng(n)
+    pos = np.mod(0.99 + rng.normal(0, spread, (n, 3)), 1.0)
+    mass = np.full(n, 0.7 / n) if equal else rng.uniform(0.5, 1.5, n) / n
+    pm = pm3d.PMPeriodic3D(64, 1.0, 1.0, 0, 2, 1.0, short_range=True, softening=eps, x_cut=x_cut)
+    st = pm.load_state(pos, np.zeros_like(pos), 0.7 / n if equal else mass)
+    a = _pair_only(pm, st)
+    sel = rng.choice(n, min(n, 100), replace=False)
+    ref = opm.p3m_short(pos, mass, pos[sel], pm.alpha, pm.r_cut, eps=eps, self_index=sel)
+    d = pos[None, :, :] - pos[sel][:, None, :]
+    d -= np.round(d)
+    r = np.sqrt((d * d).sum(2))
+    r[np.arange(len(sel)), sel] = np.inf
+    newton = np.where(r < 1.001 * pm.r_cut, mass / (r * r), 0.0)
+    cell = 1.0 / int(1.0 / pm.r_cut)
+    tol = (newton * (1e-6 + 3.0 * np.sqrt(3.0) * 2.0 * cell * 2.0 ** -24 / r)).sum(1)
+    tol += newton.sum(1) * (newton > 0).sum(1) * 2.0 ** -24
+    assert np.all(np.abs(a[sel] - ref).max(1) <= tol + 1e-30)
