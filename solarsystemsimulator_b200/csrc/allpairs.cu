@@ -50,6 +50,19 @@ constexpr int MIX_MINB = 2;
 
 constexpr int WAVES = 16;       // target number of CTA waves per evaluation
 
+// warp-split kernels (fewer than SPLIT_PAIRS pairs): 8 warps share 64 or 128
+// targets and split the CTA's sources. The limits are where the two forms cross
+// (us per evaluation, split / general; 2-D mixed crosses later, at 1e9):
+//   mixed 3-D  10,007^2 57 / 88, 17,000^2 148 / 156, 20,000^2 199 / 207, 25,000^2 294 / 290, 40,000^2 748 / 671
+//   f64 3-D    10,007^2 125 / 133, 17,000^2 316 / 326, 20,000^2 438 / 437, 30,000^2 960 / 927
+constexpr int WS_W = 8;
+constexpr int WS_NT = WS_W * 32;
+constexpr int WS_TS = 512;      // sources per tile (mixed: the tile with one centre)
+constexpr int WS_MAXCHUNKS = 16;
+constexpr int WS_R_F64 = 2, WS_R_MIX = 4;
+constexpr int WS_MINB_F64 = 4, WS_MINB_MIX = 2;
+constexpr double SPLIT_PAIRS_F64 = 3e8, SPLIT_PAIRS_MIX = 4.5e8;
+
 // r2 below this is outside the integer-seeded rsqrt's range (2^-126)
 constexpr double kIseedMinR2 = 1.1754943508222875e-38;
 
@@ -507,6 +520,250 @@ __global__ void __launch_bounds__(NT, MINB) k_force_mixed(const ForceArgs a) {
     finish_block<D, R, NT>(a, tb, ch, ax, ay, az);
 }
 
+// ----------------------------------------------- few pairs: split by warps
+//
+// With few bodies the kernels above leave the device idle: 3,000 targets are
+// three blocks of 1,024, and cutting the sources finer only moves the time
+// into the partial sums one CTA has to add. Here a CTA takes 32 R targets
+// (every warp the same ones, R per lane) and its 8 warps a slice each of the
+// CTA's sources, so a block of targets meets 8 sources at a time; the warps'
+// sums are added through shared memory in slice order, the chunks' (at most 16)
+// by the last CTA of the target block as above. Latency-bound below ~2,000
+// bodies (an evaluation of 300 or 1,000 bodies: under 8.5 us a call, host
+// included, against 23-55), FP32 / FP64 pipe above (3,000 sources on 23,000
+// targets, 2-D mixed: 33 us against 45; 10,007 bodies, f64 3-D: 125 against 133).
+// 128 registers for the mixed form, 64 for f64: 3,000^2 3-D mixed 12.3 us against
+// 15.8 with 80; 3,000 x 23,000 3-D f64 89 against 103 with 80. The mixed form centres and
+// rounds its tiles itself (bounding-box centre of at most 512 consecutive
+// sources, as k_prep_mixed), which saves that kernel's launch.
+
+// Block-wide bounding box of the tile's sources (f32 offsets v from the first
+// one, `base`) and its centre; whether all Gm are equal.
+template <int D>
+__device__ __forceinline__ void ws_centre(const float (&v)[2][3], const bool (&ok)[2], bool same,
+                                          const double4& base, double (&cen)[3], bool& uni) {
+    __shared__ float s_box[6][WS_W];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    float lo[3], hi[3];
+#pragma unroll
+    for (int c = 0; c < D; ++c) {
+        lo[c] = fminf(ok[0] ? v[0][c] : 3e38f, ok[1] ? v[1][c] : 3e38f);
+        hi[c] = fmaxf(ok[0] ? v[0][c] : -3e38f, ok[1] ? v[1][c] : -3e38f);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            lo[c] = fminf(lo[c], __shfl_xor_sync(0xffffffffu, lo[c], o));
+            hi[c] = fmaxf(hi[c], __shfl_xor_sync(0xffffffffu, hi[c], o));
+        }
+        if (lane == 0) { s_box[c][w] = lo[c]; s_box[3 + c][w] = hi[c]; }
+    }
+    uni = __syncthreads_and(same) != 0;
+    cen[0] = base.x;
+    cen[1] = base.y;
+    cen[2] = D == 3 ? base.z : 0.0;
+#pragma unroll
+    for (int c = 0; c < D; ++c) {
+        float l = s_box[c][0], h = s_box[3 + c][0];
+#pragma unroll
+        for (int q = 1; q < WS_W; ++q) { l = fminf(l, s_box[c][q]); h = fmaxf(h, s_box[3 + c][q]); }
+        cen[c] += 0.5 * ((double)l + (double)h);
+    }
+}
+
+// Sum over the warps (ascending slices) of acc[R][3], chunk partials, epilogue.
+// red: [3][WS_W][32 R] doubles of shared memory, free to overwrite.
+template <int D, int R>
+__device__ __forceinline__ void ws_finish(const ForceArgs& a, int tb, int ch, double* red, const double (&ax)[R],
+                                          const double (&ay)[R], const double (&az)[R]) {
+    constexpr int TB = 32 * R;
+    __shared__ unsigned s_last;
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        red[(0 * WS_W + w) * TB + 32 * r + lane] = ax[r];
+        red[(1 * WS_W + w) * TB + 32 * r + lane] = ay[r];
+        if (D == 3) red[(2 * WS_W + w) * TB + 32 * r + lane] = az[r];
+    }
+    __syncthreads();
+    const int64_t i = (int64_t)tb * TB + tid;
+    const bool mine = tid < TB && i < a.n_tgt;
+    double sx = 0.0, sy = 0.0, sz = 0.0;
+    if (mine) {
+#pragma unroll
+        for (int q = 0; q < WS_W; ++q) {
+            sx += red[(0 * WS_W + q) * TB + tid];
+            sy += red[(1 * WS_W + q) * TB + tid];
+            if (D == 3) sz += red[(2 * WS_W + q) * TB + tid];
+        }
+    }
+    if (a.n_chunks == 1) {
+        if (mine) epilogue<D>(a.epi, i, sx, sy, sz, a.tgt[i]);
+        return;
+    }
+    if (mine) {
+        double2* q = reinterpret_cast<double2*>(a.part + (int64_t)ch * a.n_tgt + i);
+        __stcg(q, make_double2(sx, sy));
+        __stcg(q + 1, make_double2(sz, 0.0));
+    }
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) {
+        const unsigned prev = atomicAdd(&a.counters[tb], 1u);
+        s_last = (prev == (unsigned)(a.n_chunks - 1)) ? 1u : 0u;
+        if (s_last) a.counters[tb] = 0u;   // ready for the next launch
+    }
+    __syncthreads();
+    if (!s_last || !mine) return;
+    __threadfence();
+    double2 p0[WS_MAXCHUNKS], p1[WS_MAXCHUNKS];
+#pragma unroll
+    for (int c = 0; c < WS_MAXCHUNKS; ++c)
+        if (c < a.n_chunks) {
+            const double2* q = reinterpret_cast<const double2*>(a.part + (int64_t)c * a.n_tgt + i);
+            p0[c] = __ldcg(q);
+            p1[c] = __ldcg(q + 1);
+        }
+    sx = sy = sz = 0.0;
+#pragma unroll
+    for (int c = 0; c < WS_MAXCHUNKS; ++c)
+        if (c < a.n_chunks) {
+            sx += p0[c].x;
+            sy += p0[c].y;
+            sz += p1[c].x;
+        }
+    epilogue<D>(a.epi, i, sx, sy, sz, a.tgt[i]);
+}
+
+template <int D, int R, int VAR>
+__global__ void __launch_bounds__(WS_NT, WS_MINB_F64) k_force_f64_ws(const ForceArgs a) {
+    constexpr int TB = 32 * R;
+    constexpr int RED = 3 * WS_W * TB * (int)sizeof(double), SRC = WS_TS * (int)sizeof(double4);
+    __shared__ __align__(16) unsigned char smem[RED > SRC ? RED : SRC];
+    double4* tile = reinterpret_cast<double4*>(smem);
+    const int S = a.n_chunks, tb = blockIdx.x / S, ch = blockIdx.x - tb * S;
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    double px[R], py[R], pz[R], ax[R], ay[R], az[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int64_t i = (int64_t)tb * TB + 32 * r + lane;
+        const double4 p = (i < a.n_tgt) ? a.tgt[i] : make_double4(0.0, 0.0, 0.0, 0.0);
+        px[r] = p.x; py[r] = p.y; pz[r] = p.z;
+        ax[r] = 0.0; ay[r] = 0.0; az[r] = 0.0;
+    }
+    const int64_t c0 = ch * a.n_src / S, c1 = (ch + 1) * a.n_src / S;
+    for (int64_t j0 = c0; j0 < c1; j0 += WS_TS) {
+        const int cnt = (int)min((int64_t)WS_TS, c1 - j0);
+        const double w0 = a.src[j0].w;
+        bool same = true;
+        if (j0 > c0) __syncthreads();                       // the previous tile is consumed
+        for (int j = tid; j < cnt; j += WS_NT) {
+            const double4 v = a.src[j0 + j];
+            tile[j] = v;
+            same &= (v.w == w0);
+        }
+        const bool uni = __syncthreads_and(same) != 0;
+        const int b = w * cnt / WS_W, e = (w + 1) * cnt / WS_W;
+        double tx[R], ty[R], tz[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) { tx[r] = 0.0; ty[r] = 0.0; tz[r] = 0.0; }
+        if (uni) tile_f64<D, R, VAR, true, F64_UNROLL>(tile + b, e - b, a.eps2, px, py, pz, tx, ty, tz);
+        else tile_f64<D, R, VAR, false, F64_UNROLL>(tile + b, e - b, a.eps2, px, py, pz, tx, ty, tz);
+        const double wt = uni ? w0 : 1.0;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            ax[r] = fma(wt, tx[r], ax[r]);
+            ay[r] = fma(wt, ty[r], ay[r]);
+            az[r] = fma(wt, tz[r], az[r]);
+        }
+    }
+    __syncthreads();                                        // the last tile is consumed
+    ws_finish<D, R>(a, tb, ch, reinterpret_cast<double*>(smem), ax, ay, az);
+}
+
+template <int D, int R>
+__global__ void __launch_bounds__(WS_NT, WS_MINB_MIX) k_force_mixed_ws(const ForceArgs a) {
+    static_assert(WS_TS == 2 * WS_NT, "two sources per thread and tile");
+    constexpr int TB = 32 * R, P = R / 2;
+    constexpr int RED = 3 * WS_W * TB * (int)sizeof(double), SRC = WS_TS * 2 * (int)sizeof(float4);
+    __shared__ __align__(16) unsigned char smem[RED > SRC ? RED : SRC];
+    const int S = a.n_chunks, tb = blockIdx.x / S, ch = blockIdx.x - tb * S;
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    double px[R], py[R], pz[R], ax[R], ay[R], az[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int64_t i = (int64_t)tb * TB + 32 * r + lane;
+        const double4 p = (i < a.n_tgt) ? a.tgt[i] : make_double4(0.0, 0.0, 0.0, 0.0);
+        px[r] = p.x; py[r] = p.y; pz[r] = p.z;
+        ax[r] = 0.0; ay[r] = 0.0; az[r] = 0.0;
+    }
+    const float eps2f = (float)a.eps2;
+    const f2x eps2x = pk2(eps2f, eps2f);
+    const int64_t c0 = ch * a.n_src / S, c1 = (ch + 1) * a.n_src / S;
+    for (int64_t j0 = c0; j0 < c1; j0 += WS_TS) {
+        const int cnt = (int)min((int64_t)WS_TS, c1 - j0);
+        const double4 base = a.src[j0];
+        const double w0 = base.w;
+        double4 v[2];
+        float f[2][3];
+        bool ok[2], same = true;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int j = tid + h * WS_NT;
+            ok[h] = j < cnt;
+            v[h] = ok[h] ? a.src[j0 + j] : make_double4(0.0, 0.0, 0.0, 0.0);
+            f[h][0] = (float)(v[h].x - base.x);
+            f[h][1] = (float)(v[h].y - base.y);
+            f[h][2] = (float)(v[h].z - base.z);
+            if (ok[h]) same &= (v[h].w == w0);
+        }
+        double cen[3];
+        bool uni;
+        ws_centre<D>(f, ok, same, base, cen, uni);               // (its barrier: the previous tile is consumed)
+        float4* out = reinterpret_cast<float4*>(smem);
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+            if (ok[h]) {
+                const int j = tid + h * WS_NT;
+                const float x = __double2float_rn(v[h].x - cen[0]), y = __double2float_rn(v[h].y - cen[1]);
+                const float z = (D == 3) ? __double2float_rn(v[h].z - cen[2]) : 0.f, m = __double2float_rn(v[h].w);
+                out[2 * j] = make_float4(x, x, y, y);
+                out[2 * j + 1] = make_float4(z, z, m, m);
+            }
+        f2x ox[P], oy[P], oz[P], fx[P], fy[P], fz[P];
+#pragma unroll
+        for (int q = 0; q < P; ++q) {
+            ox[q] = pk2(__double2float_rn(cen[0] - px[2 * q]), __double2float_rn(cen[0] - px[2 * q + 1]));
+            oy[q] = pk2(__double2float_rn(cen[1] - py[2 * q]), __double2float_rn(cen[1] - py[2 * q + 1]));
+            oz[q] = (D == 3) ? pk2(__double2float_rn(cen[2] - pz[2 * q]), __double2float_rn(cen[2] - pz[2 * q + 1]))
+                             : pk2(0.f, 0.f);
+            fx[q] = 0ull; fy[q] = 0ull; fz[q] = 0ull;
+        }
+        __syncthreads();                                    // the tile is staged
+        // a warp's slice is at most WS_TS / WS_W = 64 sources: one f32 partial sum (MIX_SUB = 128 above)
+        const int b = w * cnt / WS_W, e = (w + 1) * cnt / WS_W;
+        const ulonglong2* s = reinterpret_cast<const ulonglong2*>(smem);
+        if (uni) subtile_mixed<D, P, true>(s, b, e, eps2x, ox, oy, oz, fx, fy, fz);
+        else subtile_mixed<D, P, false>(s, b, e, eps2x, ox, oy, oz, fx, fy, fz);
+        const double wt = uni ? w0 : 1.0;
+#pragma unroll
+        for (int q = 0; q < P; ++q) {
+            float l0, l1;
+            upk2(fx[q], l0, l1);
+            ax[2 * q] = fma(wt, (double)l0, ax[2 * q]);
+            ax[2 * q + 1] = fma(wt, (double)l1, ax[2 * q + 1]);
+            upk2(fy[q], l0, l1);
+            ay[2 * q] = fma(wt, (double)l0, ay[2 * q]);
+            ay[2 * q + 1] = fma(wt, (double)l1, ay[2 * q + 1]);
+            if (D == 3) {
+                upk2(fz[q], l0, l1);
+                az[2 * q] = fma(wt, (double)l0, az[2 * q]);
+                az[2 * q + 1] = fma(wt, (double)l1, az[2 * q + 1]);
+            }
+        }
+    }
+    __syncthreads();                                        // the last tile is consumed
+    ws_finish<D, R>(a, tb, ch, reinterpret_cast<double*>(smem), ax, ay, az);
+}
+
 // ------------------------------------------------------------- potential
 
 // phi_t = -sum_s Gm_s / sqrt(|d|^2 + eps2), f64, one target per thread,
@@ -578,18 +835,58 @@ Plan make_plan(int64_t n_src, int64_t n_tgt, int targets_per_block, int ts, int 
     return p;
 }
 
+// Chunks per target block of a warp-split kernel: the split that takes the
+// fewest rounds of CTAs times their length, a CTA's fixed part (launch,
+// targets, sums over warps and chunks) counted as WS_FIXED sources; no chunk
+// shorter than 8 sources a warp.
+Plan make_plan_ws(int64_t n_src, int64_t n_tgt, int targets_per_block, int slots) {
+    constexpr int64_t WS_FIXED = 96;
+    Plan p;
+    p.n_tblocks = (int)((n_tgt + targets_per_block - 1) / targets_per_block);
+    p.n_tiles = p.tiles_per_chunk = 0;
+    p.n_chunks = 1;
+    int64_t best = -1;
+    for (int64_t s = 1; s <= WS_MAXCHUNKS && (s == 1 || n_src / s >= 8 * WS_W); ++s) {
+        const int64_t rounds = (p.n_tblocks * s + slots - 1) / slots;
+        const int64_t cost = rounds * ((n_src + s - 1) / s + WS_FIXED + 4 * s);
+        if (best < 0 || cost < best) {
+            best = cost;
+            p.n_chunks = (int)s;
+        }
+    }
+    return p;
+}
+
 // The force kernel a launch uses and its launch shape.
 struct KSel {
     void* fn;
     int nt, tpb, ts;
     size_t smem;       // dynamic shared memory
-    int key;           // index of its cached occupancy (0..5)
-    bool mixed;
+    int key;           // index of its cached occupancy (0 .. SSS_AP_KERNELS - 1)
+    bool mixed;        // takes the tiles k_prep_mixed writes
+    bool ws;           // warp-split (make_plan_ws)
 };
 
-KSel select_kernel(int dim, int precision, double eps2) {
+KSel select_kernel(int dim, int precision, double eps2, int64_t n_src, int64_t n_tgt) {
     KSel k;
     k.mixed = (precision == SSS_PREC_MIXED);
+    k.ws = (double)n_src * (double)n_tgt < (k.mixed ? SPLIT_PAIRS_MIX : SPLIT_PAIRS_F64);
+    if (k.ws) {
+        const bool iseed = eps2 >= kIseedMinR2;
+        if (k.mixed)
+            k.fn = (dim == 3) ? (void*)k_force_mixed_ws<3, WS_R_MIX> : (void*)k_force_mixed_ws<2, WS_R_MIX>;
+        else if (iseed)
+            k.fn = (dim == 3) ? (void*)k_force_f64_ws<3, WS_R_F64, 2> : (void*)k_force_f64_ws<2, WS_R_F64, 2>;
+        else
+            k.fn = (dim == 3) ? (void*)k_force_f64_ws<3, WS_R_F64, 1> : (void*)k_force_f64_ws<2, WS_R_F64, 1>;
+        k.nt = WS_NT;
+        k.tpb = 32 * (k.mixed ? WS_R_MIX : WS_R_F64);
+        k.ts = WS_TS;
+        k.smem = 0;
+        k.key = 8 + (k.mixed ? 4 : (iseed ? 0 : 2)) + (dim == 3);
+        k.mixed = false;
+        return k;
+    }
     if (k.mixed) {
         k.fn = (dim == 3) ? (void*)k_force_mixed<3, MIX_R, MIX_NT, MIX_TS, MIX_SUB, MIX_MINB>
                           : (void*)k_force_mixed<2, MIX_R, MIX_NT, MIX_TS, MIX_SUB, MIX_MINB>;
@@ -647,13 +944,14 @@ int force_eval(sss_ctx* ctx, int dim, int precision, const double4* src, int64_t
         return sss_set_err(ctx, SSS_ERR_ARG, "all-pairs: size out of range");
     if (precision == SSS_PREC_MIXED_TC)
         return sss_ap::force_eval_tc(ctx, dim, src, n_src, tgt, n_tgt, eps2, epi, stream);
-    const KSel ks = select_kernel(dim, precision, eps2);
+    const KSel ks = select_kernel(dim, precision, eps2, n_src, n_tgt);
     if (ctx->occ[ks.key] == 0) {
         int per_sm = 0;
         SSS_CUDA_TRY(ctx, query_occupancy(ks, &per_sm));
         ctx->occ[ks.key] = per_sm;
     }
-    const Plan pl = make_plan(n_src, n_tgt, ks.tpb, ks.ts, ctx->occ[ks.key] * ctx->num_sms);
+    const int slots = ctx->occ[ks.key] * ctx->num_sms;
+    const Plan pl = ks.ws ? make_plan_ws(n_src, n_tgt, ks.tpb, slots) : make_plan(n_src, n_tgt, ks.tpb, ks.ts, slots);
 
     ForceArgs a;
     memset(&a, 0, sizeof(a));
@@ -874,7 +1172,7 @@ struct NoAllocDevice {
     int ready;
     unsigned char* base;  // device address of g_sss_noalloc_scratch on this device
     int num_sms;
-    int occ[6];           // CTAs per SM of the force kernels (KSel::key)
+    int occ[SSS_AP_KERNELS];   // CTAs per SM of the force kernels (KSel::key)
 };
 
 constexpr int kNoAllocMaxDevices = 64;
@@ -908,13 +1206,16 @@ int noalloc_setup(int device, NoAllocDevice** out, char* eb, size_t el) {
             d->base = (unsigned char*)p;
             e = cudaDeviceGetAttribute(&d->num_sms, cudaDevAttrMultiProcessorCount, device);
             // one representative eps2 per f64 seed variant selects each kernel once
+            // and one size for the few-pairs and the general kernels
             const double probe_eps2[2] = {1.0, 0.0};
+            const int64_t probe_n[2] = {1, (int64_t)1 << 20};
             for (int prec = 0; prec < 2 && e == cudaSuccess; ++prec)
                 for (int dim = 2; dim <= 3 && e == cudaSuccess; ++dim)
-                    for (int v = 0; v < (prec ? 1 : 2) && e == cudaSuccess; ++v) {
-                        const KSel ks = select_kernel(dim, prec, probe_eps2[v]);
-                        e = query_occupancy(ks, &d->occ[ks.key]);
-                    }
+                    for (int v = 0; v < (prec ? 1 : 2) && e == cudaSuccess; ++v)
+                        for (int q = 0; q < 2 && e == cudaSuccess; ++q) {
+                            const KSel ks = select_kernel(dim, prec, probe_eps2[v], probe_n[q], probe_n[q]);
+                            e = query_occupancy(ks, &d->occ[ks.key]);
+                        }
             if (e != cudaSuccess)
                 rc = noalloc_err(eb, el, SSS_ERR_CUDA, "no-alloc setup: %s", cudaGetErrorString(e));
             else
@@ -953,8 +1254,9 @@ extern "C" int sss_allpairs_accel_noalloc(int device, int dim, int precision, co
     int rc = noalloc_setup(device, &d, eb, el);
     if (rc) return rc;
 
-    const KSel ks = select_kernel(dim, precision, eps2);
-    Plan pl = make_plan(n_src, n_tgt, ks.tpb, ks.ts, d->occ[ks.key] * d->num_sms);
+    const KSel ks = select_kernel(dim, precision, eps2, n_src, n_tgt);
+    const int slots = d->occ[ks.key] * d->num_sms;
+    Plan pl = ks.ws ? make_plan_ws(n_src, n_tgt, ks.tpb, slots) : make_plan(n_src, n_tgt, ks.tpb, ks.ts, slots);
 
     // scratch layout: [status 256 B][counters 64 KiB][tiles][centres][partials]
     const size_t data_off = SSS_NOALLOC_STATUS_BYTES + SSS_NOALLOC_COUNTERS * sizeof(unsigned);
@@ -962,7 +1264,8 @@ extern "C" int sss_allpairs_accel_noalloc(int device, int dim, int precision, co
     const size_t bytes_tiles = ks.mixed ? mixed_tile_bytes(pl.n_tiles) : 0;
     const size_t bytes_cent = ks.mixed ? mixed_centre_bytes(pl.n_tiles) : 0;
     const size_t fixed = bytes_tiles + bytes_cent;
-    if (fixed > avail)
+    // (the mixed limit holds for every mixed call, whichever kernel takes it)
+    if (fixed > avail || (precision == SSS_PREC_MIXED && n_src > SSS_NOALLOC_MAX_MIXED_SOURCES))
         return noalloc_err(eb, el, SSS_ERR_CAPACITY,
                            "n_src = %lld needs %zu bytes of mixed-precision tiles; the no-allocation "
                            "scratch holds %zu (at most %d sources)", (long long)n_src, fixed, avail,
@@ -973,7 +1276,9 @@ extern "C" int sss_allpairs_accel_noalloc(int device, int dim, int precision, co
         size_t s_fit = (avail - fixed) / per_chunk;
         if (pl.n_tblocks > (int)SSS_NOALLOC_COUNTERS) s_fit = 1;
         if (s_fit < (size_t)pl.n_chunks) {
-            if (s_fit <= 1) {
+            if (ks.ws) {
+                pl.n_chunks = s_fit < 1 ? 1 : (int)s_fit;
+            } else if (s_fit <= 1) {
                 pl.tiles_per_chunk = pl.n_tiles;
                 pl.n_chunks = 1;
             } else {

@@ -11,6 +11,8 @@
 
 #include "../../include/sss.h"
 
+#define SSS_AP_KERNELS 14   // all-pairs force kernels by dimension, precision and size
+
 struct sss_ctx {
     int device;
     int num_sms;
@@ -25,7 +27,7 @@ struct sss_ctx {
     unsigned* d_counters;
     size_t n_counters;
     // cached CTAs-per-SM of the all-pairs kernels (0 = not yet queried)
-    int occ[8];
+    int occ[SSS_AP_KERNELS];
     // the broadphase pipeline as an instantiated graph (broadphase.cu)
     struct sss_bp_graph* bp_graph;
 };

@@ -276,3 +276,30 @@ def test_step_batch_argument_errors():
         sim.step_batch(None, 0.01, 1)
     with pytest.raises(ValueError):
         sg.NBodySelfGrav(0, softening_au=0.0)
+
+
+@pytest.mark.parametrize("dim", [2, 3])
+@pytest.mark.parametrize("n_src,n_tgt", [(1, 65), (7, 64), (63, 63), (65, 129), (512, 127), (513, 1), (1025, 300),
+                                         (8200, 1000), (20000, 25000)])
+@pytest.mark.parametrize("equal", [True, False])
+def test_few_pairs_kernels(dim, n_src, n_tgt, equal):
+    """Edges of the kernels that split the sources by warps (target blocks of 64
+    and 128, tiles of 512, chunks, one size beyond their limit) with equal and
+    own masses. f64: the parity bar. Mixed, per component: every pair term m /
+    (r^2 + eps^2) times 1e-6 (the factor) plus 3 sqrt(3) roundings of an offset
+    (extent 2, f32) over the softened distance (>= eps = 0.05)."""
+    sg = _sg()
+    src, tgt = cloud(n_src, dim, seed=n_src), cloud(n_tgt, dim, seed=n_tgt + 1)
+    if equal:
+        src[:, 3] = 0.7 / n_src
+    sel = np.random.default_rng(0).choice(n_tgt, min(n_tgt, 400), replace=False)
+    eps = 0.05
+    ref = osg.accel(src, tgt[sel], eps * eps, dim=dim)
+    dev = [torch.from_numpy(v).cuda() for v in (src, tgt)]
+    a = sg.allpairs_accel(*dev, eps * eps, dim=dim, precision="f64").cpu().numpy()[sel]
+    ok, worst = parity_ok(a, ref, dim)
+    assert ok, worst
+    r2 = ((src[None, :, :dim] - tgt[sel][:, None, :dim]) ** 2).sum(2) + eps * eps
+    scale = (src[None, :, 3] / r2 * (1e-6 + 3.0 * np.sqrt(3.0) * 2.0 * 2.0 ** -24 / np.sqrt(r2))).sum(1)
+    a = sg.allpairs_accel(*dev, eps * eps, dim=dim, precision="mixed").cpu().numpy()[sel]
+    assert np.all(np.abs(a[:, :dim] - ref[:, :dim]).max(1) <= scale)
