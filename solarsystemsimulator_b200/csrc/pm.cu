@@ -1,15 +1,29 @@
 // Particle-mesh forces for sm_100a: replaces the 2-D isolated PM of the
-// reference (backend/pm_kernel.py:34-293). cuFFT performs only the
-// transforms; deposit, kernel build, spectrum multiply, gather and the KDK
-// integration are kernels of this file.
+// reference (backend/pm_kernel.py:34-293). Deposit, kernel build, the
+// convolution, gather and the KDK integration are kernels of this file.
 //
-// 2-D isolated (Hockney-James): masses are deposited by cloud-in-cell
-// straight into the zero-padded 2N x 2N grid, transformed (D2Z), multiplied
-// by the transforms of the softened force kernels K_x, K_y (with the inverse
-// transform's 1/(2N)^2 folded in), transformed back (2x Z2D) and read back
-// bilinearly with the deposit's stencil. f64 throughout, as the reference.
+// 2-D isolated (Hockney-James): masses are deposited by cloud-in-cell, the
+// zero-padded 2N x 2N density is transformed, multiplied by the transforms of
+// the softened force kernels K_x, K_y (with the inverse transform's 1/(2N)^2
+// folded in), transformed back and read bilinearly with the deposit's
+// stencil. f64 throughout, as the reference.
+//
+// The convolution (2N = 2^a, 3 2^a or 1000 2^a up to 8192) is three kernels
+// over the block transforms of fft.cuh:
+//   k_rows_fwd : two real rows a, b as one complex transform a + i b; only
+//                the N rows and the N columns that hold mass are read
+//   k_cols     : one column: forward, times each kernel spectrum, inverse,
+//                only the N rows of the crop written
+//   k_rows_inv : the two force components of a row as one complex transform
+//                f_x + i f_y, stored as pairs that the gather reads whole
+// K(d; h, eps) = G / h^2 K(d / h; 1, eps / h), and offsets of +-N never meet
+// two grid points, so the spectra are those of the unit kernel with those
+// offsets zeroed: purely imaginary, odd along the force's axis and even along
+// the other, one (N + 1)^2 table of reals (kept with its transpose) that a
+// plan remakes only when eps / h changes, not with every new h.
+// Other sizes go through cuFFT with the kernels of the current h.
 
-#include "sss_internal.cuh"
+#include "fft.cuh"
 
 #include <cufft.h>
 
@@ -47,10 +61,10 @@ __device__ __forceinline__ void cic2(double gx, double gy, double x0, double y0,
     ty = __dsub_rn(fy, (double)j);
 }
 
-// deposit into the padded (2N x 2N, row stride 2N) array
+// deposit into the grid of row stride s (2N where the padded array is transformed whole)
 __global__ void k_cic_deposit_2d(const double* __restrict__ gx, const double* __restrict__ gy,
-                                 const double* __restrict__ gm, long long np_, int n, double x0, double y0,
-                                 double h, double* __restrict__ rho_pad) {
+                                 const double* __restrict__ gm, long long np_, int n, long long s, double x0,
+                                 double y0, double h, double* __restrict__ rho_pad) {
     const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= np_) return;
     int i, j;
@@ -58,7 +72,6 @@ __global__ void k_cic_deposit_2d(const double* __restrict__ gx, const double* __
     cic2(gx[p], gy[p], x0, y0, h, n, i, j, tx, ty);
     const double m = gm[p];
     const double ux = __dsub_rn(1.0, tx), uy = __dsub_rn(1.0, ty);
-    const long long s = 2LL * n;
     atomicAdd(&rho_pad[(long long)i * s + j], __dmul_rn(__dmul_rn(m, ux), uy));
     atomicAdd(&rho_pad[(long long)(i + 1) * s + j], __dmul_rn(__dmul_rn(m, tx), uy));
     atomicAdd(&rho_pad[(long long)i * s + (j + 1)], __dmul_rn(__dmul_rn(m, ux), ty));
@@ -109,6 +122,182 @@ __global__ void k_cic_gather_2d(const double* __restrict__ px, const double* __r
     ay[p] = out[1];
 }
 
+// the same read of the N x N field of pairs (f_x, f_y)
+__global__ void k_cic_gather_pairs_2d(const double* __restrict__ px, const double* __restrict__ py, long long np_,
+                                      int n, double x0, double y0, double h, const double2* __restrict__ f,
+                                      double* __restrict__ ax, double* __restrict__ ay) {
+    const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= np_) return;
+    int i, j;
+    double tx, ty;
+    cic2(px[p], py[p], x0, y0, h, n, i, j, tx, ty);
+    const double ux = __dsub_rn(1.0, tx), uy = __dsub_rn(1.0, ty);
+    const long long c00 = (long long)i * n + j;
+    const double2 f00 = f[c00], f10 = f[c00 + n], f01 = f[c00 + 1], f11 = f[c00 + n + 1];
+    ax[p] = __dadd_rn(__dadd_rn(__dadd_rn(__dmul_rn(__dmul_rn(f00.x, ux), uy), __dmul_rn(__dmul_rn(f10.x, tx), uy)),
+                                __dmul_rn(__dmul_rn(f01.x, ux), ty)), __dmul_rn(__dmul_rn(f11.x, tx), ty));
+    ay[p] = __dadd_rn(__dadd_rn(__dadd_rn(__dmul_rn(__dmul_rn(f00.y, ux), uy), __dmul_rn(__dmul_rn(f10.y, tx), uy)),
+                                __dmul_rn(__dmul_rn(f01.y, ux), ty)), __dmul_rn(__dmul_rn(f11.y, tx), ty));
+}
+
+__global__ void k_split_pairs_2d(const double2* __restrict__ f, long long m, double* __restrict__ ax,
+                                 double* __restrict__ ay) {
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= m) return;
+    ax[t] = f[t].x;
+    ay[t] = f[t].y;
+}
+
+// ---------------------------------------------------- convolution, own FFTs
+
+// K_x of unit cell size and G = 1, zero at the offsets +-N
+__global__ void k_unit_kernel_2d(int n, double e2, double* __restrict__ kx) {
+    const int np = 2 * n;
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= (long long)np * np) return;
+    const int i = (int)(t / np), j = (int)(t % np);
+    if (i == n || j == n) { kx[t] = 0.0; return; }
+    const double dx = (double)(i < n ? i : i - np), dy = (double)(j < n ? j : j - np);
+    const double r2 = dx * dx + dy * dy + e2;
+    kx[t] = -dx / (r2 * sqrt(r2));
+}
+
+// U[a][b] = Im of the spectrum at (a, b), a, b <= N, and its transpose V
+__global__ void __launch_bounds__(256) k_kernel_tables_2d(const double2* __restrict__ fk, int n,
+                                                          double* __restrict__ u, double* __restrict__ v) {
+    __shared__ double tile[32][33];
+    const int m = n + 1, tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    for (int r = ty; r < 32; r += 8) {
+        const int a = blockIdx.y * 32 + r, b = blockIdx.x * 32 + tx;
+        double q = 0.0;
+        if (a < m && b < m) {
+            q = (a == 0 || a == n) ? 0.0 : fk[(long long)a * m + b].y;      // odd in a
+            u[(long long)a * m + b] = q;
+        }
+        tile[r][tx] = q;
+    }
+    __syncthreads();
+    for (int r = ty; r < 32; r += 8) {
+        const int b = blockIdx.x * 32 + r, a = blockIdx.y * 32 + tx;
+        if (a < m && b < m) v[(long long)b * m + a] = tile[tx][r];
+    }
+}
+
+// Rows 2p and 2p + 1 of the density -> their spectra, out[k][row], k <= N
+// (two neighbouring rows: 32-byte sectors of the transposed output).
+template <int L>
+__global__ void __launch_bounds__(fft_threads(L, 1), 512 / fft_threads(L, 1))
+k_rows_fwd(const double2* __restrict__ tw, const double* __restrict__ rho, double2* __restrict__ out) {
+    constexpr int n = L / 2;
+    extern __shared__ double2 sm2[];
+    using Map = fft::One;
+    for (int p = blockIdx.x; p < (n + 1) / 2; p += gridDim.x) {
+        const double* ra = rho + (long long)(2 * p) * n;
+        const bool two = 2 * p + 1 < n;
+        __syncthreads();
+        fft::run<L, -1, Map>(tw, sm2,
+                     [&](int i, int, bool hi) {
+                         double2 z = make_double2(0.0, 0.0);
+                         if (!hi) {
+                             z.x = __ldg(ra + i);
+                             if (two) z.y = __ldg(ra + n + i);
+                         }
+                         return z;
+                     },
+                     [&](int i, int, double2 z, bool) { sm2[Map::at(i, 0)] = z; });
+        __syncthreads();
+        for (int k = threadIdx.x; k <= n; k += blockDim.x) {
+            const double2 z = sm2[Map::at(k, 0)], w = sm2[Map::at(k == 0 ? 0 : L - k, 0)];
+            double2* o = out + (long long)k * n + 2 * p;
+            o[0] = make_double2(0.5 * (z.x + w.x), 0.5 * (z.y - w.y));
+            if (two) o[1] = make_double2(0.5 * (z.y + w.y), 0.5 * (w.x - z.x));
+        }
+    }
+}
+
+// Column kj of the density's row spectra -> the N crop rows of the two force
+// spectra' columns, out[kj][row] = (F_x, F_y). The column's spectrum waits in
+// `slot` (this CTA's L columns of scratch, L2 resident) for the second kernel.
+template <int L>
+__global__ void __launch_bounds__(fft_threads(L, 1), 512 / fft_threads(L, 1))
+k_cols(const double2* __restrict__ tw, const double2* __restrict__ in, const double* __restrict__ u,
+       const double* __restrict__ v, double scale, double2* slots, double2* __restrict__ out) {
+    constexpr int n = L / 2;
+    extern __shared__ double2 sm2[];
+    using Map = fft::One;
+    double2* slot = slots + (long long)blockIdx.x * L;
+    for (int kj = blockIdx.x; kj <= n; kj += gridDim.x) {
+        const double2* col = in + (long long)kj * n;
+        double2* o = out + (long long)kj * n * 2;
+        __syncthreads();
+        fft::run<L, -1, Map>(tw, sm2,
+                     [&](int i, int, bool hi) { return hi ? make_double2(0.0, 0.0) : __ldg(col + i); },
+                     [&](int i, int, double2 z, bool) { slot[i] = z; });
+        __syncthreads();
+        // F_x: odd in the column index, F_y = its mirror image: even
+#pragma unroll 1
+        for (int d = 0; d < 2; ++d) {
+            const double* q = (d ? u : v) + (long long)kj * (n + 1);
+            const double up = d ? scale : -scale;
+            fft::run<L, 1, Map>(tw, sm2,
+                                [&](int i, int, bool hi) {
+                                    const double2 a = slot[i];
+                                    const double g = hi ? up * __ldg(q + (L - i)) : scale * __ldg(q + i);
+                                    return make_double2(-a.y * g, a.x * g);
+                                },
+                                [&](int i, int, double2 z, bool hi) { if (!hi) o[2 * i + d] = z; });
+            __syncthreads();
+        }
+    }
+}
+
+// Row i: f_x + i f_y from the half spectra of its two real components.
+template <int L>
+__global__ void __launch_bounds__(fft_threads(L, 1), 512 / fft_threads(L, 1))
+k_rows_inv(const double2* __restrict__ tw, const double2* __restrict__ in, double2* __restrict__ field) {
+    constexpr int n = L / 2;
+    extern __shared__ double2 sm2[];
+    using Map = fft::One;
+    for (int row = blockIdx.x; row < n; row += gridDim.x) {
+        __syncthreads();
+        fft::run<L, 1, Map>(tw, sm2,
+                    [&](int i, int, bool hi) {
+                        const int k = hi ? L - i : i;
+                        const double2* q = in + ((long long)k * n + row) * 2;
+                        double2 a = __ldg(q), b = __ldg(q + 1);
+                        if (k == 0 || k == n) { a.y = 0.0; b.y = 0.0; }     // real rows
+                        return hi ? make_double2(a.x + b.y, b.x - a.y) : make_double2(a.x - b.y, a.y + b.x);
+                    },
+                    [&](int i, int, double2 z, bool hi) { if (!hi) field[(long long)row * n + i] = z; });
+    }
+}
+
+struct Convolve2d {
+    void (*rows_fwd)(const double2*, const double*, double2*);
+    void (*cols)(const double2*, const double2*, const double*, const double*, double, double2*, double2*);
+    void (*rows_inv)(const double2*, const double2*, double2*);
+    int threads;
+};
+
+template <int L>
+Convolve2d convolve_of() {
+    return {k_rows_fwd<L>, k_cols<L>, k_rows_inv<L>, fft_threads(L, 1)};
+}
+
+// Padded lengths 2N with kernels: 2^a, 3 2^a and 1000 2^a from 64 to 8192
+// (the transform and its 16 values per thread bound the length: 139 KB of
+// shared memory and 512 threads of 128 registers at 8192). Measured against
+// cuFFT's five transforms a field: see k_cols.
+bool convolve_for(int L, Convolve2d* c) {
+    switch (L) {
+#define CASE(n) case n: *c = convolve_of<n>(); return true
+        CASE(64); CASE(96); CASE(128); CASE(192); CASE(256); CASE(384); CASE(512); CASE(768); CASE(1000);
+        CASE(1024); CASE(1536); CASE(2000); CASE(2048); CASE(3072); CASE(4000); CASE(4096); CASE(6144); CASE(8192);
+#undef CASE
+        default: return false;
+    }
+}
+
 // bilinear read of one caller-held N x N field with row stride ld (_cic_gather, pm_kernel.py:93-107)
 __global__ void k_cic_gather_field_2d(const double* __restrict__ px, const double* __restrict__ py, long long np_,
                                       int n, long long ld, double x0, double y0, double h,
@@ -157,12 +346,18 @@ __global__ void k_bbox_2d(const double* __restrict__ x, const double* __restrict
 }
 
 __global__ void k_bbox_final(const double* __restrict__ part, int nb, double* __restrict__ out) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
     double a = 1e308, b = -1e308, c = 1e308, d = -1e308;
-    for (int k = 0; k < nb; ++k) {
+    for (int k = threadIdx.x; k < nb; k += 32) {
         a = fmin(a, part[4 * k]); b = fmax(b, part[4 * k + 1]);
         c = fmin(c, part[4 * k + 2]); d = fmax(d, part[4 * k + 3]);
     }
+    for (int o = 16; o > 0; o >>= 1) {
+        a = fmin(a, __shfl_xor_sync(0xffffffffu, a, o));
+        b = fmax(b, __shfl_xor_sync(0xffffffffu, b, o));
+        c = fmin(c, __shfl_xor_sync(0xffffffffu, c, o));
+        d = fmax(d, __shfl_xor_sync(0xffffffffu, d, o));
+    }
+    if (threadIdx.x != 0) return;
     out[0] = a; out[1] = b; out[2] = c; out[3] = d;
 }
 
@@ -200,8 +395,23 @@ int cufft_err(sss_ctx* ctx, cufftResult r, const char* what) {
 struct sss_pm2d {
     sss_ctx* ctx;
     int n;                 // grid_n
-    cufftHandle fwd, inv;  // D2Z / Z2D on (2N, 2N)
-    double* kx;            // real work (2N x 2N) for the kernels / deposit
+    bool own;              // the convolution by the kernels of this file
+    long long ld;          // row stride of the deposit: N (own) or 2N
+    Convolve2d conv;
+    int grid[3];           // CTAs of k_rows_fwd, k_cols, k_rows_inv
+    double2* tw;           // twiddles of length 2N
+    size_t smem;
+    double* u;             // (N+1)^2 kernel spectrum and its transpose
+    double* v;
+    double e2_unit;        // (eps / h)^2 they were made for (-1: none yet)
+    double scale;          // G / h^2 / (2N)^2 of the last build
+    double2* t1;           // (N+1, N) row spectra of the density
+    double2* t2;           // (N+1, N, 2) columns of the force spectra
+    double2* slots;        // k_cols: 2N values per CTA
+    double2* pairs;        // (N, N) field (f_x, f_y)
+    cufftHandle fwd, inv;  // D2Z / Z2D on (2N, 2N); inv only without own
+    double* rho;           // deposit
+    double* kx;            // real work (2N x 2N): the force kernels
     double* ky;
     double2* fkx;          // (2N, N+1) spectra of the force kernels
     double2* fky;
@@ -211,18 +421,46 @@ struct sss_pm2d {
     double* fieldx;        // (2N x 2N) real fields
     double* fieldy;
     double* bb_part;       // bbox partials
-    double* bb;            // bbox result (4)
 };
 
 static int pm2d_free(sss_pm2d* p) {
     if (!p) return SSS_OK;
     if (p->fwd) cufftDestroy(p->fwd);
     if (p->inv) cufftDestroy(p->inv);
+    if (p->own) {
+        cudaFree(p->rho); cudaFree(p->u); cudaFree(p->v); cudaFree(p->t1); cudaFree(p->t2); cudaFree(p->slots);
+        cudaFree(p->pairs); cudaFree(p->tw);
+    }
     cudaFree(p->kx); cudaFree(p->ky); cudaFree(p->fkx); cudaFree(p->fky); cudaFree(p->fr);
     cudaFree(p->sx); cudaFree(p->sy); cudaFree(p->fieldx); cudaFree(p->fieldy);
-    cudaFree(p->bb_part); cudaFree(p->bb);
+    cudaFree(p->bb_part);
     free(p);
     return SSS_OK;
+}
+
+static cudaError_t pm2d_own_setup(sss_pm2d* p) {
+    const int L = 2 * p->n;
+    const void* fn[3] = {(const void*)p->conv.rows_fwd, (const void*)p->conv.cols, (const void*)p->conv.rows_inv};
+    const int items[3] = {(p->n + 1) / 2, p->n + 1, p->n};
+    const size_t n = (size_t)p->n, m = n + 1;
+    p->smem = (size_t)(L + L / 16 + 1) * sizeof(double2);
+    cudaError_t e = fft_table(L, &p->tw);
+    for (int k = 0; k < 3; ++k) {
+        int per_sm = 0;
+        e = e ? e : cudaFuncSetAttribute(fn[k], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p->smem);
+        e = e ? e : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn[k], p->conv.threads, p->smem);
+        const long long cap = (long long)(per_sm > 0 ? per_sm : 1) * p->ctx->num_sms;
+        p->grid[k] = (int)(items[k] < cap ? items[k] : cap);
+    }
+    e = e ? e : cudaMalloc(&p->rho, n * n * sizeof(double));
+    e = e ? e : cudaMalloc(&p->u, m * m * sizeof(double));
+    e = e ? e : cudaMalloc(&p->v, m * m * sizeof(double));
+    e = e ? e : cudaMalloc(&p->t1, m * n * sizeof(double2));
+    e = e ? e : cudaMalloc(&p->t2, 2 * m * n * sizeof(double2));
+    e = e ? e : cudaMalloc(&p->slots, (size_t)p->grid[1] * L * sizeof(double2));
+    e = e ? e : cudaMalloc(&p->pairs, n * n * sizeof(double2));
+    e = e ? e : cudaMalloc(&p->kx, 4 * n * n * sizeof(double));
+    return e;
 }
 
 extern "C" int sss_pm2d_create(sss_ctx* ctx, int grid_n, sss_pm2d** out) {
@@ -233,27 +471,34 @@ extern "C" int sss_pm2d_create(sss_ctx* ctx, int grid_n, sss_pm2d** out) {
     sss_pm2d* p = (sss_pm2d*)calloc(1, sizeof(sss_pm2d));
     p->ctx = ctx;
     p->n = grid_n;
+    p->e2_unit = -1.0;
+    p->own = convolve_for(2 * grid_n, &p->conv);
+    p->ld = p->own ? grid_n : 2LL * grid_n;
     const long long np = 2LL * grid_n;
     const size_t real_b = (size_t)np * np * sizeof(double);
     const size_t cplx_b = (size_t)np * (grid_n + 1) * sizeof(double2);
     cudaError_t e = cudaSuccess;
-    e = e ? e : cudaMalloc(&p->kx, real_b);
-    e = e ? e : cudaMalloc(&p->ky, real_b);
-    e = e ? e : cudaMalloc(&p->fkx, cplx_b);
-    e = e ? e : cudaMalloc(&p->fky, cplx_b);
-    e = e ? e : cudaMalloc(&p->fr, cplx_b);
-    e = e ? e : cudaMalloc(&p->sx, cplx_b);
-    e = e ? e : cudaMalloc(&p->sy, cplx_b);
-    e = e ? e : cudaMalloc(&p->fieldx, real_b);
-    e = e ? e : cudaMalloc(&p->fieldy, real_b);
+    if (p->own) {
+        e = pm2d_own_setup(p);
+    } else {
+        e = e ? e : cudaMalloc(&p->kx, real_b);
+        e = e ? e : cudaMalloc(&p->ky, real_b);
+        e = e ? e : cudaMalloc(&p->fkx, cplx_b);
+        e = e ? e : cudaMalloc(&p->fky, cplx_b);
+        e = e ? e : cudaMalloc(&p->fr, cplx_b);
+        e = e ? e : cudaMalloc(&p->sx, cplx_b);
+        e = e ? e : cudaMalloc(&p->sy, cplx_b);
+        e = e ? e : cudaMalloc(&p->fieldx, real_b);
+        e = e ? e : cudaMalloc(&p->fieldy, real_b);
+        p->rho = p->kx;
+    }
     e = e ? e : cudaMalloc(&p->bb_part, 4 * 1024 * sizeof(double));
-    e = e ? e : cudaMalloc(&p->bb, 4 * sizeof(double));
     if (e != cudaSuccess) {
         pm2d_free(p);
         return sss_cuda_err(ctx, e, "cudaMalloc (pm2d)");
     }
     cufftResult r = cufftPlan2d(&p->fwd, (int)np, (int)np, CUFFT_D2Z);
-    if (r == CUFFT_SUCCESS) r = cufftPlan2d(&p->inv, (int)np, (int)np, CUFFT_Z2D);
+    if (r == CUFFT_SUCCESS && !p->own) r = cufftPlan2d(&p->inv, (int)np, (int)np, CUFFT_Z2D);
     if (r != CUFFT_SUCCESS) {
         pm2d_free(p);
         return cufft_err(ctx, r, "cufftPlan2d");
@@ -292,6 +537,25 @@ extern "C" int sss_pm2d_build_kernels(sss_pm2d* p, double h, double eps2, double
     if (!(h > 0.0)) return sss_set_err(ctx, SSS_ERR_ARG, "h must be > 0");
     cudaStream_t s = (cudaStream_t)stream;
     const long long np = 2LL * p->n;
+    if (p->own) {
+        // eps^2 / h^2 of a softening tied to h differs from step to step by a few roundings: within
+        // 1e-15 it is the same kernel
+        const double e2 = eps2 / (h * h);
+        p->scale = G / (h * h) / (double)(np * np);
+        if (fabs(e2 - p->e2_unit) <= 1e-15 * e2) return SSS_OK;
+        p->e2_unit = -1.0;
+        k_unit_kernel_2d<<<blocks_for(np * np, 256), 256, 0, s>>>(p->n, e2, p->kx);
+        SSS_LAUNCH_CHECK(ctx, "k_unit_kernel_2d");
+        cufftSetStream(p->fwd, s);
+        // the spectrum (2N x (N + 1)) fits t2 exactly
+        cufftResult r = cufftExecD2Z(p->fwd, p->kx, (cufftDoubleComplex*)p->t2);
+        if (r != CUFFT_SUCCESS) return cufft_err(ctx, r, "cufftExecD2Z (kernel)");
+        const unsigned tiles = (unsigned)(p->n / 32 + 1);
+        k_kernel_tables_2d<<<dim3(tiles, tiles), 256, 0, s>>>(p->t2, p->n, p->u, p->v);
+        SSS_LAUNCH_CHECK(ctx, "k_kernel_tables_2d");
+        p->e2_unit = e2;
+        return SSS_OK;
+    }
     k_force_kernels_2d<<<blocks_for(np * np, 256), 256, 0, s>>>(p->n, h, eps2, G, p->kx, p->ky);
     SSS_LAUNCH_CHECK(ctx, "k_force_kernels_2d");
     cufftSetStream(p->fwd, s);
@@ -311,14 +575,23 @@ extern "C" int sss_pm2d_field(sss_pm2d* p, const double* gx, const double* gy, c
     if (n < 0 || (n > 0 && (!gx || !gy || !gm))) return sss_set_err(ctx, SSS_ERR_ARG, "field: bad input");
     cudaStream_t s = (cudaStream_t)stream;
     const long long np = 2LL * p->n;
-    SSS_CUDA_TRY(ctx, cudaMemsetAsync(p->kx, 0, (size_t)np * np * sizeof(double), s));
+    SSS_CUDA_TRY(ctx, cudaMemsetAsync(p->rho, 0, (size_t)p->ld * p->ld * sizeof(double), s));
     if (n > 0) {
-        k_cic_deposit_2d<<<blocks_for(n, 256), 256, 0, s>>>(gx, gy, gm, n, p->n, x0, y0, h, p->kx);
+        k_cic_deposit_2d<<<blocks_for(n, 256), 256, 0, s>>>(gx, gy, gm, n, p->n, p->ld, x0, y0, h, p->rho);
         SSS_LAUNCH_CHECK(ctx, "k_cic_deposit_2d");
+    }
+    if (p->own) {
+        p->conv.rows_fwd<<<p->grid[0], p->conv.threads, p->smem, s>>>(p->tw, p->rho, p->t1);
+        SSS_LAUNCH_CHECK(ctx, "k_rows_fwd");
+        p->conv.cols<<<p->grid[1], p->conv.threads, p->smem, s>>>(p->tw, p->t1, p->u, p->v, p->scale, p->slots, p->t2);
+        SSS_LAUNCH_CHECK(ctx, "k_cols");
+        p->conv.rows_inv<<<p->grid[2], p->conv.threads, p->smem, s>>>(p->tw, p->t2, p->pairs);
+        SSS_LAUNCH_CHECK(ctx, "k_rows_inv");
+        return SSS_OK;
     }
     cufftSetStream(p->fwd, s);
     cufftSetStream(p->inv, s);
-    cufftResult r = cufftExecD2Z(p->fwd, p->kx, (cufftDoubleComplex*)p->fr);
+    cufftResult r = cufftExecD2Z(p->fwd, p->rho, (cufftDoubleComplex*)p->fr);
     if (r != CUFFT_SUCCESS) return cufft_err(ctx, r, "cufftExecD2Z (density)");
     const long long m = np * (p->n + 1);
     k_spectrum_mul_2d<<<blocks_for(m, 256), 256, 0, s>>>(p->fr, p->fkx, p->fky, m, 1.0 / (double)(np * np), p->sx,
@@ -336,8 +609,12 @@ extern "C" int sss_pm2d_gather(sss_pm2d* p, const double* px, const double* py, 
     if (!p) return SSS_ERR_ARG;
     if (n <= 0) return SSS_OK;
     if (!px || !py || !ax || !ay) return sss_set_err(p->ctx, SSS_ERR_ARG, "gather: NULL");
-    k_cic_gather_2d<<<blocks_for(n, 256), 256, 0, (cudaStream_t)stream>>>(px, py, n, p->n, x0, y0, h, p->fieldx,
-                                                                         p->fieldy, ax, ay);
+    if (p->own)
+        k_cic_gather_pairs_2d<<<blocks_for(n, 128), 128, 0, (cudaStream_t)stream>>>(px, py, n, p->n, x0, y0, h,
+                                                                                   p->pairs, ax, ay);
+    else
+        k_cic_gather_2d<<<blocks_for(n, 256), 256, 0, (cudaStream_t)stream>>>(px, py, n, p->n, x0, y0, h, p->fieldx,
+                                                                             p->fieldy, ax, ay);
     SSS_LAUNCH_CHECK(p->ctx, "k_cic_gather_2d");
     return SSS_OK;
 }
@@ -361,6 +638,11 @@ extern "C" int sss_pm2d_fields(sss_pm2d* p, double* ax, double* ay, void* stream
     if (!p || !ax || !ay) return SSS_ERR_ARG;
     const size_t n = (size_t)p->n;
     cudaStream_t s = (cudaStream_t)stream;
+    if (p->own) {
+        k_split_pairs_2d<<<blocks_for((long long)(n * n), 256), 256, 0, s>>>(p->pairs, (long long)(n * n), ax, ay);
+        SSS_LAUNCH_CHECK(p->ctx, "k_split_pairs_2d");
+        return SSS_OK;
+    }
     SSS_CUDA_TRY(p->ctx, cudaMemcpy2DAsync(ax, n * sizeof(double), p->fieldx, 2 * n * sizeof(double),
                                            n * sizeof(double), n, cudaMemcpyDeviceToDevice, s));
     SSS_CUDA_TRY(p->ctx, cudaMemcpy2DAsync(ay, n * sizeof(double), p->fieldy, 2 * n * sizeof(double),
@@ -372,7 +654,7 @@ extern "C" int sss_pm2d_fields(sss_pm2d* p, double* ax, double* ay, void* stream
 extern "C" int sss_pm2d_density(sss_pm2d* p, double* rho, void* stream) {
     if (!p || !rho) return SSS_ERR_ARG;
     const size_t n = (size_t)p->n;
-    SSS_CUDA_TRY(p->ctx, cudaMemcpy2DAsync(rho, n * sizeof(double), p->kx, 2 * n * sizeof(double),
+    SSS_CUDA_TRY(p->ctx, cudaMemcpy2DAsync(rho, n * sizeof(double), p->rho, p->ld * sizeof(double),
                                            n * sizeof(double), n, cudaMemcpyDeviceToDevice, (cudaStream_t)stream));
     return SSS_OK;
 }

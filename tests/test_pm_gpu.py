@@ -153,3 +153,37 @@ def test_dynamics_conserve_energy_and_momentum():
     p_rel = np.hypot(np.sum(m * f[2 * n:3 * n]), np.sum(m * f[3 * n:])) / np.hypot(np.sum(m * np.abs(vx)),
                                                                                      np.sum(m * np.abs(vy)))
     assert abs(e1 - e0) / abs(e0) < 0.03 and p_rel < 1e-6
+
+
+@pytest.mark.parametrize("n", [31, 32, 48, 64, 130, 384, 500, 512, 1000, 1024, 1536, 2048, 4096])
+def test_convolution_of_every_length(n):
+    """pm_force_field against the zero-padded convolution in torch's f64 FFTs
+    with the kernels of the same cell size, at the smallest and largest padded
+    lengths with their own kernels, of each family of lengths, and at lengths
+    without (31, 130). Each plan is used with two cell sizes whose softening
+    is tied to them (the kept kernel spectra serve both), then with a fixed
+    softening (remade). 1e-10 of the largest force: the bar of the parity
+    tests, FFT rounding."""
+    pk = _pk()
+    rng = np.random.default_rng(n)
+    x, y = rng.uniform(0, 1, 300), rng.uniform(0, 1, 300)
+    x[:3], y[:3] = (0.0, 1.0, 0.0), (0.0, 1.0, 1.0)
+    m = rng.uniform(0.5, 1.5, 300)
+    o = torch.arange(2 * n, device="cuda", dtype=torch.float64)
+    o = torch.where(o < n, o, o - 2 * n)
+    for size, soft in ((1.0, None), (7.3, None), (7.3, 0.02)):
+        x0, y0, h = pk.grid_fuer(x * size, y * size, n, 1.5)
+        eps2 = (1.5 * h) ** 2 if soft is None else soft ** 2
+        ax, ay = pk.pm_force_field(x * size, y * size, m, n, x0, y0, h, eps2)
+        rho = pk._cic_deposit(x * size, y * size, m, n, x0, y0, h)
+        assert abs(float(rho.sum()) - m.sum()) <= 1e-12 * m.sum()
+        pad = torch.zeros((2 * n, 2 * n), device="cuda", dtype=torch.float64)
+        pad[:n, :n] = rho
+        rk = torch.fft.rfft2(pad)
+        dx, dy = (o * h)[:, None], (o * h)[None, :]
+        inv = (dx * dx + dy * dy + eps2) ** -1.5
+        want = [torch.fft.irfft2(rk * torch.fft.rfft2(-pk.G_AU * d * inv), s=(2 * n, 2 * n))[:n, :n]
+                for d in (dx, dy)]
+        scale = max(float(w.abs().max()) for w in want)
+        for got, ref in zip((ax, ay), want):
+            assert float((got - ref).abs().max()) <= 1e-10 * scale
