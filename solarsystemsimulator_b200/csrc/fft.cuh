@@ -221,9 +221,9 @@ struct Outer {                         // COUNT transforms one after another, ST
 
 // Stage S of length N: `get(i, c, hi)` reads input i of transform c, `put(i, c,
 // v, hi)` writes output i; hi = (i >= N / 2), a constant of the unrolled code in
-// the first and the last stage where the radix is even. From the second stage on the inputs are in the buffer that
-// the outputs go to.
-template <int N, int S, int DIR, class Map, class C, class Get, class Put>
+// the first and the last stage where the radix is even. INPLACE: the inputs are
+// in the buffer that the outputs go to.
+template <int N, int S, int DIR, class Map, bool INPLACE, class C, class Get, class Put>
 __device__ __forceinline__ void stage(const C* __restrict__ tw, Get get, Put put) {
     constexpr int R = fft_radix(N, S), B = FFT_E / R, NB = N / R, SPAN = fft_span(N, S);
     constexpr int ITEMS = NB * Map::batch, NT = fft_threads(N, Map::batch);
@@ -241,7 +241,7 @@ __device__ __forceinline__ void stage(const C* __restrict__ tw, Get get, Put put
 #pragma unroll
         for (int t = 0; t < R; ++t) v[b * R + t] = get(j + t * NB, c, S == 0 && R % 2 == 0 ? 2 * t >= R : 2 * (j + t * NB) >= N);
     }
-    if (S > 0) __syncthreads();
+    if (INPLACE) __syncthreads();
 #pragma unroll
     for (int b = 0; b < B; ++b) {
         const int w = tid + b * NT;
@@ -250,11 +250,16 @@ __device__ __forceinline__ void stage(const C* __restrict__ tw, Get get, Put put
         Map::template split<NB>(w, j, c);
         const int k = j % SPAN;
         if (S > 0) {
+            // the powers 1, 2, 4, 8 of the butterfly's twiddle from the table, the others as
+            // their products (at most three factors): 15 loads of radix 16 were more L1
+            // traffic than the exchange itself
             const C* q = tw + fft_off(N, S) + k;
+            C f[R];
 #pragma unroll
             for (int t = 1; t < R; ++t) {
-                const C f = __ldg(q + (t - 1) * SPAN);
-                v[b * R + t] = DIR < 0 ? mul(v[b * R + t], f) : mulc(v[b * R + t], f);
+                const int top = t >= 8 ? 8 : t >= 4 ? 4 : t >= 2 ? 2 : 1;
+                f[t] = t == top ? __ldg(q + (t - 1) * SPAN) : mul(f[top], f[t - top]);
+                v[b * R + t] = DIR < 0 ? mul(v[b * R + t], f[t]) : mulc(v[b * R + t], f[t]);
             }
         }
         dft<R, DIR>(v + b * R);
@@ -269,9 +274,9 @@ template <int N, int S, int DIR, class Map, class C, class Put>
 __device__ __forceinline__ void stages(const C* __restrict__ tw, C* sm, Put put) {
     auto rd = [&](int i, int c, bool) { return sm[Map::at(i, c)]; };
     if constexpr (S + 1 == fft_stages(N)) {
-        stage<N, S, DIR, Map>(tw, rd, put);
+        stage<N, S, DIR, Map, true>(tw, rd, put);
     } else {
-        stage<N, S, DIR, Map>(tw, rd, [&](int i, int c, C v, bool) { sm[Map::at(i, c)] = v; });
+        stage<N, S, DIR, Map, true>(tw, rd, [&](int i, int c, C v, bool) { sm[Map::at(i, c)] = v; });
         __syncthreads();
         stages<N, S + 1, DIR, Map>(tw, sm, put);
     }
@@ -281,11 +286,12 @@ __device__ __forceinline__ void stages(const C* __restrict__ tw, C* sm, Put put)
 // fft_threads(N, Map::batch) threads: DIR -1 forward, +1 inverse (unscaled).
 // `sm` holds Map::at() of every element; earlier reads of it by other threads
 // must lie before a __syncthreads() of the caller. Outputs that `put` writes
-// to `sm` are safe: all inputs of the last stage have been read.
-template <int N, int DIR, class Map, class C, class Get, class Put>
+// to `sm` are safe: all inputs of the last stage have been read. INPLACE: `get`
+// reads `sm` too.
+template <int N, int DIR, class Map, bool INPLACE = false, class C, class Get, class Put>
 __device__ __forceinline__ void run(const C* __restrict__ tw, C* sm, Get get, Put put) {
     static_assert(fft_stages(N) >= 2, "one stage only");
-    stage<N, 0, DIR, Map>(tw, get, [&](int i, int c, C v, bool) { sm[Map::at(i, c)] = v; });
+    stage<N, 0, DIR, Map, INPLACE>(tw, get, [&](int i, int c, C v, bool) { sm[Map::at(i, c)] = v; });
     __syncthreads();
     stages<N, 1, DIR, Map>(tw, sm, put);
 }

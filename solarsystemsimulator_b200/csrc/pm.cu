@@ -183,6 +183,15 @@ __global__ void __launch_bounds__(256) k_kernel_tables_2d(const double2* __restr
     }
 }
 
+// One 32-byte access per lane for scattered pairs of complex values (half the
+// L1 passes of two 16-byte ones).
+__device__ __forceinline__ void st_pair(double2* p, double2 a, double2 b) {
+    asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" :: "l"(p), "d"(a.x), "d"(a.y), "d"(b.x), "d"(b.y) : "memory");
+}
+__device__ __forceinline__ void ld_pair(const double2* p, double2& a, double2& b) {
+    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(a.x), "=d"(a.y), "=d"(b.x), "=d"(b.y) : "l"(p));
+}
+
 // Rows 2p and 2p + 1 of the density -> their spectra, out[k][row], k <= N
 // (two neighbouring rows: 32-byte sectors of the transposed output).
 template <int L>
@@ -209,8 +218,14 @@ k_rows_fwd(const double2* __restrict__ tw, const double* __restrict__ rho, doubl
         for (int k = threadIdx.x; k <= n; k += blockDim.x) {
             const double2 z = sm2[Map::at(k, 0)], w = sm2[Map::at(k == 0 ? 0 : L - k, 0)];
             double2* o = out + (long long)k * n + 2 * p;
-            o[0] = make_double2(0.5 * (z.x + w.x), 0.5 * (z.y - w.y));
-            if (two) o[1] = make_double2(0.5 * (z.y + w.y), 0.5 * (w.x - z.x));
+            const double2 a = make_double2(0.5 * (z.x + w.x), 0.5 * (z.y - w.y));
+            const double2 b = make_double2(0.5 * (z.y + w.y), 0.5 * (w.x - z.x));
+            if (n % 2 == 0) {
+                st_pair(o, a, b);
+            } else {
+                o[0] = a;
+                if (two) o[1] = b;
+            }
         }
     }
 }
@@ -260,15 +275,17 @@ k_rows_inv(const double2* __restrict__ tw, const double2* __restrict__ in, doubl
     using Map = fft::One;
     for (int row = blockIdx.x; row < n; row += gridDim.x) {
         __syncthreads();
-        fft::run<L, 1, Map>(tw, sm2,
-                    [&](int i, int, bool hi) {
-                        const int k = hi ? L - i : i;
-                        const double2* q = in + ((long long)k * n + row) * 2;
-                        double2 a = __ldg(q), b = __ldg(q + 1);
-                        if (k == 0 || k == n) { a.y = 0.0; b.y = 0.0; }     // real rows
-                        return hi ? make_double2(a.x + b.y, b.x - a.y) : make_double2(a.x - b.y, a.y + b.x);
-                    },
-                    [&](int i, int, double2 z, bool hi) { if (!hi) field[(long long)row * n + i] = z; });
+#pragma unroll 4
+        for (int k = threadIdx.x; k <= n; k += fft_threads(L, 1)) {
+            double2 a, b;
+            ld_pair(in + ((long long)k * n + row) * 2, a, b);
+            if (k == 0 || k == n) { a.y = 0.0; b.y = 0.0; }     // real rows
+            sm2[Map::at(k, 0)] = make_double2(a.x - b.y, a.y + b.x);
+            if (k > 0 && k < n) sm2[Map::at(L - k, 0)] = make_double2(a.x + b.y, b.x - a.y);
+        }
+        __syncthreads();
+        fft::run<L, 1, Map, true>(tw, sm2, [&](int i, int, bool) { return sm2[Map::at(i, 0)]; },
+                                  [&](int i, int, double2 z, bool hi) { if (!hi) field[(long long)row * n + i] = z; });
     }
 }
 
