@@ -62,7 +62,7 @@ struct FrameArgs {
     unsigned char* sub_n;     // [K][n_ast]
     float* hit_t;             // [n_ast], < 0: none
     int* hit_m;               // [n_ast] compact massive index
-    double* part;             // [2][grid][3][M_MAX] back-reaction partials
+    double* part;             // [2][M_MAX][3][grid] back-reaction partials
     unsigned* gbar;           // [2] arrival count, generation
     int* status;
     int* guard_out;           // substeps used (written by CTA 0)
@@ -73,8 +73,10 @@ struct FrameArgs {
 
 struct FrameShared {
     double mx[3][M_MAX], mv[3][M_MAX], macc[3][M_MAX], mnew[3][M_MAX], mx0[3][M_MAX];
-    double mm[M_MAX], mrad[M_MAX];
+    double gm[M_MAX], mrad[M_MAX];   // G m, contact radius
+    float gmf[M_MAX];                // G m in f32
     double bk[3][M_MAX];
+    double wsum[FR_WARPS][32];       // back-reaction: the warps' sums of a pass
     double red[FR_WARPS];
     double dtH, rem;
     int done, guard, abort_;
@@ -123,19 +125,33 @@ __device__ __forceinline__ void chunk_of(int n, int& lo, int& hi) {
     hi = min(n, lo + per);
 }
 
-// Acceleration of a body at p from the visible massive bodies at `mpos`.
-// Same expression order as the reference: f = G/(r2 sqrt r2); a += f m dx.
+// G / (r2 sqrt r2) times a mass: the f64 pair factor from one reciprocal square root (within an ulp;
+// a square root and a division behind one another were the longest chain of every pass).
+__device__ __forceinline__ double pair_factor(double gm, double r2) {
+    const double inv = rsqrt(r2);
+    return gm * (inv * inv * inv);
+}
+
+// dist / vrel / 20 of an offset and a relative velocity (nbody_kernel.py:247-275): dist at least
+// 1e-12, +inf where vrel <= 1e-9. NaN offsets stay NaN (no comparison picks them).
+__device__ __forceinline__ double encounter(double d2, double v2, double& dist) {
+    const double dc = d2 < 1e-24 ? 1e-24 : d2;
+    dist = dc * rsqrt(dc);
+    return v2 > 1e-18 ? dist * rsqrt(v2) * 0.05 : (double)INFINITY;
+}
+
+// Acceleration of a body at p from the visible massive bodies (branch-free, so that the pairs of
+// several bodies are in flight: with a branch per body each pair waited for the one before).
 template <int D>
-__device__ __forceinline__ void massive_field(const FrameShared& s, const double (*mpos)[M_MAX], int M,
-                                              double G, double soft, const double* p, double* acc) {
+__device__ __forceinline__ void massive_field(const FrameShared& s, int M, double soft, const double* p,
+                                              double* acc) {
     for (int c = 0; c < D; ++c) acc[c] = 0.0;
+#pragma unroll 4
     for (int k = 0; k < M; ++k) {
-        if (!s.mvis[k]) continue;
-        double dx[3], r2 = 0.0;
-        for (int c = 0; c < D; ++c) { dx[c] = mpos[c][k] - p[c]; r2 += dx[c] * dx[c]; }
-        r2 += soft;
-        const double f = G / (r2 * sqrt(r2));
-        for (int c = 0; c < D; ++c) acc[c] += f * s.mm[k] * dx[c];
+        double dx[3], r2 = soft;
+        for (int c = 0; c < D; ++c) { dx[c] = s.mx[c][k] - p[c]; r2 += dx[c] * dx[c]; }
+        const double f = pair_factor(s.gm[k], s.mvis[k] ? r2 : 1.0);
+        for (int c = 0; c < D; ++c) acc[c] += s.mvis[k] ? f * dx[c] : 0.0;
     }
 }
 
@@ -143,124 +159,173 @@ __device__ __forceinline__ void massive_field(const FrameShared& s, const double
 // FP64 state): the offset formed in f64 and rounded to f32, r^2, the f32
 // reciprocal square root and the pair factor in f32, the sum in f64.
 template <int D>
-__device__ __forceinline__ void massive_field_f32(const FrameShared& s, const double (*mpos)[M_MAX], int M,
-                                                  double G, double soft, const double* p, double* acc) {
+__device__ __forceinline__ void massive_field_f32(const FrameShared& s, int M, double soft, const double* p,
+                                                  double* acc) {
     for (int c = 0; c < D; ++c) acc[c] = 0.0;
-    const float Gf = (float)G, sf = (float)soft;
+    const float sf = (float)soft;
+#pragma unroll 4
     for (int k = 0; k < M; ++k) {
-        if (!s.mvis[k]) continue;
         float dx[3], r2 = sf;
-        for (int c = 0; c < D; ++c) { dx[c] = (float)(mpos[c][k] - p[c]); r2 = fmaf(dx[c], dx[c], r2); }
-        const float inv = rsqrtf(r2);
-        const float f = Gf * (float)s.mm[k] * inv * inv * inv;
-        for (int c = 0; c < D; ++c) acc[c] += (double)(f * dx[c]);
+        for (int c = 0; c < D; ++c) { dx[c] = (float)(s.mx[c][k] - p[c]); r2 = fmaf(dx[c], dx[c], r2); }
+        const float inv = rsqrtf(s.mvis[k] ? r2 : 1.0f);
+        const float f = s.gmf[k] * inv * inv * inv;
+        for (int c = 0; c < D; ++c) acc[c] += s.mvis[k] ? (double)(f * dx[c]) : 0.0;
     }
+}
+
+// Sum over the FG lanes of a group (the same bits in every lane).
+template <int D>
+__device__ __forceinline__ void group_sum(double* acc, unsigned gmask) {
+#pragma unroll
+    for (int o = FG / 2; o > 0; o >>= 1)
+        for (int c = 0; c < D; ++c) acc[c] += __shfl_xor_sync(gmask, acc[c], o, FG);
 }
 
 // massive_field on the FG lanes of a group (mask gmask, this lane gl): lane
-// gl forms the pair factor f m and the offset of bodies k = k0 + gl, then
-// every lane adds the terms in ascending k, so each lane holds the sum in the
-// serial order of massive_field. INTERP: the massive positions interpolated
-// between mx0 and mx at fraction al.
+// gl takes the bodies k = gl, gl + FG, ..., the lane sums meet in a fixed
+// butterfly. INTERP: the massive positions interpolated between mx0 and mx at
+// fraction al.
 template <int D, bool INTERP>
-__device__ __forceinline__ void field_grp(const FrameShared& s, int M, double G, double soft, double al,
-                                          const double* p, double* acc, int gl, unsigned gmask) {
+__device__ __forceinline__ void field_grp(const FrameShared& s, int M, double soft, double al, const double* p,
+                                          double* acc, int gl, unsigned gmask) {
     for (int c = 0; c < D; ++c) acc[c] = 0.0;
-    for (int k0 = 0; k0 < M; k0 += FG) {
-        const int k = k0 + gl;
-        double fm = 0.0, dx[3] = {0.0, 0.0, 0.0};
-        if (k < M && s.mvis[k]) {
-            double r2 = 0.0;
-            for (int c = 0; c < D; ++c) {
-                double mi;
-                if constexpr (INTERP) mi = s.mx0[c][k] + (s.mx[c][k] - s.mx0[c][k]) * al;
-                else mi = s.mx[c][k];
-                dx[c] = mi - p[c];
-                r2 += dx[c] * dx[c];
-            }
-            r2 += soft;
-            const double f = G / (r2 * sqrt(r2));
-            fm = f * s.mm[k];
+    for (int k = gl; k < M; k += FG) {
+        if (!s.mvis[k]) continue;
+        double dx[3], r2 = soft;
+        for (int c = 0; c < D; ++c) {
+            double mi;
+            if constexpr (INTERP) mi = s.mx0[c][k] + (s.mx[c][k] - s.mx0[c][k]) * al;
+            else mi = s.mx[c][k];
+            dx[c] = mi - p[c];
+            r2 += dx[c] * dx[c];
         }
-        const int kn = min(FG, M - k0);
-        for (int j = 0; j < kn; ++j) {
-            if (!s.mvis[k0 + j]) continue;
-            const double fj = __shfl_sync(gmask, fm, j, FG);
-            for (int c = 0; c < D; ++c) acc[c] += fj * __shfl_sync(gmask, dx[c], j, FG);
-        }
+        const double f = pair_factor(s.gm[k], r2);
+        for (int c = 0; c < D; ++c) acc[c] += f * dx[c];
     }
+    group_sum<D>(acc, gmask);
 }
 
-// Back-reaction of this CTA's visible asteroids on every massive body:
-// warp w owns bodies k = w, w+8, ...; lanes run over the asteroids in a fixed
-// order and the warp sum is a fixed butterfly -> partial in a.part[slot].
+// Back-reaction of this CTA's visible asteroids on every massive body, in
+// passes over BK bodies: a thread sums its asteroids (lo + tid, ...) in
+// registers, the warp sums in a fixed order that halves the values each lane
+// carries (BK D instead of 5 BK D shuffles), the warps' sums are added in
+// ascending order -> partial [value][CTA] in a.part. A warp per body over all
+// asteroids read the asteroids M / 8 times from memory and took as long as the
+// rest of a stage.
+constexpr int BK = 8;
+
 template <int D>
-__device__ void back_partial(const FrameArgs& a, const FrameShared& s, int lo, int hi, int slot) {
+__device__ void back_partial(const FrameArgs& a, FrameShared& s, int lo, int hi, int slot) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    double* out = a.part + ((size_t)slot * gridDim.x + blockIdx.x) * 3 * M_MAX;
-    for (int k = warp; k < a.M; k += FR_WARPS) {
-        double b[3] = {0.0, 0.0, 0.0};
-        if (s.mvis[k]) {
-            for (int i = lo + lane; i < hi; i += 32) {
-                if (!a.avis[i]) continue;
-                if (a.pair_f32) {
-                    float dx[3], r2 = (float)a.soft;
+    constexpr int V = BK * D, VP = D == 2 ? 16 : 32;          // values, padded to a power of two
+    for (int k0 = 0; k0 < a.M; k0 += BK) {
+        double b[VP];
+#pragma unroll
+        for (int q = 0; q < VP; ++q) b[q] = 0.0;
+        for (int i = lo + (int)threadIdx.x; i < hi; i += FR_NT) {
+            if (!a.avis[i]) continue;
+            double p[3];
+            for (int c = 0; c < D; ++c) p[c] = a.ax[c][i];
+            const double am = a.am[i];
+            if (a.pair_f32) {
+                const float gmf = (float)a.G * (float)am, sf = (float)a.soft;
+#pragma unroll
+                for (int j = 0; j < BK; ++j) {
+                    const int k = k0 + j < M_MAX ? k0 + j : 0;
+                    float dx[3], r2 = sf;
                     for (int c = 0; c < D; ++c) {
-                        dx[c] = (float)(s.mx[c][k] - a.ax[c][i]);
+                        dx[c] = (float)(s.mx[c][k] - p[c]);
                         r2 = fmaf(dx[c], dx[c], r2);
                     }
-                    const float inv = rsqrtf(r2);
-                    const float f = (float)a.G * (float)a.am[i] * inv * inv * inv;
-                    for (int c = 0; c < D; ++c) b[c] -= (double)(f * dx[c]);
-                    continue;
+                    const bool on = k0 + j < a.M && s.mvis[k];
+                    const float inv = rsqrtf(on ? r2 : 1.0f);
+                    const float f = gmf * inv * inv * inv;
+#pragma unroll
+                    for (int c = 0; c < D; ++c) b[j * D + c] -= on ? (double)(f * dx[c]) : 0.0;
                 }
-                double dx[3], r2 = 0.0;
-                for (int c = 0; c < D; ++c) { dx[c] = s.mx[c][k] - a.ax[c][i]; r2 += dx[c] * dx[c]; }
-                r2 += a.soft;
-                const double f = a.G / (r2 * sqrt(r2));
-                for (int c = 0; c < D; ++c) b[c] += -f * a.am[i] * dx[c];
+            } else {
+                const double gm = a.G * am;
+#pragma unroll
+                for (int j = 0; j < BK; ++j) {
+                    const int k = k0 + j < M_MAX ? k0 + j : 0;
+                    double dx[3], r2 = a.soft;
+                    for (int c = 0; c < D; ++c) { dx[c] = s.mx[c][k] - p[c]; r2 += dx[c] * dx[c]; }
+                    const bool on = k0 + j < a.M && s.mvis[k];
+                    const double f = pair_factor(gm, on ? r2 : 1.0);
+#pragma unroll
+                    for (int c = 0; c < D; ++c) b[j * D + c] -= on ? f * dx[c] : 0.0;
+                }
             }
         }
-        for (int c = 0; c < D; ++c) {
-            const double t = warp_sum(b[c]);
-            if (lane == 0) __stcg(out + c * M_MAX + k, t);
+        // after the step of width w a lane holds VP w / 32 values: those whose index agrees with its lane bits
+        int n = VP;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            if (n > 1) {
+                n >>= 1;
+                const bool up = (lane & o) != 0;
+#pragma unroll
+                for (int q = 0; q < VP / 2; ++q) {
+                    if (q >= n) break;
+                    const double send = up ? b[q] : b[q + n], keep = up ? b[q + n] : b[q];
+                    b[q] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+                }
+            } else {
+                b[0] += __shfl_xor_sync(0xffffffffu, b[0], o);
+            }
         }
+        // VP = 32: lane L holds value L (its bits 4..0 chose the halves); VP = 16: lanes L, L ^ 1 hold value L / 2
+        const int val = VP == 32 ? lane : lane >> 1;
+        if (VP == 32 || !(lane & 1)) s.wsum[warp][val] = b[0];
+        __syncthreads();
+        if (threadIdx.x < V) {
+            double t = s.wsum[0][threadIdx.x];
+            for (int w = 1; w < FR_WARPS; ++w) t += s.wsum[w][threadIdx.x];
+            const int k = k0 + (int)threadIdx.x / D, c = (int)threadIdx.x % D;
+            if (k < a.M) __stcg(a.part + ((size_t)(slot * M_MAX + k) * 3 + c) * gridDim.x + blockIdx.x, t);
+        }
+        __syncthreads();
     }
 }
 
-// bk[c][k] = sum over CTAs (ascending) of the partials in `slot`.
+// bk[c][k] = sum over CTAs of the partials in `slot`: a warp per value, its
+// lanes over the CTAs, the same butterfly in every CTA (D M threads that each
+// added all partials one load behind the other took 8.5 us a stage).
 template <int D>
 __device__ void back_sum(const FrameArgs& a, FrameShared& s, int slot) {
-    for (int t = threadIdx.x; t < D * a.M; t += blockDim.x) {
-        const int c = t / a.M, k = t - c * a.M;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int t = warp; t < D * a.M; t += FR_WARPS) {
+        const int k = t / D, c = t - k * D;
+        const double* base = a.part + ((size_t)(slot * M_MAX + k) * 3 + c) * gridDim.x;
         double acc = 0.0;
-        const double* base = a.part + (size_t)slot * gridDim.x * 3 * M_MAX + c * M_MAX + k;
-        for (unsigned b = 0; b < gridDim.x; ++b) acc += __ldcg(base + (size_t)b * 3 * M_MAX);
-        s.bk[c][k] = acc;
+#pragma unroll 4
+        for (unsigned b = lane; b < gridDim.x; b += 32) acc += __ldcg(base + b);
+        acc = warp_sum(acc);
+        if (lane == 0) s.bk[c][k] = acc;
     }
 }
 
-// mnew = bk + sum over visible massive pairs (one warp per body, lanes over
-// partners, fixed butterfly order).
+// mnew = sum over visible massive pairs (one warp per body from the last
+// warp down: few asteroids leave those idle; lanes over partners, fixed
+// butterfly order).
 template <int D>
 __device__ void massive_accel(const FrameArgs& a, FrameShared& s) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = FR_WARPS - 1 - (int)(threadIdx.x >> 5), lane = threadIdx.x & 31;
     for (int i = warp; i < a.M; i += FR_WARPS) {
         double acc[3] = {0.0, 0.0, 0.0};
         if (s.mvis[i]) {
             for (int j = lane; j < a.M; j += 32) {
                 if (j == i || !s.mvis[j]) continue;
-                double dx[3], r2 = 0.0;
+                double dx[3], r2 = a.soft;
                 for (int c = 0; c < D; ++c) { dx[c] = s.mx[c][j] - s.mx[c][i]; r2 += dx[c] * dx[c]; }
-                r2 += a.soft;
-                const double f = a.G / (r2 * sqrt(r2));
-                for (int c = 0; c < D; ++c) acc[c] += f * s.mm[j] * dx[c];
+                const double f = pair_factor(s.gm[j], r2);
+                for (int c = 0; c < D; ++c) acc[c] += f * dx[c];
             }
         }
-        for (int c = 0; c < D; ++c) {
-            const double t = warp_sum(acc[c]);
-            if (lane == 0) s.mnew[c][i] = s.bk[c][i] + t;
-        }
+        for (int o = a.M > 16 ? 16 : 8; o > 0; o >>= 1)
+            for (int c = 0; c < D; ++c) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], o);
+        if (lane == 0)
+            for (int c = 0; c < D; ++c) s.mnew[c][i] = acc[c];
     }
 }
 
@@ -270,99 +335,82 @@ template <int D>
 __device__ double pair_dt(const FrameArgs& a, FrameShared& s) {
     double best = a.max_sub_dt;
     const int M = a.M;
-    for (int t = threadIdx.x; t < M * M; t += blockDim.x) {
+    for (int t = threadIdx.x; t < M * M; t += FR_NT) {
         const int i = t / M, j = t - i * M;
         if (j <= i || !s.mvis[i] || !s.mvis[j]) continue;
-        double d2 = 0.0, v2 = 0.0;
+        double d2 = 0.0, v2 = 0.0, dist;
         for (int c = 0; c < D; ++c) {
             const double dx = s.mx[c][j] - s.mx[c][i], dv = s.mv[c][j] - s.mv[c][i];
             d2 += dx * dx;
             v2 += dv * dv;
         }
-        double dist = sqrt(d2);
-        if (dist < 1e-12) dist = 1e-12;
-        const double vrel = sqrt(v2);
-        if (vrel > 1e-9) {
-            const double te = dist / vrel / 20.0;
-            if (te < best) best = te;
-        }
+        const double te = encounter(d2, v2, dist);
+        if (te < best) best = te;
     }
     for (int o = 16; o > 0; o >>= 1) best = fmin(best, __shfl_xor_sync(0xffffffffu, best, o));
     if ((threadIdx.x & 31) == 0) s.red[threadIdx.x >> 5] = best;
     __syncthreads();
     double r = s.red[0];
+#pragma unroll
     for (int w = 1; w < FR_WARPS; ++w) r = fmin(r, s.red[w]);
-    __syncthreads();
     return r;
 }
 
 // Hot asteroid i: private adaptive Yoshida over [0, dtH] (nbody_kernel.py:416-535)
-// on the FG lanes of a group. The massive bodies are spread over the lanes
-// (field_grp); the step size is the group minimum of the encounter times, a
-// contact the first body in k order (the ballot's lowest bit). Every lane
-// carries the same position, velocity and step, formed in the same order as
-// the serial loop; lane 0 writes.
+// on the FG lanes of a group. The massive bodies are spread over the lanes; the
+// step size is the group minimum of the encounter times, a contact the first
+// body in k order. Every lane carries the same position, velocity and step;
+// lane 0 writes. Bound by the latency of a step (one asteroid passing a planet
+// keeps its CTA, and with back-reaction the whole grid, waiting): the chain
+// was 2.9 us a step with square roots, divisions and the pair terms handed
+// from lane to lane in order.
 template <int D>
 __device__ void fine_loop(const FrameArgs& a, const FrameShared& s, int i, int ks, double dtH, double tSeg0,
                           int gl, unsigned gmask) {
     const double wd[3] = {a.w1, a.w0, a.w1};
-    const int gbase = (threadIdx.x & 31) & ~(FG - 1);
     double p[3], v[3];
     for (int c = 0; c < D; ++c) { p[c] = a.ax[c][i]; v[c] = a.av[c][i]; }
     const double sgn = dtH >= 0.0 ? 1.0 : -1.0;
-    const double span = fabs(dtH);
+    const double span = fabs(dtH), rspan = 1.0 / span;
     const double subDt = a.m_sub > 0 ? a.dt_raster / a.m_sub : 0.0;
-    const double rad = a.arad[i];
+    const double rad = a.arad[i], dt_min = a.max_sub_dt / 1000.0;
     bool open = a.hit_t[i] < 0.0f;      // no contact time recorded yet
     double tau = 0.0;
+    double q = a.m_sub > 0 ? tSeg0 / subDt : 0.0;       // (tSeg0 + tau) / subDt
     int guardF = 0;
     while (tau < span - 1e-15 && guardF++ < a.fine_guard) {
-        const double al = tau / span;
+        const double al = tau * rspan;
         double dtF = a.max_sub_dt;
-        int first = -1, last = -1;      // bodies in contact, lowest and highest k
+        int first = M_MAX, last = -1;   // this lane's bodies in contact, lowest and highest k
         // one pass over the bodies at fraction al: the encounter times, the contacts and the
-        // first stage's acceleration (field_grp at tau, from the same offsets)
-        double acc[3];
-        for (int c = 0; c < D; ++c) acc[c] = 0.0;
-        for (int k0 = 0; k0 < a.M; k0 += FG) {
-            const int k = k0 + gl;
-            bool touch = false;
-            double fm = 0.0, dx[3] = {0.0, 0.0, 0.0};
-            if (k < a.M && s.mvis[k]) {
-                double d2 = 0.0, v2 = 0.0;
-                for (int c = 0; c < D; ++c) {
-                    const double mi = s.mx0[c][k] + (s.mx[c][k] - s.mx0[c][k]) * al;
-                    dx[c] = mi - p[c];
-                    const double dv = s.mv[c][k] - v[c];
-                    d2 += dx[c] * dx[c];
-                    v2 += dv * dv;
-                }
-                double dist = sqrt(d2);
-                if (dist < 1e-12) dist = 1e-12;
-                touch = dist <= s.mrad[k] + rad;
-                const double vrel = sqrt(v2);
-                if (vrel > 1e-9) {
-                    const double te = dist / vrel / 20.0;
-                    if (te < dtF) dtF = te;
-                }
-                const double r2 = d2 + a.soft;
-                const double f = a.G / (r2 * sqrt(r2));
-                fm = f * s.mm[k];
+        // first stage's acceleration
+        double acc[3] = {0.0, 0.0, 0.0};
+        for (int k = gl; k < a.M; k += FG) {
+            if (!s.mvis[k]) continue;
+            double d2 = 0.0, v2 = 0.0, dx[3], dist;
+            for (int c = 0; c < D; ++c) {
+                const double mi = s.mx0[c][k] + (s.mx[c][k] - s.mx0[c][k]) * al;
+                dx[c] = mi - p[c];
+                const double dv = s.mv[c][k] - v[c];
+                d2 += dx[c] * dx[c];
+                v2 += dv * dv;
             }
-            const unsigned b = (__ballot_sync(gmask, touch) >> gbase) & ((1u << FG) - 1u);
-            if (b) {
-                if (first < 0) first = k0 + __ffs(b) - 1;
-                last = k0 + 31 - __clz(b);
-            }
-            const int kn = min(FG, a.M - k0);
-            for (int j = 0; j < kn; ++j) {
-                if (!s.mvis[k0 + j]) continue;
-                const double fj = __shfl_sync(gmask, fm, j, FG);
-                for (int c = 0; c < D; ++c) acc[c] += fj * __shfl_sync(gmask, dx[c], j, FG);
-            }
+            const double te = encounter(d2, v2, dist);
+            if (dist <= s.mrad[k] + rad) { first = min(first, k); last = k; }
+            if (te < dtF) dtF = te;
+            const double f = pair_factor(s.gm[k], d2 + a.soft);
+            for (int c = 0; c < D; ++c) acc[c] += f * dx[c];
         }
-        for (int o = FG / 2; o > 0; o >>= 1) dtF = fmin(dtF, __shfl_xor_sync(gmask, dtF, o, FG));
-        if (open && first >= 0) {
+#pragma unroll
+        for (int o = FG / 2; o > 0; o >>= 1) {
+            dtF = fmin(dtF, __shfl_xor_sync(gmask, dtF, o, FG));
+            for (int c = 0; c < D; ++c) acc[c] += __shfl_xor_sync(gmask, acc[c], o, FG);
+        }
+        if (open && __any_sync(gmask, last >= 0)) {
+            for (int o = FG / 2; o > 0; o >>= 1) {
+                first = min(first, __shfl_xor_sync(gmask, first, o, FG));
+                last = max(last, __shfl_xor_sync(gmask, last, o, FG));
+            }
             // the serial test `hit_t < 0` per body: the first body in contact closes it,
             // unless the recorded time is itself negative (then every later body overwrites)
             const float h = (float)(ks * a.dt_raster + tSeg0 + tau);
@@ -372,35 +420,35 @@ __device__ void fine_loop(const FrameArgs& a, const FrameShared& s, int i, int k
             }
             open = h < 0.0f;
         }
-        if (dtF < a.max_sub_dt / 1000.0) dtF = a.max_sub_dt / 1000.0;
+        if (dtF < dt_min) dtF = dt_min;
         if (dtF > span - tau) dtF = span - tau;
         if (a.m_sub > 0) {
-            const double tAbs = tSeg0 + tau;
-            const int jn = (int)floor(tAbs / subDt + 1e-9) + 1;
+            const int jn = (int)floor(q + 1e-9) + 1;
             if (jn <= a.m_sub) {
-                const double rest = jn * subDt - tAbs;
+                const double rest = jn * subDt - (tSeg0 + tau);
                 if (rest > 0.0 && dtF > rest) dtF = rest;
             }
         }
         // the three velocity-Verlet stages; a stage's closing acceleration (same time, same
         // position) is the next stage's opening one
         double tSub = tau;
+#pragma unroll
         for (int wf = 0; wf < 3; ++wf) {
             const double df = wd[wf] * dtF * sgn;
             double ncc[3];
             for (int c = 0; c < D; ++c) p[c] += v[c] * df + 0.5 * acc[c] * df * df;
             tSub += wd[wf] * dtF;
-            field_grp<D, true>(s, a.M, a.G, a.soft, tSub / span, p, ncc, gl, gmask);
+            field_grp<D, true>(s, a.M, a.soft, tSub * rspan, p, ncc, gl, gmask);
             for (int c = 0; c < D; ++c) {
                 v[c] += 0.5 * (acc[c] + ncc[c]) * df;
                 acc[c] = ncc[c];
             }
         }
         tau += dtF;
-        if (a.m_sub > 0 && gl == 0) {
-            const double q = (tSeg0 + tau) / subDt;
+        if (a.m_sub > 0) {
+            q = (tSeg0 + tau) / subDt;
             const int j = (int)floor(q + 0.5);
-            if (j >= 1 && j <= a.m_sub && fabs(q - j) < 1e-6) {
+            if (gl == 0 && j >= 1 && j <= a.m_sub && fabs(q - j) < 1e-6) {
                 const int64_t b = ((int64_t)ks * a.m_sub + (j - 1)) * D * a.n_ast;
                 for (int c = 0; c < D; ++c) a.sub_pos[b + (int64_t)c * a.n_ast + i] = (float)p[c];
                 a.sub_n[(int64_t)ks * a.n_ast + i]++;
@@ -408,7 +456,7 @@ __device__ void fine_loop(const FrameArgs& a, const FrameShared& s, int i, int k
         }
     }
     double acc[3];
-    field_grp<D, false>(s, a.M, a.G, a.soft, 0.0, p, acc, gl, gmask);
+    field_grp<D, false>(s, a.M, a.soft, 0.0, p, acc, gl, gmask);
     if (gl == 0) {
         // the guard ran out before the interval was covered: the reference stops there silently
         // (nbody_kernel.py:424); the state keeps it, the status word records it
@@ -447,15 +495,12 @@ __device__ void hot_pass(const FrameArgs& a, FrameShared& s, int lo, int hi, int
 // CTAs identical). Returns false if the grid barrier timed out.
 template <int D>
 __device__ bool back_reaction(const FrameArgs& a, FrameShared& s, int lo, int hi, int& slot) {
-    if (a.massless) {
-        for (int t = threadIdx.x; t < 3 * M_MAX; t += blockDim.x) (&s.bk[0][0])[t] = 0.0;
-        __syncthreads();
-        return true;
+    if (!a.massless) {
+        back_partial<D>(a, s, lo, hi, slot);
+        if (!grid_sync(a, s)) return false;
+        back_sum<D>(a, s, slot);
+        slot ^= 1;
     }
-    back_partial<D>(a, s, lo, hi, slot);
-    if (!grid_sync(a, s)) return false;
-    back_sum<D>(a, s, slot);
-    slot ^= 1;
     __syncthreads();
     return true;
 }
@@ -467,9 +512,10 @@ __global__ void __launch_bounds__(FR_NT) k_frame(const FrameArgs a) {
     int lo, hi;
     chunk_of(a.n_ast, lo, hi);
     if (tid == 0) { s.abort_ = 0; s.guard = 0; }
-    for (int k = tid; k < a.M; k += blockDim.x) {
-        for (int c = 0; c < D; ++c) { s.mx[c][k] = a.mx[c][k]; s.mv[c][k] = a.mv[c][k]; }
-        s.mm[k] = a.mm[k];
+    for (int k = tid; k < a.M; k += FR_NT) {
+        for (int c = 0; c < D; ++c) { s.mx[c][k] = a.mx[c][k]; s.mv[c][k] = a.mv[c][k]; s.bk[c][k] = 0.0; }
+        s.gm[k] = a.G * a.mm[k];
+        s.gmf[k] = (float)a.G * (float)a.mm[k];
         s.mrad[k] = a.mrad[k];
         s.mvis[k] = a.mvis[k];
     }
@@ -477,27 +523,26 @@ __global__ void __launch_bounds__(FR_NT) k_frame(const FrameArgs a) {
     int slot = 0;
 
     // initial accelerations (nbody_kernel.py:151-216)
-    for (int i = lo + tid; i < hi; i += blockDim.x) {
+    for (int i = lo + tid; i < hi; i += FR_NT) {
         double p[3], acc[3] = {0.0, 0.0, 0.0};
         for (int c = 0; c < D; ++c) p[c] = a.ax[c][i];
         if (a.avis[i]) {
-            if (a.pair_f32) massive_field_f32<D>(s, s.mx, a.M, a.G, a.soft, p, acc);
-            else massive_field<D>(s, s.mx, a.M, a.G, a.soft, p, acc);
+            if (a.pair_f32) massive_field_f32<D>(s, a.M, a.soft, p, acc);
+            else massive_field<D>(s, a.M, a.soft, p, acc);
         }
         for (int c = 0; c < D; ++c) a.aacc[c][i] = acc[c];
     }
-    if (!back_reaction<D>(a, s, lo, hi, slot)) return;
     massive_accel<D>(a, s);
-    __syncthreads();
-    for (int k = tid; k < a.M; k += blockDim.x)
-        for (int c = 0; c < D; ++c) s.macc[c][k] = s.mnew[c][k];
+    if (!back_reaction<D>(a, s, lo, hi, slot)) return;
+    for (int k = tid; k < a.M; k += FR_NT)
+        for (int c = 0; c < D; ++c) s.macc[c][k] = s.bk[c][k] + s.mnew[c][k];
     __syncthreads();
 
     const double wd[3] = {a.w1, a.w0, a.w1};
     for (int ks = 0; ks < a.K; ++ks) {
         if (tid == 0) { s.rem = a.dt_raster; s.done = 0; }
         if (a.m_sub > 0)
-            for (int i = lo + tid; i < hi; i += blockDim.x) a.sub_n[(int64_t)ks * a.n_ast + i] = 0;
+            for (int i = lo + tid; i < hi; i += FR_NT) a.sub_n[(int64_t)ks * a.n_ast + i] = 0;
         __syncthreads();
         for (;;) {
             // dtH (nbody_kernel.py:247-275)
@@ -518,71 +563,74 @@ __global__ void __launch_bounds__(FR_NT) k_frame(const FrameArgs a) {
             __syncthreads();
             if (s.done) break;
             const double dtH = s.dtH;
-            // hot classification (:283-301)
-            for (int i = lo + tid; i < hi; i += blockDim.x) {
-                unsigned char h = 0;
+            // hot classification (:283-301): dist / vrel / 20 < dtH, squared
+            int hot = 0;
+            const double lim = dtH > 0.0 ? 400.0 * dtH * dtH : -1.0;
+            for (int i = lo + tid; i < hi; i += FR_NT) {
+                bool h = false;
                 if (a.avis[i]) {
-                    for (int k = 0; k < a.M && !h; ++k) {
-                        if (!s.mvis[k]) continue;
+                    double p[3], v[3];
+                    for (int c = 0; c < D; ++c) { p[c] = a.ax[c][i]; v[c] = a.av[c][i]; }
+#pragma unroll 4
+                    for (int k = 0; k < a.M; ++k) {
                         double d2 = 0.0, v2 = 0.0;
                         for (int c = 0; c < D; ++c) {
-                            const double dx = s.mx[c][k] - a.ax[c][i], dv = s.mv[c][k] - a.av[c][i];
+                            const double dx = s.mx[c][k] - p[c], dv = s.mv[c][k] - v[c];
                             d2 += dx * dx;
                             v2 += dv * dv;
                         }
-                        double dist = sqrt(d2);
-                        if (dist < 1e-12) dist = 1e-12;
-                        const double vrel = sqrt(v2);
-                        if (vrel > 1e-9 && dist / vrel / 20.0 < dtH) h = 1;
+                        if (d2 < 1e-24) d2 = 1e-24;
+                        h |= s.mvis[k] && v2 > 1e-18 && d2 < lim * v2;
                     }
                 }
                 a.hot[i] = h;
+                hot |= h;
             }
-            for (int k = tid; k < a.M; k += blockDim.x)
+            for (int k = tid; k < a.M; k += FR_NT)
                 for (int c = 0; c < D; ++c) s.mx0[c][k] = s.mx[c][k];
-            __syncthreads();
+            hot = __syncthreads_or(hot);
 
             for (int w = 0; w < 3; ++w) {
                 const double dt = wd[w] * dtH;
-                // phase A: positions of calm asteroids and massive bodies (:317-331)
-                for (int i = lo + tid; i < hi; i += blockDim.x) {
-                    if (!a.avis[i] || a.hot[i]) continue;
-                    for (int c = 0; c < D; ++c) a.ax[c][i] += a.av[c][i] * dt + 0.5 * a.aacc[c][i] * dt * dt;
-                }
-                for (int k = tid; k < a.M; k += blockDim.x) {
+                // positions of the massive bodies (:317-331); the thread that owns body k wrote its
+                // velocity and acceleration
+                for (int k = tid; k < a.M; k += FR_NT) {
                     if (!s.mvis[k]) continue;
                     for (int c = 0; c < D; ++c) s.mx[c][k] += s.mv[c][k] * dt + 0.5 * s.macc[c][k] * dt * dt;
                 }
                 __syncthreads();
-                // phase B: asteroid forces + velocities of calm asteroids (:343-362)
-                for (int i = lo + tid; i < hi; i += blockDim.x) {
-                    if (!a.avis[i]) continue;
-                    double p[3], acc[3];
-                    for (int c = 0; c < D; ++c) p[c] = a.ax[c][i];
-                    if (a.pair_f32 && !a.hot[i]) massive_field_f32<D>(s, s.mx, a.M, a.G, a.soft, p, acc);
-                    else massive_field<D>(s, s.mx, a.M, a.G, a.soft, p, acc);
-                    if (!a.hot[i]) {
-                        for (int c = 0; c < D; ++c) {
-                            a.av[c][i] += 0.5 * (a.aacc[c][i] + acc[c]) * dt;
-                            a.aacc[c][i] = acc[c];
-                        }
+                // calm asteroids: position (:317-331), force at it and velocity (:343-362)
+                for (int i = lo + tid; i < hi; i += FR_NT) {
+                    if (!a.avis[i] || a.hot[i]) continue;
+                    double p[3], v[3], a0[3], acc[3];
+                    for (int c = 0; c < D; ++c) {
+                        v[c] = a.av[c][i];
+                        a0[c] = a.aacc[c][i];
+                        p[c] = a.ax[c][i] + (v[c] * dt + 0.5 * a0[c] * dt * dt);
+                        a.ax[c][i] = p[c];
+                    }
+                    if (a.pair_f32) massive_field_f32<D>(s, a.M, a.soft, p, acc);
+                    else massive_field<D>(s, a.M, a.soft, p, acc);
+                    for (int c = 0; c < D; ++c) {
+                        a.av[c][i] = v[c] + 0.5 * (a0[c] + acc[c]) * dt;
+                        a.aacc[c][i] = acc[c];
                     }
                 }
+                massive_accel<D>(a, s);
                 // back-reaction of all visible asteroids (hot ones at their segment start)
                 if (!back_reaction<D>(a, s, lo, hi, slot)) return;
-                // phase C: massive accelerations and velocities (:377-399)
-                massive_accel<D>(a, s);
-                __syncthreads();
-                for (int k = tid; k < a.M; k += blockDim.x) {
+                // massive velocities (:377-399)
+                for (int k = tid; k < a.M; k += FR_NT) {
                     for (int c = 0; c < D; ++c) {
-                        if (s.mvis[k]) s.mv[c][k] += 0.5 * (s.macc[c][k] + s.mnew[c][k]) * dt;
-                        s.macc[c][k] = s.mnew[c][k];
+                        const double an = s.bk[c][k] + s.mnew[c][k];
+                        if (s.mvis[k]) s.mv[c][k] += 0.5 * (s.macc[c][k] + an) * dt;
+                        s.macc[c][k] = an;
                     }
                 }
-                __syncthreads();
             }
+            __syncthreads();
             // private fine loop of the hot asteroids (:416-535)
-            hot_pass<D>(a, s, lo, hi, ks, dtH, a.dt_raster - s.rem - dtH);
+            if (hot) hot_pass<D>(a, s, lo, hi, ks, dtH, a.dt_raster - s.rem - dtH);
         }
         // snapshot of this raster sample, original body order (:540-557)
         float* row = a.snap + (int64_t)ks * 2 * D * a.n_total;
@@ -720,7 +768,10 @@ extern "C" int sss_frame_launch(sss_ctx* ctx, const sss_frame_state* st, double 
     int per_sm = 0;
     SSS_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, FR_NT, 0));
     if (per_sm < 1) return sss_set_err(ctx, SSS_ERR_CUDA, "frame kernel does not fit on an SM");
-    const int need = (int)((st->n_ast + FR_NT - 1) / FR_NT);
+    // massless asteroids: no CTA waits for another, so few asteroids are spread thin (a warp's worth
+    // each) and the CTA's other warps integrate the massive bodies meanwhile
+    const int per_cta = a.massless ? 32 : FR_NT;
+    const int need = (int)((st->n_ast + per_cta - 1) / per_cta);
     int grid = need < 1 ? 1 : need;
     const int cap = per_sm * ctx->num_sms;
     if (grid > cap) grid = cap;

@@ -345,3 +345,39 @@ def test_f32_pair_forces_on_the_asteroid_clouds():
     n = len(x)
     assert np.abs(f64s[1][:2 * n] - f64s[0][:2 * n]).max() <= 1e-9
     assert outs[0].shape == outs[1].shape
+
+
+@pytest.mark.parametrize("dim", [2, 3])
+@pytest.mark.parametrize("massive_ast", [False, True])
+@pytest.mark.parametrize("M,n_ast", [(1, 33), (2, 1), (8, 257), (9, 700), (17, 64), (64, 31)])
+def test_massive_counts_match_oracle(M, n_ast, massive_ast, dim):
+    """Body counts at the edges of the passes over massive bodies (8 a pass of
+    the back-reaction and of a hot asteroid's lanes) and of the asteroid
+    chunks (32 a CTA without mass, 256 with), one body of each kind hidden;
+    f64 state within the 1e-9 of the parity tests."""
+    nk = _nk()
+    rng = np.random.default_rng(100 * M + n_ast)
+    n = M + n_ast
+    r = np.concatenate([[0.0], 0.5 + 0.4 * np.arange(M - 1), rng.uniform(0.6, 6.0, n_ast)])
+    th = rng.uniform(0, 2 * np.pi, n)
+    x, y = r * np.cos(th), r * np.sin(th)
+    v = np.sqrt(of.G_AU / np.maximum(r, 1e-9)) * (r > 0)
+    vx, vy = -v * np.sin(th), v * np.cos(th)
+    z = vz = None
+    if dim == 3:
+        z, vz = rng.normal(0, 0.02, n) * (r > 0), rng.normal(0, 0.05, n) * (r > 0)
+    mass = np.concatenate([[1.0], 10 ** rng.uniform(-7, -4, M - 1),
+                           np.full(n_ast, 1e-7 if massive_ast else 0.0)])
+    vis = np.ones(n, np.uint8)
+    if M > 2:
+        vis[2] = 0
+    if n_ast > 5:
+        vis[M + 3] = 0
+    is_ast = np.concatenate([np.zeros(M, np.uint8), np.ones(n_ast, np.uint8)])
+    ost, a, m = oracle_state(x, y, vx, vy, mass, vis, is_ast, None, z, vz)
+    of.frame_launch(ost, 1.0 / 365.25, 2)
+    sim = nk.NBodyCuda(0)
+    st = sim.load_state(x, y, vx, vy, mass, vis, is_ast, np.zeros(n), z=z, vz=vz)
+    sim.step_batch(st, 1.0 / 365.25, 2)
+    ref = full_order(ost, a, m, n)
+    assert np.abs(sim.export_f64(st) - ref).max() <= 1e-9 * np.abs(ref).max()
