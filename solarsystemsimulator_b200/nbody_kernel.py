@@ -264,18 +264,17 @@ class NBodyCuda:
         if self.m_sub <= 0:
             return None
         ms, na, d = self.m_sub, st["n_ast"], st["dim"]
-        frames = []
         if not na:
             return [(np.empty(0, np.int64), np.empty((ms, d, 0), np.float32)) for _ in range(k)]
-        subn = st["subn"][:k, :na]
-        for ks in range(k):
-            sel = torch.nonzero(subn[ks] == ms).flatten()
-            if sel.numel() == 0:
-                frames.append((np.empty(0, np.int64), np.empty((ms, d, 0), np.float32)))
-                continue
-            pos = st["subpos"][ks, :ms, :, :na][:, :, sel].cpu().numpy()
-            frames.append((st["a_idx_h"][sel.cpu().numpy()], pos))
-        return frames
+        # all samples in one pass: the listing costs one synchronisation a batch, not one a sample
+        rows, cols = torch.nonzero(st["subn"][:k, :na] == ms, as_tuple=True)
+        if rows.numel() == 0:
+            return [(np.empty(0, np.int64), np.empty((ms, d, 0), np.float32)) for _ in range(k)]
+        pos = st["subpos"][rows, :ms, :, cols].cpu().numpy()             # (hits, ms, d), by sample
+        ends = np.searchsorted(rows.cpu().numpy(), np.arange(k + 1))
+        cols = cols.cpu().numpy()
+        return [(st["a_idx_h"][cols[a:b]], np.ascontiguousarray(pos[a:b].transpose(1, 2, 0)))
+                for a, b in zip(ends[:-1], ends[1:])]
 
     # ------------------------------------------------------- point updates
     def _scatter(self, st, idx, vals, mode):
