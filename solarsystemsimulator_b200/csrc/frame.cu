@@ -125,13 +125,6 @@ __device__ __forceinline__ void chunk_of(int n, int& lo, int& hi) {
     hi = min(n, lo + per);
 }
 
-// G / (r2 sqrt r2) times a mass: the f64 pair factor from one reciprocal square root (within an ulp;
-// a square root and a division behind one another were the longest chain of every pass).
-__device__ __forceinline__ double pair_factor(double gm, double r2) {
-    const double inv = rsqrt(r2);
-    return gm * (inv * inv * inv);
-}
-
 // dist / vrel / 20 of an offset and a relative velocity (nbody_kernel.py:247-275): dist at least
 // 1e-12, +inf where vrel <= 1e-9. NaN offsets stay NaN (no comparison picks them).
 __device__ __forceinline__ double encounter(double d2, double v2, double& dist) {
@@ -150,7 +143,7 @@ __device__ __forceinline__ void massive_field(const FrameShared& s, int M, doubl
     for (int k = 0; k < M; ++k) {
         double dx[3], r2 = soft;
         for (int c = 0; c < D; ++c) { dx[c] = s.mx[c][k] - p[c]; r2 += dx[c] * dx[c]; }
-        const double f = pair_factor(s.gm[k], s.mvis[k] ? r2 : 1.0);
+        const double f = sss_gm_rinv3(s.gm[k], s.mvis[k] ? r2 : 1.0);
         for (int c = 0; c < D; ++c) acc[c] += s.mvis[k] ? f * dx[c] : 0.0;
     }
 }
@@ -199,7 +192,7 @@ __device__ __forceinline__ void field_grp(const FrameShared& s, int M, double so
             dx[c] = mi - p[c];
             r2 += dx[c] * dx[c];
         }
-        const double f = pair_factor(s.gm[k], r2);
+        const double f = sss_gm_rinv3(s.gm[k], r2);
         for (int c = 0; c < D; ++c) acc[c] += f * dx[c];
     }
     group_sum<D>(acc, gmask);
@@ -251,7 +244,7 @@ __device__ void back_partial(const FrameArgs& a, FrameShared& s, int lo, int hi,
                     double dx[3], r2 = a.soft;
                     for (int c = 0; c < D; ++c) { dx[c] = s.mx[c][k] - p[c]; r2 += dx[c] * dx[c]; }
                     const bool on = k0 + j < a.M && s.mvis[k];
-                    const double f = pair_factor(gm, on ? r2 : 1.0);
+                    const double f = sss_gm_rinv3(gm, on ? r2 : 1.0);
 #pragma unroll
                     for (int c = 0; c < D; ++c) b[j * D + c] -= on ? f * dx[c] : 0.0;
                 }
@@ -318,7 +311,7 @@ __device__ void massive_accel(const FrameArgs& a, FrameShared& s) {
                 if (j == i || !s.mvis[j]) continue;
                 double dx[3], r2 = a.soft;
                 for (int c = 0; c < D; ++c) { dx[c] = s.mx[c][j] - s.mx[c][i]; r2 += dx[c] * dx[c]; }
-                const double f = pair_factor(s.gm[j], r2);
+                const double f = sss_gm_rinv3(s.gm[j], r2);
                 for (int c = 0; c < D; ++c) acc[c] += f * dx[c];
             }
         }
@@ -398,7 +391,7 @@ __device__ void fine_loop(const FrameArgs& a, const FrameShared& s, int i, int k
             const double te = encounter(d2, v2, dist);
             if (dist <= s.mrad[k] + rad) { first = min(first, k); last = k; }
             if (te < dtF) dtF = te;
-            const double f = pair_factor(s.gm[k], d2 + a.soft);
+            const double f = sss_gm_rinv3(s.gm[k], d2 + a.soft);
             for (int c = 0; c < D; ++c) acc[c] += f * dx[c];
         }
 #pragma unroll

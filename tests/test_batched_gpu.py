@@ -119,3 +119,28 @@ def test_matches_reference_advance_golden(load_golden):
         rv = np.stack([g[f"rvx{s}"], g[f"rvy{s}"]])
         assert np.abs(p - rp).max() <= 1e-12 * np.abs(rp).max()
         assert np.abs(v - rv).max() <= 1e-12 * np.abs(rv).max()
+
+
+@pytest.mark.parametrize("dim", [2, 3])
+@pytest.mark.parametrize("n", [9, 16, 17, 21, 31, 32, 33, 43, 63, 64])
+def test_block_mappings_of_odd_sizes(n, dim):
+    """The block-per-system mappings pack n targets and T / n source chunks
+    (at most 8): sizes that fill the block, leave a remainder and reach the
+    chunk limit, each in a launch with more than one size, against the oracle."""
+    from solarsystemsimulator_b200 import batched
+    rng = np.random.default_rng(10 * n + dim)
+    systems = []
+    for k in (n, max(3, n - 1), n):
+        pos, vel = np.zeros((3, k)), np.zeros((3, k))
+        pos[:dim], vel[:dim] = rng.normal(0, 1, (dim, k)), rng.normal(0, 0.1, (dim, k))
+        systems.append({"pos": pos, "vel": vel, "mass": rng.uniform(0.1, 1.0, k) / k, "G": 1.5, "dt": 1e-3})
+    for mapping in batched.BLOCK_MAPS[batched.block_bucket(n)]:
+        ens = batched.BatchedSystems(systems, device=0, eps2=1e-2, dim=dim, autotune=False)
+        for g in ens.groups:
+            if g["max_n"] > 8:
+                g["map"] = mapping if batched.block_bucket(g["max_n"]) == batched.block_bucket(n) else g["map"]
+        ens.run(20)
+        for s, (p, v) in zip(systems, ens.export()):
+            rp, rv = ob.yoshida(s["pos"], s["vel"], s["mass"], s["G"], s["dt"], 20, 1e-2)
+            assert np.abs(p - rp[:dim]).max() <= 1e-12 * np.abs(rp).max()
+            assert np.abs(v - rv[:dim]).max() <= 1e-12 * np.abs(rv).max()
