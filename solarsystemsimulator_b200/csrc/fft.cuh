@@ -250,15 +250,15 @@ __device__ __forceinline__ void stage(const C* __restrict__ tw, Get get, Put put
         Map::template split<NB>(w, j, c);
         const int k = j % SPAN;
         if (S > 0) {
-            // the powers 1, 2, 4, 8 of the butterfly's twiddle from the table, the others as
+            // f64: the powers 1, 2, 4, 8 of the butterfly's twiddle from the table, the others as
             // their products (at most three factors): 15 loads of radix 16 were more L1
-            // traffic than the exchange itself
+            // traffic than the exchange itself. f32: all from the table, as exact as it is
             const C* q = tw + fft_off(N, S) + k;
             C f[R];
 #pragma unroll
             for (int t = 1; t < R; ++t) {
                 const int top = t >= 8 ? 8 : t >= 4 ? 4 : t >= 2 ? 2 : 1;
-                f[t] = t == top ? __ldg(q + (t - 1) * SPAN) : mul(f[top], f[t - top]);
+                f[t] = t == top || sizeof(C) == 8 ? __ldg(q + (t - 1) * SPAN) : mul(f[top], f[t - top]);
                 v[b * R + t] = DIR < 0 ? mul(v[b * R + t], f[t]) : mulc(v[b * R + t], f[t]);
             }
         }

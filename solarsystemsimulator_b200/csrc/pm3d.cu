@@ -6,22 +6,28 @@
 //   deposit  : CIC, positions f64, weights f32, warp-aggregated atomics:
 //              lanes of a warp whose particles share a cell add their
 //              weights in registers first and one lane issues the atomics.
-//   solve    : cuFFT R2C -> k_spectrum3 (Green's function -4 pi G / k^2,
-//              divided by the CIC window W(k)^deconv (2: deposit and
-//              gather) and filtered by exp(-k^2 r_split^2), the spectral
-//              gradient a_d = -i k_d phi, the 1/n^3 of the inverse
-//              transform; one read of rho_k, three writes) -> one batched
-//              C2R for the three components. cuFFT performs the transforms
-//              only.
+//   solve    : real transform, Green's function -4 pi G / k^2 (divided by the
+//              CIC window W(k)^deconv, 2: deposit and gather, and filtered by
+//              exp(-k^2 r_split^2)), spectral gradient a_d = -i k_d phi with
+//              the 1/n^3 of the inverse transform, three inverse transforms.
+//              Mesh sides 2^a and 3 2^a from 32 to 512 take five passes over
+//              the block transforms of fft.cuh: z forward (two rows as one
+//              complex transform), y forward, x forward + Green's function +
+//              x inverse, y inverse, z inverse. The gradient's factor along an
+//              axis is applied when that axis is transformed back, so the x
+//              pass writes two spectra (phi and i k_x phi) and only the y pass
+//              makes three of them: 18 mesh passes of memory where R2C, the
+//              spectrum kernel and a batched C2R moved 36. Other sides: cuFFT
+//              for the transforms around k_spectrum3.
 //   gather   : trilinear (CIC) interpolation of the three f32 meshes into
 //              f64 accelerations, fused with the KDK epilogue.
 //
 // HBM per step at 1,048,576 particles on 256^3: deposit reads 24 B per
-// particle and makes 8 atomic f32 updates, the spectrum kernel moves
-// 32 B per mode, the gather reads 24 B per particle plus 24 f32 mesh values
+// particle and makes 8 atomic f32 updates, the gather reads 24 B per particle plus 24 f32 mesh values
 // (L2-resident for a 64 MiB mesh) and writes the state.
 
 #include "pm3d.cuh"
+#include "fft.cuh"
 
 #include <algorithm>
 
@@ -148,6 +154,207 @@ __global__ void __launch_bounds__(128) k_spectrum3(const float2* __restrict__ rk
     ak[2 * m + t] = out[2];
 }
 
+// ------------------------------------------------------- solve, own FFTs
+
+// The transforms along y or x of one half-complex mesh, 16 to a CTA: 16
+// neighbouring z of one plane (128-byte rows), the nh % 16 last z of several
+// planes together (nh = n / 2 + 1: one z a plane would leave 15 idle).
+template <int N>
+struct Tile16 {
+    static constexpr int NH = N / 2 + 1, FULL_T = NH / 16, REST = NH % 16, TILES = N * FULL_T + N * REST / 16;
+    static_assert(N % 16 == 0, "mesh side");
+    using Map = fft::Inner<16>;
+    static constexpr int NT = fft_threads(N, 16);
+    static constexpr size_t SMEM = (size_t)N * 16 * sizeof(float2);
+    int plane, iz;
+    __device__ __forceinline__ Tile16() {
+        const int b = blockIdx.x, c = threadIdx.x & 15;
+        if (b < N * FULL_T) {
+            plane = b / (FULL_T > 0 ? FULL_T : 1);
+            iz = (b - plane * FULL_T) * 16 + c;
+        } else {
+            const int u = (b - N * FULL_T) * 16 + c;
+            plane = u / (REST > 0 ? REST : 1);
+            iz = FULL_T * 16 + u - plane * REST;
+        }
+    }
+};
+
+// 16 pairs of rows along z
+template <int N>
+struct Rows16 {
+    static constexpr int NH = N / 2 + 1, STRIDE = N + N / 16, TILES = N * N / 32;
+    using Map = fft::Outer<16, STRIDE>;
+    static constexpr int NT = fft_threads(N, 16);
+    static constexpr size_t SMEM = (size_t)16 * STRIDE * sizeof(float2);
+};
+
+template <int N>
+__global__ void __launch_bounds__(Rows16<N>::NT, 768 / Rows16<N>::NT)
+k_z_fwd(const float2* __restrict__ tw, const float* __restrict__ rho, float2* __restrict__ rk) {
+    using R = Rows16<N>;
+    using Map = typename R::Map;
+    extern __shared__ float2 smf[];
+    const long long row0 = (long long)blockIdx.x * 32;
+    const float* src = rho + row0 * N;
+    fft::run<N, -1, Map>(tw, smf,
+                         [&](int i, int c, bool) { return make_float2(__ldg(src + 2 * c * N + i), __ldg(src + (2 * c + 1) * N + i)); },
+                         [&](int i, int c, float2 z, bool) { smf[Map::at(i, c)] = z; });
+    __syncthreads();
+    float2* dst = rk + row0 * R::NH;
+    for (int q = threadIdx.x; q < 16 * R::NH; q += R::NT) {
+        const int c = q / R::NH, k = q - c * R::NH;
+        const float2 z = smf[Map::at(k, c)], w = smf[Map::at(k == 0 ? 0 : N - k, c)];
+        dst[(2 * c) * R::NH + k] = make_float2(0.5f * (z.x + w.x), 0.5f * (z.y - w.y));
+        dst[(2 * c + 1) * R::NH + k] = make_float2(0.5f * (z.y + w.y), 0.5f * (w.x - z.x));
+    }
+}
+
+template <int N>
+__global__ void __launch_bounds__(Tile16<N>::NT, 768 / Tile16<N>::NT) k_y_fwd(const float2* __restrict__ tw, float2* rk) {
+    using T = Tile16<N>;
+    extern __shared__ float2 smf[];
+    const T t;
+    float2* p = rk + (long long)t.plane * N * T::NH + t.iz;
+    fft::run<N, -1, typename T::Map>(tw, smf, [&](int i, int, bool) { return p[i * T::NH]; },
+                                     [&](int i, int, float2 z, bool) { p[i * T::NH] = z; });
+}
+
+// a_x = i k_x c rho_k and phi' = c rho_k (c as in k_spectrum3), both inverse
+// transformed along x; plane = iy.
+template <int N>
+__global__ void __launch_bounds__(Tile16<N>::NT, 768 / Tile16<N>::NT)
+k_x_solve(const float2* __restrict__ tw, const float2* __restrict__ rk, double cscale, const double* __restrict__ tab,
+          float2* __restrict__ ax, float2* __restrict__ phi) {
+    using T = Tile16<N>;
+    using Map = typename T::Map;
+    extern __shared__ float2 smf[];
+    float2* sp = smf + N * 16;
+    const T t;
+    const long long o = (long long)t.plane * T::NH + t.iz;
+    constexpr int ST = N * T::NH;
+    const double k2yz = tab[N + t.plane] + tab[N + t.iz];
+    const double cyz = cscale * (tab[2 * N + t.plane] * tab[2 * N + t.iz]);
+    const bool mean = t.plane == 0 && t.iz == 0;
+    fft::run<N, -1, Map>(tw, smf, [&](int i, int, bool) { return __ldg(rk + o + i * ST); },
+                         [&](int i, int c, float2 r, bool) {
+                             float2 a = make_float2(0.f, 0.f), b = a;
+                             if (!mean || i != 0) {
+                                 const double q = cyz * __ldg(tab + 2 * N + i) / (k2yz + __ldg(tab + N + i));
+                                 const double f = __ldg(tab + i) * q;
+                                 a = make_float2((float)(-f * (double)r.y), (float)(f * (double)r.x));
+                                 b = make_float2((float)(q * (double)r.x), (float)(q * (double)r.y));
+                             }
+                             smf[Map::at(i, c)] = a;
+                             sp[Map::at(i, c)] = b;
+                         });
+    __syncthreads();
+#pragma unroll 1
+    for (int d = 0; d < 2; ++d) {
+        float2* buf = d ? sp : smf;
+        float2* out = (d ? phi : ax) + o;
+        fft::run<N, 1, Map, true>(tw, buf, [&](int i, int c, bool) { return buf[Map::at(i, c)]; },
+                                  [&](int i, int, float2 z, bool) { out[i * ST] = z; });
+    }
+}
+
+// Along y: a_x, phi -> a_y = i k_y phi in phi's place, and phi to the third
+// mesh (its k_z comes with the z pass); plane = ix.
+template <int N>
+__global__ void __launch_bounds__(Tile16<N>::NT, 768 / Tile16<N>::NT)
+k_y_inv(const float2* __restrict__ tw, const double* __restrict__ tab, float2* ax, float2* phi,
+        float2* __restrict__ third) {
+    using T = Tile16<N>;
+    using Map = typename T::Map;
+    extern __shared__ float2 smf[];
+    const T t;
+    const long long o = (long long)t.plane * N * T::NH + t.iz;
+    // one body of code for the three (three in a row kept each other's addresses in registers)
+#pragma unroll 1
+    for (int d = 0; d < 3; ++d) {
+        const float2* in = (d == 0 ? ax : phi) + o;
+        float2* out = (d == 0 ? ax : d == 1 ? third : phi) + o;
+        fft::run<N, 1, Map>(tw, smf,
+                            [&](int i, int, bool) {
+                                float2 z = in[i * T::NH];
+                                if (d == 2) {
+                                    const float k = (float)__ldg(tab + i);
+                                    z = make_float2(-k * z.y, k * z.x);
+                                }
+                                return z;
+                            },
+                            [&](int i, int, float2 z, bool) { out[i * T::NH] = z; });
+        __syncthreads();
+    }
+}
+
+// Half spectra along z of two rows -> the rows: one complex transform of
+// a + i b. blockIdx.y = component; the third one takes its i k_z here.
+template <int N>
+__global__ void __launch_bounds__(Rows16<N>::NT, 768 / Rows16<N>::NT)
+k_z_inv(const float2* __restrict__ tw, const double* __restrict__ tab, const float2* __restrict__ ak,
+        float* __restrict__ acc) {
+    using R = Rows16<N>;
+    using Map = typename R::Map;
+    extern __shared__ float2 smf[];
+    const int d = blockIdx.y;
+    const long long row0 = (long long)blockIdx.x * 32;
+    const float2* src = ak + ((long long)d * N * N + row0) * R::NH;
+#pragma unroll 4
+    for (int q = threadIdx.x; q < 16 * R::NH; q += R::NT) {
+        const int c = q / R::NH, k = q - c * R::NH;
+        float2 a = __ldg(src + (2 * c) * R::NH + k), b = __ldg(src + (2 * c + 1) * R::NH + k);
+        if (d == 2) {
+            const float kz = (float)__ldg(tab + k);
+            a = make_float2(-kz * a.y, kz * a.x);
+            b = make_float2(-kz * b.y, kz * b.x);
+        }
+        if (k == 0 || k == N / 2) { a.y = 0.f; b.y = 0.f; }      // real modes
+        smf[Map::at(k, c)] = make_float2(a.x - b.y, a.y + b.x);
+        if (k > 0 && k < N / 2) smf[Map::at(N - k, c)] = make_float2(a.x + b.y, b.x - a.y);
+    }
+    __syncthreads();
+    float* dst = acc + ((long long)d * N * N + row0) * N;
+    fft::run<N, 1, Map, true>(tw, smf, [&](int i, int c, bool) { return smf[Map::at(i, c)]; },
+                              [&](int i, int c, float2 z, bool) {
+                                  dst[2 * c * N + i] = z.x;
+                                  dst[(2 * c + 1) * N + i] = z.y;
+                              });
+}
+
+template <int N>
+cudaError_t solve_of(sss_pm3* p, double cscale, bool setup, cudaStream_t st) {
+    using T = Tile16<N>;
+    using R = Rows16<N>;
+    if (setup) {
+        const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+        cudaError_t e = cudaFuncSetAttribute((const void*)k_z_fwd<N>, attr, (int)R::SMEM);
+        e = e ? e : cudaFuncSetAttribute((const void*)k_y_fwd<N>, attr, (int)T::SMEM);
+        e = e ? e : cudaFuncSetAttribute((const void*)k_x_solve<N>, attr, (int)(2 * T::SMEM));
+        e = e ? e : cudaFuncSetAttribute((const void*)k_y_inv<N>, attr, (int)T::SMEM);
+        e = e ? e : cudaFuncSetAttribute((const void*)k_z_inv<N>, attr, (int)R::SMEM);
+        return e ? e : fft_table(N, &p->tw);
+    }
+    const size_t m = (size_t)N * N * T::NH;
+    k_z_fwd<N><<<R::TILES, R::NT, R::SMEM, st>>>(p->tw, p->rho, p->rk);
+    k_y_fwd<N><<<T::TILES, T::NT, T::SMEM, st>>>(p->tw, p->rk);
+    k_x_solve<N><<<T::TILES, T::NT, 2 * T::SMEM, st>>>(p->tw, p->rk, cscale, p->tab, p->ak, p->ak + m);
+    k_y_inv<N><<<T::TILES, T::NT, T::SMEM, st>>>(p->tw, p->tab, p->ak, p->ak + m, p->ak + 2 * m);
+    k_z_inv<N><<<dim3(R::TILES, 3), R::NT, R::SMEM, st>>>(p->tw, p->tab, p->ak, p->acc);
+    return cudaGetLastError();
+}
+
+// Mesh sides with own transforms: 2^a and 3 2^a from 32 (one stage less than
+// two below) to 512 (512 threads and 128 KB for 16 columns twice above).
+bool own_solve(sss_pm3* p, double cscale, bool setup, cudaStream_t st, cudaError_t* e) {
+    switch (p->n) {
+#define CASE(q) case q: *e = solve_of<q>(p, cscale, setup, st); return true
+        CASE(32); CASE(48); CASE(64); CASE(96); CASE(128); CASE(192); CASE(256); CASE(384); CASE(512);
+#undef CASE
+        default: return false;
+    }
+}
+
 __global__ void __launch_bounds__(256) k_gather3(const Pm3Parts s, int n, double inv_h,
                                                  const float* __restrict__ acc, const Pm3Epi e) {
     const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -189,6 +396,7 @@ void pm3_free(sss_pm3* p) {
     cudaFree(p->ak);
     cudaFree(p->acc);
     cudaFree(p->tab);
+    cudaFree(p->tw);
     free(p);
 }
 
@@ -227,6 +435,15 @@ extern "C" int sss_pm3_create(sss_ctx* ctx, int mesh_n, double box, sss_pm3** ou
     if (e != cudaSuccess) {
         pm3_free(p);
         return sss_cuda_err(ctx, e, "cudaMalloc (pm3)");
+    }
+    p->own = own_solve(p, 0.0, true, nullptr, &e);
+    if (e != cudaSuccess) {
+        pm3_free(p);
+        return sss_cuda_err(ctx, e, "transforms (pm3)");
+    }
+    if (p->own) {
+        *out = p;
+        return SSS_OK;
     }
     cufftResult r = cufftPlan3d(&p->fwd, mesh_n, mesh_n, mesh_n, CUFFT_R2C);
     if (r == CUFFT_SUCCESS) {
@@ -278,10 +495,6 @@ extern "C" int sss_pm3_solve(sss_pm3* p, double G, int deconv, double r_split, v
     if (deconv < 0 || deconv > 4) return sss_set_err(ctx, SSS_ERR_ARG, "deconv must be in [0, 4]");
     if (!(r_split >= 0.0)) return sss_set_err(ctx, SSS_ERR_ARG, "r_split must be >= 0");
     cudaStream_t st = (cudaStream_t)stream;
-    cufftSetStream(p->fwd, st);
-    cufftSetStream(p->inv3, st);
-    cufftResult r = cufftExecR2C(p->fwd, p->rho, (cufftComplex*)p->rk);
-    if (r != CUFFT_SUCCESS) return cufft_err(ctx, r, "cufftExecR2C");
     const double rs2 = r_split * r_split;
     if (p->tab_deconv != deconv || p->tab_rs2 != rs2) {
         k_spectrum_tables<<<blocks_for(p->n, 128), 128, 0, st>>>(p->n, p->box, deconv, rs2, p->tab);
@@ -291,6 +504,16 @@ extern "C" int sss_pm3_solve(sss_pm3* p, double G, int deconv, double r_split, v
     }
     const int nh = p->n / 2 + 1;
     const double cscale = 4.0 * 3.14159265358979323846 * G / ((double)p->n * p->n * p->n);
+    if (p->own) {
+        cudaError_t e = cudaSuccess;
+        own_solve(p, cscale, false, st, &e);
+        if (e != cudaSuccess) return sss_cuda_err(ctx, e, "own transforms (pm3)");
+        return SSS_OK;
+    }
+    cufftSetStream(p->fwd, st);
+    cufftSetStream(p->inv3, st);
+    cufftResult r = cufftExecR2C(p->fwd, p->rho, (cufftComplex*)p->rk);
+    if (r != CUFFT_SUCCESS) return cufft_err(ctx, r, "cufftExecR2C");
     k_spectrum3<<<dim3((nh + 127) / 128, p->n, p->n), 128, 0, st>>>(p->rk, p->n, cscale, p->tab, p->ak);
     SSS_LAUNCH_CHECK(ctx, "k_spectrum3");
     r = cufftExecC2R(p->inv3, (cufftComplex*)p->ak, p->acc);

@@ -16,6 +16,8 @@ struct sss_pm3 {
     float2* rk;         // n * n * (n/2 + 1) spectrum of rho
     float2* ak;         // 3 spectra of the acceleration components (contiguous)
     float* acc;         // 3 n^3 acceleration meshes (contiguous)
+    bool own;           // the solve by the kernels of pm3d.cu, else cuFFT
+    float2* tw;         // own: twiddles of length n
     cufftHandle fwd;    // R2C n^3
     cufftHandle inv3;   // C2R n^3, batch 3
     double* tab;        // per-axis tables of the spectrum kernel: kd[n], k2[n], fac[n]
