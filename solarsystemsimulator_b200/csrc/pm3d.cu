@@ -156,12 +156,16 @@ __global__ void __launch_bounds__(128) k_spectrum3(const float2* __restrict__ rk
 
 // ------------------------------------------------------- solve, own FFTs
 
+// Values per row of the half spectra: n / 2 + 1 rounded up to a 32-byte sector (rows of 1032 bytes
+// shared sectors between CTAs).
+__host__ __device__ constexpr int pitch_of(int n) { return (n / 2 + 4) / 4 * 4; }
+
 // The transforms along y or x of one half-complex mesh, 16 to a CTA: 16
 // neighbouring z of one plane (128-byte rows), the nh % 16 last z of several
 // planes together (nh = n / 2 + 1: one z a plane would leave 15 idle).
 template <int N>
 struct Tile16 {
-    static constexpr int NH = N / 2 + 1, FULL_T = NH / 16, REST = NH % 16, TILES = N * FULL_T + N * REST / 16;
+    static constexpr int NH = N / 2 + 1, PITCH = pitch_of(N), FULL_T = NH / 16, REST = NH % 16, TILES = N * FULL_T + N * REST / 16;
     static_assert(N % 16 == 0, "mesh side");
     using Map = fft::Inner<16>;
     static constexpr int NT = fft_threads(N, 16);
@@ -183,14 +187,14 @@ struct Tile16 {
 // 16 pairs of rows along z
 template <int N>
 struct Rows16 {
-    static constexpr int NH = N / 2 + 1, STRIDE = N + N / 16, TILES = N * N / 32;
+    static constexpr int NH = N / 2 + 1, PITCH = pitch_of(N), STRIDE = N + N / 16, TILES = N * N / 32;
     using Map = fft::Outer<16, STRIDE>;
     static constexpr int NT = fft_threads(N, 16);
     static constexpr size_t SMEM = (size_t)16 * STRIDE * sizeof(float2);
 };
 
 template <int N>
-__global__ void __launch_bounds__(Rows16<N>::NT, 768 / Rows16<N>::NT)
+__global__ void __launch_bounds__(Rows16<N>::NT, 1024 / Rows16<N>::NT)
 k_z_fwd(const float2* __restrict__ tw, const float* __restrict__ rho, float2* __restrict__ rk) {
     using R = Rows16<N>;
     using Map = typename R::Map;
@@ -201,29 +205,29 @@ k_z_fwd(const float2* __restrict__ tw, const float* __restrict__ rho, float2* __
                          [&](int i, int c, bool) { return make_float2(__ldg(src + 2 * c * N + i), __ldg(src + (2 * c + 1) * N + i)); },
                          [&](int i, int c, float2 z, bool) { smf[Map::at(i, c)] = z; });
     __syncthreads();
-    float2* dst = rk + row0 * R::NH;
+    float2* dst = rk + row0 * R::PITCH;
     for (int q = threadIdx.x; q < 16 * R::NH; q += R::NT) {
         const int c = q / R::NH, k = q - c * R::NH;
         const float2 z = smf[Map::at(k, c)], w = smf[Map::at(k == 0 ? 0 : N - k, c)];
-        dst[(2 * c) * R::NH + k] = make_float2(0.5f * (z.x + w.x), 0.5f * (z.y - w.y));
-        dst[(2 * c + 1) * R::NH + k] = make_float2(0.5f * (z.y + w.y), 0.5f * (w.x - z.x));
+        dst[(2 * c) * R::PITCH + k] = make_float2(0.5f * (z.x + w.x), 0.5f * (z.y - w.y));
+        dst[(2 * c + 1) * R::PITCH + k] = make_float2(0.5f * (z.y + w.y), 0.5f * (w.x - z.x));
     }
 }
 
 template <int N>
-__global__ void __launch_bounds__(Tile16<N>::NT, 768 / Tile16<N>::NT) k_y_fwd(const float2* __restrict__ tw, float2* rk) {
+__global__ void __launch_bounds__(Tile16<N>::NT, 1024 / Tile16<N>::NT) k_y_fwd(const float2* __restrict__ tw, float2* rk) {
     using T = Tile16<N>;
     extern __shared__ float2 smf[];
     const T t;
-    float2* p = rk + (long long)t.plane * N * T::NH + t.iz;
-    fft::run<N, -1, typename T::Map>(tw, smf, [&](int i, int, bool) { return p[i * T::NH]; },
-                                     [&](int i, int, float2 z, bool) { p[i * T::NH] = z; });
+    float2* p = rk + (long long)t.plane * N * T::PITCH + t.iz;
+    fft::run<N, -1, typename T::Map>(tw, smf, [&](int i, int, bool) { return p[i * T::PITCH]; },
+                                     [&](int i, int, float2 z, bool) { p[i * T::PITCH] = z; });
 }
 
 // a_x = i k_x c rho_k and phi' = c rho_k (c as in k_spectrum3), both inverse
 // transformed along x; plane = iy.
 template <int N>
-__global__ void __launch_bounds__(Tile16<N>::NT, 768 / Tile16<N>::NT)
+__global__ void __launch_bounds__(Tile16<N>::NT, 1024 / Tile16<N>::NT)
 k_x_solve(const float2* __restrict__ tw, const float2* __restrict__ rk, double cscale, const double* __restrict__ tab,
           float2* __restrict__ ax, float2* __restrict__ phi) {
     using T = Tile16<N>;
@@ -231,8 +235,8 @@ k_x_solve(const float2* __restrict__ tw, const float2* __restrict__ rk, double c
     extern __shared__ float2 smf[];
     float2* sp = smf + N * 16;
     const T t;
-    const long long o = (long long)t.plane * T::NH + t.iz;
-    constexpr int ST = N * T::NH;
+    const long long o = (long long)t.plane * T::PITCH + t.iz;
+    constexpr int ST = N * T::PITCH;
     const double k2yz = tab[N + t.plane] + tab[N + t.iz];
     const double cyz = cscale * (tab[2 * N + t.plane] * tab[2 * N + t.iz]);
     const bool mean = t.plane == 0 && t.iz == 0;
@@ -261,14 +265,14 @@ k_x_solve(const float2* __restrict__ tw, const float2* __restrict__ rk, double c
 // Along y: a_x, phi -> a_y = i k_y phi in phi's place, and phi to the third
 // mesh (its k_z comes with the z pass); plane = ix.
 template <int N>
-__global__ void __launch_bounds__(Tile16<N>::NT, 768 / Tile16<N>::NT)
+__global__ void __launch_bounds__(Tile16<N>::NT, 1024 / Tile16<N>::NT)
 k_y_inv(const float2* __restrict__ tw, const double* __restrict__ tab, float2* ax, float2* phi,
         float2* __restrict__ third) {
     using T = Tile16<N>;
     using Map = typename T::Map;
     extern __shared__ float2 smf[];
     const T t;
-    const long long o = (long long)t.plane * N * T::NH + t.iz;
+    const long long o = (long long)t.plane * N * T::PITCH + t.iz;
     // one body of code for the three (three in a row kept each other's addresses in registers)
 #pragma unroll 1
     for (int d = 0; d < 3; ++d) {
@@ -276,14 +280,14 @@ k_y_inv(const float2* __restrict__ tw, const double* __restrict__ tab, float2* a
         float2* out = (d == 0 ? ax : d == 1 ? third : phi) + o;
         fft::run<N, 1, Map>(tw, smf,
                             [&](int i, int, bool) {
-                                float2 z = in[i * T::NH];
+                                float2 z = in[i * T::PITCH];
                                 if (d == 2) {
                                     const float k = (float)__ldg(tab + i);
                                     z = make_float2(-k * z.y, k * z.x);
                                 }
                                 return z;
                             },
-                            [&](int i, int, float2 z, bool) { out[i * T::NH] = z; });
+                            [&](int i, int, float2 z, bool) { out[i * T::PITCH] = z; });
         __syncthreads();
     }
 }
@@ -291,7 +295,7 @@ k_y_inv(const float2* __restrict__ tw, const double* __restrict__ tab, float2* a
 // Half spectra along z of two rows -> the rows: one complex transform of
 // a + i b. blockIdx.y = component; the third one takes its i k_z here.
 template <int N>
-__global__ void __launch_bounds__(Rows16<N>::NT, 768 / Rows16<N>::NT)
+__global__ void __launch_bounds__(Rows16<N>::NT, 1024 / Rows16<N>::NT)
 k_z_inv(const float2* __restrict__ tw, const double* __restrict__ tab, const float2* __restrict__ ak,
         float* __restrict__ acc) {
     using R = Rows16<N>;
@@ -299,11 +303,11 @@ k_z_inv(const float2* __restrict__ tw, const double* __restrict__ tab, const flo
     extern __shared__ float2 smf[];
     const int d = blockIdx.y;
     const long long row0 = (long long)blockIdx.x * 32;
-    const float2* src = ak + ((long long)d * N * N + row0) * R::NH;
+    const float2* src = ak + ((long long)d * N * N + row0) * R::PITCH;
 #pragma unroll 4
     for (int q = threadIdx.x; q < 16 * R::NH; q += R::NT) {
         const int c = q / R::NH, k = q - c * R::NH;
-        float2 a = __ldg(src + (2 * c) * R::NH + k), b = __ldg(src + (2 * c + 1) * R::NH + k);
+        float2 a = __ldg(src + (2 * c) * R::PITCH + k), b = __ldg(src + (2 * c + 1) * R::PITCH + k);
         if (d == 2) {
             const float kz = (float)__ldg(tab + k);
             a = make_float2(-kz * a.y, kz * a.x);
@@ -335,7 +339,7 @@ cudaError_t solve_of(sss_pm3* p, double cscale, bool setup, cudaStream_t st) {
         e = e ? e : cudaFuncSetAttribute((const void*)k_z_inv<N>, attr, (int)R::SMEM);
         return e ? e : fft_table(N, &p->tw);
     }
-    const size_t m = (size_t)N * N * T::NH;
+    const size_t m = (size_t)N * N * T::PITCH;
     k_z_fwd<N><<<R::TILES, R::NT, R::SMEM, st>>>(p->tw, p->rho, p->rk);
     k_y_fwd<N><<<T::TILES, T::NT, T::SMEM, st>>>(p->tw, p->rk);
     k_x_solve<N><<<T::TILES, T::NT, 2 * T::SMEM, st>>>(p->tw, p->rk, cscale, p->tab, p->ak, p->ak + m);
@@ -423,12 +427,12 @@ extern "C" int sss_pm3_create(sss_ctx* ctx, int mesh_n, double box, sss_pm3** ou
     p->n = mesh_n;
     p->box = box;
     const size_t n3 = (size_t)mesh_n * mesh_n * mesh_n;
-    const size_t m = (size_t)mesh_n * mesh_n * (mesh_n / 2 + 1);
+    const size_t m = (size_t)mesh_n * mesh_n * (mesh_n / 2 + 1), mp = (size_t)mesh_n * mesh_n * pitch_of(mesh_n);
     cudaError_t e = cudaSuccess;
     e = e ? e : cudaMalloc(&p->rho, n3 * sizeof(float));
     e = e ? e : cudaMalloc(&p->lrho, n3 * sizeof(float));
-    e = e ? e : cudaMalloc(&p->rk, m * sizeof(float2));
-    e = e ? e : cudaMalloc(&p->ak, 3 * m * sizeof(float2));
+    e = e ? e : cudaMalloc(&p->rk, mp * sizeof(float2));
+    e = e ? e : cudaMalloc(&p->ak, 3 * mp * sizeof(float2));
     e = e ? e : cudaMalloc(&p->acc, 3 * n3 * sizeof(float));
     e = e ? e : cudaMalloc(&p->tab, 3 * (size_t)mesh_n * sizeof(double));
     p->tab_deconv = -1;
