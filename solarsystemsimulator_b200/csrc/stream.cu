@@ -176,8 +176,9 @@ size_t al(size_t b) { return (b + 255) / 256 * 256; }
 unsigned nb(long long n) { return (unsigned)((n + 255) / 256); }
 
 // ---------------------------------------------------------------- one sample
-// The whole sample is one cooperative launch of SAMPLE_THREADS-thread blocks,
-// all resident at once; its phases are separated by grid barriers:
+// The whole sample is one cooperative launch of SAMPLE_THREADS-thread blocks
+// (or its share of the blocks, with several samples at once), all resident;
+// its phases are separated by barriers over its blocks:
 //   cull      display coordinates, tier per body (keep = 0), tier counts of
 //             the whole sample and of each block's range of bodies
 //   (plan)    every block reads the tier counts and takes the reference's
@@ -244,7 +245,7 @@ struct SampleArgs {
     int* counts;                                    // 2 x K2 cell counts, one table per filter slot
     double* rate;                                   // K2 keep rates per cell
     double* part;                                   // 2 x CAND x GROUPS group sums
-    long long* blk;                                 // BLK x gridDim.x: per block of bodies, its tier counts, kept counts
+    long long* blk;                                 // BLK x nb: per block of bodies, its tier counts, kept counts
     unsigned* sel;
     unsigned short* ox;
     unsigned short* oy;
@@ -253,6 +254,20 @@ struct SampleArgs {
     int* vkey;                                      // 2 x VALUE_SLOTS: count value >= VDIR, -1 empty
     unsigned* vmul;                                 // 2 x VALUE_SLOTS: cells holding it
     double* vpre;                                   // 2 VALUE_MAX: prefix sums of the sorted values
+    unsigned nb, bid;                               // blocks of this sample, this block's number among them
+};
+
+// Samples of one launch: the grid's blocks are dealt out to them, sample g
+// taking the blocks [g nb, (g + 1) nb), its own work buffers (slot bytes after
+// the first sample's), outputs (n further) and control block.
+constexpr int SAMPLES_MAX = 8;
+
+struct SampleBatch {
+    SampleArgs s;                                   // the first sample's
+    size_t slot;
+    const float* x[SAMPLES_MAX];
+    const float* y[SAMPLES_MAX];
+    double t_cut[SAMPLES_MAX];
 };
 
 // the count tables of one filter slot (each filter of a launch has its own,
@@ -272,9 +287,9 @@ __device__ __forceinline__ Tables tables(const SampleArgs& a, int slot) {
 
 // bodies [c0, c1) of this block in the cull, keep and emit phases (c0 a
 // multiple of 8)
-__device__ __forceinline__ void body_range(long long n, long long& c0, long long& c1) {
-    const long long chunk = ((n + gridDim.x - 1) / gridDim.x + 7) / 8 * 8;
-    c0 = min((long long)blockIdx.x * chunk, n);
+__device__ __forceinline__ void body_range(const SampleArgs& a, long long& c0, long long& c1) {
+    const long long n = a.n, chunk = ((n + a.nb - 1) / a.nb + 7) / 8 * 8;
+    c0 = min((long long)a.bid * chunk, n);
     c1 = min(c0 + chunk, n);
 }
 
@@ -284,8 +299,10 @@ __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p) {
     return v;
 }
 
-// false: a wait ran out here or in another block (the caller returns)
-__device__ __forceinline__ bool grid_barrier(Ctl* ctl, unsigned& epoch, int* s_bad,
+// A barrier over the nb blocks of one sample (all blocks of the launch are
+// resident). false: a wait ran out here or in another block (the caller
+// returns)
+__device__ __forceinline__ bool grid_barrier(Ctl* ctl, unsigned nb, unsigned& epoch, int* s_bad,
                                              unsigned max_polls = BARRIER_POLLS) {
     ++epoch;
     __syncthreads();
@@ -294,7 +311,7 @@ __device__ __forceinline__ bool grid_barrier(Ctl* ctl, unsigned& epoch, int* s_b
         // block barrier) become visible with the arrival; acquire: the
         // other blocks' writes are visible once their arrivals are seen
         asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&ctl->bar) : "memory");
-        const unsigned target = epoch * gridDim.x;
+        const unsigned target = epoch * nb;
         int bad = 0;
         for (unsigned polls = 0; ld_acquire_u32(&ctl->bar) < target; ++polls) {
             if (polls >= max_polls || *(volatile int*)&ctl->err) {
@@ -367,7 +384,7 @@ struct Smem {
 // probe ends within HIST_SLOTS steps.
 __device__ void phase_hist(const SampleArgs& a, const Tables& tb, const float* qx, const float* qy, int mask,
                            Smem& sm) {
-    for (long long c0 = (long long)blockIdx.x * HIST_CHUNK; c0 < a.n; c0 += (long long)gridDim.x * HIST_CHUNK) {
+    for (long long c0 = (long long)a.bid * HIST_CHUNK; c0 < a.n; c0 += (long long)a.nb * HIST_CHUNK) {
         for (int j = threadIdx.x; j < HIST_SLOTS; j += SAMPLE_THREADS) {
             sm.u.h.key[j] = -1;
             sm.u.h.val[j] = 0;
@@ -415,9 +432,9 @@ __device__ void phase_hist(const SampleArgs& a, const Tables& tb, const float* q
 // empty cells sums to +0 for every midpoint, as its terms min(0, s * 0) = +0
 // do; in a leaf with occupied cells the +0 terms of its empty cells are added
 // like the others (exactly).
-__device__ void phase_group_sums(const Tables& tb, double lo, double hi, double* part, Smem& sm) {
+__device__ void phase_group_sums(const SampleArgs& a, const Tables& tb, double lo, double hi, double* part, Smem& sm) {
     const int leaf = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int g = blockIdx.x; g < GROUPS; g += gridDim.x) {
+    for (int g = a.bid; g < GROUPS; g += a.nb) {
         constexpr int PER_T = GROUP_CELLS / SAMPLE_THREADS;
         int cv[PER_T];
 #pragma unroll
@@ -572,15 +589,15 @@ static_assert(VALUE_SLOTS == 1 << 13, "13-bit hash");
 // tables (vdir, and vkey/vmul for the larger counts). A global table of
 // larger counts that runs out of slots sets value_over (the bisection then
 // takes the exact path).
-__device__ void phase_values(const Tables& tb, Smem& sm) {
+__device__ void phase_values(const SampleArgs& a, const Tables& tb, Smem& sm) {
     for (int j = threadIdx.x; j < VDIR; j += SAMPLE_THREADS) sm.u.v.dir[j] = 0;
     for (int j = threadIdx.x; j < LSLOTS; j += SAMPLE_THREADS) {
         sm.u.v.lkey[j] = -1;
         sm.u.v.lval[j] = 0;
     }
     __syncthreads();
-    const long long per = (K2 + gridDim.x - 1) / gridDim.x;
-    const long long c0 = (long long)blockIdx.x * per, c1 = min(c0 + per, (long long)K2);
+    const long long per = (K2 + a.nb - 1) / a.nb;
+    const long long c0 = (long long)a.bid * per, c1 = min(c0 + per, (long long)K2);
     for (long long c = c0 + threadIdx.x; c < c1; c += SAMPLE_THREADS) {
         const int v = __ldcg(tb.counts + c);
         if (v <= 0) continue;
@@ -901,11 +918,11 @@ __device__ bool filter(const SampleArgs& a, const float* qx, const float* qy, in
                        unsigned& epoch, Smem& sm) {
     const Tables tb = tables(a, slot);
     phase_hist(a, tb, qx, qy, mask, sm);
-    if (!grid_barrier(a.ctl, epoch, &sm.bad)) return false;
-    phase_values(tb, sm);
-    if (!grid_barrier(a.ctl, epoch, &sm.bad)) return false;
-    if (blockIdx.x == 0) block_fast_bisection(a, tb, (double)budget, sm);
-    if (!grid_barrier(a.ctl, epoch, &sm.bad)) return false;
+    if (!grid_barrier(a.ctl, a.nb, epoch, &sm.bad)) return false;
+    phase_values(a, tb, sm);
+    if (!grid_barrier(a.ctl, a.nb, epoch, &sm.bad)) return false;
+    if (a.bid == 0) block_fast_bisection(a, tb, (double)budget, sm);
+    if (!grid_barrier(a.ctl, a.nb, epoch, &sm.bad)) return false;
     // every thread reads the control words after a barrier: L1-cached loads,
     // so that one request per SM reaches their L2 line
     double lo = __ldca(&a.ctl->lohi[0]), hi = __ldca(&a.ctl->lohi[1]);
@@ -913,25 +930,25 @@ __device__ bool filter(const SampleArgs& a, const float* qx, const float* qy, in
     int left = 40 - __ldca(&a.ctl->fast_steps);
     for (int round = 0; left > 0; ++round) {
         double* part = a.part + (round & 1) * CAND * GROUPS;
-        phase_group_sums(tb, lo, hi, part, sm);
-        if (!grid_barrier(a.ctl, epoch, &sm.bad)) return false;
+        phase_group_sums(a, tb, lo, hi, part, sm);
+        if (!grid_barrier(a.ctl, a.nb, epoch, &sm.bad)) return false;
         const int levels = min(BISECT_D, left);
         phase_walk(part, (double)budget, lo, hi, levels, sm);
         left -= levels;
     }
-    const long long T = (long long)gridDim.x * SAMPLE_THREADS;
-    const long long gt = (long long)blockIdx.x * SAMPLE_THREADS + threadIdx.x;
+    const long long T = (long long)a.nb * SAMPLE_THREADS;
+    const long long gt = (long long)a.bid * SAMPLE_THREADS + threadIdx.x;
     // the keep rate of every cell: min(k, lo k ** 0.5) / k, 0 for an empty cell
     for (long long c = gt; c < K2; c += T) {
         const int k = __ldcg(tb.counts + c);
         a.rate[c] = k > 0 ? __ddiv_rn(fmin((double)k, __dmul_rn(lo, cell_weight(k))), (double)k) : 0.0;
     }
-    if (!grid_barrier(a.ctl, epoch, &sm.bad)) return false;
+    if (!grid_barrier(a.ctl, a.nb, epoch, &sm.bad)) return false;
     const unsigned char* __restrict__ tier = a.tier;
     unsigned char* __restrict__ keep = a.keep;
     const double* __restrict__ rate = a.rate;
     long long c0, c1;
-    body_range(a.n, c0, c1);
+    body_range(a, c0, c1);
     long long kept = 0;
     // two bodies per thread and pass, in three stages (loads, rate gathers,
     // decisions) so that both bodies' gathers are in flight together. A body
@@ -982,17 +999,38 @@ __device__ bool filter(const SampleArgs& a, const float* qx, const float* qy, in
     }
     kept = block_sum_ll(kept, sm.red);
     if (threadIdx.x == 0) {
-        a.blk[(size_t)blockIdx.x * BLK + 4 + slot] = kept;
+        a.blk[(size_t)a.bid * BLK + 4 + slot] = kept;
         if (kept) atomicAdd(a.ctl->kept + slot, (unsigned long long)kept);
     }
-    return grid_barrier(a.ctl, epoch, &sm.bad);
+    return grid_barrier(a.ctl, a.nb, epoch, &sm.bad);
 }
 
-__global__ void __launch_bounds__(SAMPLE_THREADS) k_sample(SampleArgs a) {
+__global__ void __launch_bounds__(SAMPLE_THREADS) k_sample(const __grid_constant__ SampleBatch p) {
     __shared__ Smem sm;
+    __shared__ SampleArgs mine;
+    if (threadIdx.x == 0) {
+        const unsigned g = blockIdx.x / p.s.nb;
+        const size_t d = g * p.slot;
+        auto at = [&](auto* q) { return (decltype(q))((char*)q + d); };
+        SampleArgs t = p.s;
+        t.bid = blockIdx.x - g * p.s.nb;
+        t.x = p.x[g];
+        t.y = p.y[g];
+        t.t_cut = p.t_cut[g];
+        t.qx = at(t.qx); t.qy = at(t.qy); t.tier = at(t.tier); t.keep = at(t.keep); t.counts = at(t.counts);
+        t.rate = at(t.rate); t.part = at(t.part); t.blk = at(t.blk); t.vdir = at(t.vdir); t.vkey = at(t.vkey);
+        t.vmul = at(t.vmul); t.vpre = at(t.vpre);
+        t.sel += (size_t)g * t.n;
+        t.ox += (size_t)g * t.n;
+        t.oy += (size_t)g * t.n;
+        t.ctl += g;
+        mine = t;
+    }
+    __syncthreads();
+    const SampleArgs& a = mine;
     unsigned epoch = 0;
-    const long long T = (long long)gridDim.x * SAMPLE_THREADS;
-    const long long gt = (long long)blockIdx.x * SAMPLE_THREADS + threadIdx.x;
+    const long long T = (long long)a.nb * SAMPLE_THREADS;
+    const long long gt = (long long)a.bid * SAMPLE_THREADS + threadIdx.x;
     const float* qx = a.log_zoom ? a.qx : a.x;
     const float* qy = a.log_zoom ? a.qy : a.y;
     // ---- cull (and clear both filter slots' count tables)
@@ -1004,7 +1042,7 @@ __global__ void __launch_bounds__(SAMPLE_THREADS) k_sample(SampleArgs a) {
     }
     for (long long c = gt; c < 2 * VDIR; c += T) a.vdir[c] = 0;
     long long c0, c1;
-    body_range(a.n, c0, c1);
+    body_range(a, c0, c1);
     for (long long i0 = c0 + threadIdx.x; i0 < c1; i0 += 4 * SAMPLE_THREADS) {
         float bx[4], by[4];
         double kt[4];
@@ -1048,14 +1086,14 @@ __global__ void __launch_bounds__(SAMPLE_THREADS) k_sample(SampleArgs a) {
         if (n1) atomicAdd(a.ctl->tier_cnt + 1, (unsigned long long)n1);
         if (n2) atomicAdd(a.ctl->tier_cnt + 2, (unsigned long long)n2);
         if (n3) atomicAdd(a.ctl->tier_cnt + 3, (unsigned long long)n3);
-        long long* rec = a.blk + (size_t)blockIdx.x * BLK;
+        long long* rec = a.blk + (size_t)a.bid * BLK;
         rec[1] = n1;
         rec[2] = n2;
         rec[3] = n3;
         rec[4] = 0;
         rec[5] = 0;
     }
-    if (!grid_barrier(a.ctl, epoch, &sm.bad)) return;
+    if (!grid_barrier(a.ctl, a.nb, epoch, &sm.bad)) return;
     // ---- plan (the reference's _lod_auswahl), identical in every block
     // (every thread reads the counts: L1-cached loads, one L2 request per SM)
     const long long mm = (long long)__ldca(a.ctl->tier_cnt + 1), ma = (long long)__ldca(a.ctl->tier_cnt + 2),
@@ -1108,7 +1146,7 @@ __global__ void __launch_bounds__(SAMPLE_THREADS) k_sample(SampleArgs a) {
     // 0 .. b - 1. A block emits its kept bodies and its bodies of the tiers
     // in all_mask (never a filtered tier): its record holds both numbers.
     long long before = 0;
-    for (int j = threadIdx.x; j < (int)blockIdx.x; j += SAMPLE_THREADS) {
+    for (int j = threadIdx.x; j < (int)a.bid; j += SAMPLE_THREADS) {
         const long long* rec = a.blk + (size_t)j * BLK;
         long long e = __ldca(rec + 4) + __ldca(rec + 5);            // (read by every later block: L1-cached)
 #pragma unroll
@@ -1187,7 +1225,7 @@ __global__ void __launch_bounds__(SAMPLE_THREADS) k_sample(SampleArgs a) {
         off += all;
         __syncthreads();                            // wcnt is rewritten by the next sub-range
     }
-    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) a.ctl->total = off;
+    if (a.bid == a.nb - 1 && threadIdx.x == 0) a.ctl->total = off;
 }
 
 struct Work {
@@ -1200,12 +1238,14 @@ struct Work {
     unsigned* vmul;
     double* vpre;
     long long* blk;
+    size_t slot;                                    // bytes from one sample's buffers to the next one's
     Ctl* ctl;
 };
 
-// scratch of a sample (reused by the samples of a batch, which run in
-// stream order) and n_ctl control blocks (one per sample of a batch)
-int make_work(sss_ctx* ctx, long long n, int grid, int n_ctl, Work* W) {
+// scratch of the `slots` samples that run at once (reused by the following
+// ones of a batch in stream order) and n_ctl control blocks (one per sample
+// of the batch)
+int make_work(sss_ctx* ctx, long long n, int grid, int slots, int n_ctl, Work* W) {
     size_t off = 0;
     const size_t o_qx = off; off += al((size_t)n * 4);
     const size_t o_qy = off; off += al((size_t)n * 4);
@@ -1219,6 +1259,8 @@ int make_work(sss_ctx* ctx, long long n, int grid, int n_ctl, Work* W) {
     const size_t o_vmul = off; off += al((size_t)2 * VALUE_SLOTS * 4);
     const size_t o_vpre = off; off += al((size_t)2 * (VALUE_MAX + 1) * 8);
     const size_t o_blk = off; off += al((size_t)grid * BLK * 8);
+    W->slot = off;
+    off *= (size_t)slots;
     const size_t o_ctl = off; off += al(sizeof(Ctl) * (size_t)n_ctl);
     void* scr = nullptr;
     int rc = sss_scratch(ctx, off, &scr);
@@ -1273,7 +1315,7 @@ extern "C" int sss_stream_minmax(sss_ctx* ctx, int64_t n, const float* x, const 
     if (n < 1 || !x || !y || !out4) return sss_set_err(ctx, SSS_ERR_ARG, "minmax: empty or NULL input");
     cudaStream_t st = (cudaStream_t)stream;
     Work W;
-    int rc = make_work(ctx, n, 1, 1, &W);
+    int rc = make_work(ctx, n, 1, 1, 1, &W);
     if (rc) return rc;
     const float* qx = x;
     const float* qy = y;
@@ -1303,8 +1345,15 @@ extern "C" int sss_stream_minmax(sss_ctx* ctx, int64_t n, const float* x, const 
 
 namespace {
 
-// k samples of the same bodies, one cooperative launch each in stream
-// order, one readback of the k counts at the end
+// k samples of the same bodies, up to SAMPLES_MAX to a cooperative launch,
+// the launches in stream order, one readback of the k counts at the end.
+// A sample alone is bound by its phases' latency (about a dozen barriers, one
+// block's bisection, first touches of memory): with the whole grid to each of
+// 8 samples of a million bodies in turn 51 us a sample, with 37 blocks to each
+// of the 8 at once 30. Their buffers (14 bytes a body, 5 MB
+// of tables) are held to SLOTS_BYTES.
+constexpr size_t SLOTS_BYTES = (size_t)256 << 20;
+
 int sample_batch(sss_ctx* ctx, int64_t n, int k, const float* const* x, const float* const* y,
                  const double* kill_t, const double* t_cut, const unsigned char* is_ast,
                  const unsigned char* injected, const double* box, int log_zoom, int64_t budget, unsigned* sel,
@@ -1324,9 +1373,14 @@ int sample_batch(sss_ctx* ctx, int64_t n, int k, const float* const* x, const fl
     int rc = sample_grid(ctx, &grid);
     if (rc) return rc;
     Work W;
-    rc = make_work(ctx, n, grid, k, &W);
+    int at_once = std::min(k, SAMPLES_MAX);
+    const size_t one = (size_t)n * 10 + (size_t)K2 * 16 + ((size_t)1 << 19);
+    while (at_once > 1 && (size_t)at_once * one > SLOTS_BYTES) --at_once;
+    rc = make_work(ctx, n, grid, at_once, k, &W);
     if (rc) return rc;
-    SampleArgs a;
+    SampleBatch p;
+    SampleArgs& a = p.s;
+    p.slot = W.slot;
     a.kill_t = kill_t;
     a.is_ast = is_ast;
     a.injected = injected;
@@ -1352,7 +1406,14 @@ int sample_batch(sss_ctx* ctx, int64_t n, int k, const float* const* x, const fl
     a.vmul = W.vmul;
     a.vpre = W.vpre;
     SSS_CUDA_TRY(ctx, cudaMemsetAsync(W.ctl, 0, sizeof(Ctl) * (size_t)k, st));
-    for (int i = 0; i < k; ++i) {
+    a.bid = 0;
+    for (int i = 0; i < k; i += at_once) {
+        const int m = std::min(at_once, k - i);
+        for (int g = 0; g < m; ++g) {
+            p.x[g] = x[i + g];
+            p.y[g] = y[i + g];
+            p.t_cut[g] = t_cut[i + g];
+        }
         a.x = x[i];
         a.y = y[i];
         a.t_cut = t_cut[i];
@@ -1360,9 +1421,10 @@ int sample_batch(sss_ctx* ctx, int64_t n, int k, const float* const* x, const fl
         a.ox = qx_out + (size_t)i * n;
         a.oy = qy_out + (size_t)i * n;
         a.ctl = W.ctl + i;
-        void* params[] = {&a};
-        SSS_CUDA_TRY(ctx, cudaLaunchCooperativeKernel((const void*)k_sample, dim3(grid), dim3(SAMPLE_THREADS), params,
-                                                      0, st));
+        a.nb = (unsigned)(grid / m);
+        void* params[] = {&p};
+        SSS_CUDA_TRY(ctx, cudaLaunchCooperativeKernel((const void*)k_sample, dim3(a.nb * m), dim3(SAMPLE_THREADS),
+                                                      params, 0, st));
     }
     Ctl hbuf[16];
     Ctl* h = k <= 16 ? hbuf : new Ctl[k];
@@ -1411,7 +1473,7 @@ __global__ void k_sample_barrier_selftest(Ctl* ctl, unsigned max_polls, int* sta
     __shared__ int bad;
     unsigned epoch = 0;
     if (blockIdx.x != 0) return;
-    if (!grid_barrier(ctl, epoch, &bad, max_polls) && threadIdx.x == 0)
+    if (!grid_barrier(ctl, gridDim.x, epoch, &bad, max_polls) && threadIdx.x == 0)
         atomicCAS(status, SSS_OK, *(volatile int*)&ctl->err);
 }
 

@@ -259,3 +259,26 @@ def test_count_histogram_paths(name):
     assert np.array_equal(sel.view(np.uint32), rs)
     assert np.array_equal(qx.view(np.uint16), rx) and np.array_equal(qy.view(np.uint16), ry)
     assert 80_000 < len(rs) <= 120_000
+
+
+@pytest.mark.parametrize("n,k,log_zoom", [(1, 3, False), (37, 9, True), (5_001, 2, False), (70_001, 8, True),
+                                          (200_003, 17, False), (3_100_000, 8, False)])
+def test_samples_at_once_equal_single_samples(n, k, log_zoom):
+    """Batches whose samples share one launch: fewer bodies than blocks, odd
+    counts, one more than a launch holds, and buffers large enough that fewer
+    than eight run at once. Every sample as its single-sample call."""
+    from solarsystemsimulator_b200.stream import StreamFrames
+    x, y, a, inj, kill_t = _scene(min(n, 20), n - min(n, 20) - n // 10, n // 10, seed=n)
+    sf = StreamFrames(a, inj)
+    sf.kill_t = torch.as_tensor(kill_t).cuda()
+    rng = np.random.default_rng(k)
+    shift = rng.normal(0, 1e-2, (2, k)).astype(np.float32)
+    xs = [torch.as_tensor(x + shift[0, s]).cuda() for s in range(k)]
+    ys = [torch.as_tensor(y + shift[1, s]).cuda() for s in range(k)]
+    ts = [0.1 * s - 0.5 for s in range(k)]
+    box = sf.box(xs[0], ys[0], (0.0, 0.0, -1.0, -1.0) if log_zoom else (0.0, 0.0, 2.0, 2.0), log_zoom)
+    budget = max(1, n // 8)
+    batch = [tuple(t.cpu().numpy() for t in r) for r in sf.sample_batch(xs, ys, ts, 0.1, box, log_zoom, budget)]
+    for s in range(k):
+        single = [t.cpu().numpy() for t in sf.sample(xs[s], ys[s], ts[s], 0.1, box, log_zoom, budget)]
+        assert all(np.array_equal(p, q) for p, q in zip(batch[s], single))
