@@ -230,32 +230,30 @@ __global__ void __launch_bounds__(RS_NT) k_rs_pass(const unsigned long long* __r
                                                   unsigned long long* __restrict__ keys_out,
                                                   unsigned* __restrict__ vals_out, int* err) {
     constexpr int NW = RS_NT / 32;
-    __shared__ unsigned s_wcnt[NW][RS_BINS];
+    __shared__ unsigned s_wcnt[NW][RS_BINS];   // per warp: its keys of each digit, then those of the warps before it
     __shared__ long long s_base[RS_BINS];
-    __shared__ unsigned s_cnt[RS_BINS];
     __shared__ unsigned s_tile;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (tid == 0) s_tile = atomicAdd(ticket, 1u);
-    s_cnt[tid] = 0;
+    for (int t = tid; t < NW * RS_BINS; t += RS_NT) (&s_wcnt[0][0])[t] = 0;
     __syncthreads();
     const long long tile = s_tile;
-    const long long base = tile * RS_TILE;
+    // a warp's keys are consecutive: it ranks its own without the others, and the tile needs one
+    // pass over the warps' counts (ranking row by row of the tile took 24 block barriers)
+    const long long base = tile * RS_TILE + (long long)warp * (32 * RS_ITEMS) + lane;
     const unsigned long long hc = hist[tid];
-    long long tot;
-    const long long goff = block_exclusive_scan((long long)hc, &tot);   // digit tid's first output position
-    const bool trivial = __syncthreads_or(hc == (unsigned long long)n);
     unsigned long long key[RS_ITEMS];
     unsigned val[RS_ITEMS];
 #pragma unroll
     for (int k = 0; k < RS_ITEMS; ++k) {
-        const long long i = base + (long long)k * RS_NT + tid;
+        const long long i = base + k * 32;
         key[k] = i < n ? keys_in[i] : 0ull;
         val[k] = i < n ? vals_in[i] : 0u;
     }
-    if (trivial) {   // every key has the same digit: the pass keeps the order
+    if (__syncthreads_or(hc == (unsigned long long)n)) {   // every key has the same digit: the pass keeps the order
 #pragma unroll
         for (int k = 0; k < RS_ITEMS; ++k) {
-            const long long i = base + (long long)k * RS_NT + tid;
+            const long long i = base + k * 32;
             if (i < n) {
                 keys_out[i] = key[k];
                 vals_out[i] = val[k];
@@ -263,12 +261,30 @@ __global__ void __launch_bounds__(RS_NT) k_rs_pass(const unsigned long long* __r
         }
         return;
     }
+    long long tot;
+    const long long goff = block_exclusive_scan((long long)hc, &tot);   // digit tid's first output position
+    const unsigned lt = (1u << lane) - 1u;
+    unsigned rank[RS_ITEMS];                   // among the warp's keys of this digit
 #pragma unroll
-    for (int k = 0; k < RS_ITEMS; ++k)
-        if (base + (long long)k * RS_NT + tid < n) atomicAdd(&s_cnt[digit_of(key[k], shift)], 1u);
+    for (int k = 0; k < RS_ITEMS; ++k) {
+        const bool valid = base + k * 32 < n;
+        const unsigned d = valid ? digit_of(key[k], shift) : RS_BINS;   // RS_BINS = no element
+        const unsigned peers = __match_any_sync(0xffffffffu, d);
+        const unsigned before = valid ? s_wcnt[warp][d] : 0u;
+        rank[k] = before + __popc(peers & lt);
+        __syncwarp();
+        if (valid && (peers & lt) == 0) s_wcnt[warp][d] = before + __popc(peers);
+        __syncwarp();
+    }
     __syncthreads();
     // digit tid: publish this tile's count, look back for the count before it
-    const unsigned long long c = s_cnt[tid];
+    unsigned long long c = 0;
+#pragma unroll
+    for (int w = 0; w < NW; ++w) {
+        const unsigned q = s_wcnt[w][tid];
+        s_wcnt[w][tid] = (unsigned)c;
+        c += q;
+    }
     unsigned long long excl = 0;
     volatile unsigned long long* mine = status + tile * RS_BINS + tid;
     if (tile > 0) {
@@ -284,29 +300,14 @@ __global__ void __launch_bounds__(RS_NT) k_rs_pass(const unsigned long long* __r
     }
     *mine = (excl + c) | RS_FLAG_INC;
     s_base[tid] = goff + (long long)excl;
-    const unsigned lt = (1u << lane) - 1u;
+    __syncthreads();
+#pragma unroll
     for (int k = 0; k < RS_ITEMS; ++k) {
-        for (int t = tid; t < NW * RS_BINS; t += RS_NT) (&s_wcnt[0][0])[t] = 0;
-        __syncthreads();
-        const long long i = base + (long long)k * RS_NT + tid;
-        const bool valid = i < n;
-        const unsigned d = valid ? digit_of(key[k], shift) : RS_BINS;   // RS_BINS = no element
-        const unsigned peers = __match_any_sync(0xffffffffu, d);
-        const unsigned rank = __popc(peers & lt);
-        if (valid && rank == 0) s_wcnt[warp][d] = __popc(peers);
-        __syncthreads();
-        if (valid) {
-            long long pos = s_base[d] + rank;
-            for (int w = 0; w < warp; ++w) pos += s_wcnt[w][d];
-            keys_out[pos] = key[k];
-            vals_out[pos] = val[k];
-        }
-        __syncthreads();
-        {
-            unsigned add = 0;
-            for (int w = 0; w < NW; ++w) add += s_wcnt[w][tid];
-            s_base[tid] += add;
-        }
+        if (base + k * 32 >= n) continue;
+        const unsigned d = digit_of(key[k], shift);
+        const long long pos = s_base[d] + s_wcnt[warp][d] + rank[k];
+        keys_out[pos] = key[k];
+        vals_out[pos] = val[k];
     }
 }
 
