@@ -494,6 +494,11 @@ __device__ __forceinline__ void queue_push(PairQueue& q, unsigned m, bool need, 
     }
 }
 
+// Bounding box of a tile's run bodies: positions, velocities, largest radius.
+struct RunBox {
+    float x0, x1, y0, y1, u0, u1, w0, w1, rr;
+};
+
 // The partners [j0, j0 + nj) of one surviving chunk against the lane's run
 // body (valid = false: the lane has none). Keep rule on body indices:
 // MODE 0: offset (0, 0), keep a < b; MODE 1: another offset whose key
@@ -505,8 +510,8 @@ __device__ __forceinline__ void queue_push(PairQueue& q, unsigned m, bool need, 
 // for c <= 0.
 template <int MODE>
 __device__ __forceinline__ void span_walk(const TileArgs& a, int o, const Body& A, unsigned ab, bool valid,
-                                          long long j0, int nj, float E, float kl, bool skip_ok, PairQueue& q,
-                                          int lane) {
+                                          long long j0, int nj, float E, float kl, bool skip_ok, const RunBox& R,
+                                          float brr, float dtf, PairQueue& q, int lane) {
     const float4* rp = a.rec + j0;
     const uint2* rp2 = a.rec2 + j0;
     auto keep_of = [&](int k) {
@@ -522,36 +527,46 @@ __device__ __forceinline__ void span_walk(const TileArgs& a, int o, const Body& 
         }
         return;
     }
-    int k = 0;
-    for (; k + 4 <= nj; k += 4) {
+    // the chunk skip's rule for each partner by itself (a box of one body): one lane a partner
+    unsigned pm = 0;
+    {
+        bool near = false;
+        if (lane < nj) {
+            const float4 v = __ldg(rp + lane);
+            const float dxb = fmaxf(0.0f, fmaxf(v.x - R.x1, R.x0 - v.x));
+            const float dyb = fmaxf(0.0f, fmaxf(v.y - R.y1, R.y0 - v.y));
+            const float Vx = fmaxf(v.z - R.u0, R.u1 - v.z), Vy = fmaxf(v.w - R.w0, R.w1 - v.w);
+            const float reach = (Vx + Vy) * 1.0001f * dtf + ((R.rr + 1e-6f) + brr);
+            near = !(reach < 1.0f && dxb * dxb + dyb * dyb > 4.01f * reach * reach);
+        }
+        pm = __ballot_sync(0xffffffffu, near);
+    }
+    while (pm) {
+        int ks[4];
         float4 v[4];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) v[u] = __ldg(rp + k + u);
+        for (int u = 0; u < 4; ++u) {
+            ks[u] = __ffs(pm) - 1;                     // -1: no partner left
+            pm &= pm - 1;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) v[u] = __ldg(rp + max(ks[u], 0));
         bool need[4];
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
             const float dpx = v[u].x - A.x, dpy = v[u].y - A.y;
             const float dvx = v[u].z - A.vx, dvy = v[u].w - A.vy;
             const float c = fabsf(dpx * dvy - dpy * dvx) - E;
-            need[u] = valid && !(c * fabsf(c) > kl * (dvx * dvx + dvy * dvy)) && keep_of(k + u);
+            need[u] = valid && ks[u] >= 0 && !(c * fabsf(c) > kl * (dvx * dvx + dvy * dvy)) && keep_of(max(ks[u], 0));
         }
         const unsigned any = __ballot_sync(0xffffffffu, need[0] || need[1] || need[2] || need[3]);
         if (any) {
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
                 const unsigned m = __ballot_sync(0xffffffffu, need[u]);
-                if (m) queue_push(q, m, need[u], (int)(j0 + k + u), a, o, A, ab, lane);
+                if (m) queue_push(q, m, need[u], (int)(j0 + ks[u]), a, o, A, ab, lane);
             }
         }
-    }
-    for (; k < nj; ++k) {
-        const float4 v = __ldg(rp + k);
-        const float dpx = v.x - A.x, dpy = v.y - A.y;
-        const float dvx = v.z - A.vx, dvy = v.w - A.vy;
-        const float c = fabsf(dpx * dvy - dpy * dvx) - E;
-        const bool need = valid && !(c * fabsf(c) > kl * (dvx * dvx + dvy * dvy)) && keep_of(k);
-        const unsigned m = __ballot_sync(0xffffffffu, need);
-        if (m) queue_push(q, m, need, (int)(j0 + k), a, o, A, ab, lane);
     }
 }
 
@@ -570,7 +585,10 @@ __device__ __forceinline__ void span_walk(const TileArgs& a, int o, const Body& 
 // |dp| > 2 ((|dvx| + |dvy|) dt + rs), so its closest approach over t in
 // [-dt, dt] exceeds 2 rs: the f32 test rejects it (its own rounding below
 // 1e-7 AU while the boxes' extents P and V dt stay below 0.5 AU, rs >= 1e-6
-// AU); 4.01 for 4 covers the rounding of the box arithmetic.
+// AU); 4.01 for 4 covers the rounding of the box arithmetic. In a chunk that
+// survives, the same rule skips single partners (its P and V, below 0.5 AU,
+// and its largest radius hold for each of them), so the line test runs on
+// those near the run bodies' box only.
 __global__ void __launch_bounds__(BP_NT, 3) k_tiles(const TileArgs a_in) {
     TileArgs a = a_in;
     a.tp.dtf = a_in.P->dtf;
@@ -623,6 +641,7 @@ __global__ void __launch_bounds__(BP_NT, 3) k_tiles(const TileArgs a_in) {
             const float aw0 = warp_min(valid ? A.vy : INFINITY), aw1 = warp_max(valid ? A.vy : -INFINITY);
             float arr = valid ? A.rr : 0.0f;
             for (int d = 16; d; d >>= 1) arr = nan_max(arr, __shfl_xor_sync(0xffffffffu, arr, d));
+            const RunBox R{ax0, ax1, ay0, ay1, au0, au1, aw0, aw1, arr};
             const long long jb = b0 + bi * TILE_B;
             const long long je = min(jb + TILE_B, b0 + nb);
             const long long c0 = jb >> 5;
@@ -660,9 +679,9 @@ __global__ void __launch_bounds__(BP_NT, 3) k_tiles(const TileArgs a_in) {
                 const float kl = 4.01f * rs * rs;
                 const long long cs = (c0 + c) << 5;
                 const long long js = max(cs, jb), jn = min(cs + 32, je);
-                if (mode == 0) span_walk<0>(a, o, A, ab, valid, js, (int)(jn - js), E, kl, skip_ok, q, lane);
-                else if (mode == 1) span_walk<1>(a, o, A, ab, valid, js, (int)(jn - js), E, kl, skip_ok, q, lane);
-                else span_walk<2>(a, o, A, ab, valid, js, (int)(jn - js), E, kl, skip_ok, q, lane);
+                if (mode == 0) span_walk<0>(a, o, A, ab, valid, js, (int)(jn - js), E, kl, skip_ok, R, br, dtf, q, lane);
+                else if (mode == 1) span_walk<1>(a, o, A, ab, valid, js, (int)(jn - js), E, kl, skip_ok, R, br, dtf, q, lane);
+                else span_walk<2>(a, o, A, ab, valid, js, (int)(jn - js), E, kl, skip_ok, R, br, dtf, q, lane);
             }
             if (q.cnt > 0) {                               // the rest of the tile's queue
                 queue_flush(q, q.cnt, a, o, A, ab, lane);
