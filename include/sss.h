@@ -230,6 +230,14 @@ int sss_broadphase(sss_ctx* ctx, const float* x, const float* y, const float* vx
  * each ascending in (a, b) (film_producer.py:255-290); n = the bodies of the
  * call (a, b < n < 2^30) */
 int sss_broadphase_order(sss_ctx* ctx, int* hits, int64_t k, int64_t n, void* stream);
+/* the f32 speeds hypot(vx, vy) of the bodies with is_ast and vis set, sorted:
+ * their count and what a linear percentile at fraction q (f32) of them reads,
+ * out3 (host) = the largest (NaN if there is one) and those at floor(vi) and
+ * floor(vi) + 1, vi = (count - 1) q in f32 (0 where vi >= count - 1);
+ * synchronous (the cell size of bounce_suche, film_producer.py:357-359) */
+int sss_broadphase_speeds(sss_ctx* ctx, const float* vx, const float* vy, const unsigned char* is_ast,
+                          const unsigned char* vis, int64_t n, float q, int64_t* n_alive, float* out3,
+                          void* stream);
 
 /* ------------------------------------------------------ particle mesh, 2-D
  *

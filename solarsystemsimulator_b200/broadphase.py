@@ -153,16 +153,47 @@ def percentile_linear(sorted_vals, q: float) -> float:
         got = torch.stack([sorted_vals[i] for i in need]).cpu().numpy().astype(f32)
     else:
         got = np.asarray(sorted_vals)[need].astype(f32)
+    return _interpolate(got, n, vi)
+
+
+def _interpolate(got, n: int, vi) -> float:
+    """The percentile from the largest value and the two neighbours of the
+    virtual index vi (f32) among n."""
+    f32 = np.float32
     if np.isnan(got[0]):
         return float("nan")
     if vi >= n - 1:
         return float(got[0])
     a, b = got[1], got[2]
-    t = vi - lo
+    t = vi - np.floor(vi)
     d = b - a
     if t >= 0.5:
         return float(b - d * (f32(1) - t))
     return float(a + d * t)
+
+
+def _alive_and_cell(card, gvx, gvy, dt_y: float):
+    """(number of living asteroids, search_cell of them): one native call and
+    one readback (sss_broadphase_speeds)."""
+    dev = torch.device("cuda", card.dev)
+    vx, vy = _dev_f32(gvx, dev), _dev_f32(gvy, dev)
+    n = card.g_ast.numel()
+    vis = torch.ones_like(card.g_ast) if card.g_vis is None else card.g_vis
+    if vx.numel() != n or vy.numel() != n or vis.numel() != n:
+        alive = (card.g_ast != 0) & (vis != 0)              # raises as indexing by the mask does
+        return int(alive.sum()), search_cell(gvx, gvy, alive, dt_y)
+    q = np.float32(95) / np.float32(100)
+    cnt, got = ctypes.c_int64(), (ctypes.c_float * 3)()
+    ctx = _lib.context(card.dev)
+    with torch.cuda.device(card.dev):
+        ctx.check(ctx.lib.sss_broadphase_speeds(ctx.ptr, vx.data_ptr(), vy.data_ptr(), card.g_ast.data_ptr(),
+                                                vis.data_ptr(), n, float(q), ctypes.byref(cnt), got,
+                                                ctypes.c_void_p(_lib.stream_handle(card.dev))))
+    k = int(cnt.value)
+    if k < 2:
+        return k, 0.0
+    v95 = _interpolate(np.array(got, np.float32), k, np.float32(k - 1) * q)
+    return k, max(1e-4, 2.0 * v95 * dt_y)
 
 
 def search_cell(gvx, gvy, alive, dt_y: float) -> float:
@@ -193,10 +224,9 @@ def bounce_suche(det, det_pool, rows, dt_y: float, rr_max: float, anteile=None):
     shares = list(anteile) if anteile is not None and len(anteile) == n_rows else [1.0 / n_rows] * n_rows
     card = det[0]
     gx, gy, gvx, gvy = rows[0]
-    alive = (card.g_ast != 0) & (card.g_vis != 0)
-    if int(alive.sum()) < 2:
+    alive, h = _alive_and_cell(card, gvx, gvy, dt_y)
+    if alive < 2:
         return None, 0, 0.0, shares
-    h = search_cell(gvx, gvy, alive, dt_y)
     card.streifen(-np.inf, np.inf)
     hits, cand = card.bounce_hits(gx, gy, gvx, gvy, dt_y, h, 2.0 * h + 2.0 * rr_max)
     return hits, cand, h, shares

@@ -708,6 +708,51 @@ __global__ void k_hit_gather(const Hit* __restrict__ in, const unsigned* __restr
     if (i < k) out[i] = in[order[i]];
 }
 
+// Sort keys of the f32 speeds of the alive bodies (film_producer.py:357-359):
+// squares exact in f64, one rounded sum and square root, rounded to f32; the
+// bits of a speed >= 0 order as the speed, NaN after every number, bodies that
+// are not alive after that. cnt += the alive ones.
+__global__ void __launch_bounds__(256) k_speed_keys(const float* __restrict__ vx, const float* __restrict__ vy,
+                                                    const unsigned char* __restrict__ is_ast,
+                                                    const unsigned char* __restrict__ vis, long long n,
+                                                    unsigned long long* __restrict__ key,
+                                                    unsigned* __restrict__ val, unsigned long long* __restrict__ cnt) {
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    bool on = false;
+    if (i < n) {
+        on = is_ast[i] && vis[i];
+        const double x = vx[i], y = vy[i];
+        const float v = __double2float_rn(__dsqrt_rn(__dadd_rn(__dmul_rn(x, x), __dmul_rn(y, y))));
+        key[i] = !on ? 0xFFFFFFFFull : v != v ? 0x7FFFFFFFull : (unsigned long long)__float_as_uint(v);
+        val[i] = (unsigned)i;
+    }
+    const int c = __syncthreads_count(on);
+    if (threadIdx.x == 0 && c) atomicAdd(cnt, (unsigned long long)c);
+}
+
+// The sorted speeds a linear percentile reads: the last one, and those at
+// floor(vi) and floor(vi) + 1 with vi = (n - 1) q in f32 (only where vi < n - 1).
+struct SpeedPick {
+    long long n;
+    float last, lo, hi;
+};
+
+__global__ void k_speed_pick(const unsigned long long* __restrict__ key, const unsigned long long* __restrict__ cnt,
+                             float q, SpeedPick* __restrict__ out) {
+    const long long n = (long long)*cnt;
+    SpeedPick r{n, 0.f, 0.f, 0.f};
+    if (n > 0) {
+        const float top = __ll2float_rn(n - 1), vi = __fmul_rn(top, q);
+        r.last = __uint_as_float((unsigned)key[n - 1]);
+        if (vi < top) {
+            const long long lo = min((long long)floorf(vi), n - 1);
+            r.lo = __uint_as_float((unsigned)key[lo]);
+            r.hi = __uint_as_float((unsigned)key[min(lo + 1, n - 1)]);
+        }
+    }
+    *out = r;
+}
+
 // The call's inputs into the staging arrays the captured pipeline reads.
 __global__ void k_bp_stage(const float* __restrict__ x, const float* __restrict__ y, const float* __restrict__ vx,
                            const float* __restrict__ vy, const float* __restrict__ rr,
@@ -1016,5 +1061,47 @@ extern "C" int sss_broadphase_order(sss_ctx* ctx, int* hits, int64_t k, int64_t 
     SSS_CUDA_TRY(ctx, cudaMemcpyAsync(tmp, hits, 12 * (size_t)k, cudaMemcpyDeviceToDevice, s));
     k_hit_gather<<<nb, 256, 0, s>>>(tmp, v0, k, (Hit*)hits);
     SSS_LAUNCH_CHECK(ctx, "k_hit_gather");
+    return SSS_OK;
+}
+
+extern "C" int sss_broadphase_speeds(sss_ctx* ctx, const float* vx, const float* vy, const unsigned char* is_ast,
+                                     const unsigned char* vis, int64_t n, float q, int64_t* n_alive, float* out3,
+                                     void* stream) {
+    if (!ctx) return SSS_ERR_ARG;
+    if (!n_alive || !out3) return sss_set_err(ctx, SSS_ERR_ARG, "NULL output");
+    *n_alive = 0;
+    out3[0] = out3[1] = out3[2] = 0.0f;
+    if (n < 0 || !(q >= 0.0f && q <= 1.0f)) return sss_set_err(ctx, SSS_ERR_ARG, "speeds: bad size or fraction");
+    if (n >= ((int64_t)1 << 31)) return sss_set_err(ctx, SSS_ERR_ARG, "too many bodies");
+    if (n == 0) return SSS_OK;
+    if (!vx || !vy || !is_ast || !vis) return sss_set_err(ctx, SSS_ERR_ARG, "NULL input");
+    SSS_CUDA_TRY(ctx, cudaSetDevice(ctx->device));
+    cudaStream_t s = (cudaStream_t)stream;
+    size_t off = 0;
+    auto take = [&](size_t bytes) { const size_t o = off; off += (bytes + 255) & ~(size_t)255; return o; };
+    const size_t o_k0 = take(8 * n), o_k1 = take(8 * n), o_v0 = take(4 * n), o_v1 = take(4 * n);
+    const size_t o_rs = take(8 * sss_dev::radix_scratch(n)), o_cnt = take(8), o_out = take(sizeof(SpeedPick));
+    void* scr = nullptr;
+    int rc = sss_scratch(ctx, off, &scr);
+    if (rc) return rc;
+    char* S = (char*)scr;
+    unsigned long long* k0 = (unsigned long long*)(S + o_k0);
+    unsigned* v0 = (unsigned*)(S + o_v0);
+    unsigned long long* cnt = (unsigned long long*)(S + o_cnt);
+    SpeedPick* out = (SpeedPick*)(S + o_out);
+    SSS_CUDA_TRY(ctx, cudaMemsetAsync(cnt, 0, sizeof(*cnt), s));
+    k_speed_keys<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(vx, vy, is_ast, vis, n, k0, v0, cnt);
+    SSS_LAUNCH_CHECK(ctx, "k_speed_keys");
+    SSS_CUDA_TRY(ctx, sss_dev::radix_sort(k0, v0, (unsigned long long*)(S + o_k1), (unsigned*)(S + o_v1), n,
+                                          (long long*)(S + o_rs), s, ctx->d_status, 32));
+    k_speed_pick<<<1, 1, 0, s>>>(k0, cnt, q, out);
+    SSS_LAUNCH_CHECK(ctx, "k_speed_pick");
+    SpeedPick h;
+    SSS_CUDA_TRY(ctx, cudaMemcpyAsync(&h, out, sizeof(h), cudaMemcpyDeviceToHost, s));
+    SSS_CUDA_TRY(ctx, cudaStreamSynchronize(s));
+    *n_alive = h.n;
+    out3[0] = h.last;
+    out3[1] = h.lo;
+    out3[2] = h.hi;
     return SSS_OK;
 }

@@ -7,6 +7,7 @@ degenerate inputs). Mirrors the reference's test_erkennung_streifen.py.
 """
 import numpy as np
 import pytest
+import torch
 
 from oracle import broadphase as obp
 
@@ -283,3 +284,28 @@ def test_one_alive_body_among_many():
     x2 = np.concatenate([np.full(n - 1, 50.0, np.float32), np.array([1.0], np.float32)])
     assert bp.bounce_hits(x2, x2, x2, x2, 0.01, 0.1, 0.2, rr=rr, lo=0.0, hi=2.0) == \
         obp.hits(x2, x2, x2, x2, rr, 0.01, 0.1, 0.2, lo=0.0, hi=2.0) == (None, 0)
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 21, 257, 2049, 50_000])
+@pytest.mark.parametrize("kind", ["normal", "ties", "nan", "inf", "mostly_hidden"])
+def test_cell_of_the_native_percentile(n, kind):
+    """The cell size of one native call (count and percentile of the living
+    asteroids' speeds) equals search_cell's on the same mask, bit for bit."""
+    from solarsystemsimulator_b200 import broadphase as bp
+    rng = np.random.default_rng(n)
+    vx, vy = rng.normal(0, 1, (2, n)).astype(np.float32)
+    if kind == "ties":
+        vx, vy = np.round(vx), np.round(vy)
+    vis = rng.uniform(0, 1, n) > (0.9 if kind == "mostly_hidden" else 0.1)
+    if kind in ("nan", "inf"):
+        vx[n // 2] = np.nan if kind == "nan" else np.inf
+        vis[n // 2] = True
+    ast = rng.uniform(0, 1, n) > 0.05
+    card = bp.Erkennungskarte(0, ast, -np.inf, np.inf)
+    card.stammdaten(vis, np.zeros(n))
+    alive = (card.g_ast != 0) & (card.g_vis != 0)
+    k, h = bp._alive_and_cell(card, vx, torch.as_tensor(vy).cuda(), 0.5)
+    assert k == int(alive.sum())
+    if k >= 2:
+        want = bp.search_cell(vx, vy, alive, 0.5)
+        assert h == want or (np.isnan(h) and np.isnan(want))
