@@ -63,9 +63,6 @@ constexpr int WS_R_F64 = 2, WS_R_MIX = 4;
 constexpr int WS_MINB_F64 = 4, WS_MINB_MIX = 2;
 constexpr double SPLIT_PAIRS_F64 = 3e8, SPLIT_PAIRS_MIX = 4.5e8;
 
-// r2 below this is outside the integer-seeded rsqrt's range (2^-126)
-constexpr double kIseedMinR2 = 1.1754943508222875e-38;
-
 using sss_ap::Epi;
 using sss_ap::epilogue;
 
@@ -145,31 +142,15 @@ __device__ __noinline__ void drain_after_abort(uint64_t* bar, int issued, int co
 
 // ------------------------------------------------------------------ f64
 
-// r2^(-3/2), times gm unless UNIT (the equal-mass tile loop scales later).
-//   VAR 1: CUDA's rsqrt(double) and three multiplies
-//   VAR 0: series refinement of an f32 seed formed by f64->f32 conversion
-//   VAR 2: the same with the seed argument formed by integer operations
-// (Measured on the benchmark shape: VAR 2 199.7 ms, VAR 0 198.8-202.6 ms,
-// VAR 1 245.6 ms per evaluation; evaluating the e^2 term in f32 to save one
-// f64 operation was slower, 215 ms, because of its two conversions.)
-template <int VAR, bool UNIT>
+// r2^(-3/2), times gm unless UNIT (the equal-mass tile loop scales later):
+// the series of sss_gm_rinv3 with the hardware's f64 seed. (One evaluation
+// of 10,007 bodies: 126 us; 136 with an f32 seed whose argument and result
+// were re-biased by integer operations. On the benchmark shape the f32 seed
+// took 200 ms and CUDA's rsqrt(double) with three multiplies 246 ms.)
+template <bool UNIT>
 __device__ __forceinline__ double rinv3(double gm, double r2) {
-    if (VAR == 1) {
-        const double inv = rsqrt(r2);
-        return UNIT ? (inv * inv) * inv : ((gm * inv) * inv) * inv;
-    }
     double c;
-    if (VAR == 2) {
-        // seed argument by integer re-biasing of r2's high word (valid for
-        // 2^-126 <= r2 < 2^128), widened back bit by bit
-        const unsigned hi = (unsigned)__double2hiint(r2);
-        const float yf = sss_rsqrt_approx_f32(__uint_as_float((hi << 3) + 0x40000000u));
-        const unsigned yb = __float_as_uint(yf);
-        c = __hiloint2double((int)((yb >> 3) + 0x38000000u), (int)(yb << 29));
-    } else {
-        c = (double)sss_rsqrt_approx_f32(__double2float_rn(r2));
-    }
-    // c^3 (1 + 3/2 e + 15/8 e^2), e = 1 - r2 c^2 (see sss_gm_rinv3_f64)
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(c) : "d"(r2));
     const double c2 = c * c;
     const double e = fma(-r2, c2, 1.0);
     const double g3 = UNIT ? c * c2 : (gm * c) * c2;
@@ -177,7 +158,7 @@ __device__ __forceinline__ double rinv3(double gm, double r2) {
     return fma(g3, e * p, g3);
 }
 
-template <int D, int R, int VAR, bool UNIT, int UNROLL>
+template <int D, int R, bool UNIT, int UNROLL>
 __device__ __forceinline__ void tile_f64(const double4* __restrict__ s, int cnt, double eps2,
                                          const double (&px)[R], const double (&py)[R],
                                          const double (&pz)[R], double (&tx)[R], double (&ty)[R],
@@ -197,7 +178,7 @@ __device__ __forceinline__ void tile_f64(const double4* __restrict__ s, int cnt,
             } else {
                 r2 = fma(dx, dx, fma(dy, dy, eps2));
             }
-            const double f = rinv3<VAR, UNIT>(sj.w, r2);
+            const double f = rinv3<UNIT>(sj.w, r2);
             tx[r] = fma(f, dx, tx[r]);
             ty[r] = fma(f, dy, ty[r]);
             if (D == 3) tz[r] = fma(f, dz, tz[r]);
@@ -205,7 +186,7 @@ __device__ __forceinline__ void tile_f64(const double4* __restrict__ s, int cnt,
     }
 }
 
-template <int D, int R, int NT, int TS, int VAR, int MINB, int UNROLL>
+template <int D, int R, int NT, int TS, int MINB, int UNROLL>
 __global__ void __launch_bounds__(NT, MINB) k_force_f64(const ForceArgs a) {
     extern __shared__ __align__(128) unsigned char smem[];
     double4* tiles = reinterpret_cast<double4*>(smem);
@@ -271,8 +252,8 @@ __global__ void __launch_bounds__(NT, MINB) k_force_f64(const ForceArgs a) {
         double tx[R], ty[R], tz[R];
 #pragma unroll
         for (int r = 0; r < R; ++r) { tx[r] = 0.0; ty[r] = 0.0; tz[r] = 0.0; }
-        if (uni) tile_f64<D, R, VAR, true, UNROLL>(s, cnt, eps2, px, py, pz, tx, ty, tz);
-        else tile_f64<D, R, VAR, false, UNROLL>(s, cnt, eps2, px, py, pz, tx, ty, tz);
+        if (uni) tile_f64<D, R, true, UNROLL>(s, cnt, eps2, px, py, pz, tx, ty, tz);
+        else tile_f64<D, R, false, UNROLL>(s, cnt, eps2, px, py, pz, tx, ty, tz);
         const double wt = uni ? w0 : 1.0;
 #pragma unroll
         for (int r = 0; r < R; ++r) {
@@ -633,7 +614,7 @@ __device__ __forceinline__ void ws_finish(const ForceArgs& a, int tb, int ch, do
     epilogue<D>(a.epi, i, sx, sy, sz, a.tgt[i]);
 }
 
-template <int D, int R, int VAR>
+template <int D, int R>
 __global__ void __launch_bounds__(WS_NT, WS_MINB_F64) k_force_f64_ws(const ForceArgs a) {
     constexpr int TB = 32 * R;
     constexpr int RED = 3 * WS_W * TB * (int)sizeof(double), SRC = WS_TS * (int)sizeof(double4);
@@ -665,8 +646,8 @@ __global__ void __launch_bounds__(WS_NT, WS_MINB_F64) k_force_f64_ws(const Force
         double tx[R], ty[R], tz[R];
 #pragma unroll
         for (int r = 0; r < R; ++r) { tx[r] = 0.0; ty[r] = 0.0; tz[r] = 0.0; }
-        if (uni) tile_f64<D, R, VAR, true, F64_UNROLL>(tile + b, e - b, a.eps2, px, py, pz, tx, ty, tz);
-        else tile_f64<D, R, VAR, false, F64_UNROLL>(tile + b, e - b, a.eps2, px, py, pz, tx, ty, tz);
+        if (uni) tile_f64<D, R, true, F64_UNROLL>(tile + b, e - b, a.eps2, px, py, pz, tx, ty, tz);
+        else tile_f64<D, R, false, F64_UNROLL>(tile + b, e - b, a.eps2, px, py, pz, tx, ty, tz);
         const double wt = uni ? w0 : 1.0;
 #pragma unroll
         for (int r = 0; r < R; ++r) {
@@ -867,23 +848,20 @@ struct KSel {
     bool ws;           // warp-split (make_plan_ws)
 };
 
-KSel select_kernel(int dim, int precision, double eps2, int64_t n_src, int64_t n_tgt) {
+KSel select_kernel(int dim, int precision, int64_t n_src, int64_t n_tgt) {
     KSel k;
     k.mixed = (precision == SSS_PREC_MIXED);
     k.ws = (double)n_src * (double)n_tgt < (k.mixed ? SPLIT_PAIRS_MIX : SPLIT_PAIRS_F64);
     if (k.ws) {
-        const bool iseed = eps2 >= kIseedMinR2;
         if (k.mixed)
             k.fn = (dim == 3) ? (void*)k_force_mixed_ws<3, WS_R_MIX> : (void*)k_force_mixed_ws<2, WS_R_MIX>;
-        else if (iseed)
-            k.fn = (dim == 3) ? (void*)k_force_f64_ws<3, WS_R_F64, 2> : (void*)k_force_f64_ws<2, WS_R_F64, 2>;
         else
-            k.fn = (dim == 3) ? (void*)k_force_f64_ws<3, WS_R_F64, 1> : (void*)k_force_f64_ws<2, WS_R_F64, 1>;
+            k.fn = (dim == 3) ? (void*)k_force_f64_ws<3, WS_R_F64> : (void*)k_force_f64_ws<2, WS_R_F64>;
         k.nt = WS_NT;
         k.tpb = 32 * (k.mixed ? WS_R_MIX : WS_R_F64);
         k.ts = WS_TS;
         k.smem = 0;
-        k.key = 8 + (k.mixed ? 4 : (iseed ? 0 : 2)) + (dim == 3);
+        k.key = (k.mixed ? 8 : 4) + (dim == 3);      // (6 and 7: allpairs_tc.cu)
         k.mixed = false;
         return k;
     }
@@ -894,22 +872,16 @@ KSel select_kernel(int dim, int precision, double eps2, int64_t n_src, int64_t n
         k.tpb = MIX_NT * MIX_R;
         k.ts = MIX_TS;
         k.smem = 2 * (size_t)MIX_TS * 2 * sizeof(float4);
-        k.key = 4 + (dim == 3);
+        k.key = 2 + (dim == 3);
         return k;
     }
-    // the integer-seeded series needs r2 >= 2^-126; smaller softening takes CUDA's rsqrt
-    const bool iseed = eps2 >= kIseedMinR2;
-    if (iseed)
-        k.fn = (dim == 3) ? (void*)k_force_f64<3, F64_R, F64_NT, F64_TS, 2, F64_MINB, F64_UNROLL>
-                          : (void*)k_force_f64<2, F64_R, F64_NT, F64_TS, 2, F64_MINB, F64_UNROLL>;
-    else
-        k.fn = (dim == 3) ? (void*)k_force_f64<3, F64_R, F64_NT, F64_TS, 1, F64_MINB, F64_UNROLL>
-                          : (void*)k_force_f64<2, F64_R, F64_NT, F64_TS, 1, F64_MINB, F64_UNROLL>;
+    k.fn = (dim == 3) ? (void*)k_force_f64<3, F64_R, F64_NT, F64_TS, F64_MINB, F64_UNROLL>
+                      : (void*)k_force_f64<2, F64_R, F64_NT, F64_TS, F64_MINB, F64_UNROLL>;
     k.nt = F64_NT;
     k.tpb = F64_NT * F64_R;
     k.ts = F64_TS;
     k.smem = 2 * (size_t)F64_TS * sizeof(double4);
-    k.key = (iseed ? 0 : 2) + (dim == 3);
+    k.key = dim == 3;
     return k;
 }
 
@@ -944,7 +916,7 @@ int force_eval(sss_ctx* ctx, int dim, int precision, const double4* src, int64_t
         return sss_set_err(ctx, SSS_ERR_ARG, "all-pairs: size out of range");
     if (precision == SSS_PREC_MIXED_TC)
         return sss_ap::force_eval_tc(ctx, dim, src, n_src, tgt, n_tgt, eps2, epi, stream);
-    const KSel ks = select_kernel(dim, precision, eps2, n_src, n_tgt);
+    const KSel ks = select_kernel(dim, precision, n_src, n_tgt);
     if (ctx->occ[ks.key] == 0) {
         int per_sm = 0;
         SSS_CUDA_TRY(ctx, query_occupancy(ks, &per_sm));
@@ -1205,17 +1177,14 @@ int noalloc_setup(int device, NoAllocDevice** out, char* eb, size_t el) {
         } else {
             d->base = (unsigned char*)p;
             e = cudaDeviceGetAttribute(&d->num_sms, cudaDevAttrMultiProcessorCount, device);
-            // one representative eps2 per f64 seed variant selects each kernel once
-            // and one size for the few-pairs and the general kernels
-            const double probe_eps2[2] = {1.0, 0.0};
+            // one size for the few-pairs and one for the general kernels
             const int64_t probe_n[2] = {1, (int64_t)1 << 20};
             for (int prec = 0; prec < 2 && e == cudaSuccess; ++prec)
                 for (int dim = 2; dim <= 3 && e == cudaSuccess; ++dim)
-                    for (int v = 0; v < (prec ? 1 : 2) && e == cudaSuccess; ++v)
-                        for (int q = 0; q < 2 && e == cudaSuccess; ++q) {
-                            const KSel ks = select_kernel(dim, prec, probe_eps2[v], probe_n[q], probe_n[q]);
-                            e = query_occupancy(ks, &d->occ[ks.key]);
-                        }
+                    for (int q = 0; q < 2 && e == cudaSuccess; ++q) {
+                        const KSel ks = select_kernel(dim, prec, probe_n[q], probe_n[q]);
+                        e = query_occupancy(ks, &d->occ[ks.key]);
+                    }
             if (e != cudaSuccess)
                 rc = noalloc_err(eb, el, SSS_ERR_CUDA, "no-alloc setup: %s", cudaGetErrorString(e));
             else
@@ -1254,7 +1223,7 @@ extern "C" int sss_allpairs_accel_noalloc(int device, int dim, int precision, co
     int rc = noalloc_setup(device, &d, eb, el);
     if (rc) return rc;
 
-    const KSel ks = select_kernel(dim, precision, eps2, n_src, n_tgt);
+    const KSel ks = select_kernel(dim, precision, n_src, n_tgt);
     const int slots = d->occ[ks.key] * d->num_sms;
     Plan pl = ks.ws ? make_plan_ws(n_src, n_tgt, ks.tpb, slots) : make_plan(n_src, n_tgt, ks.tpb, ks.ts, slots);
 

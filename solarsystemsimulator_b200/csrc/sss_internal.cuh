@@ -11,7 +11,7 @@
 
 #include "../../include/sss.h"
 
-#define SSS_AP_KERNELS 14   // all-pairs force kernels by dimension, precision and size
+#define SSS_AP_KERNELS 10   // all-pairs force kernels by dimension, precision and size
 
 struct sss_ctx {
     int device;
@@ -129,58 +129,25 @@ __device__ __forceinline__ bool sss_mbar_wait_bounded(uint64_t* bar, unsigned pa
 
 // ------------------------------------------------------------- f64 kernels
 
-// Gm * r2^(-3/2) in f64 from an f32 reciprocal-square-root seed.
-//
-// Method (Householder-type series refinement of 1/sqrt, e.g. Householder,
-// "The Numerical Treatment of a Single Nonlinear Equation", 1970): with a
-// seed c ~ r2^(-1/2) and e = 1 - r2*c^2, the exact value is
-//   r2^(-3/2) = c^3 (1 - e)^(-3/2) = c^3 (1 + 3/2 e + 15/8 e^2 + 35/16 e^3 + ...).
-// The seed is the hardware f32 approximation (rsqrt.approx.f32, |e| < 1e-6
-// here), so the cubic remainder is < 3e-18 and the series is cut after e^2.
-// c is an f32 value, hence c*c is exact in f64 and e carries one rounding.
-// Cost: 7 f64 operations + one f32 MUFU op + two conversions.
 __device__ __forceinline__ float sss_rsqrt_approx_f32(float x) {
     float y;
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
 
-__device__ __forceinline__ double sss_gm_rinv3_f64(double gm, double r2) {
-    const float yf = sss_rsqrt_approx_f32(__double2float_rn(r2));
-    const double c = (double)yf;
-    const double c2 = c * c;                    // exact
-    const double e = fma(-r2, c2, 1.0);         // 1 - r2 c^2
-    const double p = fma(e, 1.875, 1.5);        // 3/2 + 15/8 e
-    const double g = gm * c;
-    const double g3 = g * c2;                   // Gm c^3
-    return fma(g3, e * p, g3);                  // Gm c^3 (1 + e p)
-}
-
-// Same series with the seed's argument formed by integer operations instead
-// of an f64->f32 conversion: the high word of r2 (sign, 11-bit exponent, 20
-// mantissa bits) re-biased to an f32 bit pattern (mantissa truncated, |rel.
-// error| < 2^-20), and the f32 result widened to f64 bit by bit. Valid for
-// 2^-126 <= r2 < 2^128 (|e| < 1.3e-6, cubic remainder < 5e-18).
-__device__ __forceinline__ double sss_gm_rinv3_f64_iseed(double gm, double r2) {
-    const unsigned hi = (unsigned)__double2hiint(r2);
-    const unsigned fb = (hi << 3) + 0x40000000u;          // exponent 1023 -> 127 bias
-    const float yf = sss_rsqrt_approx_f32(__uint_as_float(fb));
-    const unsigned yb = __float_as_uint(yf);
-    const double c = __hiloint2double((int)((yb >> 3) + 0x38000000u), (int)(yb << 29));
-    const double c2 = c * c;
-    const double e = fma(-r2, c2, 1.0);
-    const double p = fma(e, 1.875, 1.5);
-    const double g = gm * c;
-    const double g3 = g * c2;
-    return fma(g3, e * p, g3);
-}
-
-// The same series over the full f64 range, from the hardware's f64 seed
-// (rsqrt.approx.ftz.f64: no conversion of r2 or of the seed). Measured over
-// 128 binades: seed |e| < 1.9e-6, so the cubic remainder is < 1.5e-17; result
-// within 2.3e-16 (rms 7.2e-17), against 5.5e-16 (1.6e-16) of the cube of CUDA's
-// rsqrt and 2.7e-16 (8.1e-17) of 1 / (r2 sqrt(r2)), at 74 clocks of latency
-// against 88 and 168 and 1.7 and 3.6 times their rate. 0 for r2 = +inf.
+// Gm * r2^(-3/2) in f64 from the hardware's approximate reciprocal square root.
+//
+// Method (Householder-type series refinement of 1/sqrt, e.g. Householder,
+// "The Numerical Treatment of a Single Nonlinear Equation", 1970): with a
+// seed c ~ r2^(-1/2) and e = 1 - r2*c^2, the exact value is
+//   r2^(-3/2) = c^3 (1 - e)^(-3/2) = c^3 (1 + 3/2 e + 15/8 e^2 + 35/16 e^3 + ...).
+// The seed is rsqrt.approx.ftz.f64 (a coarse value over the full f64 range,
+// no conversion of r2 or of the seed). Measured over 128 binades: |e| <
+// 1.9e-6, so the cubic remainder is < 1.5e-17 and the series is cut after
+// e^2; the result is within 2.3e-16 (rms 7.2e-17), against 5.5e-16 (1.6e-16)
+// of the cube of CUDA's rsqrt and 2.7e-16 (8.1e-17) of 1 / (r2 sqrt(r2)), at
+// 74 clocks of latency against 88 and 168 and 1.7 and 3.6 times their rate.
+// 0 for r2 = +inf.
 __device__ __forceinline__ double sss_gm_rinv3(double gm, double r2) {
     double c;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(c) : "d"(r2));
@@ -190,13 +157,6 @@ __device__ __forceinline__ double sss_gm_rinv3(double gm, double r2) {
     const double p = fma(e, 1.875, 1.5);
     const double g3 = (gm * c) * c2;
     return fma(g3, e * p, g3);
-}
-
-// Same value from CUDA's own f64 rsqrt (kept as a selectable variant so the
-// faster form can be chosen by measurement).
-__device__ __forceinline__ double sss_gm_rinv3_cuda(double gm, double r2) {
-    const double inv = rsqrt(r2);
-    return ((gm * inv) * inv) * inv;
 }
 
 // f32 hypot, correctly rounded as the C library's hypotf (which NumPy calls for float32
