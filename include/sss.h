@@ -273,6 +273,25 @@ int  sss_pm2d_kick_drift(sss_pm2d* p, double* x, double* y, double* vx, double* 
                          const double* ay, int64_t n, double hdt, double dt, int drift, void* stream);
 /* out[i] = (float)a[i] (snapshot rows, :274-280) */
 int  sss_pm2d_to_f32(sss_pm2d* p, const double* a, int64_t n, float* out, void* stream);
+/* `steps` whole KDK steps (:246-280) with the softening soft_cells cells, the
+ * grid's geometry (margin_cells of margin, :110-124) formed on the device.
+ * Index 0 of the arrays: the n masses, 1: the t tracers. *kernel_h (host, in
+ * and out, <= 0: none) is the cell size the force kernels stand for (:216-221).
+ * snap: steps rows f32 [x|y|vx|vy|tx|ty]. Synchronous. Only where
+ * sss_pm2d_steps_natively (2 grid_n = 2^a, 3 2^a or 1000 2^a, 64 .. 8192). */
+typedef struct sss_pm2d_bodies {
+    double* x[2];
+    double* y[2];
+    double* vx[2];
+    double* vy[2];
+    double* ax[2];
+    double* ay[2];
+    const double* m;
+    int64_t n, t;
+} sss_pm2d_bodies;
+int  sss_pm2d_step_batch(sss_pm2d* p, const sss_pm2d_bodies* st, double dt, int steps, double soft_cells,
+                         double margin_cells, double G, double* kernel_h, float* snap, void* stream);
+int  sss_pm2d_steps_natively(sss_pm2d* p);
 
 /* ------------------------------------------------- collision response
  *

@@ -68,6 +68,12 @@ class NBodyCfg(ctypes.Structure):
                 ("pair_f32", ctypes.c_int)]
 
 
+class Pm2dBodies(ctypes.Structure):
+    """Mirror of sss_pm2d_bodies."""
+    _fields_ = [("x", _dp * 2), ("y", _dp * 2), ("vx", _dp * 2), ("vy", _dp * 2), ("ax", _dp * 2), ("ay", _dp * 2),
+                ("m", _dp), ("n", _c_i64), ("t", _c_i64)]
+
+
 class Pm3Particles(ctypes.Structure):
     """Mirror of sss_pm3_particles."""
     _fields_ = [
@@ -122,6 +128,10 @@ SIGNATURES = {
     "sss_pm2d_fields": (ctypes.c_int, [_vp, _dp, _dp, _vp]),
     "sss_pm2d_kick_drift": (ctypes.c_int, [_vp, _dp, _dp, _dp, _dp, _dp, _dp, _c_i64, ctypes.c_double,
                                            ctypes.c_double, ctypes.c_int, _vp]),
+    "sss_pm2d_step_batch": (ctypes.c_int, [_vp, ctypes.POINTER(Pm2dBodies), ctypes.c_double, ctypes.c_int,
+                                           ctypes.c_double, ctypes.c_double, ctypes.c_double,
+                                           ctypes.POINTER(ctypes.c_double), _dp, _vp]),
+    "sss_pm2d_steps_natively": (ctypes.c_int, [_vp]),
     "sss_pm2d_to_f32": (ctypes.c_int, [_vp, _dp, _c_i64, _dp, _vp]),
     "sss_batched_launch": (ctypes.c_int, [_vp, ctypes.c_int, ctypes.POINTER(_dp), ctypes.POINTER(_dp), _dp, _dp,
                                           _dp, _dp, _dp, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int,

@@ -47,6 +47,13 @@ __global__ void k_force_kernels_2d(int n, double h, double eps2, double G, doubl
     ky[t] = __dmul_rn(__dmul_rn(-G, dy), inv_r3);
 }
 
+// Grid geometry of a step in device memory (pm_kernel.py:110-124), with the
+// cell size the force kernels stand for (remade when h moves by more than
+// 1e-6 of it, :216-221) and the factor of the unit kernel's spectrum.
+struct Geo {
+    double x0, y0, h, kernel_h, scale;
+};
+
 // CIC corner index/weights of the reference (pm_kernel.py:63-90): cell
 // clipped to [0, N-2], fractional offsets from the clipped cell.
 __device__ __forceinline__ void cic2(double gx, double gy, double x0, double y0, double h, int n, int& i,
@@ -64,9 +71,11 @@ __device__ __forceinline__ void cic2(double gx, double gy, double x0, double y0,
 // deposit into the grid of row stride s (2N where the padded array is transformed whole)
 __global__ void k_cic_deposit_2d(const double* __restrict__ gx, const double* __restrict__ gy,
                                  const double* __restrict__ gm, long long np_, int n, long long s, double x0,
-                                 double y0, double h, double* __restrict__ rho_pad) {
+                                 double y0, double h, double* __restrict__ rho_pad,
+                                 const Geo* __restrict__ g) {
     const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= np_) return;
+    if (g) { x0 = g->x0; y0 = g->y0; h = g->h; }
     int i, j;
     double tx, ty;
     cic2(gx[p], gy[p], x0, y0, h, n, i, j, tx, ty);
@@ -123,21 +132,30 @@ __global__ void k_cic_gather_2d(const double* __restrict__ px, const double* __r
 }
 
 // the same read of the N x N field of pairs (f_x, f_y)
+__device__ __forceinline__ double2 gather_pair(double px, double py, int n, double x0, double y0, double h,
+                                               const double2* __restrict__ f) {
+    int i, j;
+    double tx, ty;
+    cic2(px, py, x0, y0, h, n, i, j, tx, ty);
+    const double ux = __dsub_rn(1.0, tx), uy = __dsub_rn(1.0, ty);
+    const long long c00 = (long long)i * n + j;
+    const double2 f00 = f[c00], f10 = f[c00 + n], f01 = f[c00 + 1], f11 = f[c00 + n + 1];
+    double2 a;
+    a.x = __dadd_rn(__dadd_rn(__dadd_rn(__dmul_rn(__dmul_rn(f00.x, ux), uy), __dmul_rn(__dmul_rn(f10.x, tx), uy)),
+                              __dmul_rn(__dmul_rn(f01.x, ux), ty)), __dmul_rn(__dmul_rn(f11.x, tx), ty));
+    a.y = __dadd_rn(__dadd_rn(__dadd_rn(__dmul_rn(__dmul_rn(f00.y, ux), uy), __dmul_rn(__dmul_rn(f10.y, tx), uy)),
+                              __dmul_rn(__dmul_rn(f01.y, ux), ty)), __dmul_rn(__dmul_rn(f11.y, tx), ty));
+    return a;
+}
+
 __global__ void k_cic_gather_pairs_2d(const double* __restrict__ px, const double* __restrict__ py, long long np_,
                                       int n, double x0, double y0, double h, const double2* __restrict__ f,
                                       double* __restrict__ ax, double* __restrict__ ay) {
     const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= np_) return;
-    int i, j;
-    double tx, ty;
-    cic2(px[p], py[p], x0, y0, h, n, i, j, tx, ty);
-    const double ux = __dsub_rn(1.0, tx), uy = __dsub_rn(1.0, ty);
-    const long long c00 = (long long)i * n + j;
-    const double2 f00 = f[c00], f10 = f[c00 + n], f01 = f[c00 + 1], f11 = f[c00 + n + 1];
-    ax[p] = __dadd_rn(__dadd_rn(__dadd_rn(__dmul_rn(__dmul_rn(f00.x, ux), uy), __dmul_rn(__dmul_rn(f10.x, tx), uy)),
-                                __dmul_rn(__dmul_rn(f01.x, ux), ty)), __dmul_rn(__dmul_rn(f11.x, tx), ty));
-    ay[p] = __dadd_rn(__dadd_rn(__dadd_rn(__dmul_rn(__dmul_rn(f00.y, ux), uy), __dmul_rn(__dmul_rn(f10.y, tx), uy)),
-                                __dmul_rn(__dmul_rn(f01.y, ux), ty)), __dmul_rn(__dmul_rn(f11.y, tx), ty));
+    const double2 a = gather_pair(px[p], py[p], n, x0, y0, h, f);
+    ax[p] = a.x;
+    ay[p] = a.y;
 }
 
 __global__ void k_split_pairs_2d(const double2* __restrict__ f, long long m, double* __restrict__ ax,
@@ -236,8 +254,10 @@ k_rows_fwd(const double2* __restrict__ tw, const double* __restrict__ rho, doubl
 template <int L>
 __global__ void __launch_bounds__(fft_threads(L, 1), 512 / fft_threads(L, 1))
 k_cols(const double2* __restrict__ tw, const double2* __restrict__ in, const double* __restrict__ u,
-       const double* __restrict__ v, double scale, double2* slots, double2* __restrict__ out) {
+       const double* __restrict__ v, double scale, const Geo* __restrict__ geo, double2* slots,
+       double2* __restrict__ out) {
     constexpr int n = L / 2;
+    if (geo) scale = geo->scale;
     extern __shared__ double2 sm2[];
     using Map = fft::One;
     double2* slot = slots + (long long)blockIdx.x * L;
@@ -291,7 +311,8 @@ k_rows_inv(const double2* __restrict__ tw, const double2* __restrict__ in, doubl
 
 struct Convolve2d {
     void (*rows_fwd)(const double2*, const double*, double2*);
-    void (*cols)(const double2*, const double2*, const double*, const double*, double, double2*, double2*);
+    void (*cols)(const double2*, const double2*, const double*, const double*, double, const Geo*, double2*,
+                 double2*);
     void (*rows_inv)(const double2*, const double2*, double2*);
     int threads;
 };
@@ -333,15 +354,10 @@ __global__ void k_cic_gather_field_2d(const double* __restrict__ px, const doubl
     out[p] = __dadd_rn(__dadd_rn(__dadd_rn(t00, t10), t01), t11);
 }
 
-// min/max of x and y: out[0..3] = xmin, xmax, ymin, ymax (two-pass: blocks -> final)
-__global__ void k_bbox_2d(const double* __restrict__ x, const double* __restrict__ y, long long n,
-                          double* __restrict__ part) {
+// A block's min and max of x and y into its four values of part (warps of
+// 32 threads, at most 8).
+__device__ __forceinline__ void block_bbox(double a, double b, double c, double d, double* __restrict__ part) {
     __shared__ double s[4][8];
-    double a = 1e308, b = -1e308, c = 1e308, d = -1e308;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        a = fmin(a, x[i]); b = fmax(b, x[i]);
-        c = fmin(c, y[i]); d = fmax(d, y[i]);
-    }
     for (int o = 16; o > 0; o >>= 1) {
         a = fmin(a, __shfl_xor_sync(0xffffffffu, a, o));
         b = fmax(b, __shfl_xor_sync(0xffffffffu, b, o));
@@ -360,6 +376,17 @@ __global__ void k_bbox_2d(const double* __restrict__ x, const double* __restrict
         part[4 * blockIdx.x + 2] = c;
         part[4 * blockIdx.x + 3] = d;
     }
+}
+
+// min/max of x and y: out[0..3] = xmin, xmax, ymin, ymax (two-pass: blocks -> final)
+__global__ void k_bbox_2d(const double* __restrict__ x, const double* __restrict__ y, long long n,
+                          double* __restrict__ part) {
+    double a = 1e308, b = -1e308, c = 1e308, d = -1e308;
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+        a = fmin(a, x[i]); b = fmax(b, x[i]);
+        c = fmin(c, y[i]); d = fmax(d, y[i]);
+    }
+    block_bbox(a, b, c, d, part);
 }
 
 __global__ void k_bbox_final(const double* __restrict__ part, int nb, double* __restrict__ out) {
@@ -397,6 +424,85 @@ __global__ void k_kick_drift_2d(double* __restrict__ x, double* __restrict__ y, 
 __global__ void k_snap_2d(const double* __restrict__ a, long long n, float* __restrict__ out) {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) out[i] = (float)a[i];
+}
+
+// The step's geometry from the blocks' boxes (grid_fuer, pm_kernel.py:110-124;
+// its operations and their rounding): one block, the step stays on the device.
+__global__ void __launch_bounds__(256) k_geo_2d(const double* __restrict__ part, int nb, double cells, double margin,
+                                                double G, double np2, Geo* __restrict__ geo) {
+    __shared__ double box[4];
+    double a = 1e308, b = -1e308, c = 1e308, d = -1e308;
+    for (int k = threadIdx.x; k < nb; k += blockDim.x) {
+        a = fmin(a, part[4 * k]); b = fmax(b, part[4 * k + 1]);
+        c = fmin(c, part[4 * k + 2]); d = fmax(d, part[4 * k + 3]);
+    }
+    block_bbox(a, b, c, d, box);
+    if (threadIdx.x != 0) return;
+    const double span = fmax(fmax(__dsub_rn(box[1], box[0]), __dsub_rn(box[3], box[2])), 1e-30);
+    const double h = __ddiv_rn(span, cells);
+    geo->x0 = __dsub_rn(box[0], __dmul_rn(margin, h));
+    geo->y0 = __dsub_rn(box[2], __dmul_rn(margin, h));
+    geo->h = h;
+    double kh = geo->kernel_h;
+    if (!(kh > 0.0) || fabs(__dsub_rn(h, kh)) > __dmul_rn(1e-6, h)) kh = h;
+    geo->kernel_h = kh;
+    geo->scale = G / (kh * kh) / np2;
+}
+
+// Masses (first n) and tracers of a step.
+struct Bodies2d {
+    double *x[2], *y[2], *vx[2], *vy[2], *ax[2], *ay[2];    // masses, tracers
+    long long n, t;
+};
+
+// One pass over the bodies between two fields: with f the acceleration from
+// the field, the closing half kick and the snapshot row; with open the next
+// step's opening half kick and drift and the box of the moved masses. (As
+// separate launches around a host that read the box back, these took 100 us
+// of a step, against 290 of the transforms on a 2048 grid.)
+__global__ void __launch_bounds__(256) k_move_2d(const Bodies2d b, int grid_n, const Geo* __restrict__ geo,
+                                                 const double2* __restrict__ f, int open, double hdt, double dt,
+                                                 float* __restrict__ row, double* __restrict__ part) {
+    double lo[2] = {1e308, 1e308}, hi[2] = {-1e308, -1e308};
+    for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < b.n + b.t;
+         q += (long long)gridDim.x * blockDim.x) {
+        const int k = q < b.n ? 0 : 1;
+        const long long i = k ? q - b.n : q;
+        double x = b.x[k][i], y = b.y[k][i], vx = b.vx[k][i], vy = b.vy[k][i];
+        double2 a;
+        if (f) {
+            a = gather_pair(x, y, grid_n, geo->x0, geo->y0, geo->h, f);
+            b.ax[k][i] = a.x;
+            b.ay[k][i] = a.y;
+            vx = __dadd_rn(vx, __dmul_rn(hdt, a.x));
+            vy = __dadd_rn(vy, __dmul_rn(hdt, a.y));
+            float* r = row + (k ? 4 * b.n : 0);
+            const long long m = k ? b.t : b.n;
+            r[i] = (float)x;
+            r[m + i] = (float)y;
+            if (!k) {
+                r[2 * m + i] = (float)vx;
+                r[3 * m + i] = (float)vy;
+            }
+        } else {
+            a = make_double2(b.ax[k][i], b.ay[k][i]);
+        }
+        if (open) {
+            vx = __dadd_rn(vx, __dmul_rn(hdt, a.x));
+            vy = __dadd_rn(vy, __dmul_rn(hdt, a.y));
+            x = __dadd_rn(x, __dmul_rn(dt, vx));
+            y = __dadd_rn(y, __dmul_rn(dt, vy));
+            b.x[k][i] = x;
+            b.y[k][i] = y;
+            if (!k) {
+                lo[0] = fmin(lo[0], x); hi[0] = fmax(hi[0], x);
+                lo[1] = fmin(lo[1], y); hi[1] = fmax(hi[1], y);
+            }
+        }
+        b.vx[k][i] = vx;
+        b.vy[k][i] = vy;
+    }
+    if (open) block_bbox(lo[0], hi[0], lo[1], hi[1], part);
 }
 
 unsigned blocks_for(long long n, int nt) { return (unsigned)((n + nt - 1) / nt); }
@@ -438,6 +544,7 @@ struct sss_pm2d {
     double* fieldx;        // (2N x 2N) real fields
     double* fieldy;
     double* bb_part;       // bbox partials
+    Geo* geo;              // own: the current step's geometry (sss_pm2d_step_batch)
 };
 
 static int pm2d_free(sss_pm2d* p) {
@@ -446,7 +553,7 @@ static int pm2d_free(sss_pm2d* p) {
     if (p->inv) cufftDestroy(p->inv);
     if (p->own) {
         cudaFree(p->rho); cudaFree(p->u); cudaFree(p->v); cudaFree(p->t1); cudaFree(p->t2); cudaFree(p->slots);
-        cudaFree(p->pairs); cudaFree(p->tw);
+        cudaFree(p->pairs); cudaFree(p->tw); cudaFree(p->geo);
     }
     cudaFree(p->kx); cudaFree(p->ky); cudaFree(p->fkx); cudaFree(p->fky); cudaFree(p->fr);
     cudaFree(p->sx); cudaFree(p->sy); cudaFree(p->fieldx); cudaFree(p->fieldy);
@@ -477,6 +584,7 @@ static cudaError_t pm2d_own_setup(sss_pm2d* p) {
     e = e ? e : cudaMalloc(&p->slots, (size_t)p->grid[1] * L * sizeof(double2));
     e = e ? e : cudaMalloc(&p->pairs, n * n * sizeof(double2));
     e = e ? e : cudaMalloc(&p->kx, 4 * n * n * sizeof(double));
+    e = e ? e : cudaMalloc(&p->geo, sizeof(Geo));
     return e;
 }
 
@@ -546,6 +654,27 @@ extern "C" int sss_pm2d_bbox(sss_pm2d* p, const double* x, const double* y, int6
     return SSS_OK;
 }
 
+// The unit kernel's spectrum for the softening e2 = (eps / h)^2. eps^2 / h^2
+// of a softening tied to h differs from step to step by a few roundings:
+// within 1e-15 it is the same kernel.
+static int pm2d_unit_spectrum(sss_pm2d* p, double e2, cudaStream_t s) {
+    sss_ctx* ctx = p->ctx;
+    if (fabs(e2 - p->e2_unit) <= 1e-15 * e2) return SSS_OK;
+    const long long np = 2LL * p->n;
+    p->e2_unit = -1.0;
+    k_unit_kernel_2d<<<blocks_for(np * np, 256), 256, 0, s>>>(p->n, e2, p->kx);
+    SSS_LAUNCH_CHECK(ctx, "k_unit_kernel_2d");
+    cufftSetStream(p->fwd, s);
+    // the spectrum (2N x (N + 1)) fits t2 exactly
+    cufftResult r = cufftExecD2Z(p->fwd, p->kx, (cufftDoubleComplex*)p->t2);
+    if (r != CUFFT_SUCCESS) return cufft_err(ctx, r, "cufftExecD2Z (kernel)");
+    const unsigned tiles = (unsigned)(p->n / 32 + 1);
+    k_kernel_tables_2d<<<dim3(tiles, tiles), 256, 0, s>>>(p->t2, p->n, p->u, p->v);
+    SSS_LAUNCH_CHECK(ctx, "k_kernel_tables_2d");
+    p->e2_unit = e2;
+    return SSS_OK;
+}
+
 // FFTs of the softened force kernels for cell size h (pm_kernel.py:34-60);
 // kept inside the plan object until the next call.
 extern "C" int sss_pm2d_build_kernels(sss_pm2d* p, double h, double eps2, double G, void* stream) {
@@ -555,23 +684,8 @@ extern "C" int sss_pm2d_build_kernels(sss_pm2d* p, double h, double eps2, double
     cudaStream_t s = (cudaStream_t)stream;
     const long long np = 2LL * p->n;
     if (p->own) {
-        // eps^2 / h^2 of a softening tied to h differs from step to step by a few roundings: within
-        // 1e-15 it is the same kernel
-        const double e2 = eps2 / (h * h);
         p->scale = G / (h * h) / (double)(np * np);
-        if (fabs(e2 - p->e2_unit) <= 1e-15 * e2) return SSS_OK;
-        p->e2_unit = -1.0;
-        k_unit_kernel_2d<<<blocks_for(np * np, 256), 256, 0, s>>>(p->n, e2, p->kx);
-        SSS_LAUNCH_CHECK(ctx, "k_unit_kernel_2d");
-        cufftSetStream(p->fwd, s);
-        // the spectrum (2N x (N + 1)) fits t2 exactly
-        cufftResult r = cufftExecD2Z(p->fwd, p->kx, (cufftDoubleComplex*)p->t2);
-        if (r != CUFFT_SUCCESS) return cufft_err(ctx, r, "cufftExecD2Z (kernel)");
-        const unsigned tiles = (unsigned)(p->n / 32 + 1);
-        k_kernel_tables_2d<<<dim3(tiles, tiles), 256, 0, s>>>(p->t2, p->n, p->u, p->v);
-        SSS_LAUNCH_CHECK(ctx, "k_kernel_tables_2d");
-        p->e2_unit = e2;
-        return SSS_OK;
+        return pm2d_unit_spectrum(p, eps2 / (h * h), s);
     }
     k_force_kernels_2d<<<blocks_for(np * np, 256), 256, 0, s>>>(p->n, h, eps2, G, p->kx, p->ky);
     SSS_LAUNCH_CHECK(ctx, "k_force_kernels_2d");
@@ -594,13 +708,15 @@ extern "C" int sss_pm2d_field(sss_pm2d* p, const double* gx, const double* gy, c
     const long long np = 2LL * p->n;
     SSS_CUDA_TRY(ctx, cudaMemsetAsync(p->rho, 0, (size_t)p->ld * p->ld * sizeof(double), s));
     if (n > 0) {
-        k_cic_deposit_2d<<<blocks_for(n, 256), 256, 0, s>>>(gx, gy, gm, n, p->n, p->ld, x0, y0, h, p->rho);
+        k_cic_deposit_2d<<<blocks_for(n, 256), 256, 0, s>>>(gx, gy, gm, n, p->n, p->ld, x0, y0, h, p->rho,
+                                                            nullptr);
         SSS_LAUNCH_CHECK(ctx, "k_cic_deposit_2d");
     }
     if (p->own) {
         p->conv.rows_fwd<<<p->grid[0], p->conv.threads, p->smem, s>>>(p->tw, p->rho, p->t1);
         SSS_LAUNCH_CHECK(ctx, "k_rows_fwd");
-        p->conv.cols<<<p->grid[1], p->conv.threads, p->smem, s>>>(p->tw, p->t1, p->u, p->v, p->scale, p->slots, p->t2);
+        p->conv.cols<<<p->grid[1], p->conv.threads, p->smem, s>>>(p->tw, p->t1, p->u, p->v, p->scale, nullptr, p->slots,
+                                                                       p->t2);
         SSS_LAUNCH_CHECK(ctx, "k_cols");
         p->conv.rows_inv<<<p->grid[2], p->conv.threads, p->smem, s>>>(p->tw, p->t2, p->pairs);
         SSS_LAUNCH_CHECK(ctx, "k_rows_inv");
@@ -694,3 +810,55 @@ extern "C" int sss_pm2d_to_f32(sss_pm2d* p, const double* a, int64_t n, float* o
     SSS_LAUNCH_CHECK(p->ctx, "k_snap_2d");
     return SSS_OK;
 }
+
+// Steps of NBodyPM.step_batch (pm_kernel.py:246-280) with a softening tied to
+// the cell size, for the grids that convolve with the kernels of this file:
+// the geometry of every step stays on the device. *kernel_h (host, in and
+// out; <= 0: none yet) is the cell size the force kernels stand for.
+extern "C" int sss_pm2d_step_batch(sss_pm2d* p, const sss_pm2d_bodies* st, double dt, int steps, double soft_cells,
+                                   double margin_cells, double G, double* kernel_h, float* snap, void* stream) {
+    if (!p) return SSS_ERR_ARG;
+    sss_ctx* ctx = p->ctx;
+    if (!p->own) return sss_set_err(ctx, SSS_ERR_ARG, "step_batch: this grid size steps by its parts");
+    if (!st || !kernel_h || !snap || steps < 1 || st->n < 1 || st->t < 0)
+        return sss_set_err(ctx, SSS_ERR_ARG, "step_batch: bad input");
+    Bodies2d b;
+    for (int k = 0; k < 2; ++k) {
+        b.x[k] = st->x[k]; b.y[k] = st->y[k]; b.vx[k] = st->vx[k]; b.vy[k] = st->vy[k];
+        b.ax[k] = st->ax[k]; b.ay[k] = st->ay[k];
+        if ((k == 0 || st->t > 0) && (!b.x[k] || !b.y[k] || !b.vx[k] || !b.vy[k] || !b.ax[k] || !b.ay[k]))
+            return sss_set_err(ctx, SSS_ERR_ARG, "step_batch: NULL array");
+    }
+    if (!st->m) return sss_set_err(ctx, SSS_ERR_ARG, "step_batch: NULL masses");
+    b.n = st->n;
+    b.t = st->t;
+    SSS_CUDA_TRY(ctx, cudaSetDevice(ctx->device));
+    cudaStream_t s = (cudaStream_t)stream;
+    int rc = pm2d_unit_spectrum(p, soft_cells * soft_cells, s);
+    if (rc) return rc;
+    const double np = 2.0 * p->n, hdt = 0.5 * dt;
+    const long long row = 4 * b.n + 2 * b.t;
+    const unsigned want = blocks_for(b.n + b.t, 256), nb = want < 1024 ? want : 1024;
+    SSS_CUDA_TRY(ctx, cudaMemcpyAsync(&p->geo->kernel_h, kernel_h, sizeof(double), cudaMemcpyHostToDevice, s));
+    k_move_2d<<<nb, 256, 0, s>>>(b, p->n, p->geo, nullptr, 1, hdt, dt, nullptr, p->bb_part);
+    for (int k = 0; k < steps; ++k) {
+        k_geo_2d<<<1, 256, 0, s>>>(p->bb_part, (int)nb, p->n - 2.0 * margin_cells, margin_cells, G, np * np, p->geo);
+        SSS_CUDA_TRY(ctx, cudaMemsetAsync(p->rho, 0, (size_t)p->n * p->n * sizeof(double), s));
+        k_cic_deposit_2d<<<blocks_for(b.n, 256), 256, 0, s>>>(b.x[0], b.y[0], st->m, b.n, p->n, p->n, 0.0, 0.0, 1.0,
+                                                             p->rho, p->geo);
+        p->conv.rows_fwd<<<p->grid[0], p->conv.threads, p->smem, s>>>(p->tw, p->rho, p->t1);
+        p->conv.cols<<<p->grid[1], p->conv.threads, p->smem, s>>>(p->tw, p->t1, p->u, p->v, 0.0, p->geo, p->slots,
+                                                                 p->t2);
+        p->conv.rows_inv<<<p->grid[2], p->conv.threads, p->smem, s>>>(p->tw, p->t2, p->pairs);
+        k_move_2d<<<nb, 256, 0, s>>>(b, p->n, p->geo, p->pairs, k + 1 < steps, hdt, dt, snap + k * row, p->bb_part);
+        SSS_LAUNCH_CHECK(ctx, "pm2d step");
+    }
+    Geo g;
+    SSS_CUDA_TRY(ctx, cudaMemcpyAsync(&g, p->geo, sizeof(Geo), cudaMemcpyDeviceToHost, s));
+    SSS_CUDA_TRY(ctx, cudaStreamSynchronize(s));
+    *kernel_h = g.kernel_h;
+    p->scale = g.scale;
+    return SSS_OK;
+}
+
+extern "C" int sss_pm2d_steps_natively(sss_pm2d* p) { return p && p->own ? 1 : 0; }

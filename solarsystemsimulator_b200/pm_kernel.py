@@ -44,6 +44,7 @@ class PMPlan:
             self.ctx.check(self.ctx.lib.sss_pm2d_create(self.ctx.ptr, self.grid_n, ctypes.byref(ptr)))
         self.ptr = ptr
         self.kernel_key = None
+        self.native_steps = bool(self.ctx.lib.sss_pm2d_steps_natively(ptr))
 
     def __del__(self):
         try:
@@ -250,6 +251,11 @@ class NBodyPM:
         p = self._plan
         dev = torch.device("cuda", self.device)
         snap = torch.empty((steps, 4 * n + 2 * t), dtype=torch.float32, device=dev)
+        # a softening tied to the cell size: whole steps on the device (with a floor the kernels may
+        # have to be remade for the step's own h, which the host then reads)
+        if (p.native_steps and not self.softening_floor > 0.0 and self.softening_zellen > 0.0
+                and self.grid_n > 2 * self.rand_zellen and n):
+            return self._step_native(st, dt, steps, snap)
 
         def kd(xk, yk, vxk, vyk, axk, ayk, cnt, drift):
             p.call("sss_pm2d_kick_drift", st[xk].data_ptr(), st[yk].data_ptr(), st[vxk].data_ptr(),
@@ -269,6 +275,22 @@ class NBodyPM:
             if t:
                 p.call("sss_pm2d_to_f32", st["tx"].data_ptr(), t, row[4 * n:4 * n + t].data_ptr())
                 p.call("sss_pm2d_to_f32", st["ty"].data_ptr(), t, row[4 * n + t:].data_ptr())
+        return snap.cpu().numpy()
+
+    def _step_native(self, st: dict, dt: float, steps: int, snap: torch.Tensor) -> np.ndarray:
+        b = _lib.Pm2dBodies()
+        for k, pre in enumerate(("", "t")):
+            for f in ("x", "y", "vx", "vy", "ax", "ay"):
+                a = st[pre + f] if k == 0 or st["T"] else None
+                getattr(b, f)[k] = a.data_ptr() if a is not None else None
+        b.m = st["m"].data_ptr()
+        b.n, b.t = st["N"], st["T"]
+        kh = ctypes.c_double(-1.0 if self._kernel_h is None else self._kernel_h)
+        p = self._plan
+        p.kernel_key = None                     # the plan's kernels follow the steps
+        p.call("sss_pm2d_step_batch", ctypes.byref(b), dt, int(steps), self.softening_zellen, self.rand_zellen,
+               self.G, ctypes.byref(kh), snap.data_ptr())
+        self._kernel_h = kh.value
         return snap.cpu().numpy()
 
     def export_f64(self, st: dict) -> np.ndarray:

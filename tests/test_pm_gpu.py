@@ -187,3 +187,38 @@ def test_convolution_of_every_length(n):
         scale = max(float(w.abs().max()) for w in want)
         for got, ref in zip((ax, ay), want):
             assert float((got - ref).abs().max()) <= 1e-10 * scale
+
+
+@pytest.mark.parametrize("n,tracers,grid", [(1, 0, 32), (2, 1, 64), (300, 0, 96), (513, 700, 512), (5000, 260, 1000)])
+def test_native_steps_equal_the_parts(n, tracers, grid):
+    """A batch of steps in one native call against the same steps through the
+    parts (geometry read back by the host): the deposit's atomics may order
+    differently, nothing else does. Two batches, the second after the cloud
+    has shrunk by a factor (the kernels' cell size follows)."""
+    pk = _pk()
+    rng = np.random.default_rng(grid)
+    x, y, vx, vy = rng.uniform(-1, 1, (4, n + tracers))
+    m = rng.uniform(0.5, 1.5, n) * 1e-3
+    sims, sts = [], []
+    for native in (True, False):
+        sim = pk.NBodyPM([0], grid_n=grid)
+        sim._plan.native_steps = native
+        st = sim.load_state(x[:n], y[:n], vx[:n], vy[:n], m, tracer=(x[n:], y[n:], vx[n:], vy[n:]))
+        sims.append(sim)
+        sts.append(st)
+    for batch in range(2):
+        rows = []
+        for native, sim, st in zip((True, False), sims, sts):
+            sim._plan.native_steps = native
+            rows.append(sim.step_batch(st, 1e-3, 3))
+            assert sim._kernel_h is not None
+        a, b = (sim.export_f64(st) for sim, st in zip(sims, sts))
+        assert np.abs(a - b).max() <= 1e-11 * np.abs(b).max()
+        assert np.allclose(rows[0], rows[1], rtol=2e-7, atol=2e-7 * np.abs(rows[1]).max())
+        for k in ("ax", "ay") + (("tx", "tvy", "tax") if tracers else ()):
+            p, q = (st[k].cpu().numpy() for st in sts)
+            assert np.abs(p - q).max() <= 1e-10 * max(np.abs(q).max(), 1e-300)
+        for st in sts:
+            for k in ("x", "y"):
+                st[k].mul_(0.5)
+    sims[0]._plan.native_steps = True
