@@ -63,6 +63,15 @@ constexpr int WS_R_F64 = 2, WS_R_MIX = 4;
 constexpr int WS_MINB_F64 = 4, WS_MINB_MIX = 2;
 constexpr double SPLIT_PAIRS_F64 = 3e8, SPLIT_PAIRS_MIX = 4.5e8;
 
+// lane kernels (a warp per target): fewer than LANE_PAIRS pairs. Above, a target's
+// sources read by one warp from L1 cost more than the warp-split kernels' tiles
+// (us per evaluation among others, warp-split / lanes):
+//   mixed 2-D  300^2 6.2 / 4.1, 600^2 6.8 / 6.2, 1,000^2 7.9 / 8.2, 2,000^2 10.0 / 14.1
+//   mixed 3-D  100^2 6.1 / 4.1, 300^2 6.2 / 5.1, 600^2 7.6 / 6.2, 1,000^2 8.2 / 10.2
+//   f64 3-D    100^2 6.2 / 4.1, 300^2 7.1 / 6.2, 600^2 7.1 / 8.2 (2-D: 300^2 6.2 / 6.1, 600^2 6.4 / 7.8)
+constexpr int LN_NT = 256, LN_U = 4;
+constexpr double LANE_PAIRS_F64 = 1.5e5, LANE_PAIRS_MIX = 5e5;
+
 using sss_ap::Epi;
 using sss_ap::epilogue;
 
@@ -745,6 +754,63 @@ __global__ void __launch_bounds__(WS_NT, WS_MINB_MIX) k_force_mixed_ws(const For
     ws_finish<D, R>(a, tb, ch, reinterpret_cast<double*>(smem), ax, ay, az);
 }
 
+// A warp per target, its lanes over the sources: the smallest evaluations. No
+// tile, no centre, no partial sums between CTAs; a source's offset is formed
+// in f64 and rounded to f32 (mixed), the f32 sums of LN_U sources a lane fold
+// into f64, and the lanes meet in one butterfly. Bound by latency (a launch,
+// one load, n / 32 pairs, five shuffles).
+template <int D, bool MIXED>
+__global__ void __launch_bounds__(LN_NT) k_force_lanes(const ForceArgs a) {
+    const int lane = threadIdx.x & 31;
+    const int64_t i = (int64_t)blockIdx.x * (LN_NT / 32) + (threadIdx.x >> 5);
+    if (i >= a.n_tgt) return;
+    const double4 p = a.tgt[i];
+    const float epsf = (float)a.eps2;
+    double sx = 0.0, sy = 0.0, sz = 0.0;
+    for (int64_t j0 = lane; j0 < a.n_src; j0 += 32 * LN_U) {
+        double4 v[LN_U];
+        bool ok[LN_U];
+#pragma unroll
+        for (int u = 0; u < LN_U; ++u) {
+            ok[u] = j0 + 32 * u < a.n_src;
+            v[u] = ok[u] ? a.src[j0 + 32 * u] : make_double4(0.0, 0.0, 0.0, 0.0);
+        }
+        if (MIXED) {
+            float fx = 0.f, fy = 0.f, fz = 0.f;
+#pragma unroll
+            for (int u = 0; u < LN_U; ++u) {
+                const float dx = __double2float_rn(v[u].x - p.x), dy = __double2float_rn(v[u].y - p.y);
+                const float dz = D == 3 ? __double2float_rn(v[u].z - p.z) : 0.f;
+                const float r2 = D == 3 ? fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, epsf))) : fmaf(dx, dx, fmaf(dy, dy, epsf));
+                const float inv = sss_rsqrt_approx_f32(ok[u] ? r2 : 1.0f);
+                const float f = __double2float_rn(v[u].w) * ((inv * inv) * inv);     // (no source: 0)
+                fx = fmaf(f, dx, fx);
+                fy = fmaf(f, dy, fy);
+                if (D == 3) fz = fmaf(f, dz, fz);
+            }
+            sx += (double)fx;
+            sy += (double)fy;
+            if (D == 3) sz += (double)fz;
+        } else {
+#pragma unroll
+            for (int u = 0; u < LN_U; ++u) {
+                const double dx = v[u].x - p.x, dy = v[u].y - p.y, dz = D == 3 ? v[u].z - p.z : 0.0;
+                const double r2 = fma(dx, dx, fma(dy, dy, fma(dz, dz, a.eps2)));
+                const double f = rinv3<false>(v[u].w, ok[u] ? r2 : 1.0);
+                sx = fma(f, dx, sx);
+                sy = fma(f, dy, sy);
+                if (D == 3) sz = fma(f, dz, sz);
+            }
+        }
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        sx += __shfl_xor_sync(0xffffffffu, sx, o);
+        sy += __shfl_xor_sync(0xffffffffu, sy, o);
+        if (D == 3) sz += __shfl_xor_sync(0xffffffffu, sz, o);
+    }
+    if (lane == 0) epilogue<D>(a.epi, i, sx, sy, sz, p);
+}
+
 // ------------------------------------------------------------- potential
 
 // phi_t = -sum_s Gm_s / sqrt(|d|^2 + eps2), f64, one target per thread,
@@ -846,12 +912,26 @@ struct KSel {
     int key;           // index of its cached occupancy (0 .. SSS_AP_KERNELS - 1)
     bool mixed;        // takes the tiles k_prep_mixed writes
     bool ws;           // warp-split (make_plan_ws)
+    bool lanes;        // a warp per target (one chunk)
 };
 
 KSel select_kernel(int dim, int precision, int64_t n_src, int64_t n_tgt) {
     KSel k;
     k.mixed = (precision == SSS_PREC_MIXED);
-    k.ws = (double)n_src * (double)n_tgt < (k.mixed ? SPLIT_PAIRS_MIX : SPLIT_PAIRS_F64);
+    const double pairs = (double)n_src * (double)n_tgt;
+    k.ws = pairs < (k.mixed ? SPLIT_PAIRS_MIX : SPLIT_PAIRS_F64);
+    k.lanes = pairs < (k.mixed ? LANE_PAIRS_MIX : LANE_PAIRS_F64);
+    if (k.lanes) {
+        if (k.mixed) k.fn = (dim == 3) ? (void*)k_force_lanes<3, true> : (void*)k_force_lanes<2, true>;
+        else k.fn = (dim == 3) ? (void*)k_force_lanes<3, false> : (void*)k_force_lanes<2, false>;
+        k.nt = LN_NT;
+        k.tpb = LN_NT / 32;
+        k.ts = 1;
+        k.smem = 0;
+        k.key = (k.mixed ? 12 : 10) + (dim == 3);
+        k.mixed = false;
+        return k;
+    }
     if (k.ws) {
         if (k.mixed)
             k.fn = (dim == 3) ? (void*)k_force_mixed_ws<3, WS_R_MIX> : (void*)k_force_mixed_ws<2, WS_R_MIX>;
@@ -883,6 +963,11 @@ KSel select_kernel(int dim, int precision, int64_t n_src, int64_t n_tgt) {
     k.smem = 2 * (size_t)F64_TS * sizeof(double4);
     k.key = dim == 3;
     return k;
+}
+
+Plan plan_of(const KSel& ks, int64_t n_src, int64_t n_tgt, int slots) {
+    if (ks.lanes) return Plan{(int)((n_tgt + ks.tpb - 1) / ks.tpb), 0, 1, 0};
+    return ks.ws ? make_plan_ws(n_src, n_tgt, ks.tpb, slots) : make_plan(n_src, n_tgt, ks.tpb, ks.ts, slots);
 }
 
 // Bytes of mixed-precision tile copies and tile centres for n_tiles tiles.
@@ -923,7 +1008,7 @@ int force_eval(sss_ctx* ctx, int dim, int precision, const double4* src, int64_t
         ctx->occ[ks.key] = per_sm;
     }
     const int slots = ctx->occ[ks.key] * ctx->num_sms;
-    const Plan pl = ks.ws ? make_plan_ws(n_src, n_tgt, ks.tpb, slots) : make_plan(n_src, n_tgt, ks.tpb, ks.ts, slots);
+    const Plan pl = plan_of(ks, n_src, n_tgt, slots);
 
     ForceArgs a;
     memset(&a, 0, sizeof(a));
@@ -1177,11 +1262,13 @@ int noalloc_setup(int device, NoAllocDevice** out, char* eb, size_t el) {
         } else {
             d->base = (unsigned char*)p;
             e = cudaDeviceGetAttribute(&d->num_sms, cudaDevAttrMultiProcessorCount, device);
-            // one size for the few-pairs and one for the general kernels
-            const int64_t probe_n[2] = {1, (int64_t)1 << 20};
+            // one size for each kind of kernel
+            const int64_t probe_n[3] = {1, 16384, (int64_t)1 << 20};
+            static_assert(16384.0 * 16384.0 >= LANE_PAIRS_F64 && 16384.0 * 16384.0 >= LANE_PAIRS_MIX &&
+                          16384.0 * 16384.0 < SPLIT_PAIRS_F64 && 16384.0 * 16384.0 < SPLIT_PAIRS_MIX, "probe sizes");
             for (int prec = 0; prec < 2 && e == cudaSuccess; ++prec)
                 for (int dim = 2; dim <= 3 && e == cudaSuccess; ++dim)
-                    for (int q = 0; q < 2 && e == cudaSuccess; ++q) {
+                    for (int q = 0; q < 3 && e == cudaSuccess; ++q) {
                         const KSel ks = select_kernel(dim, prec, probe_n[q], probe_n[q]);
                         e = query_occupancy(ks, &d->occ[ks.key]);
                     }
@@ -1225,7 +1312,7 @@ extern "C" int sss_allpairs_accel_noalloc(int device, int dim, int precision, co
 
     const KSel ks = select_kernel(dim, precision, n_src, n_tgt);
     const int slots = d->occ[ks.key] * d->num_sms;
-    Plan pl = ks.ws ? make_plan_ws(n_src, n_tgt, ks.tpb, slots) : make_plan(n_src, n_tgt, ks.tpb, ks.ts, slots);
+    Plan pl = plan_of(ks, n_src, n_tgt, slots);
 
     // scratch layout: [status 256 B][counters 64 KiB][tiles][centres][partials]
     const size_t data_off = SSS_NOALLOC_STATUS_BYTES + SSS_NOALLOC_COUNTERS * sizeof(unsigned);

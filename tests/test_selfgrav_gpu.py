@@ -303,3 +303,14 @@ def test_few_pairs_kernels(dim, n_src, n_tgt, equal):
     scale = (src[None, :, 3] / r2 * (1e-6 + 3.0 * np.sqrt(3.0) * 2.0 * 2.0 ** -24 / np.sqrt(r2))).sum(1)
     a = sg.allpairs_accel(*dev, eps * eps, dim=dim, precision="mixed").cpu().numpy()[sel]
     assert np.all(np.abs(a[:, :dim] - ref[:, :dim]).max(1) <= scale)
+
+
+@pytest.mark.parametrize("dim", [2, 3])
+@pytest.mark.parametrize("n_src,n_tgt", [(1, 1), (31, 8), (32, 9), (127, 7), (129, 1000), (300, 300), (705, 705),
+                                         (710, 710), (63, 9001), (513, 1100), (8193, 65), (127, 5000)])
+@pytest.mark.parametrize("equal", [True, False])
+def test_smallest_evaluations(dim, n_src, n_tgt, equal):
+    """A warp per target (below 1.5e5 pairs in f64, 5e5 in mixed): fewer
+    sources than lanes, remainders of the 128 a pass takes and of the 8 targets
+    a block takes; and the warp-split kernels' edges at sizes just above."""
+    test_few_pairs_kernels(dim, n_src, n_tgt, equal)
