@@ -60,7 +60,8 @@ __device__ __forceinline__ void team_accel(const double (&px)[B][3], const doubl
             double r2 = fma(dx, dx, fma(dy, dy, fma(dz, dz, eps2)));
             const bool self = (i == j) || (i >= n);
             if (self) r2 = 1.0;
-            const double f = sss_gm_rinv3(self ? 0.0 : gm, r2);
+            const double inv = rsqrt(r2);
+            const double f = self ? 0.0 : ((gm * inv) * inv) * inv;
             acc[b][0] = fma(f, dx, acc[b][0]);
             acc[b][1] = fma(f, dy, acc[b][1]);
             if (D == 3) acc[b][2] = fma(f, dz, acc[b][2]);
@@ -126,69 +127,69 @@ __global__ void __launch_bounds__(128) k_batched(const BatchArgs a) {
     }
 }
 
-// Block of T threads per system, for the larger groups. Thread t + n c takes
-// target t and the sources j = c, c + S, ... with S = T / n chunks (at most 8):
-// packed by the system's own n, 80-100 % of the threads work where rows of 16,
-// 32 or 64 targets left up to half of them idle (n = 33 of 64). Positions and
-// G m in shared memory (one or two addresses a warp), the S partial forces of
-// a target added in chunk order. A force evaluation is n / S dependent pair
-// iterations instead of n, with S times the warps in flight. Pair formula and
-// KDK as in k_batched. Bound by the FP64 pipe: 16 instructions a pair.
-constexpr int BLK_N = 64, BLK_S = 8;
-
-template <int D, int T>
-__global__ void __launch_bounds__(T) k_batched_blk(const BatchArgs a) {
-    __shared__ double4 sp[BLK_N];
-    __shared__ double sa[BLK_S][3][BLK_N];
-    const int tid = threadIdx.x;
+// Block per system, for the larger groups (NT = 16, 32 or 64 targets):
+// thread (t, c) of NT * S takes
+// target t and the sources j = c, c + S, c + 2S, ...; positions and masses
+// in shared memory, the S partial forces of a target added in chunk order.
+// A force evaluation is n / S dependent pair iterations instead of n, with
+// S times the warps in flight. Pair formula and KDK as in k_batched.
+template <int D, int NT, int S>
+__global__ void __launch_bounds__(NT * S) k_batched_blk(const BatchArgs a) {
+    __shared__ double4 sp[NT];
+    __shared__ double sa[S][3][NT];
+    const int t = threadIdx.x % NT, c = threadIdx.x / NT;
     const double wd[3] = {a.w1, a.w0, a.w1};
     for (int q = blockIdx.x; q < a.n_list; q += gridDim.x) {
         const int sys = a.sys_list[q];
         const int64_t o = a.off[sys];
         const int n = (int)(a.off[sys + 1] - o);
-        if (n > BLK_N || n > T || n < 1) continue;     // the host maps groups to blocks that hold them
-        const int S = min(T / n, BLK_S);
-        const int c = tid / n, t = tid - c * n;
-        const double dt = a.dt[sys];
-        const bool own = tid < n;
-        double px[3] = {0.0, 0.0, 0.0}, pv[3] = {0.0, 0.0, 0.0}, gm = 0.0, acc[3] = {0.0, 0.0, 0.0};
+        if (n > NT) continue;         // the host maps groups to blocks that hold them
+        const double G = a.G[sys], dt = a.dt[sys];
+        const bool own = c == 0 && t < n;
+        double px[3] = {0.0, 0.0, 0.0}, pv[3] = {0.0, 0.0, 0.0}, pm = 0.0, acc[3] = {0.0, 0.0, 0.0};
         if (own) {
             for (int k = 0; k < D; ++k) {
                 px[k] = a.x[k][o + t];
                 pv[k] = a.v[k][o + t];
             }
-            gm = a.G[sys] * a.m[o + t];
+            pm = a.m[o + t];
         }
         __syncthreads();                              // the previous system's last reads of sp / sa
-        if (own) sp[t] = make_double4(px[0], px[1], px[2], gm);
+        if (c == 0) sp[t] = make_double4(px[0], px[1], px[2], pm);
         auto accel = [&]() {
             __syncthreads();                          // positions written
-            if (c < S) {
-                const double4 me = sp[t];
-                double ax = 0.0, ay = 0.0, az = 0.0;
-#pragma unroll 4
+            const double4 me = sp[t];
+            double ax = 0.0, ay = 0.0, az = 0.0;
+            if (t < n) {
                 for (int j = c; j < n; j += S) {
                     const double4 sj = sp[j];
                     const double dx = sj.x - me.x, dy = sj.y - me.y;
                     const double dz = (D == 3) ? sj.z - me.z : 0.0;
-                    const double r2 = fma(dx, dx, fma(dy, dy, fma(dz, dz, a.eps2)));
+                    double r2 = fma(dx, dx, fma(dy, dy, fma(dz, dz, a.eps2)));
                     const bool self = j == t;
-                    const double f = sss_gm_rinv3(self ? 0.0 : sj.w, self ? 1.0 : r2);
+                    if (self) r2 = 1.0;
+                    const double inv = rsqrt(r2);
+                    const double f = self ? 0.0 : ((G * sj.w * inv) * inv) * inv;
                     ax = fma(f, dx, ax);
                     ay = fma(f, dy, ay);
                     if (D == 3) az = fma(f, dz, az);
                 }
-                sa[c][0][t] = ax;
-                sa[c][1][t] = ay;
-                if (D == 3) sa[c][2][t] = az;
             }
-            __syncthreads();                          // partials written, positions read
-            if (own) {
-                for (int k = 0; k < D; ++k) acc[k] = sa[0][k][t];
+            sa[c][0][t] = ax;
+            sa[c][1][t] = ay;
+            sa[c][2][t] = az;
+            __syncthreads();                          // partials written
+            if (c == 0) {
+                double r0 = 0.0, r1 = 0.0, r2 = 0.0;
 #pragma unroll
-                for (int s = 1; s < BLK_S; ++s)
-                    if (s < S)
-                        for (int k = 0; k < D; ++k) acc[k] += sa[s][k][t];
+                for (int k = 0; k < S; ++k) {
+                    r0 += sa[k][0][t];
+                    r1 += sa[k][1][t];
+                    r2 += sa[k][2][t];
+                }
+                acc[0] = r0;
+                acc[1] = r1;
+                acc[2] = r2;
             }
         };
         accel();
@@ -197,15 +198,16 @@ __global__ void __launch_bounds__(T) k_batched_blk(const BatchArgs a) {
             for (int w = 0; w < 3; ++w) {
                 const double h = wd[w] * dt;
                 const double hh = 0.5 * h;
-                if (own) {
+                if (c == 0) {
                     for (int k = 0; k < D; ++k) {
                         pv[k] += acc[k] * hh;
                         px[k] += pv[k] * h;
                     }
-                    sp[t] = make_double4(px[0], px[1], px[2], gm);
                 }
+                __syncthreads();                      // everyone is done reading sp
+                if (c == 0) sp[t] = make_double4(px[0], px[1], px[2], pm);
                 accel();
-                if (own)
+                if (c == 0)
                     for (int k = 0; k < D; ++k) pv[k] += acc[k] * hh;
             }
         }
@@ -217,18 +219,13 @@ __global__ void __launch_bounds__(T) k_batched_blk(const BatchArgs a) {
     }
 }
 
-// T threads for systems of up to nt = 16, 32 or 64 bodies: 2 to 8 chunks of the largest
 template <int D>
-void* pick_blk(int nt, int T) {
-    const int S = T / nt;
-    if (S < 2 || S > 8 || (nt == 16 && S < 4)) return nullptr;
-    switch (T) {
-        case 64: return (void*)k_batched_blk<D, 64>;
-        case 128: return (void*)k_batched_blk<D, 128>;
-        case 256: return (void*)k_batched_blk<D, 256>;
-        case 512: return (void*)k_batched_blk<D, 512>;
-        default: return nullptr;
-    }
+void* pick_blk(int NT, int S) {
+#define SSS_BLK(nt, s) if (NT == nt && S == s) return (void*)k_batched_blk<D, nt, s>;
+    SSS_BLK(16, 4) SSS_BLK(16, 8) SSS_BLK(32, 2) SSS_BLK(32, 4) SSS_BLK(32, 8) SSS_BLK(64, 2) SSS_BLK(64, 4)
+    SSS_BLK(64, 8)
+#undef SSS_BLK
+    return nullptr;
 }
 
 template <int D>
@@ -255,13 +252,13 @@ extern "C" int sss_batched_launch(sss_ctx* ctx, int dim, double* const* x, doubl
     if (n_list < 0 || steps < 0) return sss_set_err(ctx, SSS_ERR_ARG, "negative count");
     if (n_list == 0 || steps == 0) return SSS_OK;
     if (!x || !v || !m || !off || !G || !dt || !sys_list) return sss_set_err(ctx, SSS_ERR_ARG, "NULL argument");
-    // team > 32: a block of that many threads per system, 2 to 8 times 16, 32 or 64 (by max_n)
+    // team > 32: a block per system, NT = 16, 32 or 64 targets (by max_n) x S = team / NT source chunks
     const bool blk = team > 32;
     const int nt = max_n <= 16 ? 16 : (max_n <= 32 ? 32 : 64);
     void* fn = nullptr;
     if (blk) {
         if (per_lane == 1 && team % nt == 0)
-            fn = (dim == 3) ? pick_blk<3>(nt, team) : pick_blk<2>(nt, team);
+            fn = (dim == 3) ? pick_blk<3>(nt, team / nt) : pick_blk<2>(nt, team / nt);
     } else {
         fn = (dim == 3) ? pick<3>(team, per_lane) : pick<2>(team, per_lane);
     }

@@ -153,7 +153,8 @@ __device__ __forceinline__ double sss_gm_rinv3(double gm, double r2) {
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(c) : "d"(r2));
     const double c2 = c * c;
     double e = fma(-r2, c2, 1.0);
-    if (__double2hiint(c) == 0) e = 0.0;         // r2 = +inf: -inf * 0
+    // r2 = +inf: -inf * 0 is NaN, whose low word alone is a number near 0
+    e = __hiloint2double(__double2hiint(c) == 0 ? 0 : __double2hiint(e), __double2loint(e));
     const double p = fma(e, 1.875, 1.5);
     const double g3 = (gm * c) * c2;
     return fma(g3, e * p, g3);
