@@ -95,7 +95,8 @@ __device__ __forceinline__ int pp_chunks(const int* first, const int* last, long
 // (cell, first target) of every item into the list of its class (thread per
 // cell; an item's length falls along its cell, so a class is one stretch)
 __global__ void k_pp_items(const int* __restrict__ first, const int* __restrict__ last, int M, long long cells,
-                           long long max_items, int2* __restrict__ items, unsigned* __restrict__ n_items) {
+                           long long max_items, bool two, int2* __restrict__ items,
+                           unsigned* __restrict__ n_items) {
     const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= cells) return;
     const int g = pp_chunks(first, last, c);
@@ -108,7 +109,7 @@ __global__ void k_pp_items(const int* __restrict__ first, const int* __restrict_
         const long long nc = ((long long)nz * M + ny) * M + nx;
         if (nc > c) near += pp_chunks(first, last, nc);
     }
-    const int step = near + g >= PP_LONG ? 1 : 2;           // groups of 32 targets an item takes
+    const int step = !two || near + g >= PP_LONG ? 1 : 2;           // groups of 32 targets an item takes
     const int tag = (int)c | (step == 2 ? PP_TWO : 0);
     const int gi = (g + step - 1) / step;
     for (int k = 0; k < gi;) {
@@ -559,7 +560,17 @@ extern "C" int sss_pm3_short(sss_pm3* p, const sss_pm3_particles* s, double G, d
     k_pp_bounds<<<blocks_for(n, 256), 256, 0, st>>>(k0, n, first, last);
     SSS_LAUNCH_CHECK(ctx, "k_pp_bounds");
     SSS_CUDA_TRY(ctx, cudaMemsetAsync(counters, 0, 4 * (PP_CLASSES + 1), st));
-    k_pp_items<<<blocks_for(cells, 128), 128, 0, st>>>(first, last, M, cells, max_items, items, counters);
+    // the polynomial's range is t <= 9; without a softening in f32 there is no r < eps test
+    const bool poly = alpha * r_cut <= 3.0000001 && (float)(eps * eps) > 0.0f;
+    void (*pairs)(const PPArgs) = poly ? (s->m ? k_pp_pairs<true, false> : k_pp_pairs<true, true>)
+                                       : (s->m ? k_pp_pairs<false, false> : k_pp_pairs<false, true>);
+    int per_sm = 0;
+    SSS_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pairs, PP_WARPS * 32, 0));
+    // items of 64 targets only where they still fill the warps twice: fewer particles are bound by the
+    // length of an item (us a pair pass, all of 32 / light cells of 64: 16,384 uniform 703 / 1083,
+    // 131,072 uniform 684 / 1055; 442,368 uniform 1796 either way)
+    const bool two = n >= 2LL * 64 * PP_WARPS * per_sm * ctx->num_sms;
+    k_pp_items<<<blocks_for(cells, 128), 128, 0, st>>>(first, last, M, cells, max_items, two, items, counters);
     SSS_LAUNCH_CHECK(ctx, "k_pp_items");
     PPArgs q;
     q.src = src;
@@ -581,12 +592,6 @@ extern "C" int sss_pm3_short(sss_pm3* p, const sss_pm3_particles* s, double G, d
     q.acc = (float*)(B + o_acc);
     q.n = n;
     SSS_CUDA_TRY(ctx, cudaMemsetAsync(q.acc, 0, 12 * (size_t)n, st));
-    // the polynomial's range is t <= 9; without a softening in f32 there is no r < eps test
-    const bool poly = alpha * r_cut <= 3.0000001 && q.eps2 > 0.0f;
-    void (*pairs)(const PPArgs) = poly ? (s->m ? k_pp_pairs<true, false> : k_pp_pairs<true, true>)
-                                       : (s->m ? k_pp_pairs<false, false> : k_pp_pairs<false, true>);
-    int per_sm = 0;
-    SSS_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pairs, PP_WARPS * 32, 0));
     const unsigned grid = (unsigned)(ctx->num_sms * std::max(per_sm, 1));
     pairs<<<grid, PP_WARPS * 32, 0, st>>>(q);
     SSS_LAUNCH_CHECK(ctx, "k_pp_pairs");
