@@ -224,6 +224,16 @@ __global__ void __launch_bounds__(Tile16<N>::NT, 1024 / Tile16<N>::NT) k_y_fwd(c
                                      [&](int i, int, float2 z, bool) { p[i * T::PITCH] = z; });
 }
 
+// 1 / d for a normal d > 0: the hardware's coarse reciprocal and two Newton
+// steps r (2 - d r). No branch, so the 16 modes of a thread overlap; with a
+// division each (its slow path a branch) the 64^3 pass took 14 us.
+__device__ __forceinline__ double recip(double d) {
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+    r = fma(r, fma(-d, r, 1.0), r);
+    return fma(r, fma(-d, r, 1.0), r);
+}
+
 // a_x = i k_x c rho_k and phi' = c rho_k (c as in k_spectrum3), both inverse
 // transformed along x; plane = iy.
 template <int N>
@@ -244,7 +254,7 @@ k_x_solve(const float2* __restrict__ tw, const float2* __restrict__ rk, double c
                          [&](int i, int c, float2 r, bool) {
                              float2 a = make_float2(0.f, 0.f), b = a;
                              if (!mean || i != 0) {
-                                 const double q = cyz * __ldg(tab + 2 * N + i) / (k2yz + __ldg(tab + N + i));
+                                 const double q = cyz * __ldg(tab + 2 * N + i) * recip(k2yz + __ldg(tab + N + i));
                                  const double f = __ldg(tab + i) * q;
                                  a = make_float2((float)(-f * (double)r.y), (float)(f * (double)r.x));
                                  b = make_float2((float)(q * (double)r.x), (float)(q * (double)r.y));
@@ -262,48 +272,46 @@ k_x_solve(const float2* __restrict__ tw, const float2* __restrict__ rk, double c
     }
 }
 
-// Along y: a_x, phi -> a_y = i k_y phi in phi's place, and phi to the third
-// mesh (its k_z comes with the z pass); plane = ix.
+// Along y, component blockIdx.y of a_x (in place), phi -> a_y = i k_y phi (the
+// density spectrum's buffer, free by now) and phi itself for the third one (its
+// k_z comes with the z pass); plane = ix. The three are blocks of their own: one
+// block after another on the same tile, a 64^3 pass took 9 us.
 template <int N>
 __global__ void __launch_bounds__(Tile16<N>::NT, 1024 / Tile16<N>::NT)
-k_y_inv(const float2* __restrict__ tw, const double* __restrict__ tab, float2* ax, float2* phi,
-        float2* __restrict__ third) {
+k_y_inv(const float2* __restrict__ tw, const double* __restrict__ tab, float2* ax, const float2* __restrict__ phi,
+        float2* __restrict__ ay, float2* __restrict__ third) {
     using T = Tile16<N>;
     using Map = typename T::Map;
     extern __shared__ float2 smf[];
     const T t;
     const long long o = (long long)t.plane * N * T::PITCH + t.iz;
-    // one body of code for the three (three in a row kept each other's addresses in registers)
-#pragma unroll 1
-    for (int d = 0; d < 3; ++d) {
-        const float2* in = (d == 0 ? ax : phi) + o;
-        float2* out = (d == 0 ? ax : d == 1 ? third : phi) + o;
-        fft::run<N, 1, Map>(tw, smf,
-                            [&](int i, int, bool) {
-                                float2 z = in[i * T::PITCH];
-                                if (d == 2) {
-                                    const float k = (float)__ldg(tab + i);
-                                    z = make_float2(-k * z.y, k * z.x);
-                                }
-                                return z;
-                            },
-                            [&](int i, int, float2 z, bool) { out[i * T::PITCH] = z; });
-        __syncthreads();
-    }
+    const int d = blockIdx.y;
+    const float2* in = (d == 0 ? ax : phi) + o;
+    float2* out = (d == 0 ? ax : d == 1 ? ay : third) + o;
+    fft::run<N, 1, Map>(tw, smf,
+                        [&](int i, int, bool) {
+                            float2 z = in[i * T::PITCH];
+                            if (d == 1) {
+                                const float k = (float)__ldg(tab + i);
+                                z = make_float2(-k * z.y, k * z.x);
+                            }
+                            return z;
+                        },
+                        [&](int i, int, float2 z, bool) { out[i * T::PITCH] = z; });
 }
 
 // Half spectra along z of two rows -> the rows: one complex transform of
 // a + i b. blockIdx.y = component; the third one takes its i k_z here.
 template <int N>
 __global__ void __launch_bounds__(Rows16<N>::NT, 1024 / Rows16<N>::NT)
-k_z_inv(const float2* __restrict__ tw, const double* __restrict__ tab, const float2* __restrict__ ak,
-        float* __restrict__ acc) {
+k_z_inv(const float2* __restrict__ tw, const double* __restrict__ tab, const float2* __restrict__ ax,
+        const float2* __restrict__ ay, const float2* __restrict__ az, float* __restrict__ acc) {
     using R = Rows16<N>;
     using Map = typename R::Map;
     extern __shared__ float2 smf[];
     const int d = blockIdx.y;
     const long long row0 = (long long)blockIdx.x * 32;
-    const float2* src = ak + ((long long)d * N * N + row0) * R::PITCH;
+    const float2* src = (d == 0 ? ax : d == 1 ? ay : az) + row0 * R::PITCH;
 #pragma unroll 4
     for (int q = threadIdx.x; q < 16 * R::NH; q += R::NT) {
         const int c = q / R::NH, k = q - c * R::NH;
@@ -343,8 +351,8 @@ cudaError_t solve_of(sss_pm3* p, double cscale, bool setup, cudaStream_t st) {
     k_z_fwd<N><<<R::TILES, R::NT, R::SMEM, st>>>(p->tw, p->rho, p->rk);
     k_y_fwd<N><<<T::TILES, T::NT, T::SMEM, st>>>(p->tw, p->rk);
     k_x_solve<N><<<T::TILES, T::NT, 2 * T::SMEM, st>>>(p->tw, p->rk, cscale, p->tab, p->ak, p->ak + m);
-    k_y_inv<N><<<T::TILES, T::NT, T::SMEM, st>>>(p->tw, p->tab, p->ak, p->ak + m, p->ak + 2 * m);
-    k_z_inv<N><<<dim3(R::TILES, 3), R::NT, R::SMEM, st>>>(p->tw, p->tab, p->ak, p->acc);
+    k_y_inv<N><<<dim3(T::TILES, 3), T::NT, T::SMEM, st>>>(p->tw, p->tab, p->ak, p->ak + m, p->rk, p->ak + 2 * m);
+    k_z_inv<N><<<dim3(R::TILES, 3), R::NT, R::SMEM, st>>>(p->tw, p->tab, p->ak, p->rk, p->ak + 2 * m, p->acc);
     return cudaGetLastError();
 }
 
