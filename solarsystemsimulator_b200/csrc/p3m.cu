@@ -15,7 +15,7 @@
 //   sort    : stable radix sort by cell (devscan.cuh), particles gathered in
 //             that order as (x, y, z, m)
 //   bounds  : first and last sorted particle of every cell
-//   items   : one work item per group of 64 or 32 particles of a cell (cells
+//   items   : one work item per group of 32 particles of a cell (cells
 //             hold from none to many thousands in a clustered state), listed
 //             by the power of two of its source chunks, longest first
 //   pairs   : persistent warps take items from a counter (a dense cell's
@@ -26,8 +26,7 @@
 //             higher index (13 or so of the 26, periodic). The sources are
 //             staged through the warp's shared memory in chunks of 32,
 //             relative to the item's cell corner, so that f32 differences
-//             keep the positions' resolution; a lane holds two targets (64
-//             particles an item); lane l meets sources (l + k)
+//             keep the positions' resolution; lane l meets sources (l + k)
 //             and (l + k + 16) mod 32 at step k, in packed f32x2 arithmetic,
 //             and the sources' sums rotate through the lanes with them, so
 //             that both sides accumulate in registers. Both go to an f32
@@ -80,13 +79,11 @@ __global__ void k_pp_bounds(const unsigned long long* __restrict__ keys, long lo
 // chunks of 32 its warp walks: the later ones of its cell and those of the
 // neighbouring cells of higher index; class = floor(log2(length)). The
 // warps take the longest class first: an item of a collapsed halo's cell is
-// one warp's work for milliseconds, and the ones taken last set the tail. Items
-// have 64 targets (two per lane, which share the sources' loads and rotation);
-// in a cell whose first item is PP_LONG chunks or longer they have 32, since
-// there one warp's walk would bound the kernel.
+// one warp's work for milliseconds, and the ones taken last set the tail. (64
+// targets an item, two per lane sharing the sources' loads and rotation, halved
+// the items and gained nothing: 442,368 uniform particles 2065 us a pair pass
+// against 1796 before.)
 constexpr int PP_CLASSES = 16;
-constexpr int PP_LONG = 256;
-constexpr int PP_TWO = 1 << 30;                     // flag beside an item's cell (< 2^30): 64 targets
 
 __device__ __forceinline__ int pp_chunks(const int* first, const int* last, long long c) {
     return (last[c] - first[c] + 31) / 32;
@@ -95,8 +92,7 @@ __device__ __forceinline__ int pp_chunks(const int* first, const int* last, long
 // (cell, first target) of every item into the list of its class (thread per
 // cell; an item's length falls along its cell, so a class is one stretch)
 __global__ void k_pp_items(const int* __restrict__ first, const int* __restrict__ last, int M, long long cells,
-                           long long max_items, bool two, int2* __restrict__ items,
-                           unsigned* __restrict__ n_items) {
+                           long long max_items, int2* __restrict__ items, unsigned* __restrict__ n_items) {
     const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= cells) return;
     const int g = pp_chunks(first, last, c);
@@ -109,16 +105,14 @@ __global__ void k_pp_items(const int* __restrict__ first, const int* __restrict_
         const long long nc = ((long long)nz * M + ny) * M + nx;
         if (nc > c) near += pp_chunks(first, last, nc);
     }
-    const int step = !two || near + g >= PP_LONG ? 1 : 2;           // groups of 32 targets an item takes
-    const int tag = (int)c | (step == 2 ? PP_TWO : 0);
-    const int gi = (g + step - 1) / step;
+    const int gi = g;
     for (int k = 0; k < gi;) {
-        const long long len = near + g - step * k;          // >= 1
+        const long long len = near + g - k;                 // >= 1
         const int cls = min(PP_CLASSES - 1, 63 - __clzll(len));
         // down to length 2^cls the class stays the same (class 15 is open above)
-        const int run = (int)min((long long)(gi - k), (len - (1ll << cls)) / step + 1);
+        const int run = (int)min((long long)(gi - k), len - (1ll << cls) + 1);
         const unsigned at = atomicAdd(n_items + cls, (unsigned)run);
-        for (int j = 0; j < run; ++j) items[cls * max_items + at + j] = make_int2(tag, first[c] + 32 * step * (k + j));
+        for (int j = 0; j < run; ++j) items[cls * max_items + at + j] = make_int2((int)c, first[c] + 32 * (k + j));
         k += run;
     }
 }
@@ -133,7 +127,6 @@ struct PPArgs {
     double box;
     double G;
     float alpha, rc2, eps2;
-    float m;                        // the particles' common mass (UNI)
     const int2* items;              // PP_CLASSES lists of max_items
     const unsigned* n_items;        // their lengths
     long long max_items;
@@ -192,38 +185,14 @@ __device__ __forceinline__ f2x shfl2(f2x v, int from) {
 // coincident particles, where the erfc form is not finite) the caller
 // selects 0. Two pairs at a time in packed f32x2 arithmetic; the reciprocal
 // square roots, the exponential and the reciprocal are f32 MUFU operations.
-//
-// Where alpha r_cut <= 3 (k_pp_pairs<POLY>) pairs at r >= eps take a cheaper
-// form: (1 - g(x)) / x^3 = S(x^2) with S(t) = (4 / sqrt(pi)) int_0^1 u^2 e^{-t u^2} du,
-// entire and positive, so the first term is -alpha^3 S(alpha^2 r^2), S on [0, 9]
-// a polynomial of degree 12 in w = 1 - t / 9 (weighted minimax fit of that
-// integral, weight max(t^{3/2}, 0.6): the error counts relative to the Newtonian
-// term): 3.7e-7 at most, 9.3e-8 rms in f32, where the erfc form has 5.9e-7 and
-// 1.1e-7. It takes 17 FMA-pipe operations and one MUFU a pair against 21 and
-// four: the special function unit no longer bounds the kernel. A step (warp
-// uniform) with a pair closer than eps takes the erfc form, which keeps close
-// pairs' rounding as it was.
+// (A polynomial of (1 - g) / x^3 in x^2 instead of the erfc form, one MUFU a pair
+// instead of four and as exact, took a halo step from 12.3 to 9.7 ms, but its
+// rounding moved the f64 state by up to 1.5e-9 of itself: left out.)
 __device__ __forceinline__ f2x dup(float v) { return pk2(v, v); }
 
 struct PPConst {
     f2x alpha, eps2;
-    f2x w1, w0, na3;             // POLY: w = w0 + w1 (r^2 + eps^2), -alpha^3
-    float hi, lo;                // POLY: r^2 + eps^2 at r_cut, at r = eps
 };
-
-__device__ __forceinline__ f2x pp_h2_poly(f2x R2E, const PPConst& k) {
-    constexpr float C[13] = {0.0370207495f,  0.0553906112f, 0.0686928646f, 0.0762103807f, 0.108367381f,
-                             -0.0975710749f, 0.928968487f,  -2.53256823f,  5.40020339f,   -7.24256426f,
-                             6.4283471f,     -3.28619025f,  0.807945481f};
-    float s0, s1;
-    upk2(R2E, s0, s1);
-    const f2x SI = pk2(sss_rsqrt_approx_f32(s0), sss_rsqrt_approx_f32(s1));
-    const f2x W = fma2(R2E, k.w1, k.w0);
-    f2x P = dup(C[12]);
-#pragma unroll
-    for (int j = 11; j >= 0; --j) P = fma2(P, W, dup(C[j]));
-    return fma2(P, k.na3, mul2(mul2(SI, SI), SI));
-}
 
 __device__ __forceinline__ f2x pp_h2(f2x R2, f2x alpha, f2x eps2) {
     float r0, r1;
@@ -272,16 +241,14 @@ struct PPTarget {
 // 32); OWN masks offset 16 on lanes 16 .. 31 (32 particles among themselves,
 // whose pairs (l, l + 16) and (l + 16, l) coincide). Both sources' sums rotate
 // through the lanes and end on their own lanes, then go to the accumulator.
-// UNI: all masses equal; the sums leave the mass out until the end. FMA-pipe
-// bound: 26 operations a pair (28 with masses; erfc form 33 and 35), with the 6
-// shuffles and two 16-byte shared loads of a step shared by its 2 G pairs.
-// 1,048,576 particles collapsed into halos (7.2e9 candidate pairs, 5.1e9 in
-// range): 10.4 ms a step against 15.4 with the erfc
-// form alone, sources packed by register moves and items in cell order (the
-// last heavy items then ran on by themselves). All items of 32 targets: 10.4; all
-// of 64: 11.2 (a heavy cell's walk is the kernel's length). Sorting particles
+// 35 FMA-pipe operations and four special-function ones a pair (the latter
+// bound it), with the 6 shuffles and two 16-byte shared loads of a step shared
+// by its 2 G pairs. 1,048,576 particles collapsed into halos (7.2e9 candidate
+// pairs, 5.1e9 in range): 12.3 ms a step against 15.4 with sources packed by
+// register moves and items in cell order (the last heavy items then ran on by
+// themselves). Sorting particles
 // inside a cell and testing chunk boxes saves only a fifth of these pairs.
-template <int G, bool POLY, bool UNI, bool OWN, int A0, int A1, int DA>
+template <int G, bool OWN, int A0, int A1, int DA>
 __device__ __forceinline__ void pp_chunk2(const ulonglong2* stage, int lane, PPTarget (&T)[2], const PPConst& k,
                                           const PPArgs& q, long long src0, int m) {
     f2x BX = 0ull, BY = 0ull, BZ = 0ull;             // sums of sources (lane + a) and (lane + a + da)
@@ -290,49 +257,23 @@ __device__ __forceinline__ void pp_chunk2(const ulonglong2* stage, int lane, PPT
     for (int a = A0; a < A1; ++a) {
         const ulonglong2 xy = stage[(lane + a) & 31], zm = stage[32 + ((lane + a) & 31)];
         f2x DX[G], DY[G], DZ[G], H[G];
-        bool near = !POLY;
-        if (POLY) {
-            float least = 3e38f;
 #pragma unroll
-            for (int g = 0; g < G; ++g) {
-                DX[g] = add2(xy.x, T[g].nx);
-                DY[g] = add2(xy.y, T[g].ny);
-                DZ[g] = add2(zm.x, T[g].nz);
-                H[g] = fma2(DX[g], DX[g], fma2(DY[g], DY[g], fma2(DZ[g], DZ[g], k.eps2)));
-                float r0, r1;
-                upk2(H[g], r0, r1);
-                least = fminf(least, fminf(r0, r1));
-            }
-            near = __any_sync(0xffffffffu, least < k.lo);
-        }
-        if (POLY && !near) {
-#pragma unroll
-            for (int g = 0; g < G; ++g) {
-                float r0, r1, h0, h1;
-                upk2(H[g], r0, r1);
-                const bool in0 = r0 < k.hi, in1 = r1 < k.hi && !(OWN && a + DA == 16 && lane >= 16);
-                upk2(pp_h2_poly(H[g], k), h0, h1);
-                H[g] = pk2(in0 ? h0 : 0.0f, in1 ? h1 : 0.0f);
-            }
-        } else {
-#pragma unroll
-            for (int g = 0; g < G; ++g) {
-                DX[g] = add2(xy.x, T[g].nx);
-                DY[g] = add2(xy.y, T[g].ny);
-                DZ[g] = add2(zm.x, T[g].nz);
-                const f2x R2 = fma2(DX[g], DX[g], fma2(DY[g], DY[g], mul2(DZ[g], DZ[g])));
-                float r0, r1, h0, h1;
-                upk2(R2, r0, r1);
-                const bool in0 = r0 < q.rc2 && r0 > 0.0f;
-                const bool in1 = r1 < q.rc2 && r1 > 0.0f && !(OWN && a + DA == 16 && lane >= 16);
-                upk2(pp_h2(R2, k.alpha, k.eps2), h0, h1);
-                H[g] = pk2(in0 ? h0 : 0.0f, in1 ? h1 : 0.0f);
-            }
+        for (int g = 0; g < G; ++g) {
+            DX[g] = add2(xy.x, T[g].nx);
+            DY[g] = add2(xy.y, T[g].ny);
+            DZ[g] = add2(zm.x, T[g].nz);
+            const f2x R2 = fma2(DX[g], DX[g], fma2(DY[g], DY[g], mul2(DZ[g], DZ[g])));
+            float r0, r1, h0, h1;
+            upk2(R2, r0, r1);
+            const bool in0 = r0 < q.rc2 && r0 > 0.0f;
+            const bool in1 = r1 < q.rc2 && r1 > 0.0f && !(OWN && a + DA == 16 && lane >= 16);
+            upk2(pp_h2(R2, k.alpha, k.eps2), h0, h1);
+            H[g] = pk2(in0 ? h0 : 0.0f, in1 ? h1 : 0.0f);
         }
 #pragma unroll
         for (int g = 0; g < G; ++g) {
             PPTarget& t = T[g];
-            const f2x HJ = UNI ? H[g] : mul2(H[g], zm.y), HI = UNI ? H[g] : mul2(H[g], t.nm);
+            const f2x HJ = mul2(H[g], zm.y), HI = mul2(H[g], t.nm);
             t.ax = fma2(HJ, DX[g], t.ax);
             t.ay = fma2(HJ, DY[g], t.ay);
             t.az = fma2(HJ, DZ[g], t.az);
@@ -356,15 +297,14 @@ __device__ __forceinline__ void pp_chunk2(const ulonglong2* stage, int lane, PPT
     upk2(shfl2(BZ, fa), za, t0);
     upk2(shfl2(BZ, fb), t1, zb);
     if (lane < m) {
-        const float nm = UNI ? -q.m : 1.0f;
-        atomicAdd(q.acc + src0 + lane, nm * (xa + xb));
-        atomicAdd(q.acc + q.n + src0 + lane, nm * (ya + yb));
-        atomicAdd(q.acc + 2 * q.n + src0 + lane, nm * (za + zb));
+        atomicAdd(q.acc + src0 + lane, xa + xb);
+        atomicAdd(q.acc + q.n + src0 + lane, ya + yb);
+        atomicAdd(q.acc + 2 * q.n + src0 + lane, za + zb);
     }
 }
 
 // The sources [s0, s1) (shifted by s) against the lanes' G targets, chunk by chunk.
-template <int G, bool POLY, bool UNI>
+template <int G>
 __device__ __forceinline__ void pp_walk(ulonglong2* stage, int lane, PPTarget (&T)[2], const PPConst& k,
                                         const PPArgs& q, int s0, int s1, double sx, double sy, double sz) {
     for (int j0 = s0; j0 < s1; j0 += 32) {
@@ -378,13 +318,13 @@ __device__ __forceinline__ void pp_walk(ulonglong2* stage, int lane, PPTarget (&
             m = (float)p.w;
         }
         pp_stage(stage, lane, 16, x, y, z, m);
-        pp_chunk2<G, POLY, UNI, false, 0, 16, 16>(stage, lane, T, k, q, j0, min(32, s1 - j0));
+        pp_chunk2<G, false, 0, 16, 16>(stage, lane, T, k, q, j0, min(32, s1 - j0));
     }
 }
 
 // An item: the targets from t0 of a cell as G = 1 or 2 groups of 32. Every target meets its sources in
 // ascending order, whatever the group it is in.
-template <int G, bool POLY, bool UNI>
+template <int G>
 __device__ __forceinline__ void pp_item(ulonglong2* stage, int lane, const PPArgs& q, int c, int t0,
                                         const PPConst& k) {
     const int M = q.M, cl = q.last[c];
@@ -417,10 +357,10 @@ __device__ __forceinline__ void pp_item(ulonglong2* stage, int lane, const PPArg
         pp_stage(stage, lane, 8, act ? -x : 1e18f, act ? -y : 1e18f, act ? -z : 1e18f, -m);
         PPTarget one[2];
         one[0] = T[g];
-        pp_chunk2<1, POLY, UNI, true, 1, 9, 8>(stage, lane, one, k, q, t0 + 32 * g, min(32, cl - t0 - 32 * g));
+        pp_chunk2<1, true, 1, 9, 8>(stage, lane, one, k, q, t0 + 32 * g, min(32, cl - t0 - 32 * g));
         T[g] = one[0];
     }
-    if (G == 2) pp_walk<1, POLY, UNI>(stage, lane, T, k, q, t0 + 32, min(cl, t0 + 64), -ox, -oy, -oz);
+    if (G == 2) pp_walk<1>(stage, lane, T, k, q, t0 + 32, min(cl, t0 + 64), -ox, -oy, -oz);
     // the later particles of the cell, then the neighbouring cells of higher index
     for (int nb = -1; nb < 27; ++nb) {
         int s0, s1;
@@ -439,9 +379,8 @@ __device__ __forceinline__ void pp_item(ulonglong2* stage, int lane, const PPArg
             s0 = q.first[nc];
             s1 = q.last[nc];
         }
-        pp_walk<G, POLY, UNI>(stage, lane, T, k, q, s0, s1, sx, sy, sz);
+        pp_walk<G>(stage, lane, T, k, q, s0, s1, sx, sy, sz);
     }
-    const float m = UNI ? q.m : 1.0f;
 #pragma unroll
     for (int g = 0; g < G; ++g) {
         const int t = t0 + 32 * g + lane;
@@ -450,14 +389,13 @@ __device__ __forceinline__ void pp_item(ulonglong2* stage, int lane, const PPArg
         upk2(T[g].ay, y0, y1);
         upk2(T[g].az, z0, z1);
         if (t < cl) {
-            atomicAdd(q.acc + t, m * (x0 + x1));
-            atomicAdd(q.acc + q.n + t, m * (y0 + y1));
-            atomicAdd(q.acc + 2 * q.n + t, m * (z0 + z1));
+            atomicAdd(q.acc + t, x0 + x1);
+            atomicAdd(q.acc + q.n + t, y0 + y1);
+            atomicAdd(q.acc + 2 * q.n + t, z0 + z1);
         }
     }
 }
 
-template <bool POLY, bool UNI>
 __global__ void __launch_bounds__(PP_WARPS * 32) k_pp_pairs(const PPArgs q) {
     __shared__ ulonglong2 sh[PP_WARPS][64];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -471,14 +409,8 @@ __global__ void __launch_bounds__(PP_WARPS * 32) k_pp_pairs(const PPArgs q) {
     const unsigned total = __shfl_sync(0xffffffffu, end, PP_CLASSES - 1);
     ulonglong2* stage = sh[w];
     PPConst k;
-    const float a9 = q.alpha * q.alpha / 9.0f;
     k.alpha = dup(q.alpha);
     k.eps2 = dup(q.eps2);
-    k.w1 = dup(-a9);
-    k.w0 = dup(fmaf(q.eps2, a9, 1.0f));
-    k.na3 = dup(-q.alpha * q.alpha * q.alpha);
-    k.hi = q.rc2 + q.eps2;
-    k.lo = 2.0f * q.eps2;
     for (;;) {
         unsigned it = 0;
         if (lane == 0) it = atomicAdd(q.next, 1u);
@@ -487,9 +419,7 @@ __global__ void __launch_bounds__(PP_WARPS * 32) k_pp_pairs(const PPArgs q) {
         const int b = __popc(__ballot_sync(0xffffffffu, lane < PP_CLASSES && end <= it));
         const unsigned before = __shfl_sync(0xffffffffu, end, max(b - 1, 0));
         const int2 item = q.items[(PP_CLASSES - 1 - b) * q.max_items + (it - (b ? before : 0u))];
-        const int c = item.x & (PP_TWO - 1);
-        if ((item.x & PP_TWO) && q.last[c] - item.y > 32) pp_item<2, POLY, UNI>(stage, lane, q, c, item.y, k);
-        else pp_item<1, POLY, UNI>(stage, lane, q, c, item.y, k);
+        pp_item<1>(stage, lane, q, item.x, item.y, k);
     }
 }
 
@@ -560,17 +490,9 @@ extern "C" int sss_pm3_short(sss_pm3* p, const sss_pm3_particles* s, double G, d
     k_pp_bounds<<<blocks_for(n, 256), 256, 0, st>>>(k0, n, first, last);
     SSS_LAUNCH_CHECK(ctx, "k_pp_bounds");
     SSS_CUDA_TRY(ctx, cudaMemsetAsync(counters, 0, 4 * (PP_CLASSES + 1), st));
-    // the polynomial's range is t <= 9; without a softening in f32 there is no r < eps test
-    const bool poly = alpha * r_cut <= 3.0000001 && (float)(eps * eps) > 0.0f;
-    void (*pairs)(const PPArgs) = poly ? (s->m ? k_pp_pairs<true, false> : k_pp_pairs<true, true>)
-                                       : (s->m ? k_pp_pairs<false, false> : k_pp_pairs<false, true>);
     int per_sm = 0;
-    SSS_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pairs, PP_WARPS * 32, 0));
-    // items of 64 targets only where they still fill the warps twice: fewer particles are bound by the
-    // length of an item (us a pair pass, all of 32 / light cells of 64: 16,384 uniform 703 / 1083,
-    // 131,072 uniform 684 / 1055; 442,368 uniform 1796 either way)
-    const bool two = n >= 2LL * 64 * PP_WARPS * per_sm * ctx->num_sms;
-    k_pp_items<<<blocks_for(cells, 128), 128, 0, st>>>(first, last, M, cells, max_items, two, items, counters);
+    SSS_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pp_pairs, PP_WARPS * 32, 0));
+    k_pp_items<<<blocks_for(cells, 128), 128, 0, st>>>(first, last, M, cells, max_items, items, counters);
     SSS_LAUNCH_CHECK(ctx, "k_pp_items");
     PPArgs q;
     q.src = src;
@@ -588,12 +510,11 @@ extern "C" int sss_pm3_short(sss_pm3* p, const sss_pm3_particles* s, double G, d
     q.n_items = counters;
     q.max_items = max_items;
     q.next = counters + PP_CLASSES;
-    q.m = (float)s->mass_const;
     q.acc = (float*)(B + o_acc);
     q.n = n;
     SSS_CUDA_TRY(ctx, cudaMemsetAsync(q.acc, 0, 12 * (size_t)n, st));
     const unsigned grid = (unsigned)(ctx->num_sms * std::max(per_sm, 1));
-    pairs<<<grid, PP_WARPS * 32, 0, st>>>(q);
+    k_pp_pairs<<<grid, PP_WARPS * 32, 0, st>>>(q);
     SSS_LAUNCH_CHECK(ctx, "k_pp_pairs");
     Pm3Epi e{mode, hdt, dt, p->box, snap};
     k_pp_finish<<<blocks_for(n, 256), 256, 0, st>>>(q, parts, e);

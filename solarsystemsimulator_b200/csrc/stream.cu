@@ -1377,6 +1377,11 @@ int sample_batch(sss_ctx* ctx, int64_t n, int k, const float* const* x, const fl
     const size_t one = (size_t)n * 10 + (size_t)K2 * 16 + ((size_t)1 << 19);
     while (at_once > 1 && (size_t)at_once * one > SLOTS_BYTES) --at_once;
     rc = make_work(ctx, n, grid, at_once, k, &W);
+    if (rc && at_once > 1) {                       // no memory for several: one at a time
+        cudaGetLastError();
+        at_once = 1;
+        rc = make_work(ctx, n, grid, at_once, k, &W);
+    }
     if (rc) return rc;
     SampleBatch p;
     SampleArgs& a = p.s;

@@ -12,7 +12,8 @@ gather, adaptive grid geometry, KDK):
 
 and the module functions build_force_kernels, grid_fuer, pm_force_field,
 gather_accel, pm_accelerations, _cic_deposit, _cic_gather on CUDA tensors.
-The work runs in libsss (sss_pm2d_*); cuFFT does the transforms only.
+The work runs in libsss (sss_pm2d_*): own transforms for grids of 2^a, 3 2^a and
+500 2^a points, cuFFT for others.
 """
 from __future__ import annotations
 
@@ -33,7 +34,7 @@ def _f64(a, dev) -> torch.Tensor:
 
 
 class PMPlan:
-    """cuFFT plans and grids of one grid size (an sss_pm2d object)."""
+    """Transforms and grids of one grid size (an sss_pm2d object)."""
 
     def __init__(self, grid_n: int, device: int = 0):
         self.ctx = _lib.context(device)
