@@ -62,6 +62,12 @@ class PMPlan:
         with torch.cuda.device(self.device):
             self.ctx.check(getattr(self.ctx.lib, name)(self.ptr, *args, self._s()))
 
+    def build(self, key: tuple[float, float, float]) -> None:
+        """Hold the force kernels of key = (h, eps2, G)."""
+        self.kernel_key = None                  # (until the build has succeeded)
+        self.call("sss_pm2d_build_kernels", *key)
+        self.kernel_key = key
+
 
 _plans: dict[tuple[int, int], PMPlan] = {}
 
@@ -99,9 +105,9 @@ def build_force_kernels(grid_n: int, h: float, eps2: float, G: float = G_AU, dev
     """Transforms of the softened force kernels on the 2N x 2N padded grid
     (pm_kernel.py:34-60), kept on the device."""
     p = plan_for(grid_n, device)
-    if p.kernel_key != (float(h), float(eps2), float(G)):
-        p.call("sss_pm2d_build_kernels", float(h), float(eps2), float(G))
-        p.kernel_key = (float(h), float(eps2), float(G))
+    key = (float(h), float(eps2), float(G))
+    if p.kernel_key != key:
+        p.build(key)
     return ForceKernels(p, h, eps2, G)
 
 
@@ -206,16 +212,21 @@ class NBodyPM:
     def name(self) -> str:
         return torch.cuda.get_device_name(self.device) + " (PM)"
 
+    def _kernel_key(self, h) -> tuple[float, float, float]:
+        """(h, eps2, G) of this object's force kernels at cell size h (pm_kernel.py:216-221)."""
+        eps = max(self.softening_zellen * h, self.softening_floor)
+        return float(h), float(eps * eps), self.G
+
     def _accel_into(self, st):
         """Field from the masses, read at masses and tracers (pm_kernel.py:212-229)."""
         p = self._plan
         x0, y0, h = grid_fuer(st["x"], st["y"], self.grid_n, self.rand_zellen, self.device)
-        eps = max(self.softening_zellen * h, self.softening_floor)
-        eps2 = eps * eps
-        if self._kernel_h is None or abs(h - self._kernel_h) > 1e-6 * h:
-            p.call("sss_pm2d_build_kernels", float(h), float(eps2), self.G)
-            p.kernel_key = (float(h), float(eps2), self.G)
-            self._kernel_h = h
+        keep = self._kernel_h is not None and not abs(h - self._kernel_h) > 1e-6 * h
+        key = self._kernel_key(self._kernel_h if keep else h)
+        # the plan is shared by every caller of its grid size: what it holds may be another's kernels
+        if p.kernel_key != key:
+            p.build(key)
+        self._kernel_h = key[0]
         x, y, m = st["x"], st["y"], st["m"]
         p.call("sss_pm2d_field", x.data_ptr(), y.data_ptr(), m.data_ptr(), st["N"], x0, y0, h)
         p.call("sss_pm2d_gather", x.data_ptr(), y.data_ptr(), st["N"], x0, y0, h, st["ax"].data_ptr(),
@@ -292,6 +303,7 @@ class NBodyPM:
         p.call("sss_pm2d_step_batch", ctypes.byref(b), dt, int(steps), self.softening_zellen, self.rand_zellen,
                self.G, ctypes.byref(kh), snap.data_ptr())
         self._kernel_h = kh.value
+        p.kernel_key = self._kernel_key(kh.value)
         return snap.cpu().numpy()
 
     def export_f64(self, st: dict) -> np.ndarray:

@@ -222,3 +222,57 @@ def test_native_steps_equal_the_parts(n, tracers, grid):
             for k in ("x", "y"):
                 st[k].mul_(0.5)
     sims[0]._plan.native_steps = True
+
+
+def test_kernels_after_native_steps_a_deposit_and_a_load():
+    """Accelerations of a state loaded after a native batch and a density of
+    the same grid size: those of the object's own softening and G (a deposit
+    on a plan without kernels makes some with softening 2 h), for the cell size
+    its kernels stand for (the box has moved by less than a millionth of it).
+    Bound: FFT rounding, as test_convolution_of_every_length."""
+    pk = _pk()
+    rng = np.random.default_rng(5)
+    x, y = rng.uniform(-1, 1, (2, 400))
+    m, z = rng.uniform(0.5, 1.5, 400) * 1e-3, np.zeros(400)
+    sim = pk.NBodyPM([0], grid_n=64, G=7.0)
+    st = sim.load_state(x, y, z, z, m)
+    sim.step_batch(st, 1e-4, 2)
+    f = sim.export_f64(st)
+    x0, y0, h = pk.grid_fuer(f[:400], f[400:800], 64, sim.rand_zellen)
+    pk._cic_deposit(f[:400], f[400:800], m, 64, x0, y0, h)
+    got = sim.load_state(f[:400], f[400:800], f[800:1200], f[1200:], m)
+    hk = sim._kernel_h
+    assert abs(h - hk) <= 1e-6 * h
+    ker = pk.build_force_kernels(64, hk, (1.5 * hk) ** 2, 7.0)
+    want = pk.pm_accelerations(f[:400], f[400:800], m, 64, x0, y0, h, (1.5 * hk) ** 2, 7.0, kernels=ker)
+    for a, b in zip((got["ax"], got["ay"]), want):
+        assert float((a - b).abs().max()) <= 1e-10 * float(b.abs().max())
+
+
+@pytest.mark.parametrize("grid", [64, 130])
+def test_simulations_sharing_a_plan_do_not_mix(grid):
+    """Two objects of one grid size (own transforms, cuFFT), one with a
+    softening floor, stepped in turn, against each stepped alone. The outer
+    bodies rest at the box's corners, so h does not move. Bound: the deposit's
+    atomics order by order, carried through 2 x 2 steps."""
+    pk = _pk()
+    rng = np.random.default_rng(grid)
+    x, y, vx, vy = rng.uniform(-0.5, 0.5, (4, 300))
+    x[:4], y[:4], vx[:4], vy[:4] = (-50, 50, -50, 50), (-50, -50, 50, 50), 0, 0
+    m = np.full(300, 1e-9)
+    out = []
+    for together in (True, False):
+        sims = [pk.NBodyPM([0], softening_au=f, grid_n=grid) for f in (0.0, 9.0)]
+        sts = [s.load_state(x, y, vx, vy, m) for s in sims] if together else [None, None]
+        for turn in range(2):
+            for k in (0, 1):
+                if not together:
+                    if turn:
+                        continue
+                    sts[k] = sims[k].load_state(x, y, vx, vy, m)
+                    sims[k].step_batch(sts[k], 1e-3, 2)
+                sims[k].step_batch(sts[k], 1e-3, 2)
+        out.append([np.stack([st["ax"].cpu().numpy(), st["ay"].cpu().numpy()]) for st in sts])
+    for a, b in zip(*out):
+        assert np.abs(a - b).max() <= 1e-9 * np.abs(b).max()
+    assert np.abs(out[0][0] - out[0][1]).max() > 1e-3 * np.abs(out[0][0]).max()     # (the two do differ)
