@@ -757,8 +757,10 @@ __global__ void __launch_bounds__(WS_NT, WS_MINB_MIX) k_force_mixed_ws(const For
 // A warp per target, its lanes over the sources: the smallest evaluations. No
 // tile, no centre, no partial sums between CTAs; a source's offset is formed
 // in f64 and rounded to f32 (mixed), the f32 sums of LN_U sources a lane fold
-// into f64, and the lanes meet in one butterfly. Bound by latency (a launch,
-// one load, n / 32 pairs, five shuffles).
+// into f64, and the lanes meet in one butterfly. Sources of equal Gm are summed
+// with weight one and Gm is applied in f64, as the tiles above do: rounded to
+// f32 it would be one common factor of every force, up to 6e-8 off. Bound by
+// latency (a launch, one load, n / 32 pairs, five shuffles).
 template <int D, bool MIXED>
 __global__ void __launch_bounds__(LN_NT) k_force_lanes(const ForceArgs a) {
     const int lane = threadIdx.x & 31;
@@ -766,6 +768,7 @@ __global__ void __launch_bounds__(LN_NT) k_force_lanes(const ForceArgs a) {
     if (i >= a.n_tgt) return;
     const double4 p = a.tgt[i];
     const float epsf = (float)a.eps2;
+    const double w0 = MIXED ? a.src[0].w : 1.0;
     double sx = 0.0, sy = 0.0, sz = 0.0;
     for (int64_t j0 = lane; j0 < a.n_src; j0 += 32 * LN_U) {
         double4 v[LN_U];
@@ -777,20 +780,24 @@ __global__ void __launch_bounds__(LN_NT) k_force_lanes(const ForceArgs a) {
         }
         if (MIXED) {
             float fx = 0.f, fy = 0.f, fz = 0.f;
+            bool uni = true;
+#pragma unroll
+            for (int u = 0; u < LN_U; ++u) uni &= !ok[u] || v[u].w == w0;
 #pragma unroll
             for (int u = 0; u < LN_U; ++u) {
                 const float dx = __double2float_rn(v[u].x - p.x), dy = __double2float_rn(v[u].y - p.y);
                 const float dz = D == 3 ? __double2float_rn(v[u].z - p.z) : 0.f;
                 const float r2 = D == 3 ? fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, epsf))) : fmaf(dx, dx, fmaf(dy, dy, epsf));
                 const float inv = sss_rsqrt_approx_f32(ok[u] ? r2 : 1.0f);
-                const float f = __double2float_rn(v[u].w) * ((inv * inv) * inv);     // (no source: 0)
+                const float f = (ok[u] && uni ? 1.0f : __double2float_rn(v[u].w)) * ((inv * inv) * inv);  // (no source: 0)
                 fx = fmaf(f, dx, fx);
                 fy = fmaf(f, dy, fy);
                 if (D == 3) fz = fmaf(f, dz, fz);
             }
-            sx += (double)fx;
-            sy += (double)fy;
-            if (D == 3) sz += (double)fz;
+            const double wt = uni ? w0 : 1.0;
+            sx = fma(wt, (double)fx, sx);
+            sy = fma(wt, (double)fy, sy);
+            if (D == 3) sz = fma(wt, (double)fz, sz);
         } else {
 #pragma unroll
             for (int u = 0; u < LN_U; ++u) {

@@ -314,3 +314,26 @@ def test_smallest_evaluations(dim, n_src, n_tgt, equal):
     sources than lanes, remainders of the 128 a pass takes and of the 8 targets
     a block takes; and the warp-split kernels' edges at sizes just above."""
     test_few_pairs_kernels(dim, n_src, n_tgt, equal)
+
+
+@pytest.mark.parametrize("dim", [2, 3])
+@pytest.mark.parametrize("n_src,n_tgt", [(1, 1), (33, 7), (129, 1000), (300, 300), (705, 705), (1025, 3000), (3000, 200000)])
+@pytest.mark.parametrize("gm", [1.0 + 2.0 ** -25, 1.0 / 300.0, 7e60])
+def test_mixed_equal_masses_apply_gm_in_f64(dim, n_src, n_tgt, gm):
+    """Equal masses in mixed precision: the forces are Gm times those of unit
+    masses, whatever Gm's f32 value (a common factor of up to 6e-8, or inf).
+    Bound: 64 f64 roundings of the sum of the terms' magnitudes (at most 12
+    folds of f32 partial sums a lane or tile, the sums over lanes, warps and
+    chunks)."""
+    sg = _sg()
+    src, tgt = cloud(n_src, dim, seed=n_src), cloud(n_tgt, dim, seed=n_tgt + 1)
+    sel = np.random.default_rng(0).choice(n_tgt, min(n_tgt, 200), replace=False)
+    eps2, out = 0.05 ** 2, []
+    for w in (1.0, gm):
+        src[:, 3] = w
+        a = sg.allpairs_accel(torch.from_numpy(src).cuda(), torch.from_numpy(tgt).cuda(), eps2, dim=dim,
+                              precision="mixed")
+        out.append(a.cpu().numpy()[sel][:, :dim])
+    d = src[None, :, :dim] - tgt[sel][:, None, :dim]
+    size = (np.abs(d) * ((d ** 2).sum(2) + eps2)[:, :, None] ** -1.5).sum(1)
+    assert np.all(np.abs(out[1] / gm - out[0]) <= 64 * 2.0 ** -53 * 1.01 * size)
