@@ -156,8 +156,18 @@ __device__ __noinline__ void drain_after_abort(uint64_t* bar, int issued, int co
 // of 10,007 bodies: 126 us; 136 with an f32 seed whose argument and result
 // were re-biased by integer operations. On the benchmark shape the f32 seed
 // took 200 ms and CUDA's rsqrt(double) with three multiplies 246 ms.)
-template <bool UNIT>
+//
+// GUARD: 0 for an r2 that overflows (distances from 1e154 on), NaN without. Only
+// softenings below GUARD_EPS2, point masses, whose scenes may have any scale, take
+// the guard: in every pair it took 10,007 bodies from 441 to 454 us a Yoshida step,
+// and a second, guarded sum of the NaN targets alone cost as much (30,000 bodies
+// 3-D: 924 -> 943 us an evaluation, by the registers of the pair loop). The
+// lanes kernel, which latency bounds, always has it.
+constexpr double GUARD_EPS2 = 0x1p-126;
+
+template <bool UNIT, bool GUARD>
 __device__ __forceinline__ double rinv3(double gm, double r2) {
+    if (GUARD) return sss_gm_rinv3(UNIT ? 1.0 : gm, r2);
     double c;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(c) : "d"(r2));
     const double c2 = c * c;
@@ -167,7 +177,7 @@ __device__ __forceinline__ double rinv3(double gm, double r2) {
     return fma(g3, e * p, g3);
 }
 
-template <int D, int R, bool UNIT, int UNROLL>
+template <int D, int R, bool UNIT, bool GUARD, int UNROLL>
 __device__ __forceinline__ void tile_f64(const double4* __restrict__ s, int cnt, double eps2,
                                          const double (&px)[R], const double (&py)[R],
                                          const double (&pz)[R], double (&tx)[R], double (&ty)[R],
@@ -187,7 +197,7 @@ __device__ __forceinline__ void tile_f64(const double4* __restrict__ s, int cnt,
             } else {
                 r2 = fma(dx, dx, fma(dy, dy, eps2));
             }
-            const double f = rinv3<UNIT>(sj.w, r2);
+            const double f = rinv3<UNIT, GUARD>(sj.w, r2);
             tx[r] = fma(f, dx, tx[r]);
             ty[r] = fma(f, dy, ty[r]);
             if (D == 3) tz[r] = fma(f, dz, tz[r]);
@@ -195,7 +205,7 @@ __device__ __forceinline__ void tile_f64(const double4* __restrict__ s, int cnt,
     }
 }
 
-template <int D, int R, int NT, int TS, int MINB, int UNROLL>
+template <int D, int R, int NT, int TS, int MINB, int UNROLL, bool GUARD>
 __global__ void __launch_bounds__(NT, MINB) k_force_f64(const ForceArgs a) {
     extern __shared__ __align__(128) unsigned char smem[];
     double4* tiles = reinterpret_cast<double4*>(smem);
@@ -261,8 +271,8 @@ __global__ void __launch_bounds__(NT, MINB) k_force_f64(const ForceArgs a) {
         double tx[R], ty[R], tz[R];
 #pragma unroll
         for (int r = 0; r < R; ++r) { tx[r] = 0.0; ty[r] = 0.0; tz[r] = 0.0; }
-        if (uni) tile_f64<D, R, true, UNROLL>(s, cnt, eps2, px, py, pz, tx, ty, tz);
-        else tile_f64<D, R, false, UNROLL>(s, cnt, eps2, px, py, pz, tx, ty, tz);
+        if (uni) tile_f64<D, R, true, GUARD, UNROLL>(s, cnt, eps2, px, py, pz, tx, ty, tz);
+        else tile_f64<D, R, false, GUARD, UNROLL>(s, cnt, eps2, px, py, pz, tx, ty, tz);
         const double wt = uni ? w0 : 1.0;
 #pragma unroll
         for (int r = 0; r < R; ++r) {
@@ -623,7 +633,7 @@ __device__ __forceinline__ void ws_finish(const ForceArgs& a, int tb, int ch, do
     epilogue<D>(a.epi, i, sx, sy, sz, a.tgt[i]);
 }
 
-template <int D, int R>
+template <int D, int R, bool GUARD>
 __global__ void __launch_bounds__(WS_NT, WS_MINB_F64) k_force_f64_ws(const ForceArgs a) {
     constexpr int TB = 32 * R;
     constexpr int RED = 3 * WS_W * TB * (int)sizeof(double), SRC = WS_TS * (int)sizeof(double4);
@@ -655,8 +665,8 @@ __global__ void __launch_bounds__(WS_NT, WS_MINB_F64) k_force_f64_ws(const Force
         double tx[R], ty[R], tz[R];
 #pragma unroll
         for (int r = 0; r < R; ++r) { tx[r] = 0.0; ty[r] = 0.0; tz[r] = 0.0; }
-        if (uni) tile_f64<D, R, true, F64_UNROLL>(tile + b, e - b, a.eps2, px, py, pz, tx, ty, tz);
-        else tile_f64<D, R, false, F64_UNROLL>(tile + b, e - b, a.eps2, px, py, pz, tx, ty, tz);
+        if (uni) tile_f64<D, R, true, GUARD, F64_UNROLL>(tile + b, e - b, a.eps2, px, py, pz, tx, ty, tz);
+        else tile_f64<D, R, false, GUARD, F64_UNROLL>(tile + b, e - b, a.eps2, px, py, pz, tx, ty, tz);
         const double wt = uni ? w0 : 1.0;
 #pragma unroll
         for (int r = 0; r < R; ++r) {
@@ -803,7 +813,7 @@ __global__ void __launch_bounds__(LN_NT) k_force_lanes(const ForceArgs a) {
             for (int u = 0; u < LN_U; ++u) {
                 const double dx = v[u].x - p.x, dy = v[u].y - p.y, dz = D == 3 ? v[u].z - p.z : 0.0;
                 const double r2 = fma(dx, dx, fma(dy, dy, fma(dz, dz, a.eps2)));
-                const double f = rinv3<false>(v[u].w, ok[u] ? r2 : 1.0);
+                const double f = rinv3<false, true>(v[u].w, ok[u] ? r2 : 1.0);
                 sx = fma(f, dx, sx);
                 sy = fma(f, dy, sy);
                 if (D == 3) sz = fma(f, dz, sz);
@@ -922,7 +932,14 @@ struct KSel {
     bool lanes;        // a warp per target (one chunk)
 };
 
-KSel select_kernel(int dim, int precision, int64_t n_src, int64_t n_tgt) {
+template <bool GUARD>
+void* f64_kernel(int dim, bool ws) {
+    if (ws) return dim == 3 ? (void*)k_force_f64_ws<3, WS_R_F64, GUARD> : (void*)k_force_f64_ws<2, WS_R_F64, GUARD>;
+    return dim == 3 ? (void*)k_force_f64<3, F64_R, F64_NT, F64_TS, F64_MINB, F64_UNROLL, GUARD>
+                    : (void*)k_force_f64<2, F64_R, F64_NT, F64_TS, F64_MINB, F64_UNROLL, GUARD>;
+}
+
+KSel select_kernel(int dim, int precision, int64_t n_src, int64_t n_tgt, double eps2) {
     KSel k;
     k.mixed = (precision == SSS_PREC_MIXED);
     const double pairs = (double)n_src * (double)n_tgt;
@@ -939,16 +956,18 @@ KSel select_kernel(int dim, int precision, int64_t n_src, int64_t n_tgt) {
         k.mixed = false;
         return k;
     }
+    const bool guard = eps2 < GUARD_EPS2;
+    void* const f64 = guard ? f64_kernel<true>(dim, k.ws) : f64_kernel<false>(dim, k.ws);
     if (k.ws) {
         if (k.mixed)
             k.fn = (dim == 3) ? (void*)k_force_mixed_ws<3, WS_R_MIX> : (void*)k_force_mixed_ws<2, WS_R_MIX>;
         else
-            k.fn = (dim == 3) ? (void*)k_force_f64_ws<3, WS_R_F64> : (void*)k_force_f64_ws<2, WS_R_F64>;
+            k.fn = f64;
         k.nt = WS_NT;
         k.tpb = 32 * (k.mixed ? WS_R_MIX : WS_R_F64);
         k.ts = WS_TS;
         k.smem = 0;
-        k.key = (k.mixed ? 8 : 4) + (dim == 3);      // (6 and 7: allpairs_tc.cu)
+        k.key = (k.mixed ? 8 : guard ? 16 : 4) + (dim == 3);      // (6 and 7: allpairs_tc.cu)
         k.mixed = false;
         return k;
     }
@@ -962,13 +981,12 @@ KSel select_kernel(int dim, int precision, int64_t n_src, int64_t n_tgt) {
         k.key = 2 + (dim == 3);
         return k;
     }
-    k.fn = (dim == 3) ? (void*)k_force_f64<3, F64_R, F64_NT, F64_TS, F64_MINB, F64_UNROLL>
-                      : (void*)k_force_f64<2, F64_R, F64_NT, F64_TS, F64_MINB, F64_UNROLL>;
+    k.fn = f64;
     k.nt = F64_NT;
     k.tpb = F64_NT * F64_R;
     k.ts = F64_TS;
     k.smem = 2 * (size_t)F64_TS * sizeof(double4);
-    k.key = dim == 3;
+    k.key = (guard ? 14 : 0) + (dim == 3);
     return k;
 }
 
@@ -1008,7 +1026,7 @@ int force_eval(sss_ctx* ctx, int dim, int precision, const double4* src, int64_t
         return sss_set_err(ctx, SSS_ERR_ARG, "all-pairs: size out of range");
     if (precision == SSS_PREC_MIXED_TC)
         return sss_ap::force_eval_tc(ctx, dim, src, n_src, tgt, n_tgt, eps2, epi, stream);
-    const KSel ks = select_kernel(dim, precision, n_src, n_tgt);
+    const KSel ks = select_kernel(dim, precision, n_src, n_tgt, eps2);
     if (ctx->occ[ks.key] == 0) {
         int per_sm = 0;
         SSS_CUDA_TRY(ctx, query_occupancy(ks, &per_sm));
@@ -1269,14 +1287,14 @@ int noalloc_setup(int device, NoAllocDevice** out, char* eb, size_t el) {
         } else {
             d->base = (unsigned char*)p;
             e = cudaDeviceGetAttribute(&d->num_sms, cudaDevAttrMultiProcessorCount, device);
-            // one size for each kind of kernel
+            // one size for each kind of kernel, each with and without the guard
             const int64_t probe_n[3] = {1, 16384, (int64_t)1 << 20};
             static_assert(16384.0 * 16384.0 >= LANE_PAIRS_F64 && 16384.0 * 16384.0 >= LANE_PAIRS_MIX &&
                           16384.0 * 16384.0 < SPLIT_PAIRS_F64 && 16384.0 * 16384.0 < SPLIT_PAIRS_MIX, "probe sizes");
             for (int prec = 0; prec < 2 && e == cudaSuccess; ++prec)
                 for (int dim = 2; dim <= 3 && e == cudaSuccess; ++dim)
-                    for (int q = 0; q < 3 && e == cudaSuccess; ++q) {
-                        const KSel ks = select_kernel(dim, prec, probe_n[q], probe_n[q]);
+                    for (int q = 0; q < 6 && e == cudaSuccess; ++q) {
+                        const KSel ks = select_kernel(dim, prec, probe_n[q / 2], probe_n[q / 2], q % 2 ? 1.0 : 0.0);
                         e = query_occupancy(ks, &d->occ[ks.key]);
                     }
             if (e != cudaSuccess)
@@ -1317,7 +1335,7 @@ extern "C" int sss_allpairs_accel_noalloc(int device, int dim, int precision, co
     int rc = noalloc_setup(device, &d, eb, el);
     if (rc) return rc;
 
-    const KSel ks = select_kernel(dim, precision, n_src, n_tgt);
+    const KSel ks = select_kernel(dim, precision, n_src, n_tgt, eps2);
     const int slots = d->occ[ks.key] * d->num_sms;
     Plan pl = plan_of(ks, n_src, n_tgt, slots);
 

@@ -11,7 +11,7 @@
 
 #include "../../include/sss.h"
 
-#define SSS_AP_KERNELS 14   // all-pairs force kernels by dimension, precision and size
+#define SSS_AP_KERNELS 18   // all-pairs force kernels by dimension, precision, size and softening
 
 struct sss_ctx {
     int device;

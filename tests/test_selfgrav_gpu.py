@@ -337,3 +337,24 @@ def test_mixed_equal_masses_apply_gm_in_f64(dim, n_src, n_tgt, gm):
     d = src[None, :, :dim] - tgt[sel][:, None, :dim]
     size = (np.abs(d) * ((d ** 2).sum(2) + eps2)[:, :, None] ** -1.5).sum(1)
     assert np.all(np.abs(out[1] / gm - out[0]) <= 64 * 2.0 ** -53 * 1.01 * size)
+
+
+@pytest.mark.parametrize("dim", [2, 3])
+@pytest.mark.parametrize("n_src,n_tgt", [(7, 9), (513, 1100), (20000, 25000)])
+@pytest.mark.parametrize("equal", [True, False])
+@pytest.mark.parametrize("eps2", [1e-60, 1e-38])
+def test_f64_source_beyond_the_range_of_r2(dim, n_src, n_tgt, equal, eps2):
+    """A source so far away that r^2 overflows adds nothing (r^-3 = 0) where the
+    softening is below 2^-126, in each f64 kernel: the forces of the others, at
+    the parity bar."""
+    sg = _sg()
+    src, tgt = cloud(n_src, dim, seed=n_src), cloud(n_tgt, dim, seed=n_tgt + 1)
+    if equal:
+        src[:, 3] = 0.7 / n_src
+    src[n_src // 2, 0] = 3e155
+    sel = np.random.default_rng(0).choice(n_tgt, min(n_tgt, 300), replace=False)
+    ref = osg.accel(np.delete(src, n_src // 2, 0), tgt[sel], eps2, dim=dim)
+    a = sg.allpairs_accel(torch.from_numpy(src).cuda(), torch.from_numpy(tgt).cuda(), eps2, dim=dim).cpu().numpy()[sel]
+    assert np.isfinite(a).all()
+    ok, worst = parity_ok(a, ref, dim)
+    assert ok, worst
