@@ -50,27 +50,48 @@ constexpr int MIX_MINB = 2;
 
 constexpr int WAVES = 16;       // target number of CTA waves per evaluation
 
-// warp-split kernels (fewer than SPLIT_PAIRS pairs): 8 warps share 64 or 128
-// targets and split the CTA's sources. The limits are where the two forms cross
-// (us per evaluation, split / general; 2-D mixed crosses later, at 1e9):
-//   mixed 3-D  10,007^2 57 / 88, 17,000^2 148 / 156, 20,000^2 199 / 207, 25,000^2 294 / 290, 40,000^2 748 / 671
-//   f64 3-D    10,007^2 125 / 133, 17,000^2 316 / 326, 20,000^2 438 / 437, 30,000^2 960 / 927
+// warp-split kernels (use_split): 8 warps share 64 or 128 targets and split the
+// CTA's sources.
 constexpr int WS_W = 8;
 constexpr int WS_NT = WS_W * 32;
 constexpr int WS_TS = 512;      // sources per tile (mixed: the tile with one centre)
 constexpr int WS_MAXCHUNKS = 16;
 constexpr int WS_R_F64 = 2, WS_R_MIX = 4;
 constexpr int WS_MINB_F64 = 4, WS_MINB_MIX = 2;
+
+// lane kernels (use_lanes): a warp per target
+constexpr int LN_NT = 256, LN_U = 4;
+
+// Which form an evaluation takes. The limits are where the forms cross, over
+// 1 .. 1,048,576 sources and 1 .. 1,000,000 targets (device us per evaluation
+// among others).
+//
+// Lanes / warp-split: a warp alone walks n_src / 128 rounds, and from ~4,000
+// targets on they queue for the SMs, so both counts are bounded:
+//   mixed 2-D  300^2 2.5 / 5.5, 512 x 1,024 3.6 / 5.4, 1,024^2 5.7 / 5.8, 1 x 4,096 2.7 / 2.8, 1 x 16,384 5.3 / 2.8,
+//              2,048 x 64 9.5 / 5.7, 65,536 x 1 225 / 36
+//   f64 3-D    100 x 1,024 2.5 / 4.0, 512 x 4,096 6.8 / 8.4, 512 x 64 5.1 / 5.3, 1,024 x 64 8.8 / 5.7, 100 x 16,384 7.6 / 5.0
+//
+// Warp-split / general. By pairs where both counts are large:
+//   mixed 3-D  10,007^2 57 / 88, 17,000^2 148 / 156, 20,000^2 199 / 207, 25,000^2 294 / 290, 40,000^2 748 / 671
+//   f64 3-D    10,007^2 125 / 133, 17,000^2 316 / 326, 20,000^2 438 / 437, 30,000^2 960 / 927
+// Few sources on many targets leave a CTA of 64 or 128 targets little but its fixed part:
+//   mixed 2-D  1 x 65,536 5.0 / 6.1, 1 x 131,072 8.5 / 6.1, 100 x 131,072 12 / 11, 100 x 1,000,000 82 / 42, 512 x 262,144 56 / 57
+//   f64 3-D    1 x 8,192 2.6 / 2.8, 1 x 65,536 6.1 / 2.9, 100 x 65,536 11.3 / 11.6, 100 x 1,000,000 130 / 111, 512 x 262,144 144 / 160
+// Many sources on a few targets give it 16 chunks only, of sources the general form spreads over all SMs:
+//   mixed 3-D  65,536 x 8 47 / 45, 131,072 x 64 91 / 82, 1,048,576 x 1 699 / 517, 131,072 x 200 92 / 94
+//   f64 3-D    32,768 x 8 34 / 53, 65,536 x 64 64 / 62, 262,144 x 64 243 / 204, 262,144 x 300 244 / 262
 constexpr double SPLIT_PAIRS_F64 = 3e8, SPLIT_PAIRS_MIX = 4.5e8;
 
-// lane kernels (a warp per target): fewer than LANE_PAIRS pairs. Above, a target's
-// sources read by one warp from L1 cost more than the warp-split kernels' tiles
-// (us per evaluation among others, warp-split / lanes):
-//   mixed 2-D  300^2 6.2 / 4.1, 600^2 6.8 / 6.2, 1,000^2 7.9 / 8.2, 2,000^2 10.0 / 14.1
-//   mixed 3-D  100^2 6.1 / 4.1, 300^2 6.2 / 5.1, 600^2 7.6 / 6.2, 1,000^2 8.2 / 10.2
-//   f64 3-D    100^2 6.2 / 4.1, 300^2 7.1 / 6.2, 600^2 7.1 / 8.2 (2-D: 300^2 6.2 / 6.1, 600^2 6.4 / 7.8)
-constexpr int LN_NT = 256, LN_U = 4;
-constexpr double LANE_PAIRS_F64 = 1.5e5, LANE_PAIRS_MIX = 5e5;
+constexpr bool use_lanes(bool mixed, int64_t n_src, int64_t n_tgt) {
+    return (n_src <= 512 && n_tgt <= 4096) || (mixed && n_src <= 1024 && n_tgt <= 1024);
+}
+
+constexpr bool use_split(bool mixed, int64_t n_src, int64_t n_tgt) {
+    if ((double)n_src * (double)n_tgt >= (mixed ? SPLIT_PAIRS_MIX : SPLIT_PAIRS_F64)) return false;
+    if (n_tgt >= (mixed ? 80000 + 500 * n_src : 20000 + 900 * n_src)) return false;
+    return !(n_tgt <= (mixed ? 128 : 256) && n_src >= (mixed ? 98304 : 65536));
+}
 
 using sss_ap::Epi;
 using sss_ap::epilogue;
@@ -942,9 +963,8 @@ void* f64_kernel(int dim, bool ws) {
 KSel select_kernel(int dim, int precision, int64_t n_src, int64_t n_tgt, double eps2) {
     KSel k;
     k.mixed = (precision == SSS_PREC_MIXED);
-    const double pairs = (double)n_src * (double)n_tgt;
-    k.ws = pairs < (k.mixed ? SPLIT_PAIRS_MIX : SPLIT_PAIRS_F64);
-    k.lanes = pairs < (k.mixed ? LANE_PAIRS_MIX : LANE_PAIRS_F64);
+    k.lanes = use_lanes(k.mixed, n_src, n_tgt);
+    k.ws = !k.lanes && use_split(k.mixed, n_src, n_tgt);
     if (k.lanes) {
         if (k.mixed) k.fn = (dim == 3) ? (void*)k_force_lanes<3, true> : (void*)k_force_lanes<2, true>;
         else k.fn = (dim == 3) ? (void*)k_force_lanes<3, false> : (void*)k_force_lanes<2, false>;
@@ -1289,8 +1309,9 @@ int noalloc_setup(int device, NoAllocDevice** out, char* eb, size_t el) {
             e = cudaDeviceGetAttribute(&d->num_sms, cudaDevAttrMultiProcessorCount, device);
             // one size for each kind of kernel, each with and without the guard
             const int64_t probe_n[3] = {1, 16384, (int64_t)1 << 20};
-            static_assert(16384.0 * 16384.0 >= LANE_PAIRS_F64 && 16384.0 * 16384.0 >= LANE_PAIRS_MIX &&
-                          16384.0 * 16384.0 < SPLIT_PAIRS_F64 && 16384.0 * 16384.0 < SPLIT_PAIRS_MIX, "probe sizes");
+            static_assert(use_lanes(true, 1, 1) && use_lanes(false, 1, 1) && !use_lanes(true, 16384, 16384) &&
+                          use_split(true, 16384, 16384) && use_split(false, 16384, 16384) &&
+                          !use_split(true, 1 << 20, 1 << 20) && !use_split(false, 1 << 20, 1 << 20), "probe sizes");
             for (int prec = 0; prec < 2 && e == cudaSuccess; ++prec)
                 for (int dim = 2; dim <= 3 && e == cudaSuccess; ++dim)
                     for (int q = 0; q < 6 && e == cudaSuccess; ++q) {

@@ -7,6 +7,9 @@ Tolerances:
 Mirrors the reference's own test_selfgrav.py questions A (circular orbit),
 B (energy), C (determinism), F (tracers).
 """
+import os
+import tempfile
+
 import numpy as np
 import pytest
 import torch
@@ -358,3 +361,48 @@ def test_f64_source_beyond_the_range_of_r2(dim, n_src, n_tgt, equal, eps2):
     assert np.isfinite(a).all()
     ok, worst = parity_ok(a, ref, dim)
     assert ok, worst
+
+
+def _form(sg, precision, n_src, n_tgt):
+    """The kernel form an evaluation takes, by the kernel's name in a captured graph."""
+    src, tgt = (torch.rand((n, 4), dtype=torch.float64, device="cuda") for n in (n_src, n_tgt))
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        sg.allpairs_accel(src, tgt, 1e-2, dim=3, precision=precision)          # (allocates its scratch)
+    side.synchronize()
+    g = torch.cuda.CUDAGraph(keep_graph=True)
+    g.enable_debug_mode()
+    with torch.cuda.graph(g, stream=side):
+        sg.allpairs_accel(src, tgt, 1e-2, dim=3, precision=precision)
+    with tempfile.TemporaryDirectory() as d:
+        path = os.path.join(d, "g.dot")
+        g.debug_dump(path)
+        with open(path) as f:
+            text = f.read()
+    return "lanes" if "k_force_lanes" in text else "split" if f"k_force_{precision}_ws" in text else \
+        "general" if f"k_force_{precision}" in text else text
+
+
+@pytest.mark.filterwarnings("ignore:DEBUG")
+@pytest.mark.parametrize("precision,n_src,n_tgt,form", [
+    ("mixed", 300, 300, "lanes"), ("mixed", 1000, 1000, "lanes"), ("f64", 100, 4000, "lanes"),
+    ("mixed", 65536, 1, "split"), ("mixed", 2048, 64, "split"), ("f64", 16384, 8, "split"), ("f64", 1024, 64, "split"),
+    ("mixed", 4, 16384, "split"), ("f64", 16, 16384, "split"), ("mixed", 3000, 23000, "split"),
+    ("f64", 10007, 10007, "split"), ("mixed", 512, 262144, "split"),
+    ("mixed", 100, 1000000, "general"), ("mixed", 4, 131072, "general"), ("f64", 4, 65536, "general"),
+    ("f64", 100, 500000, "general"), ("mixed", 262144, 64, "general"), ("f64", 262144, 64, "general"),
+    ("f64", 20000, 20000, "general"), ("mixed", 40000, 40000, "general")])
+def test_form_by_sources_and_targets(precision, n_src, n_tgt, form):
+    """Lopsided calls take the form that is the fastest at their shape, not the
+    one of their number of pairs."""
+    assert _form(_sg(), precision, n_src, n_tgt) == form
+
+
+@pytest.mark.parametrize("dim", [2, 3])
+@pytest.mark.parametrize("n_src,n_tgt", [(512, 4096), (513, 4096), (512, 4097), (1024, 1024), (1025, 1024), (1024, 1025),
+                                         (1, 20899), (1, 20900), (1, 80500), (98303, 3), (98304, 128), (98304, 129),
+                                         (65536, 256), (65535, 256)])
+@pytest.mark.parametrize("equal", [True, False])
+def test_lopsided_evaluations(dim, n_src, n_tgt, equal):
+    """Both sides of the limits between the forms."""
+    test_few_pairs_kernels(dim, n_src, n_tgt, equal)
