@@ -18,7 +18,7 @@
 #include "sss_internal.cuh"
 
 #include <cmath>
-#include <vector>
+#include <cstdlib>
 
 constexpr int FFT_E = 16;              // complex values per thread
 
@@ -63,25 +63,30 @@ constexpr int fft_threads(int n, int batch) {
     return (nt + 31) / 32 * 32;
 }
 
-// Twiddle table of length n in device memory (freed by the owner).
+// Twiddle table of length n in device memory (freed by the owner, also after an
+// error). Complete on return: a pageable copy may return before its data has
+// arrived, and the transforms run on streams that do not wait for the default one.
 template <class C>
 cudaError_t fft_table(int n, C** out) {
     *out = nullptr;
-    std::vector<C> tw;
+    const int size = fft_off(n, fft_stages(n));
+    C* tw = (C*)malloc((size_t)size * sizeof(C));
+    if (!tw) return cudaErrorMemoryAllocation;
     const long double pi = 3.14159265358979323846264338327950288L;
+    int q = 0;
     for (int s = 1; s < fft_stages(n); ++s) {
         const int r = fft_radix(n, s), span = fft_span(n, s);
         for (int t = 1; t < r; ++t)
-            for (int k = 0; k < span; ++k) {
+            for (int k = 0; k < span; ++k, ++q) {
                 const long double a = -2.0L * pi * (long double)(t * k) / (long double)(span * r);
-                C w;
-                w.x = (decltype(w.x))cosl(a);
-                w.y = (decltype(w.y))sinl(a);
-                tw.push_back(w);
+                tw[q].x = (decltype(tw[q].x))cosl(a);
+                tw[q].y = (decltype(tw[q].y))sinl(a);
             }
     }
-    cudaError_t e = cudaMalloc(out, tw.size() * sizeof(C));
-    if (e == cudaSuccess) e = cudaMemcpy(*out, tw.data(), tw.size() * sizeof(C), cudaMemcpyHostToDevice);
+    cudaError_t e = cudaMalloc(out, (size_t)size * sizeof(C));
+    if (e == cudaSuccess) e = cudaMemcpy(*out, tw, (size_t)size * sizeof(C), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);
+    free(tw);
     return e;
 }
 

@@ -401,3 +401,23 @@ def test_solve_of_every_mesh_side(n, deconv, rs):
         scale = max(float(w.abs().max()) for w in want)
         for got, ref in zip(pm.acc_mesh, want):
             assert float((got.double() - ref).abs().max()) <= 5e-6 * scale
+
+
+@pytest.mark.parametrize("n", [32, 64, 384])
+def test_first_solve_on_another_stream(n):
+    """The first solve of a new plan on a stream of its own, while the default
+    stream is busy, is the one every later solve makes (the plan's tables are
+    complete when its creation returns)."""
+    from solarsystemsimulator_b200.pm3d import PMPeriodic3D
+    rho = torch.randn((n, n, n), generator=torch.Generator(device="cuda").manual_seed(n), device="cuda")
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    torch.cuda._sleep(60_000_000)                           # some 30 ms of the default stream
+    pm = PMPeriodic3D(n, box=2.0, G=1.5)
+    with torch.cuda.stream(side):
+        pm.rho.copy_(rho)
+        pm._call("sss_pm3_solve", 1.5, pm.deconv, pm.r_split)
+        first = pm.acc_mesh.clone()
+    torch.cuda.synchronize()
+    pm._call("sss_pm3_solve", 1.5, pm.deconv, pm.r_split)
+    assert torch.equal(first, pm.acc_mesh)

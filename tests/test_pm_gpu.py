@@ -276,3 +276,25 @@ def test_simulations_sharing_a_plan_do_not_mix(grid):
     for a, b in zip(*out):
         assert np.abs(a - b).max() <= 1e-9 * np.abs(b).max()
     assert np.abs(out[0][0] - out[0][1]).max() > 1e-3 * np.abs(out[0][0]).max()     # (the two do differ)
+
+
+@pytest.mark.parametrize("n", [32, 500, 1024])
+def test_first_field_on_another_stream(n):
+    """The first field of a new plan on a stream of its own, while the default
+    stream is busy, is the one every later call makes (one particle: its deposit
+    has no order)."""
+    pk = _pk()
+    x = torch.tensor([0.37 * n], dtype=torch.float64, device="cuda")
+    out = [torch.empty((4, n, n), dtype=torch.float64, device="cuda") for _ in range(2)]
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    torch.cuda._sleep(60_000_000)
+    p = pk.PMPlan(n)
+    for k, stream in enumerate((side, torch.cuda.default_stream())):
+        with torch.cuda.stream(stream):
+            p.build((1.0, 2.25 + k, 1.0))                   # (both softenings' tables are made)
+            p.build((1.0, 2.25, 1.0))
+            p.call("sss_pm2d_field", x.data_ptr(), x.data_ptr(), x.data_ptr(), 1, 0.0, 0.0, 1.0)
+            p.call("sss_pm2d_fields", out[k][0].data_ptr(), out[k][1].data_ptr())
+        torch.cuda.synchronize()
+    assert torch.equal(out[0][:2], out[1][:2])
