@@ -101,7 +101,8 @@ __global__ void __launch_bounds__(256) k_deposit3(const Pm3Parts s, int n, doubl
 // Per-axis tables of the spectrum kernel, index i of a full axis (frequency
 // f = i for i < n/2, i - n otherwise): kd = k_i (0 on the Nyquist index:
 // the derivative of that mode is dropped so the spectra stay Hermitian),
-// k2 = k_i^2, fac = sinc(pi f / n)^(-2 deconv) * exp(-k_i^2 rs2). The
+// k2 = k_i^2, fac = sinc(pi f / n)^(-2 deconv) * exp(-k_i^2 rs2), then kd as
+// the sum of two f32. The
 // Green's function factorises: W(k)^-deconv e^{-k^2 rs2} = fac_x fac_y fac_z.
 // The half axis of the real transform (iz <= n/2) reads the same tables.
 __global__ void k_spectrum_tables(int n, double box, int deconv, double rs2, double* __restrict__ tab) {
@@ -117,7 +118,9 @@ __global__ void k_spectrum_tables(int n, double box, int deconv, double rs2, dou
         for (int q = 0; q < deconv; ++q) fac /= s2;
     }
     if (rs2 > 0.0) fac *= exp(-k * k * rs2);
-    tab[i] = (i == n / 2) ? 0.0 : k;
+    const double kd = (i == n / 2) ? 0.0 : k;
+    tab[i] = kd;
+    reinterpret_cast<float2*>(tab + 3 * n)[i] = make_float2((float)kd, (float)(kd - (double)(float)kd));
     tab[n + i] = k * k;
     tab[2 * n + i] = fac;
 }
@@ -234,6 +237,22 @@ __device__ __forceinline__ double recip(double d) {
     return fma(r, fma(-d, r, 1.0), r);
 }
 
+// k (f64) z rounded once, as the products of k_spectrum3, from k = hi + lo in two
+// f32: hi z = p + e exactly, so p + (e + lo z) is within 2^-46 of k z before its
+// rounding (Dekker, "A floating-point technique for extending the available
+// precision", 1971). A 256^3 solve takes 331 us; 360 in f64 with its conversions,
+// 335 with k rounded to f32 (512^3: 3,020, 3,268, 2,992).
+__device__ __forceinline__ float times_k(float2 k, float z) {
+    const float p = __fmul_rn(k.x, z);
+    return __fadd_rn(p, __fmaf_rn(k.y, z, __fmaf_rn(k.x, z, -p)));
+}
+__device__ __forceinline__ float2 times_ik(float2 k, float2 z) {
+    return make_float2(-times_k(k, z.y), times_k(k, z.x));
+}
+__device__ __forceinline__ const float2* split_k(const double* tab, int n) {
+    return reinterpret_cast<const float2*>(tab + 3 * n);
+}
+
 // a_x = i k_x c rho_k and phi' = c rho_k (c as in k_spectrum3), both inverse
 // transformed along x; plane = iy.
 template <int N>
@@ -290,12 +309,8 @@ k_y_inv(const float2* __restrict__ tw, const double* __restrict__ tab, float2* a
     float2* out = (d == 0 ? ax : d == 1 ? ay : third) + o;
     fft::run<N, 1, Map>(tw, smf,
                         [&](int i, int, bool) {
-                            float2 z = in[i * T::PITCH];
-                            if (d == 1) {
-                                const float k = (float)__ldg(tab + i);
-                                z = make_float2(-k * z.y, k * z.x);
-                            }
-                            return z;
+                            const float2 z = in[i * T::PITCH];
+                            return d == 1 ? times_ik(__ldg(split_k(tab, N) + i), z) : z;
                         },
                         [&](int i, int, float2 z, bool) { out[i * T::PITCH] = z; });
 }
@@ -317,9 +332,9 @@ k_z_inv(const float2* __restrict__ tw, const double* __restrict__ tab, const flo
         const int c = q / R::NH, k = q - c * R::NH;
         float2 a = __ldg(src + (2 * c) * R::PITCH + k), b = __ldg(src + (2 * c + 1) * R::PITCH + k);
         if (d == 2) {
-            const float kz = (float)__ldg(tab + k);
-            a = make_float2(-kz * a.y, kz * a.x);
-            b = make_float2(-kz * b.y, kz * b.x);
+            const float2 kz = __ldg(split_k(tab, N) + k);
+            a = times_ik(kz, a);
+            b = times_ik(kz, b);
         }
         if (k == 0 || k == N / 2) { a.y = 0.f; b.y = 0.f; }      // real modes
         smf[Map::at(k, c)] = make_float2(a.x - b.y, a.y + b.x);
@@ -442,7 +457,7 @@ extern "C" int sss_pm3_create(sss_ctx* ctx, int mesh_n, double box, sss_pm3** ou
     e = e ? e : cudaMalloc(&p->rk, mp * sizeof(float2));
     e = e ? e : cudaMalloc(&p->ak, 3 * mp * sizeof(float2));
     e = e ? e : cudaMalloc(&p->acc, 3 * n3 * sizeof(float));
-    e = e ? e : cudaMalloc(&p->tab, 3 * (size_t)mesh_n * sizeof(double));
+    e = e ? e : cudaMalloc(&p->tab, 4 * (size_t)mesh_n * sizeof(double));
     p->tab_deconv = -1;
     if (e != cudaSuccess) {
         pm3_free(p);

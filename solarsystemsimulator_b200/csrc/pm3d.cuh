@@ -20,7 +20,7 @@ struct sss_pm3 {
     float2* tw;         // own: twiddles of length n
     cufftHandle fwd;    // R2C n^3
     cufftHandle inv3;   // C2R n^3, batch 3
-    double* tab;        // per-axis tables of the spectrum kernel: kd[n], k2[n], fac[n]
+    double* tab;        // per-axis tables of the spectrum kernel: kd[n], k2[n], fac[n], kd as two f32 [n]
     int tab_deconv;     // parameters the tables were built for (-1: none yet)
     double tab_rs2;
 };

@@ -421,3 +421,36 @@ def test_first_solve_on_another_stream(n):
     torch.cuda.synchronize()
     pm._call("sss_pm3_solve", 1.5, pm.deconv, pm.r_split)
     assert torch.equal(first, pm.acc_mesh)
+
+
+@pytest.mark.parametrize("n", [32, 64, 128, 256, 512])
+def test_gradient_factors_are_not_rounded(n):
+    """i k phi is k (f64) times phi, rounded once, along every axis: one mode
+    (n / 4, whose density is 1, 0, -1, 0, ... and whose transform is exact), a
+    box and a G that make its k some f64 value K and its phi an f32 value P,
+    against a box and a G that make k a power of two and k phi the same V =
+    f32(K P). Every operation is the same one from there on, so the meshes are
+    equal bit by bit. K and P are draws where rounding K first would give
+    another V."""
+    from solarsystemsimulator_b200.pm3d import PMPeriodic3D
+    rng = np.random.default_rng(n)
+    f32, cases = np.float32, []
+    while len(cases) < 4:
+        K, P = rng.uniform(1.0, 2.0), float(f32(rng.uniform(1.0, 2.0)))
+        V = float(f32(K * P))
+        off = abs(K * P - V) / 2.0 ** (np.floor(np.log2(V)) - 23)           # steps of f32 off; 0.5 is a tie
+        if off < 0.49 and float(f32(float(f32(K)) * P)) != V:
+            cases.append((K, P, V))
+    wave = torch.tensor([1.0, 0.0, -1.0, 0.0], device="cuda").repeat(n // 4)
+
+    def mesh(axis, k, phi):
+        pm = PMPeriodic3D(n, box=2.0 * np.pi * (n // 4) / k, G=phi * k * k / (2.0 * np.pi), deconv=0, r_split_cells=0.0)
+        pm.rho.copy_(wave.view([n if d == axis else 1 for d in range(3)]).expand(n, n, n))
+        pm._call("sss_pm3_solve", pm.G, 0, 0.0)
+        return pm.acc_mesh[axis].clone()
+
+    for axis in range(3):
+        for K, P, V in cases[: 4 if n < 512 else 1]:
+            a, b = mesh(axis, K, P), mesh(axis, 1.0, V)
+            assert abs(float(a.abs().max()) / (2.0 * V) - 1.0) < 1e-6
+            assert torch.equal(a, b), (axis, K, P, V)
