@@ -278,7 +278,8 @@ int  sss_pm2d_to_f32(sss_pm2d* p, const double* a, int64_t n, float* out, void* 
  * Index 0 of the arrays: the n masses, 1: the t tracers. *kernel_h (host, in
  * and out, <= 0: none) is the cell size the force kernels stand for (:216-221).
  * snap: steps rows f32 [x|y|vx|vy|tx|ty]. Synchronous. Only where
- * sss_pm2d_steps_natively (2 grid_n = 2^a, 3 2^a or 1000 2^a, 64 .. 8192). */
+ * sss_pm2d_steps_natively (grid_n = 2^a or 3 2^a, 32 .. 4096, or 500, 1000,
+ * 2000). */
 typedef struct sss_pm2d_bodies {
     double* x[2];
     double* y[2];

@@ -8,7 +8,7 @@
 // folded in), transformed back and read bilinearly with the deposit's
 // stencil. f64 throughout, as the reference.
 //
-// The convolution (2N = 2^a, 3 2^a or 1000 2^a up to 8192) is three kernels
+// The convolution (2N = 2^a, 3 2^a, 1000, 2000 or 4000 up to 8192) is three kernels
 // over the block transforms of fft.cuh:
 //   k_rows_fwd : two real rows a, b as one complex transform a + i b; only
 //                the N rows and the N columns that hold mass are read
@@ -322,10 +322,14 @@ Convolve2d convolve_of() {
     return {k_rows_fwd<L>, k_cols<L>, k_rows_inv<L>, fft_threads(L, 1)};
 }
 
-// Padded lengths 2N with kernels: 2^a, 3 2^a and 1000 2^a from 64 to 8192
-// (the transform and its 16 values per thread bound the length: 139 KB of
-// shared memory and 512 threads of 128 registers at 8192). Measured against
-// cuFFT's five transforms a field: see k_cols.
+// Padded lengths 2N with kernels: 2^a and 3 2^a from 64 to 8192, and 1000, 2000
+// and 4000, the decimal grids of 500, 1,000 and 2,000 points. Every length is
+// three kernels of its own, so only sizes that simulations ask for have them;
+// any other grid (640, 1,200, ...) convolves through cuFFT as well. 8192 is the
+// longest: 139 KB of shared memory and 512 threads of 128 registers. 8000 (a grid
+// of 4,000) is none: its radix-5 stages, three butterflies a thread, need 544
+// threads. A step on a 2048 grid: 343 us; through cuFFT, kernels remade for its
+// h, 1,083.
 bool convolve_for(int L, Convolve2d* c) {
     switch (L) {
 #define CASE(n) case n: *c = convolve_of<n>(); return true

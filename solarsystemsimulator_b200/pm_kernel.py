@@ -12,8 +12,8 @@ gather, adaptive grid geometry, KDK):
 
 and the module functions build_force_kernels, grid_fuer, pm_force_field,
 gather_accel, pm_accelerations, _cic_deposit, _cic_gather on CUDA tensors.
-The work runs in libsss (sss_pm2d_*): own transforms for grids of 2^a, 3 2^a and
-500 2^a points, cuFFT for others.
+The work runs in libsss (sss_pm2d_*): own transforms for grids of 2^a and 3 2^a
+points from 32 to 4096 and of 500, 1000 and 2000 points, cuFFT for others.
 """
 from __future__ import annotations
 

@@ -224,6 +224,15 @@ def test_native_steps_equal_the_parts(n, tracers, grid):
     sims[0]._plan.native_steps = True
 
 
+@pytest.mark.parametrize("n,own", [(96, True), (128, True), (192, True), (768, True), (2000, True), (3072, True),
+                                   (4000, False), (640, False)])
+def test_convolution_of_the_other_lengths(n, own):
+    """The other lengths with kernels of their own (2 n = 192 .. 6144), and 8000,
+    whose transform needs too many threads, and 1280, through cuFFT."""
+    assert _pk().plan_for(n).native_steps is own
+    test_convolution_of_every_length(n)
+
+
 def test_kernels_after_native_steps_a_deposit_and_a_load():
     """Accelerations of a state loaded after a native batch and a density of
     the same grid size: those of the object's own softening and G (a deposit
