@@ -89,30 +89,50 @@ __device__ __forceinline__ int pp_chunks(const int* first, const int* last, long
     return (last[c] - first[c] + 31) / 32;
 }
 
-// (cell, first target) of every item into the list of its class (thread per
-// cell; an item's length falls along its cell, so a class is one stretch)
+// (cell, first target) of every item into the list, the classes one after
+// another, the longest first (thread per cell; an item's length falls along its
+// cell, so a class is one stretch). Two launches: COUNT adds up the classes'
+// lengths, the other writes behind its class's cursor. (A list of full length a
+// class in one launch took 16 times the memory, 128 bytes a particle.)
+template <bool COUNT>
 __global__ void k_pp_items(const int* __restrict__ first, const int* __restrict__ last, int M, long long cells,
-                           long long max_items, int2* __restrict__ items, unsigned* __restrict__ n_items) {
+                           unsigned* __restrict__ n_items, unsigned* __restrict__ cursor, int2* __restrict__ items) {
+    __shared__ unsigned base[PP_CLASSES];
+    if (!COUNT) {
+        if (threadIdx.x < PP_CLASSES) {
+            unsigned b = 0;
+            for (int k = PP_CLASSES - 1; k > (int)threadIdx.x; --k) b += n_items[k];
+            base[threadIdx.x] = b;
+        }
+        __syncthreads();
+    }
     const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= cells) return;
     const int g = pp_chunks(first, last, c);
     if (g == 0) return;
     const int cx = (int)(c % M), cy = (int)((c / M) % M), cz = (int)(c / ((long long)M * M));
+    const int xs[3] = {cx ? cx - 1 : M - 1, cx, cx + 1 < M ? cx + 1 : 0};
+    const int ys[3] = {cy ? cy - 1 : M - 1, cy, cy + 1 < M ? cy + 1 : 0};
+    const int zs[3] = {cz ? cz - 1 : M - 1, cz, cz + 1 < M ? cz + 1 : 0};
     long long near = 0;
+#pragma unroll
     for (int nb = 0; nb < 27; ++nb) {
         if (nb == 13) continue;
-        const int nx = (cx + nb % 3 - 1 + M) % M, ny = (cy + (nb / 3) % 3 - 1 + M) % M, nz = (cz + nb / 9 - 1 + M) % M;
-        const long long nc = ((long long)nz * M + ny) * M + nx;
-        if (nc > c) near += pp_chunks(first, last, nc);
+        const long long nc = ((long long)zs[nb / 9] * M + ys[nb / 3 % 3]) * M + xs[nb % 3];
+        const int q = pp_chunks(first, last, nc);
+        near += nc > c ? q : 0;
     }
-    const int gi = g;
-    for (int k = 0; k < gi;) {
+    for (int k = 0; k < g;) {
         const long long len = near + g - k;                 // >= 1
         const int cls = min(PP_CLASSES - 1, 63 - __clzll(len));
         // down to length 2^cls the class stays the same (class 15 is open above)
-        const int run = (int)min((long long)(gi - k), len - (1ll << cls) + 1);
-        const unsigned at = atomicAdd(n_items + cls, (unsigned)run);
-        for (int j = 0; j < run; ++j) items[cls * max_items + at + j] = make_int2((int)c, first[c] + 32 * (k + j));
+        const int run = (int)min((long long)(g - k), len - (1ll << cls) + 1);
+        if (COUNT) {
+            atomicAdd(n_items + cls, (unsigned)run);
+        } else {
+            const unsigned at = base[cls] + atomicAdd(cursor + cls, (unsigned)run);
+            for (int j = 0; j < run; ++j) items[at + j] = make_int2((int)c, first[c] + 32 * (k + j));
+        }
         k += run;
     }
 }
@@ -127,9 +147,8 @@ struct PPArgs {
     double box;
     double G;
     float alpha, rc2, eps2;
-    const int2* items;              // PP_CLASSES lists of max_items
-    const unsigned* n_items;        // their lengths
-    long long max_items;
+    const int2* items;              // longest first
+    const unsigned* n_items;        // by class
     unsigned* next;                 // work counter (zero at launch)
     float* acc;                     // 3 x n, by cell-order position (zero at launch)
     long long n;
@@ -399,14 +418,7 @@ __device__ __forceinline__ void pp_item(ulonglong2* stage, int lane, const PPArg
 __global__ void __launch_bounds__(PP_WARPS * 32) k_pp_pairs(const PPArgs q) {
     __shared__ ulonglong2 sh[PP_WARPS][64];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    // lane k < PP_CLASSES: end of class 15 - k in the order the items are taken
-    unsigned end = lane < PP_CLASSES ? q.n_items[PP_CLASSES - 1 - lane] : 0;
-#pragma unroll
-    for (int o = 1; o < PP_CLASSES; o <<= 1) {
-        const unsigned y = __shfl_up_sync(0xffffffffu, end, o);
-        if (lane >= o) end += y;
-    }
-    const unsigned total = __shfl_sync(0xffffffffu, end, PP_CLASSES - 1);
+    const unsigned total = __reduce_add_sync(0xffffffffu, lane < PP_CLASSES ? q.n_items[lane] : 0u);
     ulonglong2* stage = sh[w];
     PPConst k;
     k.alpha = dup(q.alpha);
@@ -416,9 +428,7 @@ __global__ void __launch_bounds__(PP_WARPS * 32) k_pp_pairs(const PPArgs q) {
         if (lane == 0) it = atomicAdd(q.next, 1u);
         it = __shfl_sync(0xffffffffu, it, 0);
         if (it >= total) break;
-        const int b = __popc(__ballot_sync(0xffffffffu, lane < PP_CLASSES && end <= it));
-        const unsigned before = __shfl_sync(0xffffffffu, end, max(b - 1, 0));
-        const int2 item = q.items[(PP_CLASSES - 1 - b) * q.max_items + (it - (b ? before : 0u))];
+        const int2 item = q.items[it];
         pp_item<1>(stage, lane, q, item.x, item.y, k);
     }
 }
@@ -463,7 +473,7 @@ extern "C" int sss_pm3_short(sss_pm3* p, const sss_pm3_particles* s, double G, d
     const size_t o_src = take(32 * n), o_first = take(4 * cells), o_last = take(4 * cells);
     const size_t o_rs = take(8 * sss_dev::radix_scratch(n));
     const long long max_items = n / 32 + std::min<long long>(cells, n);
-    const size_t o_items = take(8 * (size_t)max_items * PP_CLASSES), o_cnt = take(4 * (PP_CLASSES + 1));
+    const size_t o_items = take(8 * (size_t)max_items), o_cnt = take(4 * (2 * PP_CLASSES + 1));
     const size_t o_acc = take(12 * n);
     void* scr = nullptr;
     int rc = sss_scratch(ctx, off, &scr);
@@ -477,7 +487,7 @@ extern "C" int sss_pm3_short(sss_pm3* p, const sss_pm3_particles* s, double G, d
     int* first = (int*)(B + o_first);
     int* last = (int*)(B + o_last);
     int2* items = (int2*)(B + o_items);
-    unsigned* counters = (unsigned*)(B + o_cnt);                  // items per class, work counter
+    unsigned* counters = (unsigned*)(B + o_cnt);                  // items per class, cursors, work counter
     const Pm3Parts parts = pm3_parts(s);
     const double l = p->box / M;
     k_pp_keys<<<blocks_for(n, 256), 256, 0, st>>>(parts, M, 1.0 / l, k0, v0);
@@ -489,10 +499,13 @@ extern "C" int sss_pm3_short(sss_pm3* p, const sss_pm3_particles* s, double G, d
     SSS_CUDA_TRY(ctx, cudaMemsetAsync(last, 0, 4 * (size_t)cells, st));
     k_pp_bounds<<<blocks_for(n, 256), 256, 0, st>>>(k0, n, first, last);
     SSS_LAUNCH_CHECK(ctx, "k_pp_bounds");
-    SSS_CUDA_TRY(ctx, cudaMemsetAsync(counters, 0, 4 * (PP_CLASSES + 1), st));
+    SSS_CUDA_TRY(ctx, cudaMemsetAsync(counters, 0, 4 * (2 * PP_CLASSES + 1), st));
     int per_sm = 0;
     SSS_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pp_pairs, PP_WARPS * 32, 0));
-    k_pp_items<<<blocks_for(cells, 128), 128, 0, st>>>(first, last, M, cells, max_items, items, counters);
+    const unsigned ib = blocks_for(cells, 128);
+    k_pp_items<true><<<ib, 128, 0, st>>>(first, last, M, cells, counters, counters + PP_CLASSES, items);
+    SSS_LAUNCH_CHECK(ctx, "k_pp_items (count)");
+    k_pp_items<false><<<ib, 128, 0, st>>>(first, last, M, cells, counters, counters + PP_CLASSES, items);
     SSS_LAUNCH_CHECK(ctx, "k_pp_items");
     PPArgs q;
     q.src = src;
@@ -508,8 +521,7 @@ extern "C" int sss_pm3_short(sss_pm3* p, const sss_pm3_particles* s, double G, d
     q.eps2 = (float)(eps * eps);
     q.items = items;
     q.n_items = counters;
-    q.max_items = max_items;
-    q.next = counters + PP_CLASSES;
+    q.next = counters + 2 * PP_CLASSES;
     q.acc = (float*)(B + o_acc);
     q.n = n;
     SSS_CUDA_TRY(ctx, cudaMemsetAsync(q.acc, 0, 12 * (size_t)n, st));

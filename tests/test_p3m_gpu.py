@@ -111,3 +111,22 @@ def test_pair_term_item_shapes(n, spread, x_cut, eps, equal):
     tol = (newton * (1e-6 + 3.0 * np.sqrt(3.0) * 2.0 * cell * 2.0 ** -24 / r)).sum(1)
     tol += newton.sum(1) * (newton > 0).sum(1) * 2.0 ** -24
     assert np.all(np.abs(a[sel] - ref).max(1) <= tol + 1e-30)
+
+
+def test_pair_term_scratch(monkeypatch):
+    """The pair pass's working memory with as many cells as particles: keys and
+    order twice (24 bytes a particle), records (32), accumulator (12), bounds
+    (8 a cell), one list of items (8 a cell, 8 per 32 particles), the sort's
+    counts (8 passes of 256 for every 2,048 particles: 8) and 4 MB."""
+    from solarsystemsimulator_b200 import _lib, pm3d
+    n = 1_000_000
+    ctx = _lib.Context(0)                                   # (with no scratch yet)
+    monkeypatch.setattr(_lib, "context", lambda device: ctx)
+    pm = pm3d.PMPeriodic3D(384, 1.0, 1.0, 0, 2, 0.64, short_range=True, softening=1e-3, x_cut=2.999)
+    assert int(pm.box / pm.r_cut) ** 3 == n
+    st = pm.load_state(np.random.default_rng(0).uniform(0, 1, (n, 3)), np.zeros((n, 3)), 1.0 / n)
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    pm.short(st)
+    torch.cuda.synchronize()
+    assert free - torch.cuda.mem_get_info()[0] <= 93 * n + (4 << 20)
