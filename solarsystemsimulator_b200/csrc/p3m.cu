@@ -255,58 +255,48 @@ struct PPTarget {
     f2x ax, ay, az;
 };
 
-// One chunk of sources against the lanes' G targets, two sources per step:
-// offsets (a, a + da) for steps a = a0 .. a1 - 1 (source (lane + offset) mod
+// One chunk of sources against the lanes' targets, two sources per step:
+// offsets (a, a + DA) for steps a = A0 .. A1 - 1 (source (lane + offset) mod
 // 32); OWN masks offset 16 on lanes 16 .. 31 (32 particles among themselves,
 // whose pairs (l, l + 16) and (l + 16, l) coincide). Both sources' sums rotate
 // through the lanes and end on their own lanes, then go to the accumulator.
 // 35 FMA-pipe operations and four special-function ones a pair (the latter
 // bound it), with the 6 shuffles and two 16-byte shared loads of a step shared
-// by its 2 G pairs. 1,048,576 particles collapsed into halos (7.2e9 candidate
-// pairs, 5.1e9 in range): 12.3 ms a step against 15.4 with sources packed by
+// by its 2 pairs. 1,048,576 particles collapsed into halos (7.2e9 candidate
+// pairs, 5.1e9 in range): 12.5 ms a step against 15.4 with sources packed by
 // register moves and items in cell order (the last heavy items then ran on by
-// themselves). Sorting particles
-// inside a cell and testing chunk boxes saves only a fifth of these pairs.
-template <int G, bool OWN, int A0, int A1, int DA>
-__device__ __forceinline__ void pp_chunk2(const ulonglong2* stage, int lane, PPTarget (&T)[2], const PPConst& k,
+// themselves). Sorting particles inside a cell and testing chunk boxes saves
+// only a fifth of these pairs.
+template <bool OWN, int A0, int A1, int DA>
+__device__ __forceinline__ void pp_chunk2(const ulonglong2* stage, int lane, PPTarget& t, const PPConst& k,
                                           const PPArgs& q, long long src0, int m) {
-    f2x BX = 0ull, BY = 0ull, BZ = 0ull;             // sums of sources (lane + a) and (lane + a + da)
+    f2x BX = 0ull, BY = 0ull, BZ = 0ull;             // sums of sources (lane + a) and (lane + a + DA)
     const int from = (lane + 1) & 31;
-#pragma unroll (G == 1 ? 2 : 1)
+#pragma unroll 2
     for (int a = A0; a < A1; ++a) {
         const ulonglong2 xy = stage[(lane + a) & 31], zm = stage[32 + ((lane + a) & 31)];
-        f2x DX[G], DY[G], DZ[G], H[G];
-#pragma unroll
-        for (int g = 0; g < G; ++g) {
-            DX[g] = add2(xy.x, T[g].nx);
-            DY[g] = add2(xy.y, T[g].ny);
-            DZ[g] = add2(zm.x, T[g].nz);
-            const f2x R2 = fma2(DX[g], DX[g], fma2(DY[g], DY[g], mul2(DZ[g], DZ[g])));
-            float r0, r1, h0, h1;
-            upk2(R2, r0, r1);
-            const bool in0 = r0 < q.rc2 && r0 > 0.0f;
-            const bool in1 = r1 < q.rc2 && r1 > 0.0f && !(OWN && a + DA == 16 && lane >= 16);
-            upk2(pp_h2(R2, k.alpha, k.eps2), h0, h1);
-            H[g] = pk2(in0 ? h0 : 0.0f, in1 ? h1 : 0.0f);
-        }
-#pragma unroll
-        for (int g = 0; g < G; ++g) {
-            PPTarget& t = T[g];
-            const f2x HJ = mul2(H[g], zm.y), HI = mul2(H[g], t.nm);
-            t.ax = fma2(HJ, DX[g], t.ax);
-            t.ay = fma2(HJ, DY[g], t.ay);
-            t.az = fma2(HJ, DZ[g], t.az);
-            BX = fma2(HI, DX[g], BX);
-            BY = fma2(HI, DY[g], BY);
-            BZ = fma2(HI, DZ[g], BZ);
-        }
+        const f2x DX = add2(xy.x, t.nx), DY = add2(xy.y, t.ny), DZ = add2(zm.x, t.nz);
+        const f2x R2 = fma2(DX, DX, fma2(DY, DY, mul2(DZ, DZ)));
+        float r0, r1, h0, h1;
+        upk2(R2, r0, r1);
+        const bool in0 = r0 < q.rc2 && r0 > 0.0f;
+        const bool in1 = r1 < q.rc2 && r1 > 0.0f && !(OWN && a + DA == 16 && lane >= 16);
+        upk2(pp_h2(R2, k.alpha, k.eps2), h0, h1);
+        const f2x H = pk2(in0 ? h0 : 0.0f, in1 ? h1 : 0.0f);
+        const f2x HJ = mul2(H, zm.y), HI = mul2(H, t.nm);
+        t.ax = fma2(HJ, DX, t.ax);
+        t.ay = fma2(HJ, DY, t.ay);
+        t.az = fma2(HJ, DZ, t.az);
+        BX = fma2(HI, DX, BX);
+        BY = fma2(HI, DY, BY);
+        BZ = fma2(HI, DZ, BZ);
         if (a + 1 < A1) {                                          // take the next lane's sums (sources + 1)
             BX = shfl2(BX, from);
             BY = shfl2(BY, from);
             BZ = shfl2(BZ, from);
         }
     }
-    // lane l holds sources (l + a1 - 1) and (l + a1 - 1 + da): deliver both to their lanes
+    // lane l holds sources (l + A1 - 1) and (l + A1 - 1 + DA): deliver both to their lanes
     const int fa = (lane - (A1 - 1)) & 31, fb = (lane - (A1 - 1 + DA)) & 31;
     float xa, xb, ya, yb, za, zb, t0, t1;
     upk2(shfl2(BX, fa), xa, t0);
@@ -322,10 +312,9 @@ __device__ __forceinline__ void pp_chunk2(const ulonglong2* stage, int lane, PPT
     }
 }
 
-// The sources [s0, s1) (shifted by s) against the lanes' G targets, chunk by chunk.
-template <int G>
-__device__ __forceinline__ void pp_walk(ulonglong2* stage, int lane, PPTarget (&T)[2], const PPConst& k,
-                                        const PPArgs& q, int s0, int s1, double sx, double sy, double sz) {
+// The sources [s0, s1) (shifted by s) against the lanes' targets, chunk by chunk.
+__device__ __forceinline__ void pp_walk(ulonglong2* stage, int lane, PPTarget& t, const PPConst& k, const PPArgs& q,
+                                        int s0, int s1, double sx, double sy, double sz) {
     for (int j0 = s0; j0 < s1; j0 += 32) {
         const int j = j0 + lane;
         float x = 1e18f, y = 1e18f, z = 1e18f, m = 0.0f;            // padding: out of range of everything
@@ -337,55 +326,36 @@ __device__ __forceinline__ void pp_walk(ulonglong2* stage, int lane, PPTarget (&
             m = (float)p.w;
         }
         pp_stage(stage, lane, 16, x, y, z, m);
-        pp_chunk2<G, false, 0, 16, 16>(stage, lane, T, k, q, j0, min(32, s1 - j0));
+        pp_chunk2<false, 0, 16, 16>(stage, lane, t, k, q, j0, min(32, s1 - j0));
     }
 }
 
-// An item: the targets from t0 of a cell as G = 1 or 2 groups of 32. Every target meets its sources in
-// ascending order, whatever the group it is in.
-template <int G>
+// An item: the 32 targets from t0 of a cell. Every target meets its sources in ascending order.
 __device__ __forceinline__ void pp_item(ulonglong2* stage, int lane, const PPArgs& q, int c, int t0,
                                         const PPConst& k) {
     const int M = q.M, cl = q.last[c];
     const int cx = c % M, cy = (c / M) % M, cz = c / (M * M);
     const double ox = cx * q.l, oy = cy * q.l, oz = cz * q.l;
-    PPTarget T[2];
-#pragma unroll
-    for (int g = 0; g < G; ++g) {
-        const int t = t0 + 32 * g + lane;
-        float tx = -1e18f, ty = -1e18f, tz = -1e18f, tm = 0.0f;     // padding: out of range, of padding sources too
-        if (t < cl) {
-            const double4 p = q.src[t];
-            tx = (float)(p.x - ox);
-            ty = (float)(p.y - oy);
-            tz = (float)(p.z - oz);
-            tm = (float)p.w;
-        }
-        T[g] = PPTarget{dup(-tx), dup(-ty), dup(-tz), dup(-tm), 0ull, 0ull, 0ull};
+    const int t = t0 + lane;
+    const bool act = t < cl;
+    float tx = -1e18f, ty = -1e18f, tz = -1e18f, tm = 0.0f;         // padding: out of range, of padding sources too
+    if (act) {
+        const double4 p = q.src[t];
+        tx = (float)(p.x - ox);
+        ty = (float)(p.y - oy);
+        tz = (float)(p.z - oz);
+        tm = (float)p.w;
     }
-    // each group's particles with each other (offsets 1 .. 16 as (j, j + 8), j = 1 .. 8), then the first with the second
-#pragma unroll
-    for (int g = 0; g < G; ++g) {
-        const int t = t0 + 32 * g + lane;
-        const bool act = t < cl;
-        float x, y, z, m, h;
-        upk2(T[g].nx, x, h);
-        upk2(T[g].ny, y, h);
-        upk2(T[g].nz, z, h);
-        upk2(T[g].nm, m, h);
-        pp_stage(stage, lane, 8, act ? -x : 1e18f, act ? -y : 1e18f, act ? -z : 1e18f, -m);
-        PPTarget one[2];
-        one[0] = T[g];
-        pp_chunk2<1, true, 1, 9, 8>(stage, lane, one, k, q, t0 + 32 * g, min(32, cl - t0 - 32 * g));
-        T[g] = one[0];
-    }
-    if (G == 2) pp_walk<1>(stage, lane, T, k, q, t0 + 32, min(cl, t0 + 64), -ox, -oy, -oz);
+    PPTarget T{dup(-tx), dup(-ty), dup(-tz), dup(-tm), 0ull, 0ull, 0ull};
+    // the particles with each other (offsets 1 .. 16 as (j, j + 8), j = 1 .. 8)
+    pp_stage(stage, lane, 8, act ? tx : 1e18f, act ? ty : 1e18f, act ? tz : 1e18f, tm);
+    pp_chunk2<true, 1, 9, 8>(stage, lane, T, k, q, t0, min(32, cl - t0));
     // the later particles of the cell, then the neighbouring cells of higher index
     for (int nb = -1; nb < 27; ++nb) {
         int s0, s1;
         double sx = -ox, sy = -oy, sz = -oz;                    // source shift: periodic image - corner
         if (nb < 0) {
-            s0 = t0 + 32 * G;
+            s0 = t0 + 32;
             s1 = cl;
         } else {
             if (nb == 13) continue;                            // the cell itself
@@ -398,20 +368,16 @@ __device__ __forceinline__ void pp_item(ulonglong2* stage, int lane, const PPArg
             s0 = q.first[nc];
             s1 = q.last[nc];
         }
-        pp_walk<G>(stage, lane, T, k, q, s0, s1, sx, sy, sz);
+        pp_walk(stage, lane, T, k, q, s0, s1, sx, sy, sz);
     }
-#pragma unroll
-    for (int g = 0; g < G; ++g) {
-        const int t = t0 + 32 * g + lane;
-        float x0, x1, y0, y1, z0, z1;
-        upk2(T[g].ax, x0, x1);
-        upk2(T[g].ay, y0, y1);
-        upk2(T[g].az, z0, z1);
-        if (t < cl) {
-            atomicAdd(q.acc + t, x0 + x1);
-            atomicAdd(q.acc + q.n + t, y0 + y1);
-            atomicAdd(q.acc + 2 * q.n + t, z0 + z1);
-        }
+    float x0, x1, y0, y1, z0, z1;
+    upk2(T.ax, x0, x1);
+    upk2(T.ay, y0, y1);
+    upk2(T.az, z0, z1);
+    if (act) {
+        atomicAdd(q.acc + t, x0 + x1);
+        atomicAdd(q.acc + q.n + t, y0 + y1);
+        atomicAdd(q.acc + 2 * q.n + t, z0 + z1);
     }
 }
 
@@ -429,7 +395,7 @@ __global__ void __launch_bounds__(PP_WARPS * 32) k_pp_pairs(const PPArgs q) {
         it = __shfl_sync(0xffffffffu, it, 0);
         if (it >= total) break;
         const int2 item = q.items[it];
-        pp_item<1>(stage, lane, q, item.x, item.y, k);
+        pp_item(stage, lane, q, item.x, item.y, k);
     }
 }
 
