@@ -436,10 +436,12 @@ extern "C" int sss_pm3_short(sss_pm3* p, const sss_pm3_particles* s, double G, d
     size_t off = 0;
     auto take = [&](size_t bytes) { const size_t o = off; off += (bytes + 255) & ~(size_t)255; return o; };
     const size_t o_k0 = take(8 * n), o_k1 = take(8 * n), o_v0 = take(4 * n), o_v1 = take(4 * n);
-    const size_t o_src = take(32 * n), o_first = take(4 * cells), o_last = take(4 * cells);
+    const size_t o_src = take(32 * n);
     const size_t o_rs = take(8 * sss_dev::radix_scratch(n));
     const long long max_items = n / 32 + std::min<long long>(cells, n);
-    const size_t o_items = take(8 * (size_t)max_items), o_cnt = take(4 * (2 * PP_CLASSES + 1));
+    const size_t o_items = take(8 * (size_t)max_items);
+    // zero at the start, so next to one another: one memset for the four
+    const size_t o_first = take(4 * cells), o_last = take(4 * cells), o_cnt = take(4 * (2 * PP_CLASSES + 1));
     const size_t o_acc = take(12 * n);
     void* scr = nullptr;
     int rc = sss_scratch(ctx, off, &scr);
@@ -461,11 +463,9 @@ extern "C" int sss_pm3_short(sss_pm3* p, const sss_pm3_particles* s, double G, d
     SSS_CUDA_TRY(ctx, sss_dev::radix_sort(k0, v0, k1, v1, n, (long long*)(B + o_rs), st, ctx->d_status, bits));
     k_pp_gather<<<blocks_for(n, 256), 256, 0, st>>>(parts, v0, src);
     SSS_LAUNCH_CHECK(ctx, "k_pp_gather");
-    SSS_CUDA_TRY(ctx, cudaMemsetAsync(first, 0, 4 * (size_t)cells, st));
-    SSS_CUDA_TRY(ctx, cudaMemsetAsync(last, 0, 4 * (size_t)cells, st));
+    SSS_CUDA_TRY(ctx, cudaMemsetAsync(first, 0, off - o_first, st));
     k_pp_bounds<<<blocks_for(n, 256), 256, 0, st>>>(k0, n, first, last);
     SSS_LAUNCH_CHECK(ctx, "k_pp_bounds");
-    SSS_CUDA_TRY(ctx, cudaMemsetAsync(counters, 0, 4 * (2 * PP_CLASSES + 1), st));
     int per_sm = 0;
     SSS_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pp_pairs, PP_WARPS * 32, 0));
     const unsigned ib = blocks_for(cells, 128);
@@ -490,7 +490,6 @@ extern "C" int sss_pm3_short(sss_pm3* p, const sss_pm3_particles* s, double G, d
     q.next = counters + 2 * PP_CLASSES;
     q.acc = (float*)(B + o_acc);
     q.n = n;
-    SSS_CUDA_TRY(ctx, cudaMemsetAsync(q.acc, 0, 12 * (size_t)n, st));
     const unsigned grid = (unsigned)(ctx->num_sms * std::max(per_sm, 1));
     k_pp_pairs<<<grid, PP_WARPS * 32, 0, st>>>(q);
     SSS_LAUNCH_CHECK(ctx, "k_pp_pairs");
