@@ -216,34 +216,24 @@ template <int L>
 __global__ void __launch_bounds__(fft_threads(L, 1), 512 / fft_threads(L, 1))
 k_rows_fwd(const double2* __restrict__ tw, const double* __restrict__ rho, double2* __restrict__ out) {
     constexpr int n = L / 2;
+    static_assert(n % 2 == 0, "pairs of rows");
     extern __shared__ double2 sm2[];
     using Map = fft::One;
-    for (int p = blockIdx.x; p < (n + 1) / 2; p += gridDim.x) {
+    for (int p = blockIdx.x; p < n / 2; p += gridDim.x) {
         const double* ra = rho + (long long)(2 * p) * n;
-        const bool two = 2 * p + 1 < n;
         __syncthreads();
         fft::run<L, -1, Map>(tw, sm2,
                      [&](int i, int, bool hi) {
                          double2 z = make_double2(0.0, 0.0);
-                         if (!hi) {
-                             z.x = __ldg(ra + i);
-                             if (two) z.y = __ldg(ra + n + i);
-                         }
+                         if (!hi) z = make_double2(__ldg(ra + i), __ldg(ra + n + i));
                          return z;
                      },
                      [&](int i, int, double2 z, bool) { sm2[Map::at(i, 0)] = z; });
         __syncthreads();
         for (int k = threadIdx.x; k <= n; k += blockDim.x) {
             const double2 z = sm2[Map::at(k, 0)], w = sm2[Map::at(k == 0 ? 0 : L - k, 0)];
-            double2* o = out + (long long)k * n + 2 * p;
-            const double2 a = make_double2(0.5 * (z.x + w.x), 0.5 * (z.y - w.y));
-            const double2 b = make_double2(0.5 * (z.y + w.y), 0.5 * (w.x - z.x));
-            if (n % 2 == 0) {
-                st_pair(o, a, b);
-            } else {
-                o[0] = a;
-                if (two) o[1] = b;
-            }
+            st_pair(out + (long long)k * n + 2 * p, make_double2(0.5 * (z.x + w.x), 0.5 * (z.y - w.y)),
+                    make_double2(0.5 * (z.y + w.y), 0.5 * (w.x - z.x)));
         }
     }
 }
@@ -569,7 +559,7 @@ static int pm2d_free(sss_pm2d* p) {
 static cudaError_t pm2d_own_setup(sss_pm2d* p) {
     const int L = 2 * p->n;
     const void* fn[3] = {(const void*)p->conv.rows_fwd, (const void*)p->conv.cols, (const void*)p->conv.rows_inv};
-    const int items[3] = {(p->n + 1) / 2, p->n + 1, p->n};
+    const int items[3] = {p->n / 2, p->n + 1, p->n};
     const size_t n = (size_t)p->n, m = n + 1;
     p->smem = (size_t)(L + L / 16 + 1) * sizeof(double2);
     cudaError_t e = fft_table(L, &p->tw);
