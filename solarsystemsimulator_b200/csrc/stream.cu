@@ -1242,10 +1242,14 @@ struct Work {
     Ctl* ctl;
 };
 
-// scratch of the `slots` samples that run at once (reused by the following
-// ones of a batch in stream order) and n_ctl control blocks (one per sample
-// of the batch)
-int make_work(sss_ctx* ctx, long long n, int grid, int slots, int n_ctl, Work* W) {
+// scratch of the *slots samples that run at once (reused by the following
+// ones of a batch in stream order; fewer where SLOTS_BYTES hold no more, one
+// where there is no memory for several) and n_ctl control blocks (one per
+// sample of the batch). A sample's buffers take 10 bytes a body and 5 MB of
+// tables. The context keeps its scratch, hence the bound.
+constexpr size_t SLOTS_BYTES = (size_t)256 << 20;
+
+int make_work(sss_ctx* ctx, long long n, int grid, int* slots, int n_ctl, Work* W) {
     size_t off = 0;
     const size_t o_qx = off; off += al((size_t)n * 4);
     const size_t o_qy = off; off += al((size_t)n * 4);
@@ -1260,10 +1264,15 @@ int make_work(sss_ctx* ctx, long long n, int grid, int slots, int n_ctl, Work* W
     const size_t o_vpre = off; off += al((size_t)2 * (VALUE_MAX + 1) * 8);
     const size_t o_blk = off; off += al((size_t)grid * BLK * 8);
     W->slot = off;
-    off *= (size_t)slots;
-    const size_t o_ctl = off; off += al(sizeof(Ctl) * (size_t)n_ctl);
+    while (*slots > 1 && (size_t)*slots * W->slot > SLOTS_BYTES) --*slots;
+    const size_t ctl = al(sizeof(Ctl) * (size_t)n_ctl);
     void* scr = nullptr;
-    int rc = sss_scratch(ctx, off, &scr);
+    int rc = sss_scratch(ctx, (size_t)*slots * W->slot + ctl, &scr);
+    if (rc && *slots > 1) {
+        cudaGetLastError();
+        *slots = 1;
+        rc = sss_scratch(ctx, W->slot + ctl, &scr);
+    }
     if (rc) return rc;
     char* p = (char*)scr;
     W->qx = (float*)(p + o_qx);
@@ -1278,7 +1287,7 @@ int make_work(sss_ctx* ctx, long long n, int grid, int slots, int n_ctl, Work* W
     W->vmul = (unsigned*)(p + o_vmul);
     W->vpre = (double*)(p + o_vpre);
     W->blk = (long long*)(p + o_blk);
-    W->ctl = (Ctl*)(p + o_ctl);
+    W->ctl = (Ctl*)(p + (size_t)*slots * W->slot);
     return SSS_OK;
 }
 
@@ -1315,7 +1324,8 @@ extern "C" int sss_stream_minmax(sss_ctx* ctx, int64_t n, const float* x, const 
     if (n < 1 || !x || !y || !out4) return sss_set_err(ctx, SSS_ERR_ARG, "minmax: empty or NULL input");
     cudaStream_t st = (cudaStream_t)stream;
     Work W;
-    int rc = make_work(ctx, n, 1, 1, 1, &W);
+    int slots = 1;
+    int rc = make_work(ctx, n, 1, &slots, 1, &W);
     if (rc) return rc;
     const float* qx = x;
     const float* qy = y;
@@ -1350,10 +1360,7 @@ namespace {
 // A sample alone is bound by its phases' latency (about a dozen barriers, one
 // block's bisection, first touches of memory): with the whole grid to each of
 // 8 samples of a million bodies in turn 51 us a sample, with 37 blocks to each
-// of the 8 at once 30. Their buffers (14 bytes a body, 5 MB
-// of tables) are held to SLOTS_BYTES.
-constexpr size_t SLOTS_BYTES = (size_t)256 << 20;
-
+// of the 8 at once 30.
 int sample_batch(sss_ctx* ctx, int64_t n, int k, const float* const* x, const float* const* y,
                  const double* kill_t, const double* t_cut, const unsigned char* is_ast,
                  const unsigned char* injected, const double* box, int log_zoom, int64_t budget, unsigned* sel,
@@ -1374,14 +1381,7 @@ int sample_batch(sss_ctx* ctx, int64_t n, int k, const float* const* x, const fl
     if (rc) return rc;
     Work W;
     int at_once = std::min(k, SAMPLES_MAX);
-    const size_t one = (size_t)n * 10 + (size_t)K2 * 16 + ((size_t)1 << 19);
-    while (at_once > 1 && (size_t)at_once * one > SLOTS_BYTES) --at_once;
-    rc = make_work(ctx, n, grid, at_once, k, &W);
-    if (rc && at_once > 1) {                       // no memory for several: one at a time
-        cudaGetLastError();
-        at_once = 1;
-        rc = make_work(ctx, n, grid, at_once, k, &W);
-    }
+    rc = make_work(ctx, n, grid, &at_once, k, &W);
     if (rc) return rc;
     SampleBatch p;
     SampleArgs& a = p.s;
