@@ -227,16 +227,6 @@ __global__ void __launch_bounds__(Tile16<N>::NT, 1024 / Tile16<N>::NT) k_y_fwd(c
                                      [&](int i, int, float2 z, bool) { p[i * T::PITCH] = z; });
 }
 
-// 1 / d for a normal d > 0: the hardware's coarse reciprocal and two Newton
-// steps r (2 - d r). No branch, so the 16 modes of a thread overlap; with a
-// division each (its slow path a branch) the 64^3 pass took 14 us.
-__device__ __forceinline__ double recip(double d) {
-    double r;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
-    r = fma(r, fma(-d, r, 1.0), r);
-    return fma(r, fma(-d, r, 1.0), r);
-}
-
 // k (f64) z rounded once, as the products of k_spectrum3, from k = hi + lo in two
 // f32: hi z = p + e exactly, so p + (e + lo z) is within 2^-46 of k z before its
 // rounding (Dekker, "A floating-point technique for extending the available
@@ -273,7 +263,7 @@ k_x_solve(const float2* __restrict__ tw, const float2* __restrict__ rk, double c
                          [&](int i, int c, float2 r, bool) {
                              float2 a = make_float2(0.f, 0.f), b = a;
                              if (!mean || i != 0) {
-                                 const double q = cyz * __ldg(tab + 2 * N + i) * recip(k2yz + __ldg(tab + N + i));
+                                 const double q = cyz * __ldg(tab + 2 * N + i) * sss_recip_f64(k2yz + __ldg(tab + N + i));
                                  const double f = __ldg(tab + i) * q;
                                  a = make_float2((float)(-f * (double)r.y), (float)(f * (double)r.x));
                                  b = make_float2((float)(q * (double)r.x), (float)(q * (double)r.y));
