@@ -130,3 +130,9 @@ def test_pair_term_scratch(monkeypatch):
     pm.short(st)
     torch.cuda.synchronize()
     assert free - torch.cuda.mem_get_info()[0] <= 93 * n + (4 << 20)
+
+
+def test_pair_term_of_more_items_than_warps():
+    """120,000 particles in 10^3 cells, some 4,500 items: more than there are
+    warps, so the items come from the counter (fewer go by the warp's place)."""
+    test_pair_term_item_shapes(120_000, 0.3, 3.0, 1e-3, False)
