@@ -262,7 +262,10 @@ struct PPTarget {
 // through the lanes and end on their own lanes, then go to the accumulator.
 // 35 FMA-pipe operations and four special-function ones a pair (the latter
 // bound it), with the 6 shuffles and two 16-byte shared loads of a step shared
-// by its 2 pairs. 1,048,576 particles collapsed into halos (7.2e9 candidate
+// by its 2 pairs. Steps without a pair in range are skipped by a vote: particles that
+// come in spatial order, a lattice above all, lie together in the chunks (1,048,576
+// on a lattice, r_split 2.25 cells, r_cut 3 / alpha: 3.88 ms a pass, 5.21 without;
+// uniform at random 4.63, 5.21). 1,048,576 particles collapsed into halos (7.2e9 candidate
 // pairs, 5.1e9 in range): 12.5 ms a step against 15.4 with sources packed by
 // register moves and items in cell order (the last heavy items then ran on by
 // themselves). Sorting particles inside a cell and testing chunk boxes saves
@@ -281,15 +284,17 @@ __device__ __forceinline__ void pp_chunk2(const ulonglong2* stage, int lane, PPT
         upk2(R2, r0, r1);
         const bool in0 = r0 < q.rc2 && r0 > 0.0f;
         const bool in1 = r1 < q.rc2 && r1 > 0.0f && !(OWN && a + DA == 16 && lane >= 16);
-        upk2(pp_h2(R2, k.alpha, k.eps2), h0, h1);
-        const f2x H = pk2(in0 ? h0 : 0.0f, in1 ? h1 : 0.0f);
-        const f2x HJ = mul2(H, zm.y), HI = mul2(H, t.nm);
-        t.ax = fma2(HJ, DX, t.ax);
-        t.ay = fma2(HJ, DY, t.ay);
-        t.az = fma2(HJ, DZ, t.az);
-        BX = fma2(HI, DX, BX);
-        BY = fma2(HI, DY, BY);
-        BZ = fma2(HI, DZ, BZ);
+        if (__any_sync(0xffffffffu, in0 || in1)) {                  // (warp-uniform)
+            upk2(pp_h2(R2, k.alpha, k.eps2), h0, h1);
+            const f2x H = pk2(in0 ? h0 : 0.0f, in1 ? h1 : 0.0f);
+            const f2x HJ = mul2(H, zm.y), HI = mul2(H, t.nm);
+            t.ax = fma2(HJ, DX, t.ax);
+            t.ay = fma2(HJ, DY, t.ay);
+            t.az = fma2(HJ, DZ, t.az);
+            BX = fma2(HI, DX, BX);
+            BY = fma2(HI, DY, BY);
+            BZ = fma2(HI, DZ, BZ);
+        }
         if (a + 1 < A1) {                                          // take the next lane's sums (sources + 1)
             BX = shfl2(BX, from);
             BY = shfl2(BY, from);
