@@ -254,7 +254,21 @@ struct SampleArgs {
     int* vkey;                                      // 2 x VALUE_SLOTS: count value >= VDIR, -1 empty
     unsigned* vmul;                                 // 2 x VALUE_SLOTS: cells holding it
     double* vpre;                                   // 2 VALUE_MAX: prefix sums of the sorted values
-    unsigned nb, bid;                               // blocks of this sample, this block's number among them
+};
+
+// nb(): blocks of this sample, bid(): this block's number among them. A sample
+// that has the launch to itself reads its arguments as kernel parameters: 49.4 us
+// of kernel for 1,000,000 bodies, 9.2 for 1,000; from shared memory, where a block
+// of several at once puts its sample's, 53.0 and 10.5.
+struct AloneArgs : SampleArgs {
+    __device__ __forceinline__ unsigned nb() const { return gridDim.x; }
+    __device__ __forceinline__ unsigned bid() const { return blockIdx.x; }
+};
+
+struct SharedArgs : SampleArgs {
+    unsigned nb_, bid_;
+    __device__ __forceinline__ unsigned nb() const { return nb_; }
+    __device__ __forceinline__ unsigned bid() const { return bid_; }
 };
 
 // Samples of one launch: the grid's blocks are dealt out to them, sample g
@@ -264,6 +278,7 @@ constexpr int SAMPLES_MAX = 8;
 
 struct SampleBatch {
     SampleArgs s;                                   // the first sample's
+    unsigned nb;
     size_t slot;
     const float* x[SAMPLES_MAX];
     const float* y[SAMPLES_MAX];
@@ -287,9 +302,10 @@ __device__ __forceinline__ Tables tables(const SampleArgs& a, int slot) {
 
 // bodies [c0, c1) of this block in the cull, keep and emit phases (c0 a
 // multiple of 8)
-__device__ __forceinline__ void body_range(const SampleArgs& a, long long& c0, long long& c1) {
-    const long long n = a.n, chunk = ((n + a.nb - 1) / a.nb + 7) / 8 * 8;
-    c0 = min((long long)a.bid * chunk, n);
+template <class A>
+__device__ __forceinline__ void body_range(const A& a, long long& c0, long long& c1) {
+    const long long n = a.n, chunk = ((n + a.nb() - 1) / a.nb() + 7) / 8 * 8;
+    c0 = min((long long)a.bid() * chunk, n);
     c1 = min(c0 + chunk, n);
 }
 
@@ -382,9 +398,10 @@ struct Smem {
 // put many bodies of a chunk into a few cells) and adds every distinct cell
 // to the global counts once. The table has twice the chunk's slots, so a
 // probe ends within HIST_SLOTS steps.
-__device__ void phase_hist(const SampleArgs& a, const Tables& tb, const float* qx, const float* qy, int mask,
+template <class A>
+__device__ void phase_hist(const A& a, const Tables& tb, const float* qx, const float* qy, int mask,
                            Smem& sm) {
-    for (long long c0 = (long long)a.bid * HIST_CHUNK; c0 < a.n; c0 += (long long)a.nb * HIST_CHUNK) {
+    for (long long c0 = (long long)a.bid() * HIST_CHUNK; c0 < a.n; c0 += (long long)a.nb() * HIST_CHUNK) {
         for (int j = threadIdx.x; j < HIST_SLOTS; j += SAMPLE_THREADS) {
             sm.u.h.key[j] = -1;
             sm.u.h.val[j] = 0;
@@ -432,9 +449,10 @@ __device__ void phase_hist(const SampleArgs& a, const Tables& tb, const float* q
 // empty cells sums to +0 for every midpoint, as its terms min(0, s * 0) = +0
 // do; in a leaf with occupied cells the +0 terms of its empty cells are added
 // like the others (exactly).
-__device__ void phase_group_sums(const SampleArgs& a, const Tables& tb, double lo, double hi, double* part, Smem& sm) {
+template <class A>
+__device__ void phase_group_sums(const A& a, const Tables& tb, double lo, double hi, double* part, Smem& sm) {
     const int leaf = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int g = a.bid; g < GROUPS; g += a.nb) {
+    for (int g = a.bid(); g < GROUPS; g += a.nb()) {
         constexpr int PER_T = GROUP_CELLS / SAMPLE_THREADS;
         int cv[PER_T];
 #pragma unroll
@@ -589,15 +607,16 @@ static_assert(VALUE_SLOTS == 1 << 13, "13-bit hash");
 // tables (vdir, and vkey/vmul for the larger counts). A global table of
 // larger counts that runs out of slots sets value_over (the bisection then
 // takes the exact path).
-__device__ void phase_values(const SampleArgs& a, const Tables& tb, Smem& sm) {
+template <class A>
+__device__ void phase_values(const A& a, const Tables& tb, Smem& sm) {
     for (int j = threadIdx.x; j < VDIR; j += SAMPLE_THREADS) sm.u.v.dir[j] = 0;
     for (int j = threadIdx.x; j < LSLOTS; j += SAMPLE_THREADS) {
         sm.u.v.lkey[j] = -1;
         sm.u.v.lval[j] = 0;
     }
     __syncthreads();
-    const long long per = (K2 + a.nb - 1) / a.nb;
-    const long long c0 = (long long)a.bid * per, c1 = min(c0 + per, (long long)K2);
+    const long long per = (K2 + a.nb() - 1) / a.nb();
+    const long long c0 = (long long)a.bid() * per, c1 = min(c0 + per, (long long)K2);
     for (long long c = c0 + threadIdx.x; c < c1; c += SAMPLE_THREADS) {
         const int v = __ldcg(tb.counts + c);
         if (v <= 0) continue;
@@ -914,15 +933,16 @@ __device__ void block_fast_bisection(const SampleArgs& a, const Tables& tb, doub
 // points (size > budget); keep[i] = 1 for the kept bodies, their number in
 // ctl->kept[slot] and, per block of bodies, in its record. Returns false
 // when a barrier gave up.
-__device__ bool filter(const SampleArgs& a, const float* qx, const float* qy, int mask, long long budget, int slot,
+template <class A>
+__device__ bool filter(const A& a, const float* qx, const float* qy, int mask, long long budget, int slot,
                        unsigned& epoch, Smem& sm) {
     const Tables tb = tables(a, slot);
     phase_hist(a, tb, qx, qy, mask, sm);
-    if (!grid_barrier(a.ctl, a.nb, epoch, &sm.bad)) return false;
+    if (!grid_barrier(a.ctl, a.nb(), epoch, &sm.bad)) return false;
     phase_values(a, tb, sm);
-    if (!grid_barrier(a.ctl, a.nb, epoch, &sm.bad)) return false;
-    if (a.bid == 0) block_fast_bisection(a, tb, (double)budget, sm);
-    if (!grid_barrier(a.ctl, a.nb, epoch, &sm.bad)) return false;
+    if (!grid_barrier(a.ctl, a.nb(), epoch, &sm.bad)) return false;
+    if (a.bid() == 0) block_fast_bisection(a, tb, (double)budget, sm);
+    if (!grid_barrier(a.ctl, a.nb(), epoch, &sm.bad)) return false;
     // every thread reads the control words after a barrier: L1-cached loads,
     // so that one request per SM reaches their L2 line
     double lo = __ldca(&a.ctl->lohi[0]), hi = __ldca(&a.ctl->lohi[1]);
@@ -931,19 +951,19 @@ __device__ bool filter(const SampleArgs& a, const float* qx, const float* qy, in
     for (int round = 0; left > 0; ++round) {
         double* part = a.part + (round & 1) * CAND * GROUPS;
         phase_group_sums(a, tb, lo, hi, part, sm);
-        if (!grid_barrier(a.ctl, a.nb, epoch, &sm.bad)) return false;
+        if (!grid_barrier(a.ctl, a.nb(), epoch, &sm.bad)) return false;
         const int levels = min(BISECT_D, left);
         phase_walk(part, (double)budget, lo, hi, levels, sm);
         left -= levels;
     }
-    const long long T = (long long)a.nb * SAMPLE_THREADS;
-    const long long gt = (long long)a.bid * SAMPLE_THREADS + threadIdx.x;
+    const long long T = (long long)a.nb() * SAMPLE_THREADS;
+    const long long gt = (long long)a.bid() * SAMPLE_THREADS + threadIdx.x;
     // the keep rate of every cell: min(k, lo k ** 0.5) / k, 0 for an empty cell
     for (long long c = gt; c < K2; c += T) {
         const int k = __ldcg(tb.counts + c);
         a.rate[c] = k > 0 ? __ddiv_rn(fmin((double)k, __dmul_rn(lo, cell_weight(k))), (double)k) : 0.0;
     }
-    if (!grid_barrier(a.ctl, a.nb, epoch, &sm.bad)) return false;
+    if (!grid_barrier(a.ctl, a.nb(), epoch, &sm.bad)) return false;
     const unsigned char* __restrict__ tier = a.tier;
     unsigned char* __restrict__ keep = a.keep;
     const double* __restrict__ rate = a.rate;
@@ -999,38 +1019,17 @@ __device__ bool filter(const SampleArgs& a, const float* qx, const float* qy, in
     }
     kept = block_sum_ll(kept, sm.red);
     if (threadIdx.x == 0) {
-        a.blk[(size_t)a.bid * BLK + 4 + slot] = kept;
+        a.blk[(size_t)a.bid() * BLK + 4 + slot] = kept;
         if (kept) atomicAdd(a.ctl->kept + slot, (unsigned long long)kept);
     }
-    return grid_barrier(a.ctl, a.nb, epoch, &sm.bad);
+    return grid_barrier(a.ctl, a.nb(), epoch, &sm.bad);
 }
 
-__global__ void __launch_bounds__(SAMPLE_THREADS) k_sample(const __grid_constant__ SampleBatch p) {
-    __shared__ Smem sm;
-    __shared__ SampleArgs mine;
-    if (threadIdx.x == 0) {
-        const unsigned g = blockIdx.x / p.s.nb;
-        const size_t d = g * p.slot;
-        auto at = [&](auto* q) { return (decltype(q))((char*)q + d); };
-        SampleArgs t = p.s;
-        t.bid = blockIdx.x - g * p.s.nb;
-        t.x = p.x[g];
-        t.y = p.y[g];
-        t.t_cut = p.t_cut[g];
-        t.qx = at(t.qx); t.qy = at(t.qy); t.tier = at(t.tier); t.keep = at(t.keep); t.counts = at(t.counts);
-        t.rate = at(t.rate); t.part = at(t.part); t.blk = at(t.blk); t.vdir = at(t.vdir); t.vkey = at(t.vkey);
-        t.vmul = at(t.vmul); t.vpre = at(t.vpre);
-        t.sel += (size_t)g * t.n;
-        t.ox += (size_t)g * t.n;
-        t.oy += (size_t)g * t.n;
-        t.ctl += g;
-        mine = t;
-    }
-    __syncthreads();
-    const SampleArgs& a = mine;
+template <class A>
+__device__ __forceinline__ void sample(const A& a, Smem& sm) {
     unsigned epoch = 0;
-    const long long T = (long long)a.nb * SAMPLE_THREADS;
-    const long long gt = (long long)a.bid * SAMPLE_THREADS + threadIdx.x;
+    const long long T = (long long)a.nb() * SAMPLE_THREADS;
+    const long long gt = (long long)a.bid() * SAMPLE_THREADS + threadIdx.x;
     const float* qx = a.log_zoom ? a.qx : a.x;
     const float* qy = a.log_zoom ? a.qy : a.y;
     // ---- cull (and clear both filter slots' count tables)
@@ -1086,14 +1085,14 @@ __global__ void __launch_bounds__(SAMPLE_THREADS) k_sample(const __grid_constant
         if (n1) atomicAdd(a.ctl->tier_cnt + 1, (unsigned long long)n1);
         if (n2) atomicAdd(a.ctl->tier_cnt + 2, (unsigned long long)n2);
         if (n3) atomicAdd(a.ctl->tier_cnt + 3, (unsigned long long)n3);
-        long long* rec = a.blk + (size_t)a.bid * BLK;
+        long long* rec = a.blk + (size_t)a.bid() * BLK;
         rec[1] = n1;
         rec[2] = n2;
         rec[3] = n3;
         rec[4] = 0;
         rec[5] = 0;
     }
-    if (!grid_barrier(a.ctl, a.nb, epoch, &sm.bad)) return;
+    if (!grid_barrier(a.ctl, a.nb(), epoch, &sm.bad)) return;
     // ---- plan (the reference's _lod_auswahl), identical in every block
     // (every thread reads the counts: L1-cached loads, one L2 request per SM)
     const long long mm = (long long)__ldca(a.ctl->tier_cnt + 1), ma = (long long)__ldca(a.ctl->tier_cnt + 2),
@@ -1146,7 +1145,7 @@ __global__ void __launch_bounds__(SAMPLE_THREADS) k_sample(const __grid_constant
     // 0 .. b - 1. A block emits its kept bodies and its bodies of the tiers
     // in all_mask (never a filtered tier): its record holds both numbers.
     long long before = 0;
-    for (int j = threadIdx.x; j < (int)a.bid; j += SAMPLE_THREADS) {
+    for (int j = threadIdx.x; j < (int)a.bid(); j += SAMPLE_THREADS) {
         const long long* rec = a.blk + (size_t)j * BLK;
         long long e = __ldca(rec + 4) + __ldca(rec + 5);            // (read by every later block: L1-cached)
 #pragma unroll
@@ -1225,7 +1224,38 @@ __global__ void __launch_bounds__(SAMPLE_THREADS) k_sample(const __grid_constant
         off += all;
         __syncthreads();                            // wcnt is rewritten by the next sub-range
     }
-    if (a.bid == a.nb - 1 && threadIdx.x == 0) a.ctl->total = off;
+    if (a.bid() == a.nb() - 1 && threadIdx.x == 0) a.ctl->total = off;
+}
+
+__global__ void __launch_bounds__(SAMPLE_THREADS) k_sample_alone(const __grid_constant__ AloneArgs a) {
+    __shared__ Smem sm;
+    sample(a, sm);
+}
+
+__global__ void __launch_bounds__(SAMPLE_THREADS) k_sample(const __grid_constant__ SampleBatch p) {
+    __shared__ Smem sm;
+    __shared__ SharedArgs mine;
+    if (threadIdx.x == 0) {
+        const unsigned g = blockIdx.x / p.nb;
+        const size_t d = g * p.slot;
+        auto at = [&](auto* q) { return (decltype(q))((char*)q + d); };
+        SampleArgs t = p.s;
+        t.x = p.x[g];
+        t.y = p.y[g];
+        t.t_cut = p.t_cut[g];
+        t.qx = at(t.qx); t.qy = at(t.qy); t.tier = at(t.tier); t.keep = at(t.keep); t.counts = at(t.counts);
+        t.rate = at(t.rate); t.part = at(t.part); t.blk = at(t.blk); t.vdir = at(t.vdir); t.vkey = at(t.vkey);
+        t.vmul = at(t.vmul); t.vpre = at(t.vpre);
+        t.sel += (size_t)g * t.n;
+        t.ox += (size_t)g * t.n;
+        t.oy += (size_t)g * t.n;
+        t.ctl += g;
+        (SampleArgs&)mine = t;
+        mine.nb_ = p.nb;
+        mine.bid_ = blockIdx.x - g * p.nb;
+    }
+    __syncthreads();
+    sample(mine, sm);
 }
 
 struct Work {
@@ -1297,7 +1327,10 @@ int sample_grid(sss_ctx* ctx, int* grid) {
     const int dev = ctx->device;
     int per_sm = dev >= 0 && dev < 64 ? per_sm_of[dev] : 0;
     if (per_sm == 0) {
+        int alone = 0;
         SSS_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sample, SAMPLE_THREADS, 0));
+        SSS_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&alone, k_sample_alone, SAMPLE_THREADS, 0));
+        per_sm = std::min(per_sm, alone);
         if (per_sm < 1) return sss_set_err(ctx, SSS_ERR_CUDA, "k_sample: no resident block per SM");
         if (dev >= 0 && dev < 64) per_sm_of[dev] = per_sm;
     }
@@ -1411,7 +1444,6 @@ int sample_batch(sss_ctx* ctx, int64_t n, int k, const float* const* x, const fl
     a.vmul = W.vmul;
     a.vpre = W.vpre;
     SSS_CUDA_TRY(ctx, cudaMemsetAsync(W.ctl, 0, sizeof(Ctl) * (size_t)k, st));
-    a.bid = 0;
     for (int i = 0; i < k; i += at_once) {
         const int m = std::min(at_once, k - i);
         for (int g = 0; g < m; ++g) {
@@ -1426,9 +1458,17 @@ int sample_batch(sss_ctx* ctx, int64_t n, int k, const float* const* x, const fl
         a.ox = qx_out + (size_t)i * n;
         a.oy = qy_out + (size_t)i * n;
         a.ctl = W.ctl + i;
-        a.nb = (unsigned)(grid / m);
+        if (m == 1) {
+            AloneArgs one;
+            (SampleArgs&)one = a;
+            void* params[] = {&one};
+            SSS_CUDA_TRY(ctx, cudaLaunchCooperativeKernel((const void*)k_sample_alone, dim3(grid),
+                                                          dim3(SAMPLE_THREADS), params, 0, st));
+            continue;
+        }
+        p.nb = (unsigned)(grid / m);
         void* params[] = {&p};
-        SSS_CUDA_TRY(ctx, cudaLaunchCooperativeKernel((const void*)k_sample, dim3(a.nb * m), dim3(SAMPLE_THREADS),
+        SSS_CUDA_TRY(ctx, cudaLaunchCooperativeKernel((const void*)k_sample, dim3(p.nb * m), dim3(SAMPLE_THREADS),
                                                       params, 0, st));
     }
     Ctl hbuf[16];
