@@ -84,9 +84,11 @@ int sss_num_sms(const sss_ctx* ctx);
  * Body records are double4 {x, y, z, Gm} (z ignored when dim == 2; Gm is the
  * source's G*mass and is ignored for targets). Output acc4 is double4
  * {ax, ay, az, 0}. The self term contributes exactly 0 (zero offset).
- * Sources are summed in ascending index order inside each source chunk; the
- * chunk partials are added in ascending chunk order, so a result depends only
- * on the inputs and on (n_src, n_tgt, number of SMs), never on scheduling.
+ * Sources are summed in ascending index order inside each source chunk (with
+ * few pairs: inside each of a chunk's 8 slices, or by the lanes of a warp); the
+ * partial sums are added in a fixed order, so a result depends only on the
+ * inputs and on (n_src, n_tgt, number of SMs), never on scheduling. f64: a pair
+ * whose r^2 overflows adds 0 where eps2 < 2^-126, and may give NaN above.
  * All pointers are device pointers with 16-byte alignment.
  */
 int sss_allpairs_accel(sss_ctx* ctx, int dim, int precision,

@@ -124,9 +124,9 @@ def test_matches_reference_advance_golden(load_golden):
 @pytest.mark.parametrize("dim", [2, 3])
 @pytest.mark.parametrize("n", [9, 16, 17, 21, 31, 32, 33, 43, 63, 64])
 def test_block_mappings_of_odd_sizes(n, dim):
-    """The block-per-system mappings pack n targets and T / n source chunks
-    (at most 8): sizes that fill the block, leave a remainder and reach the
-    chunk limit, each in a launch with more than one size, against the oracle."""
+    """The block-per-system mappings (16, 32 or 64 targets x source chunks):
+    sizes that fill the targets' columns and leave idle ones, each in a launch
+    with more than one size, against the oracle."""
     from solarsystemsimulator_b200 import batched
     rng = np.random.default_rng(10 * n + dim)
     systems = []

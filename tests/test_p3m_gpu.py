@@ -86,9 +86,9 @@ def test_bad_arguments():
 @pytest.mark.parametrize("x_cut,eps", [(3.0, 1e-3), (3.0, 0.0), (3.5, 1e-3)])
 @pytest.mark.parametrize("equal", [True, False])
 def test_pair_term_item_shapes(n, spread, x_cut, eps, equal):
-    """Group, item and work-list remainders (one and two groups of 32, a cell
-    above the long-walk limit), the polynomial and the erfc form, equal and
-    own masses. Per target the error is bounded by the sums over its pairs of
+    """Remainders of the 32-target items, walks of one chunk and of many (the
+    class of an item's length changes along a cell), cutoffs, with and without
+    softening, equal and own masses. Per target the error is bounded by the sums over its pairs of
     the Newtonian term times 1e-6 (the factor's error) plus three times the
     rounding of an offset (2 cells to f32) over r, plus one rounding per
     accumulated term."""

@@ -454,3 +454,9 @@ def test_gradient_factors_are_not_rounded(n):
             a, b = mesh(axis, K, P), mesh(axis, 1.0, V)
             assert abs(float(a.abs().max()) / (2.0 * V) - 1.0) < 1e-6
             assert torch.equal(a, b), (axis, K, P, V)
+
+
+def test_solve_of_the_largest_own_side():
+    """Side 512: the only one of 512-thread blocks, 128 KB of shared memory in
+    the x pass."""
+    test_solve_of_every_mesh_side(512, 2, 0.6)

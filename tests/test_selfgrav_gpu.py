@@ -313,8 +313,8 @@ def test_few_pairs_kernels(dim, n_src, n_tgt, equal):
                                          (710, 710), (63, 9001), (513, 1100), (8193, 65), (127, 5000)])
 @pytest.mark.parametrize("equal", [True, False])
 def test_smallest_evaluations(dim, n_src, n_tgt, equal):
-    """A warp per target (below 1.5e5 pairs in f64, 5e5 in mixed): fewer
-    sources than lanes, remainders of the 128 a pass takes and of the 8 targets
+    """A warp per target (up to 512 sources on 4,096 targets, mixed also 1,024
+    on 1,024): fewer sources than lanes, remainders of the 128 a pass takes and of the 8 targets
     a block takes; and the warp-split kernels' edges at sizes just above."""
     test_few_pairs_kernels(dim, n_src, n_tgt, equal)
 
