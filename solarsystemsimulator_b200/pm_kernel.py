@@ -111,13 +111,20 @@ def build_force_kernels(grid_n: int, h: float, eps2: float, G: float = G_AU, dev
     return ForceKernels(p, h, eps2, G)
 
 
+def _hold(p: PMPlan, kernels: ForceKernels | None, key) -> None:
+    """The caller's kernels on the plan (made again where another caller has
+    put others there), those of key = (h, eps2, G) without any."""
+    key = kernels.key if kernels is not None and kernels.plan is p else tuple(float(v) for v in key)
+    if p.kernel_key != key:
+        p.build(key)
+
+
 def pm_force_field(gx, gy, gm, grid_n, x0, y0, h, eps2, G: float = G_AU, kernels=None, device: int = 0):
     """The acceleration field on the N x N grid (pm_kernel.py:127-147).
     Returns (ax_grid, ay_grid) as (N, N) float64 CUDA tensors."""
     dev = torch.device("cuda", device)
     p = plan_for(grid_n, device)
-    if kernels is None or kernels.plan is not p or p.kernel_key != kernels.key:
-        kernels = build_force_kernels(grid_n, h, eps2, G, device)
+    _hold(p, kernels, (h, eps2, G))
     x, y, m = _f64(gx, dev), _f64(gy, dev), _f64(gm, dev)
     p.call("sss_pm2d_field", x.data_ptr(), y.data_ptr(), m.data_ptr(), x.numel(), float(x0), float(y0), float(h))
     return _crop_fields(p, dev)
@@ -168,8 +175,7 @@ def pm_accelerations(gx, gy, gm, grid_n, x0, y0, h, eps2, G: float = G_AU, kerne
     """Acceleration of each mass via PM (pm_kernel.py:157-163)."""
     dev = torch.device("cuda", device)
     p = plan_for(grid_n, device)
-    if kernels is None or kernels.plan is not p or p.kernel_key != kernels.key:
-        build_force_kernels(grid_n, h, eps2, G, device)
+    _hold(p, kernels, (h, eps2, G))
     x, y, m = _f64(gx, dev), _f64(gy, dev), _f64(gm, dev)
     p.call("sss_pm2d_field", x.data_ptr(), y.data_ptr(), m.data_ptr(), x.numel(), float(x0), float(y0), float(h))
     ax, ay = torch.empty_like(x), torch.empty_like(x)

@@ -96,3 +96,20 @@ def test_kernels_stay_within_a_millionth_of_h_and_survive_a_failed_build(plan):
     plan.box = 1.0
     fresh.load_state([0.0, 1.0], [0.0, 1.0], [0.0, 0.0], [0.0, 0.0], [1.0, 1.0])
     assert plan.fields[-1] == _held(fresh, fresh._kernel_h)
+
+
+def test_a_callers_kernels_are_made_again_as_they_were(plan, monkeypatch):
+    """Kernels handed to a field are the ones it is made with, also after
+    another caller has put its own on the plan (the reference's arrays cannot
+    change either), and whatever h the field itself has."""
+    monkeypatch.setattr(pk, "_crop_fields", lambda p, dev: None)
+    mine = pk.build_force_kernels(64, 0.5, 0.25, 2.0)
+    args = ([0.0], [0.0], [1.0], 64, 0.0, 0.0, 0.75, 0.3)
+    for other in (False, True):
+        if other:
+            pk.build_force_kernels(64, 0.6, 0.1, 3.0)
+        pk.pm_force_field(*args, kernels=mine)
+        pk.pm_accelerations(*args, kernels=mine)
+        assert plan.fields[-2:] == [mine.key, mine.key]
+    pk.pm_force_field(*args, G=4.0)
+    assert plan.fields[-1] == (0.75, 0.3, 4.0)
