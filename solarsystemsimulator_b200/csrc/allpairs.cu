@@ -75,8 +75,10 @@ constexpr int LN_NT = 256, LN_U = 4;
 // Warp-split / general. By pairs where both counts are large:
 //   mixed 3-D  10,007^2 57 / 88, 17,000^2 148 / 156, 20,000^2 199 / 207, 25,000^2 294 / 290, 40,000^2 748 / 671
 //   f64 3-D    10,007^2 125 / 133, 17,000^2 316 / 326, 20,000^2 438 / 437, 30,000^2 960 / 927
-// Few sources on many targets leave a CTA of 64 or 128 targets little but its fixed part:
-//   mixed 2-D  1 x 65,536 5.0 / 6.1, 1 x 131,072 8.5 / 6.1, 100 x 131,072 12 / 11, 100 x 1,000,000 82 / 42, 512 x 262,144 56 / 57
+// Few sources on many targets leave a CTA of 64 or 128 targets little but its fixed part, while the general form's time
+// rises by the round of 148 CTAs of 1,024 (f64: 512) targets; us of both as fitted to the sweep (within 7 %):
+//   mixed 2-D  1 x 65,536 5.0 / 6.1, 1 x 131,072 8.5 / 6.1, 100 x 131,072 12 / 11, 192 x 196,608 24 / 26 (two rounds),
+//              500 x 300,000 67 / 61, 100 x 1,000,000 82 / 42, 512 x 262,144 56 / 57
 //   f64 3-D    1 x 8,192 2.6 / 2.8, 1 x 65,536 6.1 / 2.9, 100 x 65,536 11.3 / 11.6, 100 x 1,000,000 130 / 111, 512 x 262,144 144 / 160
 // Many sources on a few targets give it 16 chunks only, of sources the general form spreads over all SMs:
 //   mixed 3-D  65,536 x 8 47 / 45, 131,072 x 64 91 / 82, 1,048,576 x 1 699 / 517, 131,072 x 200 92 / 94
@@ -87,10 +89,17 @@ constexpr bool use_lanes(bool mixed, int64_t n_src, int64_t n_tgt) {
     return (n_src <= 512 && n_tgt <= 4096) || (mixed && n_src <= 1024 && n_tgt <= 1024);
 }
 
-constexpr bool use_split(bool mixed, int64_t n_src, int64_t n_tgt) {
-    if ((double)n_src * (double)n_tgt >= (mixed ? SPLIT_PAIRS_MIX : SPLIT_PAIRS_F64)) return false;
-    if (n_tgt >= (mixed ? 80000 + 500 * n_src : 20000 + 900 * n_src)) return false;
-    return !(n_tgt <= (mixed ? 128 : 256) && n_src >= (mixed ? 98304 : 65536));
+constexpr bool use_split(bool mixed, int dim, int64_t n_src, int64_t n_tgt) {
+    const double n = (double)n_src, t = (double)n_tgt;
+    if (n * t >= (mixed ? SPLIT_PAIRS_MIX : SPLIT_PAIRS_F64)) return false;
+    if (n_src <= 512) {
+        const double w = (double)((n_tgt + (mixed ? 151551 : 75775)) / (mixed ? 151552 : 75776));     // rounds
+        const double general = mixed ? 4.8 + w * (1.1 + 0.049 * n) : 2.0 + 0.7 * w + n * (0.0615 * w + 0.006);
+        const double split = mixed ? 2.0 + t * (5.0e-5 + 3.0e-7 * n) : 1.7 + t * ((dim == 3 ? 4.8e-5 : 3.7e-5) + 8.0e-7 * n);
+        if (general < split) return false;
+    }
+    const int64_t few = !mixed || (dim == 3 && n_src >= 131072) ? 256 : 128;
+    return !(n_tgt <= few && n_src >= (mixed && dim == 2 ? 98304 : 65536));
 }
 
 using sss_ap::Epi;
@@ -964,7 +973,7 @@ KSel select_kernel(int dim, int precision, int64_t n_src, int64_t n_tgt, double 
     KSel k;
     k.mixed = (precision == SSS_PREC_MIXED);
     k.lanes = use_lanes(k.mixed, n_src, n_tgt);
-    k.ws = !k.lanes && use_split(k.mixed, n_src, n_tgt);
+    k.ws = !k.lanes && use_split(k.mixed, dim, n_src, n_tgt);
     if (k.lanes) {
         if (k.mixed) k.fn = (dim == 3) ? (void*)k_force_lanes<3, true> : (void*)k_force_lanes<2, true>;
         else k.fn = (dim == 3) ? (void*)k_force_lanes<3, false> : (void*)k_force_lanes<2, false>;
@@ -1310,8 +1319,8 @@ int noalloc_setup(int device, NoAllocDevice** out, char* eb, size_t el) {
             // one size for each kind of kernel, each with and without the guard
             const int64_t probe_n[3] = {1, 16384, (int64_t)1 << 20};
             static_assert(use_lanes(true, 1, 1) && use_lanes(false, 1, 1) && !use_lanes(true, 16384, 16384) &&
-                          use_split(true, 16384, 16384) && use_split(false, 16384, 16384) &&
-                          !use_split(true, 1 << 20, 1 << 20) && !use_split(false, 1 << 20, 1 << 20), "probe sizes");
+                          use_split(true, 3, 16384, 16384) && use_split(false, 3, 16384, 16384) &&
+                          !use_split(true, 3, 1 << 20, 1 << 20) && !use_split(false, 3, 1 << 20, 1 << 20), "probe sizes");
             for (int prec = 0; prec < 2 && e == cudaSuccess; ++prec)
                 for (int dim = 2; dim <= 3 && e == cudaSuccess; ++dim)
                     for (int q = 0; q < 6 && e == cudaSuccess; ++q) {

@@ -386,12 +386,14 @@ def _form(sg, precision, n_src, n_tgt):
 @pytest.mark.filterwarnings("ignore:DEBUG")
 @pytest.mark.parametrize("precision,n_src,n_tgt,form", [
     ("mixed", 300, 300, "lanes"), ("mixed", 1000, 1000, "lanes"), ("f64", 100, 4000, "lanes"),
-    ("mixed", 65536, 1, "split"), ("mixed", 2048, 64, "split"), ("f64", 16384, 8, "split"), ("f64", 1024, 64, "split"),
+    ("mixed", 16384, 1, "split"), ("mixed", 2048, 64, "split"), ("f64", 16384, 8, "split"), ("f64", 1024, 64, "split"),
     ("mixed", 4, 16384, "split"), ("f64", 16, 16384, "split"), ("mixed", 3000, 23000, "split"),
     ("f64", 10007, 10007, "split"), ("mixed", 512, 262144, "split"),
     ("mixed", 100, 1000000, "general"), ("mixed", 4, 131072, "general"), ("f64", 4, 65536, "general"),
     ("f64", 100, 500000, "general"), ("mixed", 262144, 64, "general"), ("f64", 262144, 64, "general"),
-    ("f64", 20000, 20000, "general"), ("mixed", 40000, 40000, "general")])
+    ("f64", 20000, 20000, "general"), ("mixed", 40000, 40000, "general"), ("mixed", 500, 300000, "general"),
+    ("mixed", 192, 196608, "split"), ("mixed", 262144, 200, "general"),
+    ("mixed", 65536, 1, "general"), ("f64", 256, 100000, "split")])
 def test_form_by_sources_and_targets(precision, n_src, n_tgt, form):
     """Lopsided calls take the form that is the fastest at their shape, not the
     one of their number of pairs."""
