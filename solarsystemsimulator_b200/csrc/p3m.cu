@@ -395,7 +395,7 @@ __global__ void __launch_bounds__(PP_WARPS * 32) k_pp_pairs(const PPArgs q) {
     k.alpha = dup(q.alpha);
     k.eps2 = dup(q.eps2);
     // no more items than warps: by the warp's place, which spreads them over all SMs (taken from the counter,
-    // 4 each by the blocks that start first, 32,768 particles in 7^3 cells took 1,020 us a step; now 727)
+    // 4 each by the blocks that start first, 32,768 particles in 7^3 cells took 1,020 us a step, placed 727)
     const unsigned warps = gridDim.x * PP_WARPS, placed = total <= warps ? warps : 0u;
     auto take = [&]() {
         unsigned it = 0;
