@@ -262,44 +262,67 @@ struct PPTarget {
 // through the lanes and end on their own lanes, then go to the accumulator.
 // 35 FMA-pipe operations and four special-function ones a pair (the latter
 // bound it), with the 6 shuffles and two 16-byte shared loads of a step shared
-// by its 2 pairs. Steps without a pair in range are skipped by a vote: particles that
-// come in spatial order, a lattice above all, lie together in the chunks (1,048,576
-// on a lattice, r_split 2.25 cells, r_cut 3 / alpha: 3.88 ms a pass, 5.21 without;
-// uniform at random 4.63, 5.21). 1,048,576 particles collapsed into halos (7.2e9 candidate
-// pairs, 5.1e9 in range): 12.5 ms a step against 15.4 with sources packed by
-// register moves and items in cell order (the last heavy items then ran on by
-// themselves). Sorting particles inside a cell and testing chunk boxes saves
-// only a fifth of these pairs.
+// by its 2 pairs. Two steps at a time, skipped by one vote where no pair is in range:
+// particles that come in spatial order, a lattice above all, lie together in the
+// chunks (1,048,576 on a lattice, r_split 2.25 cells, r_cut 3 / alpha: 3.80 ms a pass,
+// 5.20 without the vote, 3.87 with one a step; uniform at random 4.53, 5.18, 4.62). A
+// vote a step holds up the longest items, a halo's, which two steps' work hides again
+// (262,144 particles in 192 halos 1,386 us a step, 1,594 without, 1,670 with one a
+// step). 1,048,576 particles collapsed into halos (7.2e9 candidate pairs, 5.1e9 in
+// range): 11.0 ms a step against 15.2 with sources packed by register moves and
+// items in cell order (the last heavy items then ran on by themselves). Sorting
+// particles inside a cell and testing chunk boxes saves only a fifth of these pairs.
 template <bool OWN, int A0, int A1, int DA>
 __device__ __forceinline__ void pp_chunk2(const ulonglong2* stage, int lane, PPTarget& t, const PPConst& k,
                                           const PPArgs& q, long long src0, int m) {
+    static_assert((A1 - A0) % 2 == 0, "steps by two");
     f2x BX = 0ull, BY = 0ull, BZ = 0ull;             // sums of sources (lane + a) and (lane + a + DA)
     const int from = (lane + 1) & 31;
-#pragma unroll 2
-    for (int a = A0; a < A1; ++a) {
-        const ulonglong2 xy = stage[(lane + a) & 31], zm = stage[32 + ((lane + a) & 31)];
-        const f2x DX = add2(xy.x, t.nx), DY = add2(xy.y, t.ny), DZ = add2(zm.x, t.nz);
-        const f2x R2 = fma2(DX, DX, fma2(DY, DY, mul2(DZ, DZ)));
-        float r0, r1, h0, h1;
-        upk2(R2, r0, r1);
-        const bool in0 = r0 < q.rc2 && r0 > 0.0f;
-        const bool in1 = r1 < q.rc2 && r1 > 0.0f && !(OWN && a + DA == 16 && lane >= 16);
-        if (__any_sync(0xffffffffu, in0 || in1)) {                  // (warp-uniform)
-            upk2(pp_h2(R2, k.alpha, k.eps2), h0, h1);
-            const f2x H = pk2(in0 ? h0 : 0.0f, in1 ? h1 : 0.0f);
-            const f2x HJ = mul2(H, zm.y), HI = mul2(H, t.nm);
-            t.ax = fma2(HJ, DX, t.ax);
-            t.ay = fma2(HJ, DY, t.ay);
-            t.az = fma2(HJ, DZ, t.az);
-            BX = fma2(HI, DX, BX);
-            BY = fma2(HI, DY, BY);
-            BZ = fma2(HI, DZ, BZ);
+    auto rotate = [&]() {                            // take the next lane's sums (sources + 1)
+        BX = shfl2(BX, from);
+        BY = shfl2(BY, from);
+        BZ = shfl2(BZ, from);
+    };
+#pragma unroll 1
+    for (int a = A0; a < A1; a += 2) {
+        f2x DX[2], DY[2], DZ[2], R2[2], M[2];
+        bool in0[2], in1[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const ulonglong2 xy = stage[(lane + a + u) & 31], zm = stage[32 + ((lane + a + u) & 31)];
+            DX[u] = add2(xy.x, t.nx);
+            DY[u] = add2(xy.y, t.ny);
+            DZ[u] = add2(zm.x, t.nz);
+            M[u] = zm.y;
+            R2[u] = fma2(DX[u], DX[u], fma2(DY[u], DY[u], mul2(DZ[u], DZ[u])));
+            float r0, r1;
+            upk2(R2[u], r0, r1);
+            in0[u] = r0 < q.rc2 && r0 > 0.0f;
+            in1[u] = r1 < q.rc2 && r1 > 0.0f && !(OWN && a + u + DA == 16 && lane >= 16);
         }
-        if (a + 1 < A1) {                                          // take the next lane's sums (sources + 1)
-            BX = shfl2(BX, from);
-            BY = shfl2(BY, from);
-            BZ = shfl2(BZ, from);
+        if (__any_sync(0xffffffffu, in0[0] || in1[0] || in0[1] || in1[1])) {       // (warp-uniform)
+            f2x H[2];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                float h0, h1;
+                upk2(pp_h2(R2[u], k.alpha, k.eps2), h0, h1);
+                H[u] = pk2(in0[u] ? h0 : 0.0f, in1[u] ? h1 : 0.0f);
+            }
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const f2x HJ = mul2(H[u], M[u]), HI = mul2(H[u], t.nm);
+                t.ax = fma2(HJ, DX[u], t.ax);
+                t.ay = fma2(HJ, DY[u], t.ay);
+                t.az = fma2(HJ, DZ[u], t.az);
+                BX = fma2(HI, DX[u], BX);
+                BY = fma2(HI, DY[u], BY);
+                BZ = fma2(HI, DZ[u], BZ);
+                if (u == 0) rotate();
+            }
+        } else {
+            rotate();
         }
+        if (a + 2 < A1) rotate();
     }
     // lane l holds sources (l + A1 - 1) and (l + A1 - 1 + DA): deliver both to their lanes
     const int fa = (lane - (A1 - 1)) & 31, fb = (lane - (A1 - 1 + DA)) & 31;
